@@ -22,7 +22,7 @@ REFERENCE_DIR = os.environ.get("IBM_REFERENCE_DIR", "/root/reference")
 
 def build(with_reference: bool = True) -> None:
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-    if with_reference and os.path.isdir(REFERENCE_DIR):
+    if with_reference and os.path.isfile(os.path.join(REFERENCE_DIR, "common.hpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "refcubin", f"REFERENCE={REFERENCE_DIR}"], check=True)
 
 
