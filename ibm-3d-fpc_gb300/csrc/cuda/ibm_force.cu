@@ -81,14 +81,13 @@ __global__ void __launch_bounds__(kThreads) k_forces_cut(const uint8_t *code, co
   __syncthreads();
   if (!last) return;
   __threadfence();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < 3; ++q) {
-      double a = 0.0;
-      for (int b = 0; b < (int)gridDim.x; ++b) a += __ldcg(&part[3 * b + q]);
-      dg->force[q] = a;
-    }
-    dg->fticket = 0;
+  if (warp < 3) {  // one warp per component over the blocks' partials
+    double a = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) a += __ldcg(&part[3 * b + warp]);
+    a = warp_sum(a);
+    if (lane == 0) dg->force[warp] = a;
   }
+  if (threadIdx.x == 0) dg->fticket = 0;
 }
 
 // Adjoint of the x force: lambda_p += weight w (pressure entries), lambda_u

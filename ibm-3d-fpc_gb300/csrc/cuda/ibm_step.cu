@@ -651,12 +651,36 @@ __global__ void __launch_bounds__(kThreads, 4) k_diagnostics(DiagArgs A) {
   __syncthreads();
   if (!last) return;
   __threadfence();
+  // The last block sums the blocks' partials with all its threads: each thread
+  // takes every 256th block (independent loads), then a fixed tree. One thread
+  // walking the 608 partials took 130 us, more than the sweep itself on grids
+  // below about a million cells.
+  double a = 0.0;
+  unsigned long long b = 0, c = 0, e = 0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
+    a += __ldcg(&A.part[4 * q]);
+    const unsigned long long pb = (unsigned long long)__double_as_longlong(__ldcg(&A.part[4 * q + 1]));
+    const unsigned long long pc = (unsigned long long)__double_as_longlong(__ldcg(&A.part[4 * q + 2]));
+    const unsigned long long pe = (unsigned long long)__double_as_longlong(__ldcg(&A.part[4 * q + 3]));
+    b = pb > b ? pb : b;
+    c = pc > c ? pc : c;
+    e = pe > e ? pe : e;
+  }
+  a = warp_sum(a);
+  b = warp_max_u64(b); c = warp_max_u64(c); e = warp_max_u64(e);
+  if (lane == 0) { s_div[warp] = a; s_max[0][warp] = b; s_max[1][warp] = c; s_max[2][warp] = e; }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0, c = 0.0, e = 0.0;
-    for (int q = 0; q < (int)gridDim.x; ++q) {
-      a += A.part[4 * q]; b = fmax(b, A.part[4 * q + 1]); c = fmax(c, A.part[4 * q + 2]); e = fmax(e, A.part[4 * q + 3]);
+    for (int q = 1; q < kWarps; ++q) {
+      a += s_div[q];
+      b = s_max[0][q] > b ? s_max[0][q] : b;
+      c = s_max[1][q] > c ? s_max[1][q] : c;
+      e = s_max[2][q] > e ? s_max[2][q] : e;
     }
-    A.dg->div2 = a; A.dg->umax = b; A.dg->vmax = c; A.dg->wmax = e;
+    A.dg->div2 = a;
+    A.dg->umax = __longlong_as_double((long long)b);
+    A.dg->vmax = __longlong_as_double((long long)c);
+    A.dg->wmax = __longlong_as_double((long long)e);
     A.dg->ticket = 0;
   }
 }
@@ -881,14 +905,13 @@ __global__ void __launch_bounds__(kThreads) k_forces(ForceArgs A) {
   __syncthreads();
   if (!last) return;
   __threadfence();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < 3; ++q) {
-      double a = 0.0;
-      for (int b = 0; b < (int)gridDim.x; ++b) a += A.part[3 * b + q];
-      A.dg->force[q] = a;
-    }
-    A.dg->fticket = 0;
+  if (warp < 3) {  // one warp per component over the blocks' partials
+    double a = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) a += __ldcg(&A.part[3 * b + warp]);
+    a = warp_sum(a);
+    if (lane == 0) A.dg->force[warp] = a;
   }
+  if (threadIdx.x == 0) A.dg->fticket = 0;
 }
 
 void launch_forces(ibm_ctx *c) {
