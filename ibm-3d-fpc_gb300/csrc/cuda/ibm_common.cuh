@@ -162,6 +162,7 @@ struct KScal {
   double cyc_eps;     // the current cycle also ends when the estimate reaches this
   double cyc_rtol;    // cyc_eps = max(eps, cyc_rtol * true residual at the cycle start)
   double nu[kMaxKdim + 1];            // norms of the stored (unnormalised) basis vectors
+  double inu[kMaxKdim + 1];           // their reciprocals (one division per vector, not one per thread)
   double H[(kMaxKdim + 1) * kMaxKdim];  // H(i,j) at [i*kMaxKdim + j]
   double cs[kMaxKdim], sn[kMaxKdim], g[kMaxKdim + 1], y[kMaxKdim];
   double coef[kMaxKdim + 1];          // coefficients of the next basis update

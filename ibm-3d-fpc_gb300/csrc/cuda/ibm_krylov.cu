@@ -102,8 +102,8 @@ __device__ bool block_partials_and_last(double *sacc, int nd, double *part, unsi
 }
 
 // r = b - Ar x; V_0 = r; |b|^2, |r|^2. Last block: norms, tolerance, state.
-__global__ void __launch_bounds__(kThreads) k_init(KSys *sys, int nsys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_init(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   __shared__ double sacc[2 * kWarps];
   if (threadIdx.x < 2 * kWarps) sacc[threadIdx.x] = 0.0;
@@ -183,150 +183,232 @@ __global__ void __launch_bounds__(kThreads) k_init(KSys *sys, int nsys) {
     else if (sc->maxit <= 0) { sc->status = 2; sc->active = 0; }
     else { sc->status = 0; sc->active = 1; }
     sc->nu[0] = rn;
+    sc->inu[0] = 1.0 / rn;
     sc->g[0] = rn;
   }
 }
 
-// w = A z_j (z_j = M v_j by the system's preconditioner mode), d1_k = (V_k, w).
-// Closes Arnoldi step j (one thread): h(j+1,j) = |v_{j+1}| = hn, the previous
-// rotations applied to the new Hessenberg column, a new Givens rotation, the
-// residual estimate and the stop tests; at the end of a cycle the
-// back-substitution H y = g and the update coefficients y / nu.
+// Closes Arnoldi step j: h(j+1,j) = |v_{j+1}| = hn, the previous rotations
+// applied to the new Hessenberg column, a new Givens rotation, the residual
+// estimate and the stop tests; at the end of a cycle the back-substitution
+// H y = g and the update coefficients y / nu. Called by every thread of the
+// last block: what the serial part needs is loaded into shared memory by as
+// many threads at once (one memory latency each for the column and, at a
+// cycle's end, the triangle), and one thread then works there. One thread
+// walking global memory paid a latency per rotation and per matrix entry.
 __device__ void arnoldi_finalize(KScal *sc, int j, double hn) {
-  const int K = kMaxKdim;
-  sc->nu[j + 1] = hn;
-  sc->H[(j + 1) * K + j] = hn;
-  // apply previous rotations to the new column, then a new rotation
-  for (int q = 0; q < j; ++q) {
-    const double t = sc->H[q * K + j];
-    sc->H[q * K + j] = sc->sn[q] * sc->H[(q + 1) * K + j] + sc->cs[q] * t;
-    sc->H[(q + 1) * K + j] = -sc->sn[q] * t + sc->cs[q] * sc->H[(q + 1) * K + j];
+  constexpr int K = kMaxKdim;
+  __shared__ double col[K + 1], rc[K], rs[K], tri[K * (K + 1) / 2];
+  __shared__ int ended;
+  const int tid = threadIdx.x;
+  const double gj = sc->g[j], eps = sc->eps, cyc_eps = sc->cyc_eps;
+  const int kdim = sc->kdim, iters = sc->iters + 1, maxit = sc->maxit, m = j + 1;
+  for (int q = tid; q <= j; q += blockDim.x) {
+    col[q] = sc->H[q * K + j];
+    if (q < j) { rc[q] = sc->cs[q]; rs[q] = sc->sn[q]; }
   }
-  const double a = sc->H[j * K + j], b = sc->H[(j + 1) * K + j];
-  double gam = sqrt(b * b + a * a);
-  if (gam == 0.0) gam = 2.220446049250313e-16;
-  sc->cs[j] = a / gam;
-  sc->sn[j] = b / gam;
-  sc->g[j + 1] = -sc->sn[j] * sc->g[j];
-  sc->g[j] = sc->cs[j] * sc->g[j];
-  sc->H[j * K + j] = sc->sn[j] * b + sc->cs[j] * a;
-  sc->i = j + 1;
-  sc->iters += 1;
-  sc->r_norm = fabs(sc->g[j + 1]);
-  const bool claimed = sc->r_norm <= sc->eps || hn == 0.0;
-  const bool cycle_done = sc->r_norm <= sc->cyc_eps;
-  if (!isfinite(sc->r_norm)) sc->nonfinite = 1;
-  if (claimed || cycle_done || sc->i >= sc->kdim || sc->iters >= sc->maxit || !isfinite(sc->r_norm)) {
-    sc->claimed = claimed;
-    sc->active = 0;
-    sc->cycle_end = 1;
-    // back substitution H y = g for the i x i upper triangle
-    const int m = sc->i;
-    for (int q = m - 1; q >= 0; --q) {
-      double t = sc->g[q];
-      for (int c = q + 1; c < m; ++c) t -= sc->H[q * K + c] * sc->y[c];
-      sc->y[q] = t / sc->H[q * K + q];
-    }
-    for (int q = 0; q < m; ++q) sc->coef[q] = sc->y[q] / sc->nu[q];
-  }
-}
-
-// FP64 Arnoldi kernels with a short basis (at most kDots64 vectors) keep each
-// dot product as a per-thread sum over all the thread's rows and reduce it
-// across the warp once per kernel; a reduction per tile of rows cost about as
-// much FP64 issue as the products themselves.
-constexpr int kDots64 = 8;
-__device__ __forceinline__ void flush_dots64(const double (&pd)[kDots64], int nd, double *sacc, int warp,
-                                             int lane) {
-#pragma unroll
-  for (int kk = 0; kk < kDots64; ++kk) {
-    if (kk >= nd) break;
-    const double p = warp_sum(pd[kk]);
-    if (lane == 0) sacc[kk * kWarps + warp] += p;
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) k_arnoldi_spmv(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
-  KScal *sc = S.s;
-  if (!sc->active || S.a32) return;
-  const int j = sc->i, nd = j + 1;
-  __shared__ double sacc[(kMaxKdim + 1) * kWarps];
-  for (int t = threadIdx.x; t < nd * kWarps; t += blockDim.x) sacc[t] = 0.0;
-  __shared__ double inv_nu;
-  if (threadIdx.x == 0) inv_nu = 1.0 / sc->nu[j];
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double *vj = S.V + (long)j * S.ldv;
-  double pd[kDots64];
+  if (tid == 32) {
+    sc->nu[j + 1] = hn;
+    sc->inu[j + 1] = 1.0 / hn;
+  }
+  if (tid == 0) {
+    double a = col[0];
+    for (int q = 0; q < j; ++q) {
+      const double t = a, h = col[q + 1];
+      col[q] = rs[q] * h + rc[q] * t;
+      a = -rs[q] * t + rc[q] * h;
+    }
+    const double b = hn;
+    double gam = sqrt(b * b + a * a);
+    if (gam == 0.0) gam = 2.220446049250313e-16;
+    const double c = a / gam, s = b / gam;
+    const double gn = -s * gj;
+    const double r_norm = fabs(gn);
+    col[j] = s * b + c * a;
+    rc[0] = c * gj;  // the rotated g_j
+    sc->cs[j] = c;
+    sc->sn[j] = s;
+    sc->g[j + 1] = gn;
+    sc->g[j] = c * gj;
+    sc->i = m;
+    sc->iters = iters;
+    sc->r_norm = r_norm;
+    const bool claimed = r_norm <= eps || hn == 0.0;
+    const bool cycle_done = r_norm <= cyc_eps;
+    if (!isfinite(r_norm)) sc->nonfinite = 1;
+    const bool end = claimed || cycle_done || m >= kdim || iters >= maxit || !isfinite(r_norm);
+    if (end) {
+      sc->claimed = claimed;
+      sc->active = 0;
+      sc->cycle_end = 1;
+    }
+    ended = end;
+  }
+  __syncthreads();
+  for (int q = tid; q <= j; q += blockDim.x) sc->H[q * K + j] = col[q];
+  if (!ended) return;
+  // column c of the triangle at tri[c (c + 1) / 2]; the last column is col
+  double *y = rs;  // the rotations' sines are not needed any more
+  for (int e = tid; e < j * K; e += blockDim.x) {
+    const int c = e / K, q = e - c * K;
+    if (q <= c) tri[c * (c + 1) / 2 + q] = sc->H[q * K + c];
+  }
+  for (int q = tid; q < j; q += blockDim.x) y[q] = sc->g[q];
+  if (tid == 0) y[j] = rc[0];
+  for (int q = tid; q <= j; q += blockDim.x) tri[j * (j + 1) / 2 + q] = col[q];
+  __syncthreads();
+  if (tid == 0) {
+    for (int q = m - 1; q >= 0; --q) {
+      double t = y[q];
+      for (int c = q + 1; c < m; ++c) t -= tri[c * (c + 1) / 2 + q] * y[c];
+      y[q] = t / tri[q * (q + 1) / 2 + q];
+    }
+  }
+  __syncthreads();
+  for (int q = tid; q < m; q += blockDim.x) {
+    sc->y[q] = y[q];
+    sc->coef[q] = y[q] / sc->nu[q];
+  }
+}
+
+// The FP64 Arnoldi kernels take their dot products kDots64 basis vectors at a
+// time: each stays a per-thread sum over all the thread's rows and is reduced
+// across the warp once per kernel. A longer basis takes further passes over
+// the rows that read w back (8 bytes a row beside the 64 of the eight basis
+// vectors); reducing across the warp for each tile of rows, as a loop over all
+// vectors per tile would have to, costs as many FP64 issue slots as the
+// products.
+constexpr int kDots64 = 8;
+
+// Sums of the N values of pd over the warp: value k in lanes with lane / (32 / N) == k.
+// Halves are exchanged, so a lane adds N/2 + N/4 + ... + 1 + log2(32 / N)
+// times (9 for N = 8) instead of 5 N: GB300 issues two FP64 operations per
+// clock and SM, and eight five-step butterflies in each of 32 warps took 10 us
+// of every launch.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&pd)[N], int lane) {
+  int o = 16;
 #pragma unroll
-  for (int kk = 0; kk < kDots64; ++kk) pd[kk] = 0.0;
+  for (int h = N / 2; h > 0; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double send = up ? pd[k] : pd[k + h], keep = up ? pd[k + h] : pd[k];
+      pd[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  double v = pd[0];
+  for (; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// Adds the block's nd <= kDots64 sums of this pass to sacc[kk * kWarps + warp].
+__device__ __forceinline__ void flush_dots64(double (&pd)[kDots64], int nd, double *sacc, int warp, int lane) {
+  if (nd == 1) {
+    const double v = warp_sum(pd[0]);
+    if (lane == 0) sacc[warp] = v;
+  } else if (nd <= 4) {
+    double q[4] = {pd[0], pd[1], pd[2], pd[3]};
+    const double v = warp_sums<4>(q, lane);
+    const int k = lane >> 3;
+    if ((lane & 7) == 0 && k < nd) sacc[k * kWarps + warp] = v;
+  } else {
+    const double v = warp_sums<8>(pd, lane);
+    const int k = lane >> 2;
+    if ((lane & 3) == 0 && k < nd) sacc[k * kWarps + warp] = v;
+  }
+}
+
+// Row r of w = A z_j. Mode 0: z_j in double-float from the class table; 1: A
+// applied to the FP64 vector z times inv_nu (folded Jacobi, or the explicit
+// z); 2: A applied to the FP32 direction z_j.
+template <int MODE>
+__device__ __forceinline__ double spmv_row64(const KSys &S, long r, const double *z, const float *zj, double inv_nu) {
+  int i, jj, k;
+  sys_ijk(r, S, i, jj, k);
+  if constexpr (MODE == 0) {
+    // the seven products and their sum in double-float, widened once (two
+    // conversions and one FP64 add); a neighbour outside the box reads as 0:
+    // its product and sum are exact no-ops, so all seven loads issue together
+    const float4 *c4 = reinterpret_cast<const float4 *>(S.tabdf + 16 * (long)S.cls[r]);
+    const long sy = S.nx, sz = (long)S.nx * S.ny;
+    const float z0 = zj[r], zxm = i > 0 ? zj[r - 1] : 0.0f, zxp = i < S.nx - 1 ? zj[r + 1] : 0.0f,
+                zym = jj > 0 ? zj[r - sy] : 0.0f, zyp = jj < S.ny - 1 ? zj[r + sy] : 0.0f,
+                zzm = k > 0 ? zj[r - sz] : 0.0f, zzp = k < S.nz - 1 ? zj[r + sz] : 0.0f;
+    const float4 h0 = __ldg(c4), h1 = __ldg(c4 + 1), l0 = __ldg(c4 + 2), l1 = __ldg(c4 + 3);
+    float ah = 0.0f, al = 0.0f;
+    df_fma1(ah, al, h0.x, l0.x, z0);
+    df_fma1(ah, al, h0.y, l0.y, zxm);
+    df_fma1(ah, al, h0.z, l0.z, zxp);
+    df_fma1(ah, al, h0.w, l0.w, zym);
+    df_fma1(ah, al, h1.x, l1.x, zyp);
+    df_fma1(ah, al, h1.y, l1.y, zzm);
+    df_fma1(ah, al, h1.z, l1.z, zzp);
+    return (double)ah + (double)al;
+  } else {
+    long cs;
+    const double *c0 = a_row(S, r, cs);
+    if constexpr (MODE == 1) return stencil7_at(c0, cs, z, (int)r, i, jj, k, S.nx, S.ny, S.nz) * inv_nu;
+    else return stencil7_at(c0, cs, zj, (int)r, i, jj, k, S.nx, S.ny, S.nz);
+  }
+}
+
+// The rows of w = A z_j and their dot products with basis vectors c0 ..
+// c0 + nd - 1. The rows of a tile are computed before any is stored, so that
+// their loads are in flight together (a store between them would hold the
+// later ones back); later passes (c0 > 0) read w.
+template <int MODE>
+__device__ __forceinline__ void spmv_pass64(const KSys &S, const double *z, const float *zj, double inv_nu, int c0,
+                                            int nd, double (&pd)[kDots64]) {
   for (long t0 = (long)blockIdx.x * kTile; t0 < S.n; t0 += (long)gridDim.x * kTile) {
     double wv[kRowsPerThread];
 #pragma unroll
     for (int t = 0; t < kRowsPerThread; ++t) {
       const long r = t0 + t * kThreads + threadIdx.x;
       wv[t] = 0.0;
-      if (r < S.n) {
-        int i, jj, k;
-        sys_ijk(r, S, i, jj, k);
-        double w;
-        long cs;
-        const double *c0 = a_row(S, r, cs);
-        if (S.df_spmv) {
-          // A z_j with z_j exact in FP32: the seven products and their sum in
-          // double-float, widened once (two conversions and one FP64 add)
-          // (a neighbour outside the box reads as 0: its product and sum are
-          // exact no-ops, so all seven loads issue together)
-          const float4 *c4 = reinterpret_cast<const float4 *>(S.tabdf + 16 * (long)S.cls[r]);
-          const float *zj = S.Z + (long)j * S.ldv;
-          const long sy = S.nx, sz = (long)S.nx * S.ny;
-          const float z0 = zj[r], zxm = i > 0 ? zj[r - 1] : 0.0f, zxp = i < S.nx - 1 ? zj[r + 1] : 0.0f,
-                      zym = jj > 0 ? zj[r - sy] : 0.0f, zyp = jj < S.ny - 1 ? zj[r + sy] : 0.0f,
-                      zzm = k > 0 ? zj[r - sz] : 0.0f, zzp = k < S.nz - 1 ? zj[r + sz] : 0.0f;
-          const float4 h0 = __ldg(c4), h1 = __ldg(c4 + 1), l0 = __ldg(c4 + 2), l1 = __ldg(c4 + 3);
-          float ah = 0.0f, al = 0.0f;
-          df_fma1(ah, al, h0.x, l0.x, z0);
-          df_fma1(ah, al, h0.y, l0.y, zxm);
-          df_fma1(ah, al, h0.z, l0.z, zxp);
-          df_fma1(ah, al, h0.w, l0.w, zym);
-          df_fma1(ah, al, h1.x, l1.x, zyp);
-          df_fma1(ah, al, h1.y, l1.y, zzm);
-          df_fma1(ah, al, h1.z, l1.z, zzp);
-          w = (double)ah + (double)al;
-        } else if (S.pc == 0) w = stencil7_at(c0, cs, vj, (int)r, i, jj, k, S.nx, S.ny, S.nz) * inv_nu;
-        else if (S.pc == 1) w = stencil7_at(c0, cs, S.z, (int)r, i, jj, k, S.nx, S.ny, S.nz) * inv_nu;
-        else w = stencil7_at(c0, cs, S.Z + (long)j * S.ldv, (int)r, i, jj, k, S.nx, S.ny, S.nz);
-        S.w[r] = w;
-        wv[t] = w;
-      }
+      if (r < S.n) wv[t] = c0 ? S.w[r] : spmv_row64<MODE>(S, r, z, zj, inv_nu);
     }
-    if (nd <= kDots64) {  // per-thread sums over all the thread's rows (reduced once below)
-#pragma unroll
-      for (int kk = 0; kk < kDots64; ++kk) {
-        if (kk >= nd) break;
-        const double *vk = S.V + (long)kk * S.ldv;
-#pragma unroll
-        for (int t = 0; t < kRowsPerThread; ++t) {
-          const long r = t0 + t * kThreads + threadIdx.x;
-          if (r < S.n) pd[kk] = fma(vk[r], wv[t], pd[kk]);
-        }
-      }
-      continue;
-    }
-    for (int kk = 0; kk < nd; ++kk) {
-      const double *vk = S.V + (long)kk * S.ldv;
-      double p = 0.0;
+    if (c0 == 0) {
 #pragma unroll
       for (int t = 0; t < kRowsPerThread; ++t) {
         const long r = t0 + t * kThreads + threadIdx.x;
-        if (r < S.n) p = fma(vk[r], wv[t], p);
+        if (r < S.n) S.w[r] = wv[t];
       }
-      p = warp_sum(p);
-      if (lane == 0) sacc[kk * kWarps + warp] += p;
+    }
+#pragma unroll
+    for (int kk = 0; kk < kDots64; ++kk) {
+      if (kk >= nd) break;
+      const double *vk = S.V + (long)(c0 + kk) * S.ldv;
+#pragma unroll
+      for (int t = 0; t < kRowsPerThread; ++t) {
+        const long r = t0 + t * kThreads + threadIdx.x;
+        if (r < S.n) pd[kk] = fma(vk[r], wv[t], pd[kk]);
+      }
     }
   }
-  if (nd <= kDots64) flush_dots64(pd, nd, sacc, warp, lane);
+}
+
+// w = A z_j (z_j = M v_j by the system's preconditioner mode), d1_k = (V_k, w).
+__global__ void __launch_bounds__(kThreads) k_arnoldi_spmv(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
+  KScal *sc = S.s;
+  if (!sc->active || S.a32) return;
+  const int j = sc->i, nd = j + 1;
+  const double inv_nu = sc->inu[j];
+  __shared__ double sacc[(kMaxKdim + 1) * kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double *z = S.pc == 0 ? S.V + (long)j * S.ldv : S.z;
+  const float *zj = S.Z + (long)j * S.ldv;
+  for (int c0 = 0; c0 < nd; c0 += kDots64) {
+    const int ndc = min(nd - c0, kDots64);
+    double pd[kDots64];
+#pragma unroll
+    for (int kk = 0; kk < kDots64; ++kk) pd[kk] = 0.0;
+    if (S.df_spmv) spmv_pass64<0>(S, z, zj, inv_nu, c0, ndc, pd);
+    else if (S.pc != 2) spmv_pass64<1>(S, z, zj, inv_nu, c0, ndc, pd);
+    else spmv_pass64<2>(S, z, zj, inv_nu, c0, ndc, pd);
+    flush_dots64(pd, ndc, sacc + c0 * kWarps, warp, lane);
+  }
   if (!block_partials_and_last(sacc, nd, S.part, &sc->ticket)) return;
   __shared__ double tot[kMaxKdim + 1];
   reduce_partials(S.part, gridDim.x, nd, tot);
@@ -340,59 +422,73 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv(KSys *sys) {
   if (threadIdx.x == 0) sc->ticket = 0;
 }
 
+// w - sum_k cf_k V_k for the rows of one tile of a thread, each row's terms in
+// order of k; the rows' loads of a basis vector are in flight together.
+__device__ __forceinline__ void orth_rows64(const KSys &S, long t0, const double *cf, int nd,
+                                            double (&wv)[kRowsPerThread]) {
+#pragma unroll
+  for (int t = 0; t < kRowsPerThread; ++t) {
+    const long r = t0 + t * kThreads + threadIdx.x;
+    wv[t] = r < S.n ? S.w[r] : 0.0;
+  }
+#pragma unroll 2
+  for (int kk = 0; kk < nd; ++kk) {
+    const double *vk = S.V + (long)kk * S.ldv;
+    const double c = -cf[kk];
+#pragma unroll
+    for (int t = 0; t < kRowsPerThread; ++t) {
+      const long r = t0 + t * kThreads + threadIdx.x;
+      if (r < S.n) wv[t] = fma(c, vk[r], wv[t]);
+    }
+  }
+}
+
 // w -= sum_k coef_k V_k (first pass), d2_k = (V_k, w). Last block: the
 // second-pass coefficients and the Hessenberg column above the diagonal.
-__global__ void __launch_bounds__(kThreads) k_arnoldi_orth(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_arnoldi_orth(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || S.a32 || S.cgs1) return;
   const int j = sc->i, nd = j + 1;
   __shared__ double sacc[(kMaxKdim + 1) * kWarps];
   __shared__ double cf[kMaxKdim + 1];
-  for (int t = threadIdx.x; t < nd * kWarps; t += blockDim.x) sacc[t] = 0.0;
   for (int t = threadIdx.x; t < nd; t += blockDim.x) cf[t] = sc->coef[t];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double pd[kDots64];
+  for (int c0 = 0; c0 < nd; c0 += kDots64) {
+    const int ndc = min(nd - c0, kDots64);
+    double pd[kDots64];
 #pragma unroll
-  for (int kk = 0; kk < kDots64; ++kk) pd[kk] = 0.0;
-  for (long t0 = (long)blockIdx.x * kTile; t0 < S.n; t0 += (long)gridDim.x * kTile) {
-    double wv[kRowsPerThread];
-#pragma unroll
-    for (int t = 0; t < kRowsPerThread; ++t) {
-      const long r = t0 + t * kThreads + threadIdx.x;
-      wv[t] = 0.0;
-      if (r < S.n) {
-        double w = S.w[r];
-        for (int kk = 0; kk < nd; ++kk) w = fma(-cf[kk], S.V[(long)kk * S.ldv + r], w);
-        S.w[r] = w;
-        wv[t] = w;
-      }
-    }
-    if (nd <= kDots64) {
-#pragma unroll
-      for (int kk = 0; kk < kDots64; ++kk) {
-        if (kk >= nd) break;
+    for (int kk = 0; kk < kDots64; ++kk) pd[kk] = 0.0;
+    for (long t0 = (long)blockIdx.x * kTile; t0 < S.n; t0 += (long)gridDim.x * kTile) {
+      double wv[kRowsPerThread];
+      if (c0 == 0) {
+        orth_rows64(S, t0, cf, nd, wv);
 #pragma unroll
         for (int t = 0; t < kRowsPerThread; ++t) {
           const long r = t0 + t * kThreads + threadIdx.x;
-          if (r < S.n) pd[kk] = fma(S.V[(long)kk * S.ldv + r], wv[t], pd[kk]);
+          if (r < S.n) S.w[r] = wv[t];
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < kRowsPerThread; ++t) {
+          const long r = t0 + t * kThreads + threadIdx.x;
+          wv[t] = r < S.n ? S.w[r] : 0.0;
         }
       }
-      continue;
-    }
-    for (int kk = 0; kk < nd; ++kk) {
-      double p = 0.0;
 #pragma unroll
-      for (int t = 0; t < kRowsPerThread; ++t) {
-        const long r = t0 + t * kThreads + threadIdx.x;
-        if (r < S.n) p = fma(S.V[(long)kk * S.ldv + r], wv[t], p);
+      for (int kk = 0; kk < kDots64; ++kk) {
+        if (kk >= ndc) break;
+        const double *vk = S.V + (long)(c0 + kk) * S.ldv;
+#pragma unroll
+        for (int t = 0; t < kRowsPerThread; ++t) {
+          const long r = t0 + t * kThreads + threadIdx.x;
+          if (r < S.n) pd[kk] = fma(vk[r], wv[t], pd[kk]);
+        }
       }
-      p = warp_sum(p);
-      if (lane == 0) sacc[kk * kWarps + warp] += p;
     }
+    flush_dots64(pd, ndc, sacc + c0 * kWarps, warp, lane);
   }
-  if (nd <= kDots64) flush_dots64(pd, nd, sacc, warp, lane);
   if (!block_partials_and_last(sacc, nd, S.part, &sc->ticket)) return;
   __shared__ double tot[kMaxKdim + 1];
   reduce_partials(S.part, gridDim.x, nd, tot);
@@ -408,8 +504,8 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_orth(KSys *sys) {
 // v_{j+1} = w - sum_k coef_k V_k, stored unnormalised, with its exact norm.
 // Last block: Hessenberg column, Givens rotation, stop test, and at the end
 // of a cycle the back substitution.
-__global__ void __launch_bounds__(kThreads) k_arnoldi_next(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_arnoldi_next(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || S.a32) return;
   const int j = sc->i, nd = j + 1;
@@ -423,17 +519,17 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next(KSys *sys) {
   const bool store = nd < sc->kdim;  // the last vector of a full cycle is never used
   double p = 0.0;  // per thread over all its rows
   for (long t0 = (long)blockIdx.x * kTile; t0 < S.n; t0 += (long)gridDim.x * kTile) {
+    double wv[kRowsPerThread];
+    orth_rows64(S, t0, cf, nd, wv);
 #pragma unroll
     for (int t = 0; t < kRowsPerThread; ++t) {
       const long r = t0 + t * kThreads + threadIdx.x;
       if (r < S.n) {
-        double w = S.w[r];
-        for (int kk = 0; kk < nd; ++kk) w = fma(-cf[kk], S.V[(long)kk * S.ldv + r], w);
         if (store) {
-          vn[r] = w;
-          if (S.vcur) S.vcur[r] = (float)w;
+          vn[r] = wv[t];
+          if (S.vcur) S.vcur[r] = (float)wv[t];
         }
-        p = fma(w, w, p);
+        p = fma(wv[t], wv[t], p);
       }
     }
   }
@@ -443,16 +539,14 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next(KSys *sys) {
   __shared__ double tot[1];
   reduce_partials(S.part, gridDim.x, 1, tot);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    sc->ticket = 0;
-    arnoldi_finalize(sc, j, sqrt(tot[0]));
-  }
+  if (threadIdx.x == 0) sc->ticket = 0;
+  arnoldi_finalize(sc, j, sqrt(tot[0]));
 }
 
 // Cycle end, solution update. pc 0: x += invd * (V c); pc 1: z = V c (the
 // caller applies the preconditioner and then k_add_z); pc 2: x += Z y.
-__global__ void __launch_bounds__(kThreads) k_cycle_update(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_cycle_update(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->cycle_end) return;
   const int m = sc->i;
@@ -524,8 +618,8 @@ __global__ void __launch_bounds__(kThreads) k_cycle_update(KSys *sys) {
   }
 }
 
-__global__ void k_add_z(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void k_add_z(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   if (!S.s->cycle_end || S.pc != 1) return;
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x)
     S.x[r] = S.x[r] + S.z2[r];
@@ -543,8 +637,8 @@ constexpr double kDfRowBound = 4.547473508864641e-13;  // 2^-41
 // the per-row bounds; a decision closer to the tolerance than
 // kDfRowBound * M is taken again from an FP64 residual, and the rest of the
 // solve stays in FP64, so convergence is always decided within FP64 rounding.
-__global__ void __launch_bounds__(kThreads) k_cycle_residual(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->cycle_end) return;
   const bool df = S.df_resid && !sc->use64;
@@ -644,6 +738,7 @@ __global__ void __launch_bounds__(kThreads) k_cycle_residual(KSys *sys) {
     sc->i = 0;
     sc->claimed = 0;
     sc->nu[0] = rt;
+    sc->inu[0] = 1.0 / rt;
     sc->g[0] = rt;
     sc->active = 1;
   }
@@ -666,8 +761,8 @@ __device__ __forceinline__ float warp_sum_f(float v) {
   return v;
 }
 
-__global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || !S.a32) return;
   const int j = sc->i, nd = j + 1;
@@ -798,8 +893,8 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(KSys *sys) {
   if (threadIdx.x == 0) sc->ticket = 0;
 }
 
-__global__ void __launch_bounds__(kThreads) k_arnoldi_orth32(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_arnoldi_orth32(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || !S.a32) return;
   const int j = sc->i, nd = j + 1;
@@ -912,8 +1007,8 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_orth32(KSys *sys) {
   if (threadIdx.x == 0) sc->ticket = 0;
 }
 
-__global__ void __launch_bounds__(kThreads) k_arnoldi_next32(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_arnoldi_next32(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || !S.a32) return;
   const int j = sc->i, nd = j + 1;
@@ -976,10 +1071,8 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next32(KSys *sys) {
   __shared__ double tot[1];
   reduce_partials(S.part, gridDim.x, 1, tot);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    sc->ticket = 0;
-    arnoldi_finalize(sc, j, sqrt(tot[0]));
-  }
+  if (threadIdx.x == 0) sc->ticket = 0;
+  arnoldi_finalize(sc, j, sqrt(tot[0]));
 }
 
 // Two FP32 Jacobi sweeps from zero in one pass (momentum preconditioner of
@@ -1045,12 +1138,12 @@ __device__ __forceinline__ void jacobi_two_rows4(const KSys &S, const float *__r
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_jacobi32_two(KSys *sys) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_jacobi32_two(const __grid_constant__ KSysPack P) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || S.pc != 2 || S.pc_cb) return;
   const int j = sc->i;
-  const float inv_nu = (float)(1.0 / sc->nu[j]);
+  const float inv_nu = (float)sc->inu[j];
   float *out = S.Z + (long)j * S.ldv;
   // an FP64 basis is read through its FP32 copy when there is one: the same
   // values ((float) V_j), one conversion per row where the vector is formed
@@ -1063,12 +1156,12 @@ __global__ void __launch_bounds__(kThreads) k_jacobi32_two(KSys *sys) {
 
 // FP32 inner preconditioner for the flexible form: zf = D^-1 v (v = V_j / nu_j),
 // then `sweeps-1` Jacobi sweeps zf <- zf + D^-1 (v - A zf); result to Z_j.
-__global__ void __launch_bounds__(kThreads) k_jacobi32_first(KSys *sys, int to_z) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_jacobi32_first(const __grid_constant__ KSysPack P, int to_z) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || S.pc != 2 || S.pc_cb) return;
   const int j = sc->i;
-  const double inv_nu = 1.0 / sc->nu[j];
+  const double inv_nu = sc->inu[j];
   const double *vj = S.V + (long)j * S.ldv;
   const float *vjf = S.Vf + (long)j * S.ldv;
   float *out = to_z ? S.Z + (long)j * S.ldv : S.zf;
@@ -1082,12 +1175,13 @@ __global__ void __launch_bounds__(kThreads) k_jacobi32_first(KSys *sys, int to_z
     out[r] = (float)((S.a32 ? (double)vjf[r] : vj[r]) * inv_nu) * S.invdf[r];
 }
 
-__global__ void __launch_bounds__(kThreads) k_jacobi32_sweep(KSys *sys, int src_is_zf, int to_z) {
-  KSys &S = sys[blockIdx.y];
+__global__ void __launch_bounds__(kThreads) k_jacobi32_sweep(const __grid_constant__ KSysPack P, int src_is_zf,
+                                                             int to_z) {
+  const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || S.pc != 2 || S.pc_cb) return;
   const int j = sc->i;
-  const double inv_nu = 1.0 / sc->nu[j];
+  const double inv_nu = sc->inu[j];
   const double *vj = S.V + (long)j * S.ldv;
   const float *vjf = S.Vf + (long)j * S.ldv;
   const float *src = src_is_zf ? S.zf : S.zf2;
@@ -1104,10 +1198,10 @@ __global__ void __launch_bounds__(kThreads) k_jacobi32_sweep(KSys *sys, int src_
   }
 }
 
-__global__ void k_flags(KSys *sys, int nsys, KFlags *out) {
+__global__ void k_flags(const __grid_constant__ KSysPack P, int nsys, KFlags *out) {
   const int t = threadIdx.x;
   if (t < nsys) {
-    KScal *sc = sys[t].s;
+    KScal *sc = P.s[t].s;
     out[t].active = sc->active;
     out[t].cycle_end = sc->cycle_end;
     out[t].status = sc->status;
@@ -1121,17 +1215,17 @@ __global__ void k_flags(KSys *sys, int nsys, KFlags *out) {
 // Loop control of the graph form: WHILE runs while any system is active or
 // has a finished cycle to close; the SWITCH picks the cycle-end body (0) when
 // any system closed a cycle, else the Arnoldi body (1).
-__global__ void k_set_while(KSys *sys, int nsys, cudaGraphConditionalHandle hw) {
+__global__ void k_set_while(const __grid_constant__ KSysPack P, int nsys, cudaGraphConditionalHandle hw) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   unsigned run = 0;
-  for (int s = 0; s < nsys; ++s) run |= (sys[s].s->active | sys[s].s->cycle_end) ? 1u : 0u;
+  for (int s = 0; s < nsys; ++s) run |= (P.s[s].s->active | P.s[s].s->cycle_end) ? 1u : 0u;
   cudaGraphSetConditional(hw, run);
 }
 
-__global__ void k_set_switch(KSys *sys, int nsys, cudaGraphConditionalHandle hs, unsigned long long *loops) {
+__global__ void k_set_switch(const __grid_constant__ KSysPack P, int nsys, cudaGraphConditionalHandle hs, unsigned long long *loops) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int end = 0;
-  for (int s = 0; s < nsys; ++s) end |= sys[s].s->cycle_end;
+  for (int s = 0; s < nsys; ++s) end |= P.s[s].s->cycle_end;
   cudaGraphSetConditional(hs, end ? 0u : 1u);
   loops[end ? 0 : 1] += 1;
 }
@@ -1184,7 +1278,6 @@ void Krylov::configure(int nsys_, const KSysHost *hs) {
     sl.part.alloc(need_part);
   }
   scal.alloc(nsys);
-  dsys.alloc(nsys);
   dflags.alloc(nsys);
   if (!hflags) IBM_CUDA_TRY(cudaMallocHost((void **)&hflags, sizeof(KFlags) * kMaxSys));
 }
@@ -1207,11 +1300,10 @@ Krylov::~Krylov() {
 void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, unsigned mask, bool x_zero) {
   bound_mask = mask;
   bound_x_zero = x_zero;
-  KSys hsys[kMaxSys];
-  memset(hsys, 0, sizeof(hsys));
+  memset(&pack, 0, sizeof(pack));
   for (int s = 0; s < nsys; ++s) {
     const KSysHost &h = slot[s].host;
-    KSys &k = hsys[s];
+    KSys &k = pack.s[s];
     k.nx = h.nx; k.ny = h.ny; k.nz = h.nz; k.n = ((mask >> s) & 1u) ? h.n : 0;
     k.fdx = make_fastdiv((unsigned)h.nx); k.fdy = make_fastdiv((unsigned)h.ny);
     k.A = h.A; k.Ar = h.Ar; k.invd = h.invd; k.Af = h.Af; k.invdf = h.invdf; k.Ajf = h.Ajf;
@@ -1236,7 +1328,6 @@ void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, uns
     k.pc_cb = h.pc_cb;
     k.s = scal.p + s;
   }
-  IBM_CUDA_TRY(cudaMemcpyAsync(dsys.p, hsys, sizeof(KSys) * nsys, cudaMemcpyHostToDevice, st));
   static KScal init[kMaxSys];
   memset(init, 0, sizeof(init));
   for (int s = 0; s < nsys; ++s) {
@@ -1252,7 +1343,7 @@ void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, uns
 void Krylov::read_flags(cudaStream_t st) {
   {
     LaunchScope ls(K_GM_UPDATE, st, 0.0);
-    k_flags<<<1, 32, 0, st>>>(dsys.p, nsys, dflags.p);
+    k_flags<<<1, 32, 0, st>>>(pack, nsys, dflags.p);
   }
   IBM_CUDA_TRY(cudaMemcpyAsync(hflags, dflags.p, sizeof(KFlags) * nsys, cudaMemcpyDeviceToHost, st));
   IBM_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1264,7 +1355,6 @@ void Krylov::read_flags(cudaStream_t st) {
 // bytes are attributed.
 void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *fl, unsigned mask) {
   const dim3 grid(nblk, nsys), gridu(nblk * 2, nsys);
-  KSys *dev = dsys.p;
   auto rows = [&](int s) { return ((mask >> s) & 1u) ? (double)slot[s].host.n : 0.0; };
   double bu = 0.0, br = 0.0, ba = 0.0;
   if (fl) {
@@ -1279,7 +1369,7 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
   }
   {
     LaunchScope ls(K_GM_UPDATE, st, bu);
-    k_cycle_update<<<wave(k_cycle_update), kThreads, 0, st>>>(dev);
+    k_cycle_update<<<wave(k_cycle_update), kThreads, 0, st>>>(pack);
   }
   bool cb = false;
   for (int s = 0; s < nsys; ++s) {
@@ -1293,15 +1383,14 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
   }
   if (cb) {
     LaunchScope ls(K_GM_ADDZ, st, ba);
-    k_add_z<<<wave(k_add_z), kThreads, 0, st>>>(dev);
+    k_add_z<<<wave(k_add_z), kThreads, 0, st>>>(pack);
   }
   LaunchScope ls(K_GM_RESID, st, br);
-  k_cycle_residual<<<wave(k_cycle_residual), kThreads, 0, st>>>(dev);
+  k_cycle_residual<<<wave(k_cycle_residual), kThreads, 0, st>>>(pack);
 }
 
 void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl, unsigned mask) {
   const dim3 grid(nblk, nsys), gridu(nblk * 2, nsys);
-  KSys *dev = dsys.p;
   auto rows = [&](int s) { return ((mask >> s) & 1u) ? (double)slot[s].host.n : 0.0; };
   for (int s = 0; s < nsys; ++s) {
     if (!((mask >> s) & 1u) || (fl && !fl[s].active)) continue;
@@ -1316,7 +1405,7 @@ void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl
       VecRef in;
       if (h.a32) in.basef = slot[s].Vf.p;
       else in.base = slot[s].V.p;
-      in.ld = h.n; in.idx = &scal.p[s].i; in.nu = scal.p[s].nu;
+      in.ld = h.n; in.idx = &scal.p[s].i; in.inu = scal.p[s].inu;
       OutRef out;
       out.f = slot[s].Z.p; out.ld = h.n; out.idx = &scal.p[s].i;
       pc.apply(pc.ctx, st, s, in, out, &scal.p[s].active);
@@ -1355,19 +1444,19 @@ void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl
   if (inner_sweeps > 0) {
     if (inner_sweeps == 2) {
       LaunchScope ls(K_GM_JAC32, st, j32two);
-      k_jacobi32_two<<<wave(k_jacobi32_two), kThreads, 0, st>>>(dev);
+      k_jacobi32_two<<<wave(k_jacobi32_two), kThreads, 0, st>>>(pack);
     } else if (inner_sweeps == 1) {
       LaunchScope ls(K_GM_JAC32, st, 16.0 * r32);
-      k_jacobi32_first<<<gridu, kThreads, 0, st>>>(dev, 1);
+      k_jacobi32_first<<<gridu, kThreads, 0, st>>>(pack, 1);
     } else {
       {
         LaunchScope ls(K_GM_JAC32, st, 16.0 * r32);
-        k_jacobi32_first<<<gridu, kThreads, 0, st>>>(dev, 0);
+        k_jacobi32_first<<<gridu, kThreads, 0, st>>>(pack, 0);
       }
       int src_zf = 1;
       for (int q = 1; q < inner_sweeps; ++q) {
         LaunchScope ls(K_GM_JAC32, st, 48.0 * r32);
-        k_jacobi32_sweep<<<gridu, kThreads, 0, st>>>(dev, src_zf, q == inner_sweeps - 1);
+        k_jacobi32_sweep<<<gridu, kThreads, 0, st>>>(pack, src_zf, q == inner_sweeps - 1);
         src_zf ^= 1;
       }
     }
@@ -1375,26 +1464,26 @@ void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl
   if (any64) {
     {
       LaunchScope ls(K_GM_SPMV, st, bsp);
-      k_arnoldi_spmv<<<wave(k_arnoldi_spmv), kThreads, 0, st>>>(dev);
+      k_arnoldi_spmv<<<wave(k_arnoldi_spmv), kThreads, 0, st>>>(pack);
     }
     if (any_orth) {
       LaunchScope ls(K_GM_ORTH, st, bor_orth);
-      k_arnoldi_orth<<<wave(k_arnoldi_orth), kThreads, 0, st>>>(dev);
+      k_arnoldi_orth<<<wave(k_arnoldi_orth), kThreads, 0, st>>>(pack);
     }
     LaunchScope ls(K_GM_NEXT, st, bor + bnx);
-    k_arnoldi_next<<<wave(k_arnoldi_next), kThreads, 0, st>>>(dev);
+    k_arnoldi_next<<<wave(k_arnoldi_next), kThreads, 0, st>>>(pack);
   }
   if (any32) {
     {
       LaunchScope ls(K_GM_SPMV, st, bsp32);
-      k_arnoldi_spmv32<<<wave(k_arnoldi_spmv32), kThreads, 0, st>>>(dev);
+      k_arnoldi_spmv32<<<wave(k_arnoldi_spmv32), kThreads, 0, st>>>(pack);
     }
     {
       LaunchScope ls(K_GM_ORTH, st, bor32);
-      k_arnoldi_orth32<<<wave(k_arnoldi_orth32), kThreads, 0, st>>>(dev);
+      k_arnoldi_orth32<<<wave(k_arnoldi_orth32), kThreads, 0, st>>>(pack);
     }
     LaunchScope ls(K_GM_NEXT, st, bor32);
-    k_arnoldi_next32<<<wave(k_arnoldi_next32), kThreads, 0, st>>>(dev);
+    k_arnoldi_next32<<<wave(k_arnoldi_next32), kThreads, 0, st>>>(pack);
   }
 }
 
@@ -1418,7 +1507,7 @@ void Krylov::solve(cudaStream_t st, const double *const *b, double *const *x, co
       init_bytes += ((x_zero ? 16.0 : slot[s].host.cls ? 26.0 : 80.0) + (slot[s].vcur.p ? 4.0 : 0.0)) * slot[s].host.n;
   {
     LaunchScope ls(K_GM_INIT, st, init_bytes);
-    k_init<<<wave(k_init), kThreads, 0, st>>>(dsys.p, nsys);
+    k_init<<<wave(k_init), kThreads, 0, st>>>(pack);
   }
   for (long guard = 0;; ++guard) {
     if (guard > 4L * 1000 * 1000) throw Error(IBM_ERR_CUDA, "GMRES host loop did not terminate");
@@ -1489,17 +1578,16 @@ Krylov::GraphCounts Krylov::enqueue_graph(cudaStream_t st, const cudaStream_t bo
   GraphCounts gc;
   const long long t0 = launches();
   const dim3 grid(nblk, nsys);
-  KSys *dev = dsys.p;
   const unsigned mask = bound_mask;
   {
     LaunchScope ls(K_GM_INIT, st, 0.0);
-    k_init<<<wave(k_init), kThreads, 0, st>>>(dev, nsys);
+    k_init<<<wave(k_init), kThreads, 0, st>>>(pack);
   }
   cudaGraphConditionalHandle hw;
   IBM_CUDA_TRY(cudaGraphConditionalHandleCreate(&hw, capture_graph_of(st), 0, 0));
   {
     LaunchScope ls(K_GM_UPDATE, st, 0.0);
-    k_set_while<<<1, 32, 0, st>>>(dev, nsys, hw);
+    k_set_while<<<1, 32, 0, st>>>(pack, nsys, hw);
   }
   cudaGraph_t wbody;
   add_conditional(st, &hw, cudaGraphCondTypeWhile, 1, &wbody);
@@ -1509,18 +1597,18 @@ Krylov::GraphCounts Krylov::enqueue_graph(cudaStream_t st, const cudaStream_t bo
     IBM_CUDA_TRY(cudaGraphConditionalHandleCreate(&hs, wbody, 0, 0));
     {
       LaunchScope ls(K_GM_UPDATE, b0, 0.0);
-      k_set_switch<<<1, 32, 0, b0>>>(dev, nsys, hs, loops);
+      k_set_switch<<<1, 32, 0, b0>>>(pack, nsys, hs, loops);
     }
     cudaGraph_t cases[2];
     add_conditional(b0, &hs, cudaGraphCondTypeSwitch, 2, cases);
     end_l = capture_body(cases[0], body_st[1], [&](cudaStream_t b1) { launch_cycle_end(b1, pc, nullptr, mask); });
     arn_l = capture_body(cases[1], body_st[1], [&](cudaStream_t b1) { launch_arnoldi(b1, pc, nullptr, mask); });
     LaunchScope ls(K_GM_UPDATE, b0, 0.0);
-    k_set_while<<<1, 32, 0, b0>>>(dev, nsys, hw);
+    k_set_while<<<1, 32, 0, b0>>>(pack, nsys, hw);
   });
   {
     LaunchScope ls(K_GM_UPDATE, st, 0.0);
-    k_flags<<<1, 32, 0, st>>>(dev, nsys, dflags.p);
+    k_flags<<<1, 32, 0, st>>>(pack, nsys, dflags.p);
   }
   IBM_CUDA_TRY(cudaMemcpyAsync(host_flags, dflags.p, sizeof(KFlags) * nsys, cudaMemcpyDeviceToHost, st));
   const long long per_iter = loop_l - end_l - arn_l;  // the two control kernels

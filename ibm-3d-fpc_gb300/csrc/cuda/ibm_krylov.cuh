@@ -5,13 +5,13 @@
 namespace ibm {
 
 // A vector whose location is resolved on the device: base + (*idx) * ld,
-// optionally scaled by 1 / nu[*idx] (the unnormalised Krylov basis).
+// optionally scaled by inu[*idx] (1 / norm of the unnormalised Krylov basis vector).
 struct VecRef {
   const double *base = nullptr;
   const float *basef = nullptr;  // FP32 source (used instead of base when set)
   long ld = 0;
   const int *idx = nullptr;
-  const double *nu = nullptr;
+  const double *inu = nullptr;
 };
 struct OutRef {
   double *d = nullptr;  // FP64 destination, or
@@ -59,6 +59,13 @@ struct KSysHost {
 // FP64 cycles of the flexible form when configured. The FP64 true residual
 // at each cycle end still decides convergence.
 inline bool cgs1(const KSysHost &h) { return h.pc == 2 && !h.a32 && h.arnoldi_passes == 1; }
+
+// The systems of one batch as a kernel parameter: their fields are read from
+// constant memory, with no load through a pointer before a kernel's first
+// useful one and none repeated after its stores.
+struct KSysPack {
+  KSys s[kMaxSys];
+};
 
 struct KResult {
   int iters = 0;
@@ -112,7 +119,7 @@ class Krylov {
   int nblk_spmv32 = 0;
   Slot slot[kMaxSys];
   DBuf<KScal> scal;
-  DBuf<KSys> dsys;
+  KSysPack pack;  // the systems as bound, passed to the kernels by value
   DBuf<KFlags> dflags;
   KFlags *hflags = nullptr;
 };

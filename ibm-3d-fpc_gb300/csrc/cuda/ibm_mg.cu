@@ -239,12 +239,12 @@ template <class T>
 __global__ void k_load_input(T *bv, long n, VecRef in, const double *winv, const int *gate) {
   if (gate_off(gate)) return;
   const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
-  const double sc = in.nu ? 1.0 / in.nu[in.idx ? *in.idx : 0] : 1.0;
+  const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
   const double *src = in.base + off;
   const float *srcf = in.basef ? in.basef + off : nullptr;
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
     const double a = srcf ? (double)srcf[r] : src[r];
-    double v = in.nu ? a * sc : a;
+    double v = in.inu ? a * sc : a;
     if (winv) v = v * winv[r];
     bv[r] = (T)v;
   }
@@ -255,7 +255,7 @@ __global__ void k_load_input(T *bv, long n, VecRef in, const double *winv, const
 __global__ void k_load_input_f4(float *bv, long n, VecRef in, const float *winvf, const int *gate) {
   if (gate_off(gate)) return;
   const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
-  const float sc = in.nu ? (float)(1.0 / in.nu[in.idx ? *in.idx : 0]) : 1.0f;
+  const float sc = in.inu ? (float)in.inu[in.idx ? *in.idx : 0] : 1.0f;
   const float *srcf = in.basef + off;
   for (long r0 = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x); r0 < n; r0 += 4L * gridDim.x * blockDim.x) {
     float4 a = *reinterpret_cast<const float4 *>(srcf + r0);
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_quad_in(Recs<float, 8> R,
   if (gate_off(gate)) return;
   const long n4 = bx.n / 4;
   const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
-  const float sc = in.nu ? (float)(1.0 / in.nu[in.idx ? *in.idx : 0]) : 1.0f;
+  const float sc = in.inu ? (float)in.inu[in.idx ? *in.idx : 0] : 1.0f;
   const float *srcf = in.basef + off;
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
     const long r0 = 4 * q;
