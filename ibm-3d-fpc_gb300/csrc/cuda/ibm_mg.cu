@@ -236,28 +236,32 @@ __global__ void k_convert(const double *src, T *dst, long n) {
 
 // ---------------------------------------------------------------- V-cycle
 template <class T>
-__global__ void k_load_input(T *bv, long n, VecRef in, const double *winv, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void load_input_body(T *bv, long n, const VecRef &in, const double *winv, long t0, long ts) {
   const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
   const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
   const double *src = in.base + off;
   const float *srcf = in.basef ? in.basef + off : nullptr;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
+  for (long r = t0; r < n; r += ts) {
     const double a = srcf ? (double)srcf[r] : src[r];
     double v = in.inu ? a * sc : a;
     if (winv) v = v * winv[r];
     bv[r] = (T)v;
   }
 }
+template <class T>
+__global__ void k_load_input(T *bv, long n, VecRef in, const double *winv, const int *gate) {
+  if (gate_off(gate)) return;
+  load_input_body<T>(bv, n, in, winv, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
 // FP32 hierarchy fed from an FP32 basis: four rows per thread, scale and
 // symmetrizer applied in FP32 (n % 4 == 0, 16-byte aligned source).
-__global__ void k_load_input_f4(float *bv, long n, VecRef in, const float *winvf, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void load_input_f4_body(float *bv, long n, const VecRef &in, const float *winvf, long t0,
+                                                   long ts) {
   const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
   const float sc = in.inu ? (float)in.inu[in.idx ? *in.idx : 0] : 1.0f;
   const float *srcf = in.basef + off;
-  for (long r0 = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x); r0 < n; r0 += 4L * gridDim.x * blockDim.x) {
+  for (long r0 = 4 * t0; r0 < n; r0 += 4 * ts) {
     float4 a = *reinterpret_cast<const float4 *>(srcf + r0);
     a.x *= sc; a.y *= sc; a.z *= sc; a.w *= sc;
     if (winvf) {
@@ -267,44 +271,62 @@ __global__ void k_load_input_f4(float *bv, long n, VecRef in, const float *winvf
     *reinterpret_cast<float4 *>(bv + r0) = a;
   }
 }
+__global__ void k_load_input_f4(float *bv, long n, VecRef in, const float *winvf, const int *gate) {
+  if (gate_off(gate)) return;
+  load_input_f4_body(bv, n, in, winvf, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
 template <class T>
-__global__ void k_store_output(const T *x, long n, OutRef out, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void store_output_body(const T *x, long n, const OutRef &out, long t0, long ts) {
   const long off = out.idx ? (long)(*out.idx) * out.ld : 0;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
+  for (long r = t0; r < n; r += ts) {
     if (out.d) out.d[off + r] = (double)x[r];
     else out.f[off + r] = (float)x[r];
   }
 }
+template <class T>
+__global__ void k_store_output(const T *x, long n, OutRef out, const int *gate) {
+  if (gate_off(gate)) return;
+  store_output_body<T>(x, n, out, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
+// Kernel bodies below take their first item and stride (t0, ts) so that the
+// stand-alone kernels and the fused coarse-level kernels (k_mg_tail,
+// k_mg_cluster) run the same per-point arithmetic.
+template <class T>
+__device__ __forceinline__ void relax_zero_body(const T *wd, const T *b, T *x, long n, long t0, long ts) {
+  for (long r = t0; r < n; r += ts) x[r] = wd[r] * b[r];
+}
 template <class T>
 __global__ void k_relax_zero(const T *wd, const T *b, T *x, long n, const int *gate) {
   if (gate_off(gate)) return;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
-    x[r] = wd[r] * b[r];
+  relax_zero_body<T>(wd, b, x, n, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
 // Weighted Jacobi: t = x + wd (b - A x).
 template <class T, int NS>
-__global__ void k_relax_jacobi(const T *A, const T *wd, const T *b, const T *x, T *t, Box bx, const int *gate) {
-  if (gate_off(gate)) return;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < bx.n; r += (long)gridDim.x * blockDim.x) {
+__device__ __forceinline__ void relax_jacobi_body(const T *A, const T *wd, const T *b, const T *x, T *t, const Box &bx,
+                                                  long t0, long ts) {
+  for (long r = t0; r < bx.n; r += ts) {
     int i, j, k;
     box_ijk(r, bx, i, j, k);
     const T ax = apply_row<T, NS>(A, bx.n, x, (int)r, i, j, k, bx.nx, bx.ny, bx.nz);
     t[r] = fmat<T>(wd[r], b[r] - ax, x[r]);
   }
 }
+template <class T, int NS>
+__global__ void k_relax_jacobi(const T *A, const T *wd, const T *b, const T *x, T *t, Box bx, const int *gate) {
+  if (gate_off(gate)) return;
+  relax_jacobi_body<T, NS>(A, wd, b, x, t, bx, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
 // One colour phase of the two-colour relaxation: points of `color` take
 // x + invd (b - A x) from the phase's input; the others are copied.
 // zero_x treats the input as all zeros (first phase of a zero-guess sweep).
 template <class T, int NS>
-__global__ void k_relax_color(const T *A, const T *invd, const T *b, const T *x, T *t, Box bx, int color,
-                              int zero_x, const int *gate) {
-  if (gate_off(gate)) return;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < bx.n; r += (long)gridDim.x * blockDim.x) {
+__device__ __forceinline__ void relax_color_body(const T *A, const T *invd, const T *b, const T *x, T *t, const Box &bx,
+                                                 int color, int zero_x, long t0, long ts) {
+  for (long r = t0; r < bx.n; r += ts) {
     int i, j, k;
     box_ijk(r, bx, i, j, k);
     if (((i + j + k) & 1) != color) { t[r] = zero_x ? T(0) : x[r]; continue; }
@@ -312,6 +334,13 @@ __global__ void k_relax_color(const T *A, const T *invd, const T *b, const T *x,
     const T ax = apply_row<T, NS>(A, bx.n, x, (int)r, i, j, k, bx.nx, bx.ny, bx.nz);
     t[r] = fmat<T>(invd[r], b[r] - ax, x[r]);
   }
+}
+template <class T, int NS>
+__global__ void k_relax_color(const T *A, const T *invd, const T *b, const T *x, T *t, Box bx, int color,
+                              int zero_x, const int *gate) {
+  if (gate_off(gate)) return;
+  relax_color_body<T, NS>(A, invd, b, x, t, bx, color, zero_x, (long)blockIdx.x * blockDim.x + threadIdx.x,
+                          (long)gridDim.x * blockDim.x);
 }
 
 // Colour-split coefficients of levels with an even nx. Rows 2m and 2m+1 lie on
@@ -393,13 +422,12 @@ __global__ void k_split_colors(const T *A, const T *invd, Box bx, T *R) {
 // other colour's points). Points of one colour are not coupled to each other
 // in a 7-point stencil, so the phase reads only values it does not write.
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_relax_rb(Recs<T, 8> R, const T *__restrict__ b, T *x,
-                                                       Box bx, int color, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void relax_rb_body(const Recs<T, 8> &R, const T *b, T *x, const Box &bx, int color, long t0,
+                                              long ts) {
   const long h = bx.n / 2;
   const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
   const long sy = nx, sz = (long)nx * ny;
-  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < h; m += (long)gridDim.x * blockDim.x) {
+  for (long m = t0; m < h; m += ts) {
     int i, j, k;
     const long r = rb_row(m, color, bx, i, j, k);
     T c[8];
@@ -420,6 +448,12 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb(Recs<T, 8> R, const T *__
     x[r] = c[0] * (b[r] - acc);
   }
 }
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_relax_rb(Recs<T, 8> R, const T *__restrict__ b, T *x,
+                                                       Box bx, int color, const int *gate) {
+  if (gate_off(gate)) return;
+  relax_rb_body<T>(R, b, x, bx, color, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
 // 27-point levels: diagonal neighbours share a colour, so a phase cannot
 // update in place: it writes every point of the pair to the other buffer (the
@@ -439,9 +473,6 @@ __global__ void k_split_colors27(const T *A, const T *invd, Box bx, T *R) {
   }
 }
 
-// Kernel bodies below take their first item and stride (t0, ts) so that the
-// stand-alone kernels and the fused coarse-level kernel (k_mg_tail) run the
-// same per-point arithmetic.
 template <class T>
 __device__ __forceinline__ void relax_rb27_body(const Recs<T, 28> &R, const T *b, const T *x, T *t, const Box &bx,
                                                 int color, int zero_x, long t0, long ts) {
@@ -655,14 +686,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_residual_rb27(Recs<T, 28> R, co
 // residual is zero up to rounding and is written as 0; colour-0 points take
 // b - A x with the colour-split coefficients (centre first, as apply_row).
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_residual_rb(Recs<T, 8> R, const T *__restrict__ b,
-                                                          const T *__restrict__ x, T *__restrict__ res, Box bx,
-                                                          const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void residual_rb_body(const Recs<T, 8> &R, const T *b, const T *x, T *res, const Box &bx,
+                                                 long t0, long ts) {
   const long h = bx.n / 2;
   const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
   const long sy = nx, sz = (long)nx * ny;
-  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < h; m += (long)gridDim.x * blockDim.x) {
+  for (long m = t0; m < h; m += ts) {
     int i, j, k;
     const long r = rb_row(m, 0, bx, i, j, k);
     T c[8];
@@ -685,6 +714,13 @@ __global__ void __launch_bounds__(kThreads) k_residual_rb(Recs<T, 8> R, const T 
     res[r] = b[r] - acc;
     res[r ^ 1] = T(0);
   }
+}
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_residual_rb(Recs<T, 8> R, const T *__restrict__ b,
+                                                          const T *__restrict__ x, T *__restrict__ res, Box bx,
+                                                          const int *gate) {
+  if (gate_off(gate)) return;
+  residual_rb_body<T>(R, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
 // Quartet form of the FP32 in-place phases (nx a multiple of 4): a thread
@@ -736,7 +772,7 @@ __device__ __forceinline__ void relax_quad(const float (&c)[2][8], const float4 
 
 // One quad of an FP32 in-place phase: the four points r0 .. r0+3 of line
 // (j, k) from column i0.
-__device__ __forceinline__ void relax_quad_at(const Recs<float, 8> &R, const float *__restrict__ b, float *x,
+__device__ __forceinline__ void relax_quad_at(const Recs<float, 8> &R, const float *b, float *x,
                                               const Box &bx, int color, int zero_x, long r0, int i0, int j, int k,
                                               float *zout = nullptr) {
   const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
@@ -828,17 +864,22 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_quad_out(Recs<float, 8> R
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_relax_rb_quad(Recs<float, 8> R, const float *__restrict__ b, float *x,
-                                                            Box bx, int color, int zero_x, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void relax_rb_quad_body(const Recs<float, 8> &R, const float *b, float *x, const Box &bx,
+                                                   int color, int zero_x, long t0, long ts) {
   const long n4 = bx.n / 4;
-  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+  for (long q = t0; q < n4; q += ts) {
     const long r0 = 4 * q;
     const unsigned line = fast_div((unsigned)r0, bx.dx);
     const int i0 = (int)((unsigned)r0 - line * (unsigned)bx.nx);
     const unsigned kk = fast_div(line, bx.dy);
     relax_quad_at(R, b, x, bx, color, zero_x, r0, i0, (int)(line - kk * (unsigned)bx.ny), (int)kk);
   }
+}
+__global__ void __launch_bounds__(kThreads) k_relax_rb_quad(Recs<float, 8> R, const float *__restrict__ b, float *x,
+                                                            Box bx, int color, int zero_x, const int *gate) {
+  if (gate_off(gate)) return;
+  relax_rb_quad_body(R, b, x, bx, color, zero_x, (long)blockIdx.x * blockDim.x + threadIdx.x,
+                     (long)gridDim.x * blockDim.x);
 }
 
 // One whole two-colour sweep of a 7-point FP32 level (colour 0, then colour
@@ -998,14 +1039,12 @@ __device__ __forceinline__ void resid_quad(const float (&c)[2][8], const float4 
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_residual_rb_quad(Recs<float, 8> R, const float *__restrict__ b,
-                                                               const float *__restrict__ x, float *__restrict__ res,
-                                                               Box bx, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void residual_rb_quad_body(const Recs<float, 8> &R, const float *b, const float *x,
+                                                      float *res, const Box &bx, long t0, long ts) {
   const long n4 = bx.n / 4;
   const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
   const long sy = nx, sz = (long)nx * ny;
-  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+  for (long q = t0; q < n4; q += ts) {
     const long r0 = 4 * q;
     const unsigned line = fast_div((unsigned)r0, bx.dx);
     const int i0 = (int)((unsigned)r0 - line * (unsigned)nx);
@@ -1028,28 +1067,44 @@ __global__ void __launch_bounds__(kThreads) k_residual_rb_quad(Recs<float, 8> R,
     *reinterpret_cast<float4 *>(res + r0) = make_float4(rr[0], rr[1], rr[2], rr[3]);
   }
 }
+__global__ void __launch_bounds__(kThreads) k_residual_rb_quad(Recs<float, 8> R, const float *__restrict__ b,
+                                                               const float *__restrict__ x, float *__restrict__ res,
+                                                               Box bx, const int *gate) {
+  if (gate_off(gate)) return;
+  residual_rb_quad_body(R, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
 // First phase from a zero guess: colour-0 points take invd b, colour-1 points 0.
 template <class T>
-__global__ void k_relax_rb_zero(Recs<T, 8> R, const T *__restrict__ b, T *x, Box bx, const int *gate) {
-  if (gate_off(gate)) return;
+__device__ __forceinline__ void relax_rb_zero_body(const Recs<T, 8> &R, const T *b, T *x, const Box &bx, long t0,
+                                                   long ts) {
   const long h = bx.n / 2;
-  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < h; m += (long)gridDim.x * blockDim.x) {
+  for (long m = t0; m < h; m += ts) {
     int i, j, k;
     const long r = rb_row(m, 0, bx, i, j, k);
     x[r] = rec_ptr<T, 8>(R, m)[0] * b[r];
     x[r ^ 1] = T(0);
   }
 }
+template <class T>
+__global__ void k_relax_rb_zero(Recs<T, 8> R, const T *__restrict__ b, T *x, Box bx, const int *gate) {
+  if (gate_off(gate)) return;
+  relax_rb_zero_body<T>(R, b, x, bx, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
 
 template <class T, int NS>
-__global__ void k_residual(const T *A, const T *b, const T *x, T *res, Box bx, const int *gate) {
-  if (gate_off(gate)) return;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < bx.n; r += (long)gridDim.x * blockDim.x) {
+__device__ __forceinline__ void residual_body(const T *A, const T *b, const T *x, T *res, const Box &bx, long t0,
+                                              long ts) {
+  for (long r = t0; r < bx.n; r += ts) {
     int i, j, k;
     box_ijk(r, bx, i, j, k);
     res[r] = b[r] - apply_row<T, NS>(A, bx.n, x, (int)r, i, j, k, bx.nx, bx.ny, bx.nz);
   }
+}
+template <class T, int NS>
+__global__ void k_residual(const T *A, const T *b, const T *x, T *res, Box bx, const int *gate) {
+  if (gate_off(gate)) return;
+  residual_body<T, NS>(A, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
 template <class T>
@@ -1286,6 +1341,104 @@ __global__ void k_prolong(const T *xc, Box cb, const T *pm, const T *pp, Box fb,
                   (long)gridDim.x * blockDim.x);
 }
 
+// Transfers of a whole coarsening group: the levels between two relaxed ones
+// (one per coarsened direction) only restrict and interpolate, so a thread
+// takes a point of the group's last level (restriction) or first level
+// (interpolation) and evaluates the stages for it in registers, each with its
+// level's weights, operations and rounding, so results equal the single
+// transfers' bit for bit. The intermediate levels' vectors are neither written
+// nor read, and a group is two launches instead of six.
+template <class T>
+struct GroupStage {
+  Box b;  // the stage's fine level
+  int d = 0;
+  const T *pm = nullptr, *pp = nullptr;
+};
+template <class T>
+struct Group {
+  GroupStage<T> s[3];
+  Box cb;  // the level after the last stage
+  int n = 0;
+};
+
+// The vector after S restrictions at point (i, j, k) of its level (0, with
+// nothing loaded, when `in` is false). Every load is predicated and none waits
+// for a branch, so a thread's 27 values and their weights are in flight
+// together.
+template <class T, int S>
+__device__ __forceinline__ T restricted(const Group<T> &G, const T *r, int i, int j, int k, bool in) {
+  if constexpr (S == 0) {
+    const Box &b = G.s[0].b;
+    return in ? r[((long)k * b.ny + j) * b.nx + i] : T(0);
+  } else {
+    const GroupStage<T> &L = G.s[S - 1];
+    const int nd = L.d == 0 ? L.b.nx : L.d == 1 ? L.b.ny : L.b.nz, c2 = 2 * (L.d == 0 ? i : L.d == 1 ? j : k);
+    T acc = T(0);
+#pragma unroll
+    for (int fo = -1; fo <= 1; ++fo) {
+      const int f = c2 + fo;
+      const bool has = in && f >= 0 && f < nd;
+      const int fi = L.d == 0 ? f : i, fj = L.d == 1 ? f : j, fk = L.d == 2 ? f : k;
+      T w = T(1);
+      if (fo != 0) w = has ? (fo < 0 ? L.pp : L.pm)[((long)fk * L.b.ny + fj) * L.b.nx + fi] : T(0);
+      const T v = restricted<T, S - 1>(G, r, fi, fj, fk, has);
+      acc = has ? fmat<T>(w, v, acc) : acc;
+    }
+    return acc;
+  }
+}
+template <class T, int M>
+__device__ __forceinline__ void restrict_group_body(const Group<T> &G, const T *r, T *bc, long t0, long ts) {
+  for (long I = t0; I < G.cb.n; I += ts) {
+    int i, j, k;
+    box_ijk(I, G.cb, i, j, k);
+    bc[I] = restricted<T, M>(G, r, i, j, k, true);
+  }
+}
+template <class T, int M>
+__global__ void __launch_bounds__(kThreads) k_restrict_group(Group<T> G, const T *__restrict__ r, T *__restrict__ bc,
+                                                             const int *gate) {
+  if (gate_off(gate)) return;
+  restrict_group_body<T, M>(G, r, bc, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+}
+
+// The interpolation of xc at point (i, j, k) of the group's level S (0, with
+// nothing loaded, when `in` is false).
+template <class T, int S, int M>
+__device__ __forceinline__ T prolonged(const Group<T> &G, const T *xc, int i, int j, int k, bool in) {
+  if constexpr (S == M) {
+    return in ? xc[((long)k * G.cb.ny + j) * G.cb.nx + i] : T(0);
+  } else {
+    const GroupStage<T> &L = G.s[S];
+    const int nd = L.d == 0 ? L.b.nx : L.d == 1 ? L.b.ny : L.b.nz, f = L.d == 0 ? i : L.d == 1 ? j : k, c = f >> 1;
+    const bool odd = in && (f & 1), two = odd && c + 1 < (nd + 1) / 2;
+    const T x0 = prolonged<T, S + 1, M>(G, xc, L.d == 0 ? c : i, L.d == 1 ? c : j, L.d == 2 ? c : k, in);
+    const T x1 =
+        prolonged<T, S + 1, M>(G, xc, L.d == 0 ? c + 1 : i, L.d == 1 ? c + 1 : j, L.d == 2 ? c + 1 : k, two);
+    const long r = ((long)k * L.b.ny + j) * L.b.nx + i;
+    const T wp = odd ? L.pp[r] : T(0), wm = odd ? L.pm[r] : T(0);
+    return odd ? fmat<T>(wp, x1, wm * x0) : x0;
+  }
+}
+template <class T, int M>
+__device__ __forceinline__ void prolong_group_body(const Group<T> &G, const T *xc, T *x, int accumulate, long t0,
+                                                   long ts) {
+  const Box &b = G.s[0].b;
+  for (long r = t0; r < b.n; r += ts) {
+    int i, j, k;
+    box_ijk(r, b, i, j, k);
+    const T corr = prolonged<T, 0, M>(G, xc, i, j, k, true);
+    x[r] = accumulate ? x[r] + corr : corr;
+  }
+}
+template <class T, int M>
+__global__ void __launch_bounds__(kThreads) k_prolong_group(Group<T> G, const T *__restrict__ xc, T *x, int accumulate,
+                                                            const int *gate) {
+  if (gate_off(gate)) return;
+  prolong_group_body<T, M>(G, xc, x, accumulate, (long)blockIdx.x * blockDim.x + threadIdx.x,
+                           (long)gridDim.x * blockDim.x);
+}
+
 // Coarsest level: x = Ainv b (one warp per row).
 // Coarsest level: x = A^-1 b, one warp per row. FP64 hierarchies accumulate
 // in FP64; FP32 ones in FP32 per lane (n / 32 products each) and FP64 across
@@ -1429,6 +1582,161 @@ __global__ void __launch_bounds__(kThreads) k_mg_tail(const TailOp *__restrict__
     }
   }
 }
+
+// ---------------------------------------------------------------------------
+// The coarse end of the V-cycle on one thread-block cluster, for solves that
+// the host drives launch by launch. Below a few ten thousand points a phase's
+// work is well under a microsecond and a launch costs the host 5 to 6 us. The
+// blocks of one cluster run the recorded phases in order with the hardware
+// cluster barrier between them, whose release / acquire orders their global
+// stores and loads; the phase list is copied to shared memory once. A phase
+// then takes 2.5 to 3 us (the barrier's flush to L2 and the loads back). A
+// launch inside a captured step takes no longer than that, so captured steps
+// keep one launch per phase. Per point the arithmetic is the stand-alone
+// kernels' (the shared bodies), so results do not depend on which form ran.
+// ---------------------------------------------------------------------------
+enum ClusterKind : int {
+  CK_LOAD = 0, CK_ZERO, CK_JACOBI7, CK_JACOBI27, CK_COLOR7, CK_COLOR27, CK_RB_ZERO, CK_RB, CK_RB27, CK_RESID7,
+  CK_RESID27, CK_RESID_RB, CK_RESID_RB27, CK_RESTRICT, CK_PROLONG, CK_RESTRICT2, CK_PROLONG2, CK_RESTRICT3,
+  CK_PROLONG3, CK_DENSE, CK_STORE,
+  // FP32 only
+  CK_RB_QUAD, CK_RB27_QUAD, CK_RESID_RB_QUAD, CK_RESID_RB27_QUAD, CK_RESTRICT_YZ4, CK_RESTRICT_X4, CK_PROLONG_YZ4,
+  CK_PROLONG_X4
+};
+template <class T>
+struct alignas(16) ClusterOp {
+  int kind = 0, color = 0, zero = 0, d = 0;  // zero: zero guess (relaxation); d: direction (transfers)
+  int accumulate = 0;
+  Box fb, cb;
+  const T *rec = nullptr, *tab = nullptr;  // colour-split records: the records, or the class table
+  const uint16_t *code = nullptr;
+  const T *A = nullptr;    // planes, or the dense inverse
+  const T *wd = nullptr;   // (weighted) inverse diagonal
+  const T *b = nullptr, *src = nullptr, *pm = nullptr, *pp = nullptr;
+  T *dst = nullptr;
+  Group<T> grp;            // transfers of a coarsening group
+};
+constexpr int kClusterThreads = 512;
+constexpr int kClusterOps = 160;  // phases of one launch (their list is in shared memory)
+// Levels of at most this many points run on the cluster; FP64 levels of at most
+// this many stencil entries (an SM has two FP64 lanes, so sixteen of them need
+// 3.4 us for that many). Measured on host-driven solves, one launch per phase
+// against the cluster: default step 32x12x12 3872 -> 2350 us, 48x16x16 with
+// its 12288 points of 7 entries 2834 -> 2566; FP32 multigrid 75x21x18 1885 ->
+// 1435, 160x32x32 2065 -> 1852; FP64 160x32x32 from its level of 2560 points
+// of 27 entries 2865 -> 2904, from 20480 points 3346.
+constexpr long kClusterPoints32 = 50000, kClusterEntries64 = 110000;
+// An FP64 dense level of more points than this keeps its own launch (its n^2
+// products would take one cluster's FP64 units longer than a launch takes).
+constexpr long kClusterDense64 = 256;
+
+// All writes of the cluster's blocks before the barrier are visible to all of
+// its blocks after it. Every block runs the same number of phases.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <class T, int W>
+__device__ __forceinline__ Recs<T, W> op_recs(const ClusterOp<T> &o) {
+  Recs<T, W> r;
+  r.R = o.rec; r.code = o.code; r.tab = o.tab;
+  return r;
+}
+
+// One cluster. ops[0 .. nops): the phases; in / out / winv: the V-cycle's
+// input, output and scaling when the list holds the whole V-cycle (load4: the
+// input is read in FP32, four rows per thread).
+template <class T>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    k_mg_cluster(const ClusterOp<T> *__restrict__ ops, int nops, VecRef in, int load4, OutRef out, const double *winv,
+                 const float *winvf, const int *gate) {
+  if (gate_off(gate)) return;
+  extern __shared__ __align__(16) unsigned char smem_ops[];
+  static_assert(sizeof(ClusterOp<T>) % 16 == 0, "the list is copied 16 bytes at a time");
+  {
+    const uint4 *g = reinterpret_cast<const uint4 *>(ops);
+    uint4 *sm = reinterpret_cast<uint4 *>(smem_ops);
+    for (int e = threadIdx.x; e < nops * (int)(sizeof(ClusterOp<T>) / 16); e += kClusterThreads) sm[e] = __ldg(g + e);
+  }
+  __syncthreads();
+  const ClusterOp<T> *list = reinterpret_cast<const ClusterOp<T> *>(smem_ops);
+  const long t0 = (long)blockIdx.x * kClusterThreads + threadIdx.x, ts = (long)gridDim.x * kClusterThreads;
+  for (int o = 0; o < nops; ++o) {
+    const ClusterOp<T> &op = list[o];
+    bool done = true;
+    switch (op.kind) {
+      case CK_LOAD:
+        if constexpr (sizeof(T) == 4) {
+          if (load4) {
+            load_input_f4_body(op.dst, op.fb.n, in, winvf, t0, ts);
+            break;
+          }
+        }
+        load_input_body<T>(op.dst, op.fb.n, in, winv, t0, ts);
+        break;
+      case CK_ZERO: relax_zero_body<T>(op.wd, op.b, op.dst, op.fb.n, t0, ts); break;
+      case CK_JACOBI7: relax_jacobi_body<T, 7>(op.A, op.wd, op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_JACOBI27: relax_jacobi_body<T, 27>(op.A, op.wd, op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_COLOR7:
+        relax_color_body<T, 7>(op.A, op.wd, op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
+        break;
+      case CK_COLOR27:
+        relax_color_body<T, 27>(op.A, op.wd, op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
+        break;
+      case CK_RB_ZERO: relax_rb_zero_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, t0, ts); break;
+      case CK_RB: relax_rb_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, op.color, t0, ts); break;
+      case CK_RB27:
+        relax_rb27_body<T>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
+        break;
+      case CK_RESID7: residual_body<T, 7>(op.A, op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_RESID27: residual_body<T, 27>(op.A, op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_RESID_RB: residual_rb_body<T>(op_recs<T, 8>(op), op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_RESID_RB27: residual_rb27_body<T>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_RESTRICT: restrict_body<T>(op.src, op.pm, op.pp, op.fb, op.d, op.dst, op.cb, t0, ts); break;
+      case CK_PROLONG:
+        prolong_body<T>(op.src, op.cb, op.pm, op.pp, op.fb, op.d, op.dst, op.accumulate, t0, ts);
+        break;
+      case CK_RESTRICT2: restrict_group_body<T, 2>(op.grp, op.src, op.dst, t0, ts); break;
+      case CK_RESTRICT3: restrict_group_body<T, 3>(op.grp, op.src, op.dst, t0, ts); break;
+      case CK_PROLONG2: prolong_group_body<T, 2>(op.grp, op.src, op.dst, op.accumulate, t0, ts); break;
+      case CK_PROLONG3: prolong_group_body<T, 3>(op.grp, op.src, op.dst, op.accumulate, t0, ts); break;
+      case CK_DENSE: dense_body<T>(op.A, op.src, op.dst, op.fb.n, t0, ts); break;
+      case CK_STORE: store_output_body<T>(op.src, op.fb.n, out, t0, ts); break;
+      default: done = false; break;
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (!done) {
+        switch (op.kind) {
+          case CK_RB_QUAD:
+            relax_rb_quad_body(op_recs<T, 8>(op), op.b, op.dst, op.fb, op.color, op.zero, t0, ts);
+            break;
+          case CK_RB27_QUAD:
+            relax_rb27_quad_body(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
+            break;
+          case CK_RESID_RB_QUAD:
+            residual_rb_quad_body(op_recs<T, 8>(op), op.b, op.src, op.dst, op.fb, t0, ts);
+            break;
+          case CK_RESID_RB27_QUAD:
+            residual_rb27_quad_body(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, t0, ts);
+            break;
+          case CK_RESTRICT_YZ4: restrict_yz4_body(op.src, op.pm, op.pp, op.fb, op.d, op.dst, op.cb, t0, ts); break;
+          case CK_RESTRICT_X4: restrict_x4_body(op.src, op.pm, op.pp, op.fb, op.dst, op.cb, t0, ts); break;
+          case CK_PROLONG_YZ4:
+            prolong_yz4_body(op.src, op.cb, op.pm, op.pp, op.fb, op.d, op.dst, op.accumulate, t0, ts);
+            break;
+          case CK_PROLONG_X4:
+            prolong_x4_body(op.src, op.cb, op.pm, op.pp, op.fb, op.dst, op.accumulate, t0, ts);
+            break;
+          default: break;
+        }
+      }
+    }
+    if (o + 1 < nops) cluster_barrier();
+  }
+}
+
+// Blocks of the dense level's solve: one warp per row.
+int dense_grid(long n) { return std::max(1, (int)std::min<long>((n + 7) / 8, (long)sm_count() * 4)); }
 
 int grid_for(long n) {
   long b = (n + kThreads - 1) / kThreads;
@@ -1668,6 +1976,8 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
 
 static float *record_tail(std::vector<MgLevelT<float>> &L, int l, const MgParams &p, std::vector<TailOp> &ops,
                           double &bytes);
+template <class T>
+static void plan_cluster(cudaStream_t st, std::vector<MgLevelT<T>> &L, const MgParams &p, ClusterPlan &c);
 
 void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const float *A7f, const double h[3],
                       const MgParams &p, bool fp64, bool fp32, const double *winv) {
@@ -1714,6 +2024,12 @@ void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const flo
     IBM_CUDA_TRY(cudaStreamSynchronize(st));
   }
   build_tail(st);
+  clu32_ = ClusterPlan();
+  clu64_ = ClusterPlan();
+  if (prm.fused_coarse <= 0) {  // the fused coarse kernel takes the same levels when it is asked for
+    if (fp32) plan_cluster<float>(st, L32, prm, clu32_);
+    plan_cluster<double>(st, L64, prm, clu64_);
+  }
 }
 
 void Multigrid::build_tail(cudaStream_t st) {
@@ -1742,6 +2058,27 @@ void Multigrid::build_tail(cudaStream_t st) {
   tail_level_ = lt;
   tail_out_ = out;
   tail_bytes_ = bytes;
+}
+
+// The transfers from level l to the next relaxed (or dense) level, at most
+// `most` stages. A stage of its own is a launch of 2.9 us or more whatever its
+// size, a group's launch evaluates shared intermediate points again: above
+// kGroupPoints the single, vectorized stages are faster (steps with groups up
+// to 2M, 700k, 200k points and none: mixed 320x64x64 with 1.3M points on its
+// finest level 5660 / 5407 / 5498 / 5518 us, FP64 adjoint 256x48x48 with 590k
+// 25065 / 25062 / 25621 / 25905 us; FP64 160x32x32 4603 against 4765).
+constexpr long kGroupPoints = 700000;
+template <class T>
+static Group<T> group_of(const std::vector<MgLevelT<T>> &L, int l, int most) {
+  Group<T> G;
+  most = L[(size_t)l].b.n > kGroupPoints ? 1 : std::min(most, 3);
+  do {
+    const MgLevelT<T> &F = L[(size_t)(l + G.n)];
+    GroupStage<T> &S = G.s[G.n++];
+    S.b = F.b; S.d = F.cdir; S.pm = F.pm.p; S.pp = F.pp.p;
+  } while (G.n < most && !L[(size_t)(l + G.n)].relax && L[(size_t)(l + G.n)].cdir >= 0);
+  G.cb = L[(size_t)(l + G.n)].b;
+  return G;
 }
 
 // Runs the V-cycle from level l with zero initial guess; returns (through the
@@ -1827,6 +2164,245 @@ static float *record_tail(std::vector<MgLevelT<float>> &L, int l, const MgParams
   return cur;
 }
 
+// Records the V-cycle from level l as phases of k_mg_cluster, with the
+// operations, order and buffers that vcycle() below would launch. Returns the
+// buffer that holds level l's result.
+template <class T>
+static T *record_cluster(std::vector<MgLevelT<T>> &L, int l, const MgParams &p, std::vector<ClusterOp<T>> &ops) {
+  MgLevelT<T> &F = L[l];
+  constexpr bool f32 = sizeof(T) == 4;
+  auto base = [&](int kind) {
+    ClusterOp<T> op;
+    op.kind = kind;
+    op.fb = F.b;
+    op.b = F.bv.p;
+    return op;
+  };
+  if (F.cdir < 0) {
+    ClusterOp<T> op = base(CK_DENSE);
+    op.A = F.dense.p; op.src = F.bv.p; op.dst = F.x.p;
+    ops.push_back(op);
+    return F.x.p;
+  }
+  const Recs<T, 8> R7 = recs_of<T, 8>(F.rb, F.rbc);
+  const Recs<T, 28> R27 = recs_of<T, 28>(F.rb27, F.rbc);
+  const bool rb7 = R7.R || R7.code, rb27 = R27.R || R27.code;
+  const bool quad = f32 && p.quads && F.b.nx % 4 == 0;
+  auto recs = [&](ClusterOp<T> &op) {
+    if (rb7) { op.rec = R7.R; op.tab = R7.tab; op.code = R7.code; }
+    else { op.rec = R27.R; op.tab = R27.tab; op.code = R27.code; }
+  };
+  T *cur = F.x.p, *oth = F.t.p;
+  auto relax = [&](bool zero) {
+    if (p.relax == 2 && rb7) {
+      for (int color = 0; color < 2; ++color) {
+        const bool z = zero && color == 0;
+        ClusterOp<T> op = base(quad ? CK_RB_QUAD : z ? CK_RB_ZERO : CK_RB);
+        recs(op);
+        op.dst = cur; op.color = color; op.zero = z;
+        ops.push_back(op);
+      }
+    } else if (p.relax == 2) {
+      for (int color = 0; color < 2; ++color) {
+        ClusterOp<T> op = base(rb27 ? (quad ? CK_RB27_QUAD : CK_RB27) : F.ns == 7 ? CK_COLOR7 : CK_COLOR27);
+        if (rb27) recs(op);
+        op.A = F.A; op.wd = F.invd.p; op.src = cur; op.dst = oth; op.color = color; op.zero = zero && color == 0;
+        ops.push_back(op);
+        std::swap(cur, oth);
+      }
+    } else if (zero) {
+      ClusterOp<T> op = base(CK_ZERO);
+      op.wd = F.wd.p; op.dst = cur;
+      ops.push_back(op);
+    } else {
+      ClusterOp<T> op = base(F.ns == 7 ? CK_JACOBI7 : CK_JACOBI27);
+      op.A = F.A; op.wd = F.wd.p; op.src = cur; op.dst = oth;
+      ops.push_back(op);
+      std::swap(cur, oth);
+    }
+  };
+  const int c1 = (l > 0 && p.nu_coarse > 0) ? p.nu_coarse : p.nu1, c2 = (l > 0 && p.nu_coarse > 0) ? p.nu_coarse : p.nu2;
+  const int nu1 = F.relax ? c1 : 0, nu2 = F.relax ? c2 : 0;
+  for (int s = 0; s < nu1; ++s) relax(s == 0);
+  const T *res = F.bv.p;
+  if (nu1 > 0) {
+    const bool rb = p.relax == 2;
+    ClusterOp<T> op = base(rb && rb7    ? (quad ? CK_RESID_RB_QUAD : CK_RESID_RB)
+                           : rb && rb27 ? (quad ? CK_RESID_RB27_QUAD : CK_RESID_RB27)
+                           : F.ns == 7  ? CK_RESID7
+                                        : CK_RESID27);
+    if (rb && (rb7 || rb27)) recs(op);
+    op.A = F.A; op.src = cur; op.dst = F.r.p;
+    ops.push_back(op);
+    res = F.r.p;
+  }
+  const Group<T> G = group_of<T>(L, l, 3);
+  MgLevelT<T> &C = L[l + G.n];
+  const bool yz4 = f32 && F.cdir != 0 && F.b.nx % 4 == 0;
+  const bool x4 = f32 && !yz4 && p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0;
+  {
+    ClusterOp<T> op = base(G.n == 3   ? CK_RESTRICT3
+                           : G.n == 2 ? CK_RESTRICT2
+                           : yz4      ? CK_RESTRICT_YZ4
+                           : x4       ? CK_RESTRICT_X4
+                                      : CK_RESTRICT);
+    op.cb = C.b; op.d = F.cdir; op.src = res; op.pm = F.pm.p; op.pp = F.pp.p; op.dst = C.bv.p; op.grp = G;
+    ops.push_back(op);
+  }
+  T *xc = record_cluster<T>(L, l + G.n, p, ops);
+  {
+    ClusterOp<T> op = base(G.n == 3   ? CK_PROLONG3
+                           : G.n == 2 ? CK_PROLONG2
+                           : yz4      ? CK_PROLONG_YZ4
+                           : x4       ? CK_PROLONG_X4
+                                      : CK_PROLONG);
+    op.cb = C.b; op.d = F.cdir; op.src = xc; op.pm = F.pm.p; op.pp = F.pp.p; op.dst = cur; op.accumulate = nu1 > 0;
+    op.grp = G;
+    ops.push_back(op);
+  }
+  for (int s = 0; s < nu2; ++s) relax(false);
+  return cur;
+}
+
+// Launches phases [first, first + count) of a recorded list on one cluster.
+template <class T>
+static void launch_cluster(cudaStream_t st, const ClusterOp<T> *ops, int count, int blocks, double bytes,
+                           const Box *fine, const VecRef &in, const OutRef &out, const double *winv, const float *winvf,
+                           const int *gate) {
+  LaunchScope ls(K_MG_CLUSTER, st, bytes);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = sizeof(ClusterOp<T>) * (size_t)count;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const int n = fine ? fine->n : 0;
+  const int load4 = sizeof(T) == 4 && in.basef && n % 4 == 0 && in.ld % 4 == 0;
+  IBM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_mg_cluster<T>, ops, count, in, load4, out, winv, winvf, gate));
+}
+
+// Blocks of the cluster: 16 where the device can place such a cluster, else
+// the portable 8, else 0 (one launch per phase). Asked once per device: the
+// occupancy query takes milliseconds.
+template <class T>
+static int cluster_blocks() {
+  static std::mutex mu;
+  static std::unordered_map<int, int> known;
+  int dev = 0;
+  IBM_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  int &found = known[dev];
+  found = 0;
+  if (cudaFuncSetAttribute(k_mg_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(k_mg_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(ClusterOp<T>) * kClusterOps) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  for (int blocks : {16, 8}) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = sizeof(ClusterOp<T>) * (size_t)kClusterOps;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_mg_cluster<T>, &cfg) == cudaSuccess && n > 0) {
+      found = blocks;
+      break;
+    }
+    cudaGetLastError();
+  }
+  return found;
+}
+
+// Algorithmic bytes of the recorded phases (each operand of a phase once).
+template <class T>
+static double cluster_bytes(const std::vector<ClusterOp<T>> &ops) {
+  double b = 0.0;
+  for (const auto &o : ops) {
+    const double n = o.fb.n, t = sizeof(T);
+    if (o.kind == CK_DENSE) b += t * (n * n + 2.0 * n);
+    else if (o.cb.n > 0) b += t * ((o.accumulate ? 4.0 : 3.0) * n + o.cb.n);
+    else b += t * n * 3.0 + (o.code ? 1.0 * n : o.A ? t * n * 7.0 : 0.0);
+  }
+  return b;
+}
+
+// Plans the cluster's part of a hierarchy: from the first relaxed level that is
+// small enough. A larger FP64 dense level gets its own launch between two
+// parts.
+template <class T>
+static void plan_cluster(cudaStream_t st, std::vector<MgLevelT<T>> &L, const MgParams &p, ClusterPlan &c) {
+  c = ClusterPlan();
+  if (L.size() < 2 || L[0].cdir < 0) return;
+  int lt = 0;
+  auto fits = [](const MgLevelT<T> &F) {
+    return sizeof(T) == 4 ? F.b.n <= kClusterPoints32 : (long)F.b.n * F.ns <= kClusterEntries64;
+  };
+  while (lt < (int)L.size() && (!fits(L[lt]) || !L[lt].relax)) ++lt;
+  if (lt + 1 >= (int)L.size()) return;  // nothing but the dense level
+  std::vector<ClusterOp<T>> ops;
+  if (lt == 0) {
+    ClusterOp<T> op;
+    op.kind = CK_LOAD;
+    op.fb = L[0].b; op.dst = L[0].bv.p;
+    ops.push_back(op);
+  }
+  T *out = record_cluster<T>(L, lt, p, ops);
+  if (lt == 0) {
+    ClusterOp<T> op;
+    op.kind = CK_STORE;
+    op.fb = L[0].b; op.src = out;
+    ops.push_back(op);
+  }
+  int down = (int)ops.size();
+  if (sizeof(T) == 8 && L.back().b.n > kClusterDense64)
+    for (int o = 0; o < (int)ops.size(); ++o)
+      if (ops[(size_t)o].kind == CK_DENSE) down = o;
+  const int up = (int)ops.size() - down - 1;  // phases after the dense level, when it stands alone
+  if (down > kClusterOps || up > kClusterOps) return;
+  c.blocks = cluster_blocks<T>();
+  if (c.blocks == 0) return;
+  c.ops.alloc(sizeof(ClusterOp<T>) * ops.size());
+  IBM_CUDA_TRY(cudaMemcpyAsync(c.ops.p, ops.data(), c.ops.n, cudaMemcpyHostToDevice, st));
+  IBM_CUDA_TRY(cudaStreamSynchronize(st));
+  c.level = lt;
+  c.down = down;
+  c.up = std::max(0, up);
+  c.out = out;
+  c.bytes = cluster_bytes<T>(ops);
+}
+
+// Runs the planned part; returns the buffer with its first level's result.
+template <class T>
+static T *run_cluster(cudaStream_t st, std::vector<MgLevelT<T>> &L, const ClusterPlan &c, const VecRef &in,
+                      const OutRef &out, const double *winv, const float *winvf, const int *gate) {
+  const ClusterOp<T> *ops = reinterpret_cast<const ClusterOp<T> *>(c.ops.p);
+  launch_cluster<T>(st, ops, c.down, c.blocks, c.bytes, &L[0].b, in, out, winv, winvf, gate);
+  if (c.up > 0) {
+    MgLevelT<T> &D = L.back();
+    const long n = D.b.n;
+    {
+      LaunchScope ls(K_MG_DENSE, st, sizeof(T) * ((double)n * n + 2.0 * n));
+      k_dense<T><<<dense_grid(n), kThreads, 0, st>>>(D.dense.p, D.bv.p, D.x.p, (int)n, gate);
+    }
+    launch_cluster<T>(st, ops + c.down + 1, c.up, c.blocks, 0.0, &L[0].b, in, out, winv, winvf, gate);
+  }
+  return (T *)c.out;
+}
+
 // One cooperative launch of the fused coarse levels (a memset clears the
 // barrier state first); returns the buffer holding the first fused level's
 // correction.
@@ -1850,18 +2426,18 @@ template <class T>
 // fin / fout (finest level only, may be null): the V-cycle's input load and
 // output store, fused into the first and the last relaxation phases.
 // tail (FP32 hierarchies, may be null): the levels from tail->level on run as
-// the fused coarse kernel instead of one launch per phase.
+// the fused coarse kernel instead of one launch per phase; clu likewise for
+// the levels on one cluster.
 static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgParams &p, const int *gate,
                  const VecRef *fin = nullptr, const OutRef *fout = nullptr, const float *winvf = nullptr,
-                 const TailLaunch *tail = nullptr) {
+                 const TailLaunch *tail = nullptr, const ClusterPlan *clu = nullptr) {
   MgLevelT<T> &F = L[l];
   const long n = F.b.n;
   const double T_ = sizeof(T);
   const int g = grid_for(n);
   if (F.cdir < 0) {
     LaunchScope ls(K_MG_DENSE, st, T_ * ((double)n * n + 2.0 * n));
-    k_dense<T><<<std::max(1, (int)std::min<long>((n + 7) / 8, (long)sm_count() * 4)), kThreads, 0, st>>>(
-        F.dense.p, F.bv.p, F.x.p, (int)n, gate);
+    k_dense<T><<<dense_grid(n), kThreads, 0, st>>>(F.dense.p, F.bv.p, F.x.p, (int)n, gate);
     return F.x.p;
   }
   T *cur = F.x.p, *oth = F.t.p;
@@ -1982,10 +2558,20 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
     else k_residual<T, 27><<<grid_all(n), kThreads, 0, st>>>(F.A, F.bv.p, cur, F.r.p, F.b, gate);
     res = F.r.p;
   }
-  MgLevelT<T> &C = L[l + 1];
+  // the stages of this level's coarsening group, up to where a fused part begins
+  int most = 3;
+  if (tail && l < tail->level) most = tail->level - l;
+  if (clu && clu->blocks && l < clu->level) most = clu->level - l;
+  const Group<T> G = group_of<T>(L, l, most);
+  MgLevelT<T> &C = L[l + G.n];
   {
-    LaunchScope ls(K_MG_RESTRICT, st, T_ * (3.0 * n + C.b.n));
-    if constexpr (sizeof(T) == 4) {
+    // a group reads the level once and writes the group's last level (the weights of the levels between: n)
+    LaunchScope ls(K_MG_RESTRICT, st, T_ * ((G.n > 1 ? 2.0 : 3.0) * n + C.b.n));
+    if (G.n == 3)
+      k_restrict_group<T, 3><<<resident_grid(k_restrict_group<T, 3>, C.b.n), kThreads, 0, st>>>(G, res, C.bv.p, gate);
+    else if (G.n == 2)
+      k_restrict_group<T, 2><<<resident_grid(k_restrict_group<T, 2>, C.b.n), kThreads, 0, st>>>(G, res, C.bv.p, gate);
+    else if constexpr (sizeof(T) == 4) {
       if (F.cdir != 0 && F.b.nx % 4 == 0)
         k_restrict_yz4<<<resident_grid(k_restrict_yz4, C.b.n / 4), kThreads, 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
       else if (p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0)
@@ -1998,12 +2584,18 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   }
   T *xc = nullptr;
   if constexpr (sizeof(T) == 4) {
-    if (tail && l + 1 == tail->level) xc = launch_tail(st, *tail, gate);
+    if (tail && l + G.n == tail->level) xc = launch_tail(st, *tail, gate);
   }
-  if (!xc) xc = vcycle<T>(st, L, l + 1, p, gate, nullptr, nullptr, nullptr, tail);
+  if (!xc && clu && clu->blocks && l + G.n == clu->level)
+    xc = run_cluster<T>(st, L, *clu, VecRef(), OutRef(), nullptr, nullptr, gate);
+  if (!xc) xc = vcycle<T>(st, L, l + G.n, p, gate, nullptr, nullptr, nullptr, tail, clu);
   {
     LaunchScope ls(K_MG_PROLONG, st, T_ * ((nu1 > 0 ? 4.0 : 3.0) * n + C.b.n));
-    if constexpr (sizeof(T) == 4) {
+    if (G.n == 3)
+      k_prolong_group<T, 3><<<resident_grid(k_prolong_group<T, 3>, n), kThreads, 0, st>>>(G, xc, cur, nu1 > 0, gate);
+    else if (G.n == 2)
+      k_prolong_group<T, 2><<<resident_grid(k_prolong_group<T, 2>, n), kThreads, 0, st>>>(G, xc, cur, nu1 > 0, gate);
+    else if constexpr (sizeof(T) == 4) {
       if (F.cdir != 0 && F.b.nx % 4 == 0)
         k_prolong_yz4<<<resident_grid(k_prolong_yz4, n / 4), kThreads, 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
       else if (p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0)
@@ -2021,6 +2613,11 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
 void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, const int *gate, bool use_fp32) {
   if (prm.cycles != 1) throw Error(IBM_ERR_UNSUPPORTED, "multigrid: only one V-cycle per application");
   const double ob = out.d ? 8.0 : 4.0;
+  // captured solves keep a launch per phase (see k_mg_cluster)
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  IBM_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
+  const bool cluster = capturing == cudaStreamCaptureStatusNone;
+  const ClusterPlan *c32 = cluster ? &clu32_ : nullptr, *c64 = cluster ? &clu64_ : nullptr;
   if (use_fp32) {
     if (L32.empty()) throw Error(IBM_ERR_STATE, "multigrid: FP32 hierarchy not built");
     MgLevelT<float> &F = L32[0];
@@ -2037,8 +2634,12 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
       tl.out = tail_out_; tl.bytes = tail_bytes_;
     }
     const TailLaunch *tp = tail_nops_ > 0 ? &tl : nullptr;
+    if (cluster && clu32_.blocks && clu32_.level == 0) {
+      run_cluster<float>(st, L32, clu32_, in, out, winv_, winvf_.p, gate);
+      return;
+    }
     if (fuse) {
-      vcycle<float>(st, L32, 0, prm, gate, &in, &out, winvf_.p, tp);
+      vcycle<float>(st, L32, 0, prm, gate, &in, &out, winvf_.p, tp, c32);
       return;
     }
     {
@@ -2050,16 +2651,20 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
         k_load_input<float><<<grid_for(F.b.n), kThreads, 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
       }
     }
-    float *x = vcycle<float>(st, L32, 0, prm, gate, nullptr, nullptr, nullptr, tp);
+    float *x = vcycle<float>(st, L32, 0, prm, gate, nullptr, nullptr, nullptr, tp, c32);
     LaunchScope ls(K_MG_STORE, st, (4.0 + ob) * F.b.n);
     k_store_output<float><<<grid_for(F.b.n), kThreads, 0, st>>>(x, F.b.n, out, gate);
   } else {
     MgLevelT<double> &F = L64[0];
+    if (cluster && clu64_.blocks && clu64_.level == 0) {
+      run_cluster<double>(st, L64, clu64_, in, out, winv_, nullptr, gate);
+      return;
+    }
     {
       LaunchScope ls(K_MG_LOAD, st, (winv_ ? 24.0 : 16.0) * F.b.n);
       k_load_input<double><<<grid_for(F.b.n), kThreads, 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
     }
-    double *x = vcycle<double>(st, L64, 0, prm, gate);
+    double *x = vcycle<double>(st, L64, 0, prm, gate, nullptr, nullptr, nullptr, nullptr, c64);
     LaunchScope ls(K_MG_STORE, st, (8.0 + ob) * F.b.n);
     k_store_output<double><<<grid_for(F.b.n), kThreads, 0, st>>>(x, F.b.n, out, gate);
   }

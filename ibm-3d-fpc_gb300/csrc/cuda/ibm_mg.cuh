@@ -36,6 +36,16 @@ struct MgLevelT {
   Classes<T> rbc;       // the classes of rb or rb27 (W 8 or 28); the plain records are then released
 };
 
+// The part of a hierarchy that runs on one thread-block cluster (ibm_mg.cu):
+// the phases from level `level` on as a device list, cut at the dense level
+// when that has a launch of its own. blocks == 0: none.
+struct ClusterPlan {
+  DBuf<unsigned char> ops;
+  int level = 0, down = 0, up = 0, blocks = 0;
+  void *out = nullptr;   // the buffer that holds level `level`'s result
+  double bytes = 0.0;    // algorithmic bytes of all phases
+};
+
 class Multigrid {
  public:
   // Builds the hierarchy from a 7-point operator (FP64 planes, and FP32 planes
@@ -69,6 +79,7 @@ class Multigrid {
   int tail_nops_ = 0, tail_blocks_ = 0, tail_level_ = 0;
   float *tail_out_ = nullptr;
   double tail_bytes_ = 0.0;
+  ClusterPlan clu32_, clu64_;
   const double *winv_ = nullptr;
   DBuf<float> winvf_;   // FP32 copy of winv_ for the FP32 hierarchy
 };
