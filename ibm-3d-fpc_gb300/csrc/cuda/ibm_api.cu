@@ -221,7 +221,7 @@ const Box &field_box(const ibm_ctx *c, int f) {
 
 void mg_apply_cb(void *ctx, cudaStream_t st, int, const VecRef &in, const OutRef &out, const int *gate) {
   ibm_ctx *c = (ibm_ctx *)ctx;
-  c->mg.apply(st, in, out, gate, out.f != nullptr);
+  c->mg.apply(st, in, out, gate, out.f != nullptr, true);
 }
 
 void require_inputs(ibm_ctx *c) {

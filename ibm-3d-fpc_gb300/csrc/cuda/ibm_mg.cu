@@ -1585,7 +1585,9 @@ __global__ void __launch_bounds__(kThreads) k_mg_tail(const TailOp *__restrict__
 
 // ---------------------------------------------------------------------------
 // The coarse end of the V-cycle on one thread-block cluster, for solves that
-// the host drives launch by launch. Below a few ten thousand points a phase's
+// the host drives launch by launch (a single application,
+// ibm_apply_preconditioner, keeps a launch per phase, each in its class of the
+// profile). Below a few ten thousand points a phase's
 // work is well under a microsecond and a launch costs the host 5 to 6 us. The
 // blocks of one cluster run the recorded phases in order with the hardware
 // cluster barrier between them, whose release / acquire orders their global
@@ -2610,13 +2612,14 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   return cur;
 }
 
-void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, const int *gate, bool use_fp32) {
+void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, const int *gate, bool use_fp32,
+                      bool fused) {
   if (prm.cycles != 1) throw Error(IBM_ERR_UNSUPPORTED, "multigrid: only one V-cycle per application");
   const double ob = out.d ? 8.0 : 4.0;
   // captured solves keep a launch per phase (see k_mg_cluster)
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   IBM_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
-  const bool cluster = capturing == cudaStreamCaptureStatusNone;
+  const bool cluster = fused && capturing == cudaStreamCaptureStatusNone;
   const ClusterPlan *c32 = cluster ? &clu32_ : nullptr, *c64 = cluster ? &clu64_ : nullptr;
   if (use_fp32) {
     if (L32.empty()) throw Error(IBM_ERR_STATE, "multigrid: FP32 hierarchy not built");

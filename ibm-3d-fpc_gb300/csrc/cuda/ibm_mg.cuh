@@ -54,8 +54,9 @@ class Multigrid {
   // every application scales its input by winv.
   void setup(cudaStream_t st, const Box &b, const double *A7, const float *A7f, const double h[3],
              const MgParams &p, bool fp64, bool fp32, const double *winv);
-  // out = M in (every kernel gated on *gate when gate != nullptr).
-  void apply(cudaStream_t st, const VecRef &in, const OutRef &out, const int *gate, bool use_fp32);
+  // out = M in (every kernel gated on *gate when gate != nullptr). fused: small
+  // levels may run on one cluster (see k_mg_cluster) when st is not capturing.
+  void apply(cudaStream_t st, const VecRef &in, const OutRef &out, const int *gate, bool use_fp32, bool fused = false);
   int levels() const { return (int)L64.size() ? (int)L64.size() : (int)L32.size(); }
   void level_info(int l, int dims[3], int *cdir, int *ns) const;
   // Copies level l's coefficients as [n][27] (FP64 hierarchy).
