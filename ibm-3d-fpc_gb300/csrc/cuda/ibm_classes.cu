@@ -13,6 +13,7 @@
 // the host in first-seen order, the table gathered on the device, and every
 // record compared bit for bit with its class's record (a hash collision makes
 // the build fail, and the caller keeps the plain records).
+#include <algorithm>
 #include <unordered_map>
 
 #include "ibm_common.cuh"
@@ -62,6 +63,25 @@ __global__ void k_verify_classes(const unsigned *__restrict__ words, int wpr, lo
   }
 }
 
+// runs[w] = 1 when the four points of every quad 32 w .. 32 w + 31 have codes
+// `major`. One warp per run, one quad per lane.
+__global__ void k_mark_runs(const uint16_t *__restrict__ code, Box b, QuadMap Q, int major, uint8_t *__restrict__ runs,
+                            long nruns) {
+  const long w0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, ws = ((long)gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const long h = b.n / 2;
+  for (long w = w0; w < nruns; w += ws) {
+    const long q = 32 * w + lane;
+    bool same = true;
+    if (q < b.n / 4) {
+      const long m = quad_of(q, Q, b).r0 / 2;
+      same = code[m] == major && code[m + 1] == major && code[h + m] == major && code[h + m + 1] == major;
+    }
+    same = __all_sync(0xffffffffu, same);
+    if (lane == 0) runs[w] = same ? 1 : 0;
+  }
+}
+
 int grid_of(long n) { return (int)std::max<long>(1, std::min<long>((n + kThreads - 1) / kThreads, 65535L * 8)); }
 
 }  // namespace
@@ -71,6 +91,7 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
   static_assert(sizeof(T) % 4 == 0, "records are whole 32-bit words");
   out.code.release();
   out.tab.release();
+  out.runs.release();
   out.K = 0;
   out.W = W;
   if (nrec <= 0 || W <= 0) return false;
@@ -140,9 +161,26 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
     return false;
   }
   out.K = K;
+  std::vector<long> count((size_t)K, 0);
+  for (long t = 0; t < nrec; ++t) ++count[code[(size_t)t]];
+  out.major = (int)(std::max_element(count.begin(), count.end()) - count.begin());
+  out.major_rec.resize((size_t)W);
+  IBM_CUDA_TRY(cudaMemcpyAsync(out.major_rec.data(), out.tab.p + (size_t)out.major * W, sizeof(T) * W,
+                               cudaMemcpyDeviceToHost, st));
+  IBM_CUDA_TRY(cudaStreamSynchronize(st));
   return true;
 }
 
+template <class T>
+void mark_runs(cudaStream_t st, Classes<T> &c, const Box &b) {
+  const long nruns = (b.n / 4 + 31) / 32;
+  c.runs.alloc((size_t)nruns);
+  LaunchScope ls(K_SETUP, st, 0.0);
+  k_mark_runs<<<grid_of(32 * nruns), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b), c.major, c.runs.p, nruns);
+}
+
+template void mark_runs<float>(cudaStream_t, Classes<float> &, const Box &);
+template void mark_runs<double>(cudaStream_t, Classes<double> &, const Box &);
 template bool build_classes<float>(cudaStream_t, const float *, int, long, Classes<float> &);
 template bool build_classes<double>(cudaStream_t, const double *, int, long, Classes<double> &);
 

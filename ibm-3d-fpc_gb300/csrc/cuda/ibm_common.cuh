@@ -89,9 +89,17 @@ struct Classes {
   DBuf<uint16_t> code;  // class of each record
   DBuf<T> tab;          // [K][W] distinct records, first-seen order
   int K = 0, W = 0;
+  int major = 0;             // the class of most records
+  std::vector<T> major_rec;  // its record
+  DBuf<uint8_t> runs;        // per 32 quads of a level: all their records are of the major class (mark_runs)
   bool ok() const { return code.p != nullptr; }
-  size_t bytes() const { return code.bytes() + tab.bytes(); }
+  size_t bytes() const { return code.bytes() + tab.bytes() + runs.bytes(); }
 };
+struct Box;
+// Fills c.runs for colour-split codes ([colour][n / 2]) of a level of box b
+// (b.nx % 4 == 0), quads in the order of QuadMap.
+template <class T>
+void mark_runs(cudaStream_t st, Classes<T> &c, const Box &b);
 // Fills c for the records rec[t * W .. t * W + W) (device memory, t < nrec).
 // Returns false and leaves c empty when there are more than kMaxClasses
 // distinct records. Synchronises the stream.
@@ -124,6 +132,52 @@ inline Box make_box(int nx, int ny, int nz) {
   b.dx = make_fastdiv((unsigned)(nx > 0 ? nx : 1));
   b.dy = make_fastdiv((unsigned)(ny > 0 ? ny : 1));
   return b;
+}
+
+// Quads of a box with nx % 4 == 0 (four consecutive points of a line), in the
+// order the quartet kernels take them: first the quads inside the lines, then
+// the two at each line's ends. The points at the ends (inlet and outlet) carry
+// other records than those inside; taken line by line they would put one into
+// two of five runs of 32 quads at nx = 640, and into most at half of that.
+struct QuadMap {
+  int w = 0;      // quads inside a line
+  long nint = 0;  // ... of all lines
+  FastDiv dw;
+};
+inline QuadMap make_quad_map(const Box &b) {
+  QuadMap m;
+  m.w = b.nx / 4 > 2 ? b.nx / 4 - 2 : 0;
+  m.nint = (long)m.w * b.ny * b.nz;
+  m.dw = make_fastdiv((unsigned)(m.w > 0 ? m.w : 1));
+  return m;
+}
+// Quad q: the points r0 .. r0 + 3 of line (j, k) from column i0.
+struct Quad {
+  long r0;
+  int i0, j, k;
+};
+__device__ __forceinline__ unsigned fast_div(unsigned n, FastDiv f);
+__device__ __forceinline__ Quad quad_of(long q, const QuadMap &m, const Box &b) {
+  Quad g;
+  unsigned line;
+  if (q < m.nint) {
+    line = fast_div((unsigned)q, m.dw);
+    g.i0 = 4 * (int)((unsigned)q - line * (unsigned)m.w + 1u);
+  } else {
+    const unsigned e = (unsigned)(q - m.nint);
+    if (b.nx > 4) {
+      line = e >> 1;
+      g.i0 = (e & 1) ? b.nx - 4 : 0;
+    } else {  // one quad a line
+      line = e;
+      g.i0 = 0;
+    }
+  }
+  const unsigned kk = fast_div(line, b.dy);
+  g.j = (int)(line - kk * (unsigned)b.ny);
+  g.k = (int)kk;
+  g.r0 = (long)line * b.nx + g.i0;
+  return g;
 }
 
 // 7-point operator on a solve box: coefficient planes [7][n] (C,-x,+x,-y,+y,-z,+z).

@@ -770,57 +770,112 @@ __device__ __forceinline__ void relax_quad(const float (&c)[2][8], const float4 
   }
 }
 
-// One quad of an FP32 in-place phase: the four points r0 .. r0+3 of line
-// (j, k) from column i0.
-__device__ __forceinline__ void relax_quad_at(const Recs<float, 8> &R, const float *b, float *x,
-                                              const Box &bx, int color, int zero_x, long r0, int i0, int j, int k,
-                                              float *zout = nullptr) {
+// Runs of one record: 93 to 96 % of a fine level's points carry the same
+// record (every fluid cell away from walls and the body). Where 32 quads (a
+// warp's) are of that record only, its values come from the kernel's
+// parameters, FFMA operands in constant memory: no class and no table load,
+// which were 5 of a quad's 13 loads and a dependent chain of two. With the x
+// neighbours from the lanes beside and one 16-byte store a phase at
+// 640x128x128 takes 24.3 us (27.7 before), at 29 us of HBM time for what a
+// whole sweep must move. runs null: every quad reads its records.
+struct Uni8 {
+  float c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const uint8_t *runs = nullptr;
+};
+
+// Where a quad's x neighbours come from: the lanes beside, whose quads are the
+// ones before and after it in the line, or memory at the ends of a warp and of
+// a line's inner quads.
+struct QuadEdge {
+  bool load_l, load_r, has_l, has_r;
+};
+__device__ __forceinline__ QuadEdge quad_edge(const Quad &g, int nx) {
+  const int lane = threadIdx.x & 31;
+  QuadEdge e;
+  e.has_l = g.i0 > 0;
+  e.has_r = g.i0 + 4 < nx;
+  const bool end = !e.has_l || !e.has_r;
+  e.load_l = e.has_l && (end || lane == 0 || g.i0 == 4);
+  e.load_r = e.has_r && (end || lane == 31 || g.i0 + 8 == nx);
+  return e;
+}
+// x left and right of the quad whose values are v; called by whole warps.
+__device__ __forceinline__ void quad_sides(const float *xq, const float4 &v, const QuadEdge &e, float &l, float &r) {
+  float el = 0.0f, er = 0.0f;
+  if (e.load_l) el = xq[-1];
+  if (e.load_r) er = xq[4];
+  l = __shfl_up_sync(0xffffffffu, v.w, 1);
+  r = __shfl_down_sync(0xffffffffu, v.x, 1);
+  if (e.load_l || !e.has_l) l = el;
+  if (e.load_r || !e.has_r) r = er;
+}
+
+// x on the quad and its neighbours, 0 outside the box. Called by whole warps.
+struct QuadX {
+  float4 c, s, n, b, t;
+  float l, r;
+};
+__device__ __forceinline__ QuadX load_quad_x(const float *x, const Quad &g, const Box &bx) {
   const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
   const long sy = nx, sz = (long)nx * ny;
-  const int p = (j + k + color) & 1;
-  const long m0 = (long)color * (bx.n / 2) + r0 / 2;
-  float c[2][8];
-  load_quad_recs(R, m0, c);
-  const float4 bq = *reinterpret_cast<const float4 *>(b + r0);
-  if (zero_x) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p == 0) { v.x = c[0][0] * bq.x; v.z = c[1][0] * bq.z; }
-    else { v.y = c[0][0] * bq.y; v.w = c[1][0] * bq.w; }
-    *reinterpret_cast<float4 *>(x + r0) = v;
-    return;
-  }
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 xc = *reinterpret_cast<const float4 *>(x + r0);
-  const float4 xs = j > 0 ? *reinterpret_cast<const float4 *>(x + r0 - sy) : z4;
-  const float4 xn = j < ny - 1 ? *reinterpret_cast<const float4 *>(x + r0 + sy) : z4;
-  const float4 xb = k > 0 ? *reinterpret_cast<const float4 *>(x + r0 - sz) : z4;
-  const float4 xt = k < nz - 1 ? *reinterpret_cast<const float4 *>(x + r0 + sz) : z4;
-  const float xl = i0 > 0 ? x[r0 - 1] : 0.0f;
-  const float xr = i0 + 4 < nx ? x[r0 + 4] : 0.0f;
-  float out[2];
-  float4 q = xc;  // the quad after the phase
-  if (p == 0) {
-    relax_quad<0>(c, bq, xc, xs, xn, xb, xt, xl, xr, out);
-    x[r0] = out[0];
-    x[r0 + 2] = out[1];
-    q.x = out[0];
-    q.z = out[1];
-  } else {
-    relax_quad<1>(c, bq, xc, xs, xn, xb, xt, xl, xr, out);
-    x[r0 + 1] = out[0];
-    x[r0 + 3] = out[1];
-    q.y = out[0];
-    q.w = out[1];
-  }
-  if (zout) *reinterpret_cast<float4 *>(zout + r0) = q;
+  QuadX v;
+  v.c = *reinterpret_cast<const float4 *>(x + g.r0);
+  v.s = g.j > 0 ? *reinterpret_cast<const float4 *>(x + g.r0 - sy) : z4;
+  v.n = g.j < ny - 1 ? *reinterpret_cast<const float4 *>(x + g.r0 + sy) : z4;
+  v.b = g.k > 0 ? *reinterpret_cast<const float4 *>(x + g.r0 - sz) : z4;
+  v.t = g.k < nz - 1 ? *reinterpret_cast<const float4 *>(x + g.r0 + sz) : z4;
+  quad_sides(x + g.r0, v.c, quad_edge(g, nx), v.l, v.r);
+  return v;
 }
+
+// The quad after a phase: its colour's two points relaxed, the others as read.
+template <int P>
+__device__ __forceinline__ float4 relax_quad_uni(const Uni8 &U, const float4 &bq, const QuadX &v) {
+  const float c[2][8] = {{U.c[0], U.c[1], U.c[2], U.c[3], U.c[4], U.c[5], U.c[6], U.c[7]},
+                         {U.c[0], U.c[1], U.c[2], U.c[3], U.c[4], U.c[5], U.c[6], U.c[7]}};
+  float out[2];
+  relax_quad<P>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, out);
+  return P == 0 ? make_float4(out[0], v.c.y, out[1], v.c.w) : make_float4(v.c.x, out[0], v.c.z, out[1]);
+}
+__device__ __forceinline__ float4 relax_quad_new(const Recs<float, 8> &R, const Uni8 &U, const float4 &bq,
+                                                 const QuadX &v, int p, long m0, bool uni) {
+  if (uni) return p == 0 ? relax_quad_uni<0>(U, bq, v) : relax_quad_uni<1>(U, bq, v);
+  float c[2][8], out[2];
+  load_quad_recs(R, m0, c);
+  if (p == 0) {
+    relax_quad<0>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, out);
+    return make_float4(out[0], v.c.y, out[1], v.c.w);
+  }
+  relax_quad<1>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, out);
+  return make_float4(v.c.x, out[0], v.c.z, out[1]);
+}
+// The colour's inverse diagonals times b, 0 at the other points.
+__device__ __forceinline__ float4 zero_quad(const Recs<float, 8> &R, const Uni8 &U, const float4 &bq, int p, long m0,
+                                            bool uni) {
+  float d0 = U.c[0], d1 = U.c[0];
+  if (!uni) {
+    float c[2][8];
+    load_quad_recs(R, m0, c);
+    d0 = c[0][0];
+    d1 = c[1][0];
+  }
+  return p == 0 ? make_float4(d0 * bq.x, 0.f, d1 * bq.z, 0.f) : make_float4(0.f, d0 * bq.y, 0.f, d1 * bq.w);
+}
+
+// Grid-stride loop over quads by whole warps: lanes past the end take the
+// last quad and store nothing. (t0: the thread's first quad.)
+#define IBM_QUAD_LOOP(q, live, n4, t0, ts)                                                                   \
+  for (long qb__ = (t0) - (threadIdx.x & 31); qb__ < (n4); qb__ += (ts))                                       \
+    if (const bool live = qb__ + (threadIdx.x & 31) < (n4); true)                                              \
+      if (const long q = live ? qb__ + (threadIdx.x & 31) : (n4) - 1; true)
 
 // The finest level's first phase from a zero guess with the V-cycle's input
 // load fused in (k_load_input_f4's b = winv * in / nu, then k_relax_rb_quad's
 // zero phase), and its last phase with the output store fused in (the whole
 // quad also written to the preconditioned direction). Same values as the
 // separate kernels.
-__global__ void __launch_bounds__(kThreads) k_relax_rb_quad_in(Recs<float, 8> R, float *bv, float *x, Box bx,
+__global__ void __launch_bounds__(kThreads) k_relax_rb_quad_in(Recs<float, 8> R, Uni8 U, QuadMap Q, float *bv, float *x, Box bx,
                                                                VecRef in, const float *winvf, const int *gate) {
   if (gate_off(gate)) return;
   const long n4 = bx.n / 4;
@@ -828,57 +883,57 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_quad_in(Recs<float, 8> R,
   const float sc = in.inu ? (float)in.inu[in.idx ? *in.idx : 0] : 1.0f;
   const float *srcf = in.basef + off;
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
-    const long r0 = 4 * q;
-    float4 a = *reinterpret_cast<const float4 *>(srcf + r0);
+    const Quad g = quad_of(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    float4 a = *reinterpret_cast<const float4 *>(srcf + g.r0);
     a.x *= sc; a.y *= sc; a.z *= sc; a.w *= sc;
     if (winvf) {
-      const float4 w = *reinterpret_cast<const float4 *>(winvf + r0);
+      const float4 w = *reinterpret_cast<const float4 *>(winvf + g.r0);
       a.x *= w.x; a.y *= w.y; a.z *= w.z; a.w *= w.w;
     }
-    *reinterpret_cast<float4 *>(bv + r0) = a;
-    const unsigned line = fast_div((unsigned)r0, bx.dx);
-    const unsigned kk = fast_div(line, bx.dy);
-    const int j = (int)(line - kk * (unsigned)bx.ny), k = (int)kk;
-    const int p = (j + k) & 1;  // colour-0 points of the quad
-    float c[2][8];
-    load_quad_recs(R, r0 / 2, c);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p == 0) { v.x = c[0][0] * a.x; v.z = c[1][0] * a.z; }
-    else { v.y = c[0][0] * a.y; v.w = c[1][0] * a.w; }
-    *reinterpret_cast<float4 *>(x + r0) = v;
+    *reinterpret_cast<float4 *>(bv + g.r0) = a;
+    *reinterpret_cast<float4 *>(x + g.r0) = zero_quad(R, U, a, (g.j + g.k) & 1, g.r0 / 2, uni);
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_relax_rb_quad_out(Recs<float, 8> R, const float *__restrict__ b,
+// One in-place phase. The quad is written whole: the other colour's values go
+// back as they were read (no phase changes them while others read them), one
+// 16-byte store instead of two strided ones. zout (may be null) receives it
+// too.
+__device__ __forceinline__ void relax_rb_quad_body(const Recs<float, 8> &R, const Uni8 &U, const QuadMap &Q, const float *b, float *x,
+                                                   const Box &bx, int color, int zero_x, float *zout, long t0,
+                                                   long ts) {
+  const long n4 = bx.n / 4;
+  const long mc = (long)color * (bx.n / 2);
+  IBM_QUAD_LOOP(q, live, n4, t0, ts) {
+    const Quad g = quad_of(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    const int p = (g.j + g.k + color) & 1;
+    const float4 bq = *reinterpret_cast<const float4 *>(b + g.r0);
+    float4 o;
+    if (zero_x) {
+      o = zero_quad(R, U, bq, p, mc + g.r0 / 2, uni);
+    } else {
+      const QuadX v = load_quad_x(x, g, bx);
+      o = relax_quad_new(R, U, bq, v, p, mc + g.r0 / 2, uni);
+    }
+    if (live) {
+      *reinterpret_cast<float4 *>(x + g.r0) = o;
+      if (zout) *reinterpret_cast<float4 *>(zout + g.r0) = o;
+    }
+  }
+}
+__global__ void __launch_bounds__(kThreads) k_relax_rb_quad_out(Recs<float, 8> R, Uni8 U, QuadMap Q, const float *__restrict__ b,
                                                                 float *x, Box bx, int color, OutRef out,
                                                                 const int *gate) {
   if (gate_off(gate)) return;
-  const long n4 = bx.n / 4;
-  float *z = out.f + (out.idx ? (long)(*out.idx) * out.ld : 0);
-  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
-    const long r0 = 4 * q;
-    const unsigned line = fast_div((unsigned)r0, bx.dx);
-    const int i0 = (int)((unsigned)r0 - line * (unsigned)bx.nx);
-    const unsigned kk = fast_div(line, bx.dy);
-    relax_quad_at(R, b, x, bx, color, 0, r0, i0, (int)(line - kk * (unsigned)bx.ny), (int)kk, z);
-  }
+  relax_rb_quad_body(R, U, Q, b, x, bx, color, 0, out.f + (out.idx ? (long)(*out.idx) * out.ld : 0),
+                     (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
-
-__device__ __forceinline__ void relax_rb_quad_body(const Recs<float, 8> &R, const float *b, float *x, const Box &bx,
-                                                   int color, int zero_x, long t0, long ts) {
-  const long n4 = bx.n / 4;
-  for (long q = t0; q < n4; q += ts) {
-    const long r0 = 4 * q;
-    const unsigned line = fast_div((unsigned)r0, bx.dx);
-    const int i0 = (int)((unsigned)r0 - line * (unsigned)bx.nx);
-    const unsigned kk = fast_div(line, bx.dy);
-    relax_quad_at(R, b, x, bx, color, zero_x, r0, i0, (int)(line - kk * (unsigned)bx.ny), (int)kk);
-  }
-}
-__global__ void __launch_bounds__(kThreads) k_relax_rb_quad(Recs<float, 8> R, const float *__restrict__ b, float *x,
-                                                            Box bx, int color, int zero_x, const int *gate) {
+__global__ void __launch_bounds__(kThreads) k_relax_rb_quad(Recs<float, 8> R, Uni8 U, QuadMap Q, const float *__restrict__ b,
+                                                            float *x, Box bx, int color, int zero_x, const int *gate) {
   if (gate_off(gate)) return;
-  relax_rb_quad_body(R, b, x, bx, color, zero_x, (long)blockIdx.x * blockDim.x + threadIdx.x,
+  relax_rb_quad_body(R, U, Q, b, x, bx, color, zero_x, nullptr, (long)blockIdx.x * blockDim.x + threadIdx.x,
                      (long)gridDim.x * blockDim.x);
 }
 
@@ -1039,39 +1094,36 @@ __device__ __forceinline__ void resid_quad(const float (&c)[2][8], const float4 
   }
 }
 
-__device__ __forceinline__ void residual_rb_quad_body(const Recs<float, 8> &R, const float *b, const float *x,
-                                                      float *res, const Box &bx, long t0, long ts) {
+__device__ __forceinline__ void residual_rb_quad_body(const Recs<float, 8> &R, const Uni8 &U, const QuadMap &Q,
+                                                      const float *b, const float *x, float *res, const Box &bx, long t0, long ts) {
   const long n4 = bx.n / 4;
-  const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
-  const long sy = nx, sz = (long)nx * ny;
-  for (long q = t0; q < n4; q += ts) {
-    const long r0 = 4 * q;
-    const unsigned line = fast_div((unsigned)r0, bx.dx);
-    const int i0 = (int)((unsigned)r0 - line * (unsigned)nx);
-    const unsigned kk = fast_div(line, bx.dy);
-    const int j = (int)(line - kk * (unsigned)ny), k = (int)kk;
-    float c[2][8];
-    load_quad_recs(R, r0 / 2, c);
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 bq = *reinterpret_cast<const float4 *>(b + r0);
-    const float4 xc = *reinterpret_cast<const float4 *>(x + r0);
-    const float4 xs = j > 0 ? *reinterpret_cast<const float4 *>(x + r0 - sy) : z4;
-    const float4 xn = j < ny - 1 ? *reinterpret_cast<const float4 *>(x + r0 + sy) : z4;
-    const float4 xb = k > 0 ? *reinterpret_cast<const float4 *>(x + r0 - sz) : z4;
-    const float4 xt = k < nz - 1 ? *reinterpret_cast<const float4 *>(x + r0 + sz) : z4;
-    const float xl = i0 > 0 ? x[r0 - 1] : 0.0f;
-    const float xr = i0 + 4 < nx ? x[r0 + 4] : 0.0f;
+  IBM_QUAD_LOOP(q, live, n4, t0, ts) {
+    const Quad g = quad_of(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    const float4 bq = *reinterpret_cast<const float4 *>(b + g.r0);
+    const QuadX v = load_quad_x(x, g, bx);
+    const bool even = ((g.j + g.k) & 1) == 0;
     float rr[4];
-    if (((j + k) & 1) == 0) resid_quad<0>(c, bq, xc, xs, xn, xb, xt, xl, xr, rr);
-    else resid_quad<1>(c, bq, xc, xs, xn, xb, xt, xl, xr, rr);
-    *reinterpret_cast<float4 *>(res + r0) = make_float4(rr[0], rr[1], rr[2], rr[3]);
+    if (uni) {
+      const float c[2][8] = {{U.c[0], U.c[1], U.c[2], U.c[3], U.c[4], U.c[5], U.c[6], U.c[7]},
+                             {U.c[0], U.c[1], U.c[2], U.c[3], U.c[4], U.c[5], U.c[6], U.c[7]}};
+      if (even) resid_quad<0>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, rr);
+      else resid_quad<1>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, rr);
+    } else {
+      float c[2][8];
+      load_quad_recs(R, g.r0 / 2, c);
+      if (even) resid_quad<0>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, rr);
+      else resid_quad<1>(c, bq, v.c, v.s, v.n, v.b, v.t, v.l, v.r, rr);
+    }
+    if (live) *reinterpret_cast<float4 *>(res + g.r0) = make_float4(rr[0], rr[1], rr[2], rr[3]);
   }
 }
-__global__ void __launch_bounds__(kThreads) k_residual_rb_quad(Recs<float, 8> R, const float *__restrict__ b,
+__global__ void __launch_bounds__(kThreads) k_residual_rb_quad(Recs<float, 8> R, Uni8 U, QuadMap Q, const float *__restrict__ b,
                                                                const float *__restrict__ x, float *__restrict__ res,
                                                                Box bx, const int *gate) {
   if (gate_off(gate)) return;
-  residual_rb_quad_body(R, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+  residual_rb_quad_body(R, U, Q, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x,
+                        (long)gridDim.x * blockDim.x);
 }
 
 // First phase from a zero guess: colour-0 points take invd b, colour-1 points 0.
@@ -1610,6 +1662,7 @@ struct alignas(16) ClusterOp {
   int kind = 0, color = 0, zero = 0, d = 0;  // zero: zero guess (relaxation); d: direction (transfers)
   int accumulate = 0;
   Box fb, cb;
+  QuadMap quads;
   const T *rec = nullptr, *tab = nullptr;  // colour-split records: the records, or the class table
   const uint16_t *code = nullptr;
   const T *A = nullptr;    // planes, or the dense inverse
@@ -1710,13 +1763,13 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       if (!done) {
         switch (op.kind) {
           case CK_RB_QUAD:
-            relax_rb_quad_body(op_recs<T, 8>(op), op.b, op.dst, op.fb, op.color, op.zero, t0, ts);
+            relax_rb_quad_body(op_recs<T, 8>(op), Uni8(), op.quads, op.b, op.dst, op.fb, op.color, op.zero, nullptr, t0, ts);
             break;
           case CK_RB27_QUAD:
             relax_rb27_quad_body(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
             break;
           case CK_RESID_RB_QUAD:
-            residual_rb_quad_body(op_recs<T, 8>(op), op.b, op.src, op.dst, op.fb, t0, ts);
+            residual_rb_quad_body(op_recs<T, 8>(op), Uni8(), op.quads, op.b, op.src, op.dst, op.fb, t0, ts);
             break;
           case CK_RESID_RB27_QUAD:
             residual_rb27_quad_body(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, t0, ts);
@@ -1852,7 +1905,10 @@ static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
     if (F.ns == 7) k_split_colors<T><<<grid_for(F.b.n), kThreads, 0, st>>>(F.A, F.invd.p, F.b, R.p);
     else k_split_colors27<T><<<grid_for(F.b.n), kThreads, 0, st>>>(F.A, F.invd.p, F.b, R.p);
   }
-  if (prm.classes && build_classes<T>(st, R.p, W, F.b.n, F.rbc)) R.release();
+  if (prm.classes && build_classes<T>(st, R.p, W, F.b.n, F.rbc)) {
+    R.release();
+    if (sizeof(T) == 4 && F.b.nx % 4 == 0 && prm.quads) mark_runs<T>(st, F.rbc, F.b);
+  }
 }
 
 template <class T, int W>
@@ -1861,6 +1917,15 @@ static Recs<T, W> recs_of(const DBuf<T> &plain, const Classes<T> &c) {
   if (c.ok() && c.W == W) { r.code = c.code.p; r.tab = c.tab.p; }
   else r.R = plain.p;
   return r;
+}
+
+static Uni8 uni8_of(const Classes<float> &c) {
+  Uni8 u;
+  if (c.ok() && c.W == 8 && c.runs.p) {
+    std::copy(c.major_rec.begin(), c.major_rec.end(), u.c);
+    u.runs = c.runs.p;
+  }
+  return u;
 }
 
 template <>
@@ -2177,6 +2242,7 @@ static T *record_cluster(std::vector<MgLevelT<T>> &L, int l, const MgParams &p, 
     ClusterOp<T> op;
     op.kind = kind;
     op.fb = F.b;
+    op.quads = make_quad_map(F.b);
     op.b = F.bv.p;
     return op;
   };
@@ -2452,6 +2518,9 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   const Recs<T, 28> R27 = recs_of<T, 28>(F.rb27, F.rbc);
   const bool rb7 = R7.R || R7.code, rb27 = R27.R || R27.code;
   const bool quad = F.b.nx % 4 == 0 && p.quads;  // quartet kernels (FP32)
+  Uni8 U7;
+  if constexpr (sizeof(T) == 4) U7 = uni8_of(F.rbc);
+  const QuadMap Q = make_quad_map(F.b);
   const double rec7 = R7.code ? 2.0 : 8.0 * T_, rec27 = R27.code ? 2.0 : 28.0 * T_;
   auto relax = [&](bool zero, bool last) {
     if constexpr (sizeof(T) == 4) {
@@ -2469,14 +2538,14 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
           const bool z = zero && color == 0;
           if (z && fin) {
             LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? 2.0 : T_) + (winvf ? 4.0 : 3.0) * T_ * n);
-            k_relax_rb_quad_in<<<resident_grid(k_relax_rb_quad_in, n / 4), kThreads, 0, st>>>(R7, F.bv.p, cur, F.b, *fin, winvf, gate);
+            k_relax_rb_quad_in<<<resident_grid(k_relax_rb_quad_in, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, *fin, winvf, gate);
           } else if (color == 1 && last && fout) {
             LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 2.5 * T_ * n);
-            k_relax_rb_quad_out<<<resident_grid(k_relax_rb_quad_out, n / 4), kThreads, 0, st>>>(R7, F.bv.p, cur, F.b, 1, *fout, gate);
+            k_relax_rb_quad_out<<<resident_grid(k_relax_rb_quad_out, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, 1, *fout, gate);
           } else {
             LaunchScope ls(K_MG_RELAX_FINE, st, z ? 0.5 * n * (R7.code ? 2.0 : T_) + 1.5 * T_ * n
                                                   : 0.5 * n * rec7 + 1.5 * T_ * n);
-            k_relax_rb_quad<<<resident_grid(k_relax_rb_quad, n / 4), kThreads, 0, st>>>(R7, F.bv.p, cur, F.b, color, z, gate);
+            k_relax_rb_quad<<<resident_grid(k_relax_rb_quad, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, color, z, gate);
           }
         }
         return;
@@ -2537,7 +2606,7 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
     bool done = false;
     if constexpr (sizeof(T) == 4) {
       if (quad) {
-        k_residual_rb_quad<<<resident_grid(k_residual_rb_quad, n / 4), kThreads, 0, st>>>(R7, F.bv.p, cur, F.r.p, F.b, gate);
+        k_residual_rb_quad<<<resident_grid(k_residual_rb_quad, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.r.p, F.b, gate);
         done = true;
       }
     }
