@@ -237,6 +237,7 @@ struct KSys {
   long ldv;
   float *Z;             // flexible basis (FP32), vector k at Z + k*ldv
   double *w, *x, *z, *z2;
+  double *Zd;           // pc 1: the preconditioned directions M V_k at Zd + k*ldv (null: only the current one, in z)
   const double *b;
   float *zf, *zf2;      // FP32 work for the inner sweeps
   double *part;         // block partial sums [nblk][kMaxKdim + 2]

@@ -100,6 +100,7 @@ class Krylov {
   struct Slot {
     KSysHost host;
     DBuf<double> V, w, z, z2, part;
+    DBuf<double> Zd;  // pc 1: the preconditioned directions of the cycle
     DBuf<float> Z, zf, zf2, Vf, wf;
     DBuf<float> vcur;  // FP64 basis with FP32 Jacobi: FP32 copy of the current basis vector
     DBuf<float2> xs;  // double-float copy of x for the double-float residual
