@@ -250,6 +250,9 @@ void ensure_classes(ibm_ctx *c, Op7 &o) {
     o.tabdf.alloc((size_t)16 * o.cls.K);
     LaunchScope ls(K_SETUP, c->st, 0.0);
     k_pad_rows<<<grid1d(8L * o.cls.K), kThreads, 0, c->st>>>(o.cls.tab.p, o.cls.K, o.tab.p, o.tabf.p, o.tabdf.p);
+    IBM_CUDA_TRY(cudaMemcpyAsync(o.major_f, o.tabf.p + 8L * o.cls.major, sizeof(o.major_f), cudaMemcpyDeviceToHost, c->st));
+    IBM_CUDA_TRY(
+        cudaMemcpyAsync(o.major_df, o.tabdf.p + 16L * o.cls.major, sizeof(o.major_df), cudaMemcpyDeviceToHost, c->st));
   }
   rows.release();
   DBuf<float> jrec;
@@ -264,8 +267,15 @@ void ensure_classes(ibm_ctx *c, Op7 &o) {
 
 // Points a system at its operator's classes.
 void use_classes(const Op7 &o, KSysHost &h) {
-  if (o.cls.ok()) { h.cls = o.cls.code.p; h.tab = o.tab.p; h.tabf = o.tabf.p; h.tabdf = o.tabdf.p; }
-  if (o.clsj.ok()) { h.clsj = o.clsj.code.p; h.tabj = o.clsj.tab.p; }
+  if (o.cls.ok()) {
+    h.cls = o.cls.code.p; h.tab = o.tab.p; h.tabf = o.tabf.p; h.tabdf = o.tabdf.p;
+    h.major = o.cls.major;
+    std::copy(o.major_f, o.major_f + 8, h.uf);
+    std::copy(o.major_df, o.major_df + 16, h.udf);
+  }
+  if (o.clsj.ok()) {
+    h.clsj = o.clsj.code.p; h.tabj = o.clsj.tab.p;
+  }
 }
 
 // Precision key of the configured solvers: the pressure's and the momentum's.

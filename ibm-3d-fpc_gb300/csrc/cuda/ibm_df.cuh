@@ -108,6 +108,31 @@ __device__ __forceinline__ void df_split_fast(double v, float &hi, float &lo) {
   lo = tiny ? 0.0f : lm;
 }
 
+// (double) v and (float) v (round to nearest even) with integer operations for
+// normal numbers and zeros: GB300 issues a conversion instruction at its FP64
+// rate, two per clock and SM, and integer operations at 64. Same value in
+// every case; subnormals, infinities, NaN and values out of the float's normal
+// range take the conversion instruction.
+__device__ __forceinline__ double widen(float v) {
+  const unsigned u = __float_as_uint(v), a = u & 0x7fffffffu;
+  if (a - 0x00800000u < 0x7f000000u)  // exponent 1 .. 254
+    return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(u << 29));
+  if (a == 0u) return __hiloint2double((int)u, 0);
+  return (double)v;
+}
+__device__ __forceinline__ float narrow(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v), e = (hi >> 20) & 0x7ffu;
+  if (e - 898u < 252u) {  // 2^-125 <= |v| < 2^127: rounding stays normal and finite
+    // exponent and fraction down to the float's 23 bits: the kept bits, and the 29 below them
+    const unsigned m = __funnelshift_l(lo, hi & 0x7fffffffu, 3) - 0xC0000000u;  // rebias: 896 << 23 mod 2^32
+    const unsigned rest = lo & 0x1fffffffu;
+    const unsigned up = (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u;
+    return __uint_as_float((hi & 0x80000000u) | (m + up));
+  }
+  if (((hi & 0x7fffffffu) | lo) == 0u) return __uint_as_float(hi);
+  return (float)v;
+}
+
 // A double-float value and the operations the dense kernels need. Sums and
 // products carry about 2^-47 of their operands' size.
 struct DF {

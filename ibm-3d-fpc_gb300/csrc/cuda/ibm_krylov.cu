@@ -16,6 +16,8 @@
 // Basis vectors are stored unnormalised with their exact norms in nu[].
 // Reductions are deterministic: fixed per-warp order inside a block, block
 // partials summed in block order by the last block to finish.
+#include <algorithm>
+
 #include "ibm_common.cuh"
 #include "ibm_krylov.cuh"
 #include "ibm_df.cuh"
@@ -70,6 +72,68 @@ __device__ __forceinline__ void load_rows4(const float *__restrict__ tab, ushort
   }
 #pragma unroll
   for (int s = 0; s < 7; ++s) cp[s] = make_float4(v[0][s], v[1][s], v[2][s], v[3][s]);
+}
+
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ float f4(const float4 &v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
+
+// A quad: rows r0 .. r0 + 3 of one line (nx and r0 multiples of 4), with the
+// values of an FP32 vector there and around, 0 outside the box: seven loads
+// instead of 28.
+struct QuadRows {
+  float4 c, s, n, b, t;  // the quad; its neighbours at y - 1, y + 1, z - 1, z + 1
+  float l, r;            // x neighbours of the first and the last row
+  bool hl, hr, hs, hn, hb, ht;
+};
+__device__ __forceinline__ QuadRows load_quad_rows(const KSys &S, const float *z, long r0) {
+  int i, j, k;
+  sys_ijk(r0, S, i, j, k);
+  const long sy = S.nx, sz = (long)S.nx * S.ny;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  QuadRows q;
+  q.hl = i > 0; q.hr = i + 4 < S.nx; q.hs = j > 0; q.hn = j < S.ny - 1; q.hb = k > 0; q.ht = k < S.nz - 1;
+  q.c = ld4(z + r0);
+  q.s = q.hs ? ld4(z + r0 - sy) : z4;
+  q.n = q.hn ? ld4(z + r0 + sy) : z4;
+  q.b = q.hb ? ld4(z + r0 - sz) : z4;
+  q.t = q.ht ? ld4(z + r0 + sz) : z4;
+  q.l = q.hl ? z[r0 - 1] : 0.0f;
+  q.r = q.hr ? z[r0 + 4] : 0.0f;
+  return q;
+}
+// x neighbours of row q of the quad
+__device__ __forceinline__ float quad_w(const QuadRows &v, int q) { return q == 0 ? v.l : f4(v.c, q - 1); }
+__device__ __forceinline__ float quad_e(const QuadRows &v, int q) { return q == 3 ? v.r : f4(v.c, q + 1); }
+// whether all four codes are `major`
+__device__ __forceinline__ bool all_major(ushort4 c, int major) {
+  return c.x == major && c.y == major && c.z == major && c.w == major;
+}
+// A z of one row in FP32, slot order; c[s] the row's slots.
+__device__ __forceinline__ float quad_row32(const QuadRows &v, int q, float c0, float c1, float c2, float c3, float c4,
+                                            float c5, float c6) {
+  float a = 0.0f;
+  a = fmaf(c0, f4(v.c, q), a);
+  a = fmaf(c1, quad_w(v, q), a);
+  a = fmaf(c2, quad_e(v, q), a);
+  a = fmaf(c3, f4(v.s, q), a);
+  a = fmaf(c4, f4(v.n, q), a);
+  a = fmaf(c5, f4(v.b, q), a);
+  a = fmaf(c6, f4(v.t, q), a);
+  return a;
+}
+// ... in double-float (hi: slots 0 .. 6, lo: 8 .. 14 of c), widened once.
+template <class C>
+__device__ __forceinline__ double quad_row_df(const QuadRows &v, int q, const C &c) {
+  float ah = 0.0f, al = 0.0f;
+  df_fma1(ah, al, c[0], c[8], f4(v.c, q));
+  df_fma1(ah, al, c[1], c[9], quad_w(v, q));
+  df_fma1(ah, al, c[2], c[10], quad_e(v, q));
+  df_fma1(ah, al, c[3], c[11], f4(v.s, q));
+  df_fma1(ah, al, c[4], c[12], f4(v.n, q));
+  df_fma1(ah, al, c[5], c[13], f4(v.b, q));
+  df_fma1(ah, al, c[6], c[14], f4(v.t, q));
+  return widen(ah) + widen(al);
 }
 
 // Sum block partials of `nd` dot products in block order; one warp per dot.
@@ -148,9 +212,9 @@ __global__ void __launch_bounds__(kThreads) k_init(const __grid_constant__ KSysP
             rv = bv - stencil7_at(c0, cs, S.x, (int)r, i, j, k, S.nx, S.ny, S.nz);
             pr = fma(rv, rv, pr);
           }
-          if (S.a32) S.Vf[r] = (float)rv;
+          if (S.a32) S.Vf[r] = narrow(rv);
           else S.V[r] = rv;
-          if (S.vcur) S.vcur[r] = (float)rv;
+          if (S.vcur) S.vcur[r] = narrow(rv);
           pb = fma(bv, bv, pb);
         }
       }
@@ -344,7 +408,7 @@ __device__ __forceinline__ double spmv_row64(const KSys &S, long r, const double
     df_fma1(ah, al, h1.x, l1.x, zyp);
     df_fma1(ah, al, h1.y, l1.y, zzm);
     df_fma1(ah, al, h1.z, l1.z, zzp);
-    return (double)ah + (double)al;
+    return widen(ah) + widen(al);
   } else {
     long cs;
     const double *c0 = a_row(S, r, cs);
@@ -388,8 +452,57 @@ __device__ __forceinline__ void spmv_pass64(const KSys &S, const double *z, cons
   }
 }
 
+// spmv_pass64<0> with four consecutive rows per thread (S.quad). The rows of
+// most quads are all of the major class: their 14 values come from constant
+// memory. Bound: HBM (34 bytes a row at a basis of 2.5 vectors) next to FP64
+// issue (one add and nd FMAs a row). One row at a time, with two conversion
+// instructions a row, 28 loads for four rows and four 16-byte table loads for
+// each, a launch over 3 x 10.5M rows took 371 us, now 353: the v and w rows go
+// in quads, and the u rows (an odd number a line) set the time.
+__device__ __forceinline__ void spmv_pass64_quad(const KSys &S, const float *zj, int c0, int nd,
+                                                 double (&pd)[kDots64]) {
+  for (long t0 = (long)blockIdx.x * kTile; t0 < S.n; t0 += (long)gridDim.x * kTile) {
+    const long r0 = t0 + 4 * threadIdx.x;
+    if (r0 >= S.n) continue;
+    double w[4];
+    if (c0 == 0) {
+      const ushort4 c4 = __ldcs(reinterpret_cast<const ushort4 *>(S.cls + r0));
+      const QuadRows v = load_quad_rows(S, zj, r0);
+      if (all_major(c4, S.major)) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[q] = quad_row_df(v, q, S.udf);
+      } else {
+        const unsigned short ks[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 *p = reinterpret_cast<const float4 *>(S.tabdf + 16 * (long)ks[q]);
+          const float4 h0 = __ldg(p), h1 = __ldg(p + 1), l0 = __ldg(p + 2), l1 = __ldg(p + 3);
+          const float c[16] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w,
+                               l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+          w[q] = quad_row_df(v, q, c);
+        }
+      }
+      *reinterpret_cast<double2 *>(S.w + r0) = make_double2(w[0], w[1]);
+      *reinterpret_cast<double2 *>(S.w + r0 + 2) = make_double2(w[2], w[3]);
+    } else {
+      const double2 a = *reinterpret_cast<const double2 *>(S.w + r0), b = *reinterpret_cast<const double2 *>(S.w + r0 + 2);
+      w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
+    }
+#pragma unroll
+    for (int kk = 0; kk < kDots64; ++kk) {
+      if (kk >= nd) break;
+      const double *vk = S.V + (long)(c0 + kk) * S.ldv + r0;
+      const double2 a = *reinterpret_cast<const double2 *>(vk), b = *reinterpret_cast<const double2 *>(vk + 2);
+      pd[kk] = fma(a.x, w[0], pd[kk]);
+      pd[kk] = fma(a.y, w[1], pd[kk]);
+      pd[kk] = fma(b.x, w[2], pd[kk]);
+      pd[kk] = fma(b.y, w[3], pd[kk]);
+    }
+  }
+}
+
 // w = A z_j (z_j = M v_j by the system's preconditioner mode), d1_k = (V_k, w).
-__global__ void __launch_bounds__(kThreads) k_arnoldi_spmv(const __grid_constant__ KSysPack P) {
+__global__ void __launch_bounds__(kThreads, 4) k_arnoldi_spmv(const __grid_constant__ KSysPack P) {
   const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
   if (!sc->active || S.a32) return;
@@ -404,7 +517,8 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv(const __grid_constant
     double pd[kDots64];
 #pragma unroll
     for (int kk = 0; kk < kDots64; ++kk) pd[kk] = 0.0;
-    if (S.df_spmv) spmv_pass64<0>(S, z, zj, inv_nu, c0, ndc, pd);
+    if (S.df_spmv && S.quad) spmv_pass64_quad(S, zj, c0, ndc, pd);
+    else if (S.df_spmv) spmv_pass64<0>(S, z, zj, inv_nu, c0, ndc, pd);
     else if (S.pc != 2) spmv_pass64<1>(S, z, zj, inv_nu, c0, ndc, pd);
     else spmv_pass64<2>(S, z, zj, inv_nu, c0, ndc, pd);
     flush_dots64(pd, ndc, sacc + c0 * kWarps, warp, lane);
@@ -527,7 +641,7 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next(const __grid_constant
       if (r < S.n) {
         if (store) {
           vn[r] = wv[t];
-          if (S.vcur) S.vcur[r] = (float)wv[t];
+          if (S.vcur) S.vcur[r] = narrow(wv[t]);
         }
         p = fma(wv[t], wv[t], p);
       }
@@ -606,10 +720,31 @@ __global__ void __launch_bounds__(kThreads) k_cycle_update(const __grid_constant
     }
     return;
   }
+  if (S.pc == 2 && S.vec4) {
+    // four consecutive rows per thread; the directions widened on the integer
+    // pipe (the conversions took as many FP64 issue slots as the sums: 550 us
+    // over 3 x 10.5M rows and three to four directions, now 303)
+    for (long r0 = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x); r0 < S.n; r0 += 4L * gridDim.x * blockDim.x) {
+      const double2 x01 = *reinterpret_cast<const double2 *>(S.x + r0);
+      const double2 x23 = *reinterpret_cast<const double2 *>(S.x + r0 + 2);
+      double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+      for (int kk = 0; kk < m; ++kk) {
+        const float4 z = ld4(S.Z + (long)kk * S.ldv + r0);
+        a[0] = fma(cf[kk], widen(z.x), a[0]);
+        a[1] = fma(cf[kk], widen(z.y), a[1]);
+        a[2] = fma(cf[kk], widen(z.z), a[2]);
+        a[3] = fma(cf[kk], widen(z.w), a[3]);
+      }
+      *reinterpret_cast<double2 *>(S.x + r0) = make_double2(x01.x + a[0], x01.y + a[1]);
+      *reinterpret_cast<double2 *>(S.x + r0 + 2) = make_double2(x23.x + a[2], x23.y + a[3]);
+    }
+    return;
+  }
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x) {
     double acc = 0.0;
     if (S.pc == 2) {
-      for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], (double)S.Z[(long)kk * S.ldv + r], acc);
+      for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], widen(S.Z[(long)kk * S.ldv + r]), acc);
       S.x[r] = S.x[r] + acc;
     } else {
       const double *basis = S.Zd ? S.Zd : S.V;
@@ -700,9 +835,9 @@ __global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_consta
         long cs;
         const double *c0 = ar_row(S, r, cs);
         const double rv = S.b[r] - stencil7_at(c0, cs, S.x, (int)r, i, j, k, S.nx, S.ny, S.nz);
-        if (S.a32) S.Vf[r] = (float)rv;
+        if (S.a32) S.Vf[r] = narrow(rv);
         else S.V[r] = rv;
-        if (S.vcur) S.vcur[r] = (float)rv;
+        if (S.vcur) S.vcur[r] = narrow(rv);
         pr = fma(rv, rv, pr);
       }
     }
@@ -754,10 +889,6 @@ __global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_consta
 // A cycle stops once its estimate fell by cyc_rtol; the restart computes the
 // true residual in FP64, so the solve still meets the FP64 tolerance.
 
-__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
-__device__ __forceinline__ float f4(const float4 &v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
-
 __device__ __forceinline__ float warp_sum_f(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -784,6 +915,25 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(const __grid_consta
     for (long t0 = (long)blockIdx.x * kTile; t0 < n; t0 += (long)gridDim.x * kTile) {
       const long r0 = t0 + 4 * threadIdx.x;
       if (r0 >= n) continue;
+      float w[4];
+      if (S.quad && S.cls) {
+        // 85 us at 10.5M rows with 28 loads of z and eight of the table per
+        // thread, 64 as quads
+        const ushort4 c4 = __ldcs(reinterpret_cast<const ushort4 *>(S.cls + r0));
+        const QuadRows v = load_quad_rows(S, zj, r0);
+        if (all_major(c4, S.major)) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            w[q] = quad_row32(v, q, S.uf[0], S.uf[1], S.uf[2], S.uf[3], S.uf[4], S.uf[5], S.uf[6]);
+        } else {
+          float4 cp[7];
+          load_rows4(S.tabf, c4, cp);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            w[q] = quad_row32(v, q, f4(cp[0], q), f4(cp[1], q), f4(cp[2], q), f4(cp[3], q), f4(cp[4], q), f4(cp[5], q),
+                              f4(cp[6], q));
+        }
+      } else {
       float4 cp[7];
       if (S.cls) {
         load_rows4(S.tabf, __ldcs(reinterpret_cast<const ushort4 *>(S.cls + r0)), cp);
@@ -791,7 +941,6 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(const __grid_consta
 #pragma unroll
         for (int q = 0; q < 7; ++q) cp[q] = __ldcs(reinterpret_cast<const float4 *>(S.Af + (long)q * n + r0));
       }
-      float w[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const long r = r0 + q;
@@ -806,6 +955,7 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(const __grid_consta
         a = fmaf(f4(cp[5], q), k > 0 ? zj[r - sz] : 0.0f, a);
         a = fmaf(f4(cp[6], q), k < S.nz - 1 ? zj[r + sz] : 0.0f, a);
         w[q] = a;
+      }
       }
       st4(S.wf + r0, make_float4(w[0], w[1], w[2], w[3]));
 #pragma unroll
@@ -1105,8 +1255,8 @@ __device__ __forceinline__ void jacobi_two_rows(const KSys &S, const VT *__restr
   }
 }
 
-// The same, four consecutive rows per thread with 16-byte loads of the
-// coefficient planes and stores of z (FP32 basis, n % 4 == 0).
+// Four consecutive rows per thread with 16-byte loads of the coefficient
+// planes and stores of z (FP32 basis, n % 4 == 0).
 __device__ __forceinline__ void jacobi_two_rows4(const KSys &S, const float *__restrict__ vj, float inv_nu,
                                                  float *__restrict__ out) {
   const long n = S.n, sy = S.nx, sz = (long)S.nx * S.ny;
@@ -1329,6 +1479,10 @@ void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, uns
     k.A = h.A; k.Ar = h.Ar; k.invd = h.invd; k.Af = h.Af; k.invdf = h.invdf; k.Ajf = h.Ajf;
     k.cls = h.cls; k.tab = h.tab; k.tabf = h.tabf; k.clsj = h.clsj; k.tabj = h.tabj;
     k.tabdf = h.tabdf;
+    k.major = h.major;
+    std::copy(h.uf, h.uf + 8, k.uf);
+    std::copy(h.udf, h.udf + 16, k.udf);
+    k.quad = (h.nx % 4 == 0) ? 1 : 0;
     k.df_resid = (h.a32 && h.cls && h.tabdf && h.df_residual) ? 1 : 0;
     k.df_spmv = (h.pc == 2 && !h.a32 && h.cls && h.tabdf && h.A == h.Ar && h.df_spmv) ? 1 : 0;
     k.xs = slot[s].xs.p;
