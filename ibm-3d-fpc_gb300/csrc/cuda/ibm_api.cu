@@ -658,6 +658,7 @@ int ibm_assemble_momentum(ibm_ctx *c, double xcirc, double ycirc, double Rcirc, 
           sbox[r] = rid > 0 ? hs[(size_t)rid] : 0.0;
         }
         upload(c->scale_box[f], sbox, c->st);
+        c->plain_ready = false;
         invalidate_graph(c);
       }
     }
@@ -785,6 +786,7 @@ int ibm_set_masks(ibm_ctx *c, const uint8_t *active_u, const uint8_t *active_v, 
     c->h_act_u = au; c->h_act_v = av; c->h_act_w = aw; c->h_fluid = fp;
     c->body_set = false;
     c->masks_set = true;
+    c->plain_ready = false;
     c->aux_set = false;
     c->csr_set = false;
     c->solvers_ready = false;
@@ -848,6 +850,7 @@ int ibm_set_aux(ibm_ctx *c, const double *scale_u, const double *scale_v, const 
     upload(c->div_bc_cell, dcell, c->st);
     upload(c->uin, to_host(uin, (size_t)c->g.ny * c->g.nz), c->st);
     c->aux_set = true;
+    c->plain_ready = false;
     invalidate_graph(c);
     return IBM_OK;
   });
@@ -950,6 +953,7 @@ int ibm_set_projection_csr(ibm_ctx *c, const int32_t *D_rowptr, const int32_t *D
     upload(c->Dc, Dc, c->st);
     upload(c->Gu, Gu, c->st); upload(c->Gv, Gv, c->st); upload(c->Gw, Gw, c->st);
     c->csr_set = true;
+    c->plain_ready = false;
     invalidate_graph(c);
     return IBM_OK;
   });
@@ -1019,6 +1023,7 @@ void step_launch(ibm_ctx *c, double ramp) {
   require_inputs(c);
   ensure_solvers(c);
   ensure_rhs_df(c);
+  ensure_plain(c);
   cudaStream_t st = c->st;
   *c->hramp = ramp;
   KResult *rm = c->last_rm, *rp = c->last_rp;

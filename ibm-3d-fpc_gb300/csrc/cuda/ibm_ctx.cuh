@@ -11,8 +11,14 @@ constexpr uint8_t kActive = 1;   // active_{u,v,w} at the face itself
 constexpr uint8_t kQFace = 2;    // id_q > 0: part of the projection vector q
 constexpr uint8_t kRhsRow = 4;   // id > 0 && active: a solved (non-identity) momentum row
 constexpr uint8_t kBcSet = 8;    // the BC cleanup overwrites this face (boundary plane or zero list)
-// Cell flag bit.
-constexpr uint8_t kFluid = 1;    // fluid_p && id_p > 0
+// ... derived from the coefficients (ensure_plain): away from walls and the
+// body the same few values repeat on every face and cell, and the dense
+// kernels take them from their parameters instead of memory there
+constexpr uint8_t kPlainFace = 16;  // a q face between two fluid cells with the field's common G pair
+constexpr uint8_t kPlainRow = 32;   // a row with the field's common row scale and boundary term
+// Cell flag bits.
+constexpr uint8_t kFluid = 1;      // fluid_p && id_p > 0
+constexpr uint8_t kPlainCell = 2;  // fluid, common D row, no boundary lift, its faces all q faces the BC leaves alone
 
 struct StepDiag {                // written by the diagnostics kernel
   double div2, umax, vmax, wmax;
@@ -22,6 +28,13 @@ struct StepDiag {                // written by the diagnostics kernel
   double force[3];               // force of the fluid on the body (k_forces)
   unsigned fticket;
   int pad2;
+};
+
+// The common coefficients that the flags above refer to.
+struct Plain {
+  double gl[3] = {}, gr[3] = {};  // G of a face: lower and upper cell
+  double sc[3] = {}, bc[3] = {};  // row scale and boundary term
+  double D[6] = {};
 };
 
 struct Geometry {
@@ -77,6 +90,8 @@ struct ibm_ctx {
   ibm::DBuf<double> cf_w;
 
   ibm::DBuf<double> u, v, w, p, ut, vt, wt;
+  ibm::Plain plain;
+  bool plain_ready = false;      // flags and coefficients above derived from the current inputs
   ibm::DBuf<float2> df_u, df_v, df_w, df_p;  // double-float copies of u, v, w, p (df_rhs)
   ibm::DBuf<double> xb[4], bb[4];
   ibm::DBuf<double> part;        // diagnostics block partials

@@ -9,7 +9,10 @@
 // written out (fma() where the reference's device code fuses a CSR
 // accumulation, separately rounded operations elsewhere) so the CPU oracle
 // reproduces the results bit for bit.
+#include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <map>
 
 #include "ibm_ctx.cuh"
 #include "ibm_df.cuh"
@@ -173,6 +176,7 @@ struct RhsArgs {
   KnownDiv tdx, tdy, tdz;  // 2 dx, 2 dy, 2 dz
   DF da, drho, drx, dry, drz;  // double-float a, rho, 1 / (2 dx), 1 / (2 dy), 1 / (2 dz)
   const float2 *u2, *v2, *w2, *p2;  // double-float copies of u, v, w, p (RhsDF; k_split_fields)
+  Plain plain;
   int zero_guess;
 };
 
@@ -186,6 +190,7 @@ struct RhsArgs {
 struct RhsF64 {
   using T = double;
   __device__ static T in(double x) { return x; }
+  __device__ static T in_once(double x) { return x; }
   __device__ static T fld(const double *a, const float2 *, long i) { return a[i]; }
   __device__ static T zero() { return 0.0; }
   __device__ static T avg(T a, T b, T c, T d) { return avg4(a, b, c, d); }
@@ -193,13 +198,19 @@ struct RhsF64 {
     return advect(c, dm, dp, A.tdx, a2, em, ep, A.tdy, a3, fm, fp, A.tdz);
   }
   __device__ static T grad(T gl, T pl, T gr, T pr) { return grad_face(gl, pl, gr, pr); }
-  __device__ static double rhs(const RhsArgs &A, T uc, T conv, T gp, double bc, double sc) {
+  __device__ static double rhs(const RhsArgs &A, T uc, T conv, T gp, T bc, T sc) {
     return mom_rhs(A.a, A.rho, uc, conv, gp, bc, sc);
   }
 };
 struct RhsDF {
   using T = DF;
   __device__ static T in(double x) { return df_of(x); }
+  // ... of a value split once per thread: every bit two floats hold
+  __device__ static T in_once(double x) {
+    T r;
+    df_split(x, r.h, r.l);
+    return r;
+  }
   // a field value from the field's double-float copy (split once per step)
   __device__ static T fld(const double *, const float2 *a2, long i) {
     const float2 v = a2[i];
@@ -214,14 +225,18 @@ struct RhsDF {
     return df_add(df_add(t1, t2), t3);
   }
   __device__ static T grad(T gl, T pl, T gr, T pr) { return df_add(df_mul(gl, pl), df_mul(gr, pr)); }
-  __device__ static double rhs(const RhsArgs &A, T uc, T conv, T gp, double bc, double sc) {
+  __device__ static double rhs(const RhsArgs &A, T uc, T conv, T gp, T bc, T sc) {
     T t = df_sub(df_mul(A.da, uc), df_mul(A.drho, conv));
-    t = df_add(df_sub(t, gp), df_of(bc));
-    return df_to_double(df_mul(t, df_of(sc)));
+    t = df_add(df_sub(t, gp), bc);
+    return df_to_double(df_mul(t, sc));
   }
 };
 
-// One thread per solve-box row of u, v and w (flat index over the three boxes).
+// One thread per solve-box row, the u, v and w boxes one after the other. Rows
+// and faces with the common coefficients (kPlainRow, kPlainFace) read neither
+// the scale and boundary term nor G and the cells' flags: 32 of a row's 65
+// bytes, and in the double-float instance four of its splits (640x128x128 in
+// that instance: 890 -> 690 us, FP32 issue next to HBM).
 // The loads are those of the reference's bounds-guarded loads
 // (gpu_dense_ops.hpp:1-3) with the guards that a solve-box row can never fail
 // dropped: on a u row (1 <= i <= nx-1) the x neighbours of u and the four v
@@ -232,15 +247,15 @@ template <class M>
 __global__ void __launch_bounds__(kThreads, 4) k_momentum_rhs(RhsArgs A) {
   using T = typename M::T;
   const Dims &d = A.d;
-  const long total = A.nb[0] + A.nb[1] + A.nb[2];
   const long NU = (long)(d.nx + 1) * d.ny * d.nz, NV = (long)d.nx * (d.ny + 1) * d.nz,
              NW = (long)d.nx * d.ny * (d.nz + 1);
   const long su = d.nx + 1, pu = (long)(d.nx + 1) * d.ny;  // u strides along y and z
   const long sv = d.nx, pv = (long)d.nx * (d.ny + 1);     // v
   const long sw = d.nx, pw = (long)d.nx * d.ny;           // w and cells
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
-    if (t < A.nb[0]) {  // u row: face (i+1, j, k) with i in [0, nx-2]
-      const long r = t;
+  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
+  {
+    const T cgl = M::in_once(A.plain.gl[0]), cgr = M::in_once(A.plain.gr[0]), csc = M::in_once(A.plain.sc[0]), cbc = M::in_once(A.plain.bc[0]);
+    for (long r = t0; r < A.nb[0]; r += ts) {  // u row: face (i+1, j, k) with i in [0, nx-2]
       long q;
       const int i = udivmod(r, d.dnxm, q) + 1;
       long kq;
@@ -262,18 +277,29 @@ __global__ void __launch_bounds__(kThreads, 4) k_momentum_rhs(RhsArgs A) {
                         (k > 0 ? M::fld(A.u, A.u2, f - pu) : uc), (k < d.nz - 1 ? M::fld(A.u, A.u2, f + pu) : uc));
         }
         T gp = M::zero();
-        if (fl & kQFace) {
+        if (fl & kPlainFace) {
+          const long c = P3(d, i - 1, j, k);
+          gp = M::grad(cgl, M::fld(A.p, A.p2, c), cgr, M::fld(A.p, A.p2, c + 1));
+        } else if (fl & kQFace) {
           const long c = P3(d, i - 1, j, k);
           const T pl = (A.fc[c] & kFluid) ? M::fld(A.p, A.p2, c) : M::zero();
           const T pr = (A.fc[c + 1] & kFluid) ? M::fld(A.p, A.p2, c + 1) : M::zero();
           gp = M::grad(M::in(A.Gu[f]), pl, M::in(A.Gu[NU + f]), pr);
         }
-        rhs = M::rhs(A, uc, conv, gp, A.bc[0][r], A.sc[0][r]);
+        T bc = cbc, sc = csc;
+        if (!(fl & kPlainRow)) {
+          bc = M::in(A.bc[0][r]);
+          sc = M::in(A.sc[0][r]);
+        }
+        rhs = M::rhs(A, uc, conv, gp, bc, sc);
       }
       A.b[0][r] = rhs;
       A.x0[0][r] = A.zero_guess ? 0.0 : A.u[f];
-    } else if (t < A.nb[0] + A.nb[1]) {  // v row: face (i, j+1, k)
-      const long r = t - A.nb[0];
+    }
+  }
+  {
+    const T cgl = M::in_once(A.plain.gl[1]), cgr = M::in_once(A.plain.gr[1]), csc = M::in_once(A.plain.sc[1]), cbc = M::in_once(A.plain.bc[1]);
+    for (long r = t0; r < A.nb[1]; r += ts) {  // v row: face (i, j+1, k)
       long q;
       const int i = udivmod(r, d.dnx, q);
       long kq;
@@ -296,18 +322,29 @@ __global__ void __launch_bounds__(kThreads, 4) k_momentum_rhs(RhsArgs A) {
                         (k > 0 ? M::fld(A.v, A.v2, f - pv) : vc), (k < d.nz - 1 ? M::fld(A.v, A.v2, f + pv) : vc));
         }
         T gp = M::zero();
-        if (fl & kQFace) {
+        if (fl & kPlainFace) {
+          const long c = P3(d, i, j - 1, k);
+          gp = M::grad(cgl, M::fld(A.p, A.p2, c), cgr, M::fld(A.p, A.p2, c + sw));
+        } else if (fl & kQFace) {
           const long c = P3(d, i, j - 1, k);
           const T pl = (A.fc[c] & kFluid) ? M::fld(A.p, A.p2, c) : M::zero();
           const T pr = (A.fc[c + sw] & kFluid) ? M::fld(A.p, A.p2, c + sw) : M::zero();
           gp = M::grad(M::in(A.Gv[f]), pl, M::in(A.Gv[NV + f]), pr);
         }
-        rhs = M::rhs(A, vc, conv, gp, A.bc[1][r], A.sc[1][r]);
+        T bc = cbc, sc = csc;
+        if (!(fl & kPlainRow)) {
+          bc = M::in(A.bc[1][r]);
+          sc = M::in(A.sc[1][r]);
+        }
+        rhs = M::rhs(A, vc, conv, gp, bc, sc);
       }
       A.b[1][r] = rhs;
       A.x0[1][r] = A.zero_guess ? 0.0 : A.v[f];
-    } else {  // w row: face (i, j, k+1)
-      const long r = t - A.nb[0] - A.nb[1];
+    }
+  }
+  {
+    const T cgl = M::in_once(A.plain.gl[2]), cgr = M::in_once(A.plain.gr[2]), csc = M::in_once(A.plain.sc[2]), cbc = M::in_once(A.plain.bc[2]);
+    for (long r = t0; r < A.nb[2]; r += ts) {  // w row: face (i, j, k+1)
       long q;
       const int i = udivmod(r, d.dnx, q);
       long kq;
@@ -331,13 +368,21 @@ __global__ void __launch_bounds__(kThreads, 4) k_momentum_rhs(RhsArgs A) {
                         M::fld(A.w, A.w2, f - pw), M::fld(A.w, A.w2, f + pw));
         }
         T gp = M::zero();
-        if (fl & kQFace) {
+        if (fl & kPlainFace) {
+          const long c = P3(d, i, j, k - 1);
+          gp = M::grad(cgl, M::fld(A.p, A.p2, c), cgr, M::fld(A.p, A.p2, c + pw));
+        } else if (fl & kQFace) {
           const long c = P3(d, i, j, k - 1);
           const T pl = (A.fc[c] & kFluid) ? M::fld(A.p, A.p2, c) : M::zero();
           const T pr = (A.fc[c + pw] & kFluid) ? M::fld(A.p, A.p2, c + pw) : M::zero();
           gp = M::grad(M::in(A.Gw[f]), pl, M::in(A.Gw[NW + f]), pr);
         }
-        rhs = M::rhs(A, wc, conv, gp, A.bc[2][r], A.sc[2][r]);
+        T bc = cbc, sc = csc;
+        if (!(fl & kPlainRow)) {
+          bc = M::in(A.bc[2][r]);
+          sc = M::in(A.sc[2][r]);
+        }
+        rhs = M::rhs(A, wc, conv, gp, bc, sc);
       }
       A.b[2][r] = rhs;
       A.x0[2][r] = A.zero_guess ? 0.0 : A.w[f];
@@ -359,8 +404,10 @@ __global__ void __launch_bounds__(kThreads) k_split_fields(SplitArgs A) {
   float2 *dst = a == 0 ? A.dst[0] : a == 1 ? A.dst[1] : a == 2 ? A.dst[2] : A.dst[3];
   const long n = a == 0 ? A.n[0] : a == 1 ? A.n[1] : a == 2 ? A.n[2] : A.n[3];
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    // all of the significand that two floats hold: the pressure's split error,
+    // over the grid spacing, is the largest of the right-hand side's
     float h, l;
-    df_split_fast(src[i], h, l);
+    df_split(src[i], h, l);
     dst[i] = make_float2(h, l);
   }
 }
@@ -460,6 +507,7 @@ struct ProjArgs {
   const double *Gu, *Gv, *Gw;
   double factor;
   StepDiag *dg;
+  Plain plain;
 };
 
 __device__ __forceinline__ double phi_at(const ProjArgs &A, long c) { return (A.fc[c] & kFluid) ? A.phi[c] : 0.0; }
@@ -471,50 +519,46 @@ __global__ void __launch_bounds__(kThreads, 4) k_project(ProjArgs A) {
              NW = (long)d.nx * d.ny * (d.nz + 1), NP = (long)d.nx * d.ny * d.nz;
   const double nf = -A.factor;
   int bad = 0;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < NU + NV + NW + NP; t += (long)gridDim.x * blockDim.x) {
-    if (t < NU) {
-      const long f = t;
-      double val = A.ut[f];
-      if (A.fu[f] & kQFace) {
-        long q;
-        const int i = udivmod(f, d.dnx1, q);
-        long kq;
-      const int j = udivmod(q, d.dny, kq), k = (int)kq;
-        const double pl = i > 0 ? phi_at(A, P3(d, i - 1, j, k)) : 0.0;
-        const double pr = i < d.nx ? phi_at(A, P3(d, i, j, k)) : 0.0;
-        val = fma(nf, grad_face(A.Gu[f], pl, A.Gu[NU + f], pr), val);
-      }
-      A.u[f] = val;
-    } else if (t < NU + NV) {
-      const long f = t - NU;
-      double val = A.vt[f];
-      if (A.fv[f] & kQFace) {
-        long q;
-        const int i = udivmod(f, d.dnx, q);
-        long kq;
-      const int j = udivmod(q, d.dny1, kq), k = (int)kq;
-        const double pl = j > 0 ? phi_at(A, P3(d, i, j - 1, k)) : 0.0;
-        const double pr = j < d.ny ? phi_at(A, P3(d, i, j, k)) : 0.0;
-        val = fma(nf, grad_face(A.Gv[f], pl, A.Gv[NV + f], pr), val);
-      }
-      A.v[f] = val;
-    } else if (t < NU + NV + NW) {
-      const long f = t - NU - NV;
-      double val = A.wt[f];
-      if (A.fw[f] & kQFace) {
-        const long plane = (long)d.nx * d.ny;
-        const int k = (int)(f / plane);
-        const long c = f - (long)k * plane;
-        const double pl = k > 0 ? phi_at(A, c + (long)(k - 1) * plane) : 0.0;
-        const double pr = k < d.nz ? phi_at(A, c + (long)k * plane) : 0.0;
-        val = fma(nf, grad_face(A.Gw[f], pl, A.Gw[NW + f], pr), val);
-      }
-      A.w[f] = val;
-    } else {
-      const long c = t - NU - NV - NW;
-      bad |= !isfinite(A.phi[c]);
-      if (A.fc[c] & kFluid) A.p[c] = __dadd_rn(A.p[c], A.phi[c]);
-    }
+  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
+  // One loop per field. The common face reads its flag, its value and the two
+  // phi and nothing else (no G pair, no cell flags), and none of its loads
+  // waits for another but the flag. 640x128x128: 519 -> 390 us, bound by HBM
+  // (8.6 values a cell) and three FP64 operations a face.
+  auto face = [&](uint8_t fl, double val, int f, long lo, long hi, bool has_lo, bool has_hi, const double *G, long NF,
+                  long g) {
+    if (fl & kPlainFace) return fma(nf, grad_face(A.plain.gl[f], A.phi[lo], A.plain.gr[f], A.phi[hi]), val);
+    if (!(fl & kQFace)) return val;
+    const double pl = has_lo ? phi_at(A, lo) : 0.0, pr = has_hi ? phi_at(A, hi) : 0.0;
+    return fma(nf, grad_face(G[g], pl, G[NF + g], pr), val);
+  };
+  for (long f = t0; f < NU; f += ts) {
+    const uint8_t fl = A.fu[f];
+    const double val = A.ut[f];
+    long q;
+    const int i = udivmod(f, d.dnx1, q);
+    const long c = q * d.nx + i;  // cell i of the face's line
+    A.u[f] = face(fl, val, 0, c - 1, c, i > 0, i < d.nx, A.Gu, NU, f);
+  }
+  for (long f = t0; f < NV; f += ts) {
+    const uint8_t fl = A.fv[f];
+    const double val = A.vt[f];
+    long q;
+    const int i = udivmod(f, d.dnx, q);
+    long kq;
+    const int j = udivmod(q, d.dny1, kq), k = (int)kq;
+    const long c = P3(d, i, j, k);
+    A.v[f] = face(fl, val, 1, c - d.nx, c, j > 0, j < d.ny, A.Gv, NV, f);
+  }
+  const long plane = (long)d.nx * d.ny;
+  for (long f = t0; f < NW; f += ts) {
+    const uint8_t fl = A.fw[f];
+    const double val = A.wt[f];
+    A.w[f] = face(fl, val, 2, f - plane, f, f >= plane, f < NP, A.Gw, NW, f);
+  }
+  for (long c = t0; c < NP; c += ts) {
+    const double phi = A.phi[c];
+    bad |= !isfinite(phi);
+    if (A.fc[c] & kFluid) A.p[c] = __dadd_rn(A.p[c], phi);
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&A.dg->nonfinite_p, 1);
 }
@@ -531,6 +575,7 @@ struct DiagArgs {
   double *part;
   StepDiag *dg;
   int np_active;
+  Plain plain;
 };
 
 // Corrected q value of a face: the projected field holds it (k_project
@@ -583,45 +628,57 @@ __device__ __noinline__ void boundary_q(const DiagArgs &A, long c, int i, int j,
 
 __global__ void __launch_bounds__(kThreads, 4) k_diagnostics(DiagArgs A) {
   const Dims &d = A.d;
-  const long NU = (long)(d.nx + 1) * d.ny * d.nz, NV = (long)d.nx * (d.ny + 1) * d.nz,
-             NW = (long)d.nx * d.ny * (d.nz + 1), NP = (long)d.nx * d.ny * d.nz;
+  const long NP = (long)d.nx * d.ny * d.nz;
   double div2 = 0.0;
   unsigned long long um = 0, vm = 0, wm = 0;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < NP + NU + NV + NW; t += (long)gridDim.x * blockDim.x) {
-    if (t < NP) {
-      const long c = t;
-      if (!(A.fc[c] & kFluid)) continue;
-      long q;
-      const int i = udivmod(c, d.dnx, q);
-      long kq;
-      const int j = udivmod(q, d.dny, kq), k = (int)kq;
-      const long fw_ = U3(d, i, j, k), fe = U3(d, i + 1, j, k), fs = V3(d, i, j, k), fn = V3(d, i, j + 1, k),
-                 fb = W3(d, i, j, k), ft = W3(d, i, j, k + 1);
-      double qw, qe, qs, qn, qb, qt;
-      if (!((A.fu[fw_] | A.fu[fe] | A.fv[fs] | A.fv[fn] | A.fw[fb] | A.fw[ft]) & kBcSet)) {
-        // interior cell: the six corrected values are the projected field
-        qw = (A.fu[fw_] & kQFace) ? A.u[fw_] : 0.0;
-        qe = (A.fu[fe] & kQFace) ? A.u[fe] : 0.0;
-        qs = (A.fv[fs] & kQFace) ? A.v[fs] : 0.0;
-        qn = (A.fv[fn] & kQFace) ? A.v[fn] : 0.0;
-        qb = (A.fw[fb] & kQFace) ? A.w[fb] : 0.0;
-        qt = (A.fw[ft] & kQFace) ? A.w[ft] : 0.0;
+  // Each cell reads its six faces: their magnitudes (the lower three, and the
+  // upper ones on the last planes, so that every face is taken once or more),
+  // and for fluid cells their divergence. The common cell needs nothing else.
+  const long plane = (long)d.nx * d.ny;
+  auto top = [](unsigned long long &m, double x) {
+    const unsigned long long key = mag_key(x);
+    m = key > m ? key : m;
+  };
+  for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < NP; c += (long)gridDim.x * blockDim.x) {
+    const uint8_t fl = A.fc[c];
+    long q;
+    const int i = udivmod(c, d.dnx, q);
+    long kq;
+    const int j = udivmod(q, d.dny, kq), k = (int)kq;
+    const long fw_ = U3(d, i, j, k), fe = fw_ + 1, fs = V3(d, i, j, k), fn = fs + d.nx, fb = c, ft = c + plane;
+    double qw = A.u[fw_], qe = A.u[fe], qs = A.v[fs], qn = A.v[fn], qb = A.w[fb], qt = A.w[ft];
+    top(um, qw); top(vm, qs); top(wm, qb);
+    if (i == d.nx - 1) top(um, qe);
+    if (j == d.ny - 1) top(vm, qn);
+    if (k == d.nz - 1) top(wm, qt);
+    if (!(fl & kFluid)) continue;
+    double s, lift;
+    if (fl & kPlainCell) {
+      s = fma(A.plain.D[0], qw, 0.0);
+      s = fma(A.plain.D[1], qe, s);
+      s = fma(A.plain.D[2], qs, s);
+      s = fma(A.plain.D[3], qn, s);
+      s = fma(A.plain.D[4], qb, s);
+      s = fma(A.plain.D[5], qt, s);
+      lift = 0.0;
+    } else {
+      const uint8_t mw = A.fu[fw_], me = A.fu[fe], ms = A.fv[fs], mn = A.fv[fn], mb = A.fw[fb], mt = A.fw[ft];
+      if (!((mw | me | ms | mn | mb | mt) & kBcSet)) {
+        // the six corrected values are the projected field
+        qw = (mw & kQFace) ? qw : 0.0;
+        qe = (me & kQFace) ? qe : 0.0;
+        qs = (ms & kQFace) ? qs : 0.0;
+        qn = (mn & kQFace) ? qn : 0.0;
+        qb = (mb & kQFace) ? qb : 0.0;
+        qt = (mt & kQFace) ? qt : 0.0;
       } else {
         boundary_q(A, c, i, j, k, qw, qe, qs, qn, qb, qt);
       }
-      const double s = div_cell(A.Dc, NP, c, qw, qe, qs, qn, qb, qt);
-      const double dv = __dadd_rn(s, __dmul_rn(*A.ramp, A.div_bc[c]));
-      div2 = __dadd_rn(div2, __dmul_rn(dv, dv));
-    } else if (t < NP + NU) {
-      const unsigned long long m = mag_key(A.u[t - NP]);
-      um = m > um ? m : um;
-    } else if (t < NP + NU + NV) {
-      const unsigned long long m = mag_key(A.v[t - NP - NU]);
-      vm = m > vm ? m : vm;
-    } else {
-      const unsigned long long m = mag_key(A.w[t - NP - NU - NV]);
-      wm = m > wm ? m : wm;
+      s = div_cell(A.Dc, NP, c, qw, qe, qs, qn, qb, qt);
+      lift = A.div_bc[c];
     }
+    const double dv = __dadd_rn(s, __dmul_rn(*A.ramp, lift));
+    div2 = __dadd_rn(div2, __dmul_rn(dv, dv));
   }
   __shared__ double s_div[kWarps];
   __shared__ unsigned long long s_max[3][kWarps];
@@ -685,6 +742,61 @@ __global__ void __launch_bounds__(kThreads, 4) k_diagnostics(DiagArgs A) {
   }
 }
 
+// ------------------------------------------------------------------ plain flags
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+// n_samples records of W values, value w of record r at a[w * ld + r], spread over n records.
+__global__ void k_sample(const double *a, long ld, const double *a2, int W, long n, int samples, double *out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= samples) return;
+  const long r = (long)((double)n * (t + 0.5) / samples);
+  for (int w = 0; w < W; ++w) out[(long)t * W + w] = a2 && w == 1 ? a2[r] : a[w * ld + r];
+}
+// kPlainFace of one field's faces. d3: the direction of the field; the cells
+// below and above a face (none outside the box).
+__global__ void k_mark_faces(uint8_t *fl, const uint8_t *fc, const double *G, long NF, Dims d, int d3, double gl,
+                             double gr) {
+  for (long f = (long)blockIdx.x * blockDim.x + threadIdx.x; f < NF; f += (long)gridDim.x * blockDim.x) {
+    long q, kq;
+    const int i = udivmod(f, d3 == 0 ? d.dnx1 : d.dnx, q);
+    const int j = udivmod(q, d3 == 1 ? d.dny1 : d.dny, kq), k = (int)kq;
+    const int x = d3 == 0 ? i : d3 == 1 ? j : k, nd = d3 == 0 ? d.nx : d3 == 1 ? d.ny : d.nz;
+    uint8_t v = fl[f] & (uint8_t)~kPlainFace;
+    if ((v & kQFace) && x > 0 && x < nd && same_bits(G[f], gl) && same_bits(G[NF + f], gr)) {
+      const long hi = P3(d, i, j, k), lo = hi - (d3 == 0 ? 1 : d3 == 1 ? d.nx : (long)d.nx * d.ny);
+      if ((fc[lo] & kFluid) && (fc[hi] & kFluid)) v |= kPlainFace;
+    }
+    fl[f] = v;
+  }
+}
+// kPlainRow of one field's solve-box rows.
+__global__ void k_mark_rows(uint8_t *fl, const double *sc, const double *bc, long n, Dims d, int d3, double s, double b) {
+  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
+    long q, kq;
+    const int i = udivmod(r, d3 == 0 ? d.dnxm : d.dnx, q) + (d3 == 0);
+    const int j = udivmod(q, d3 == 1 ? d.dnym : d.dny, kq) + (d3 == 1), k = (int)kq + (d3 == 2);
+    const long f = d3 == 0 ? U3(d, i, j, k) : d3 == 1 ? V3(d, i, j, k) : W3(d, i, j, k);
+    const bool same = same_bits(sc[r], s) && same_bits(bc[r], b);
+    fl[f] = (uint8_t)((fl[f] & ~kPlainRow) | (same ? kPlainRow : 0));
+  }
+}
+// kPlainCell. Cells of the inlet column never are: ibm_set_inflow rewrites their lift.
+__global__ void k_mark_cells(uint8_t *fc, const uint8_t *fu, const uint8_t *fv, const uint8_t *fw, const double *Dc,
+                             const double *div_bc, Dims d, Plain p) {
+  const long NP = (long)d.nx * d.ny * d.nz;
+  for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < NP; c += (long)gridDim.x * blockDim.x) {
+    long q, kq;
+    const int i = udivmod(c, d.dnx, q);
+    const int j = udivmod(q, d.dny, kq), k = (int)kq;
+    const long fs = V3(d, i, j, k), ft = c + (long)d.nx * d.ny;
+    const uint8_t f[6] = {fu[U3(d, i, j, k)], fu[U3(d, i + 1, j, k)], fv[fs], fv[fs + d.nx], fw[c], fw[ft]};
+    bool plain = (fc[c] & kFluid) && i > 0 && same_bits(div_bc[c], 0.0);
+    for (int s = 0; s < 6; ++s) plain = plain && (f[s] & kQFace) && !(f[s] & kBcSet) && same_bits(Dc[s * NP + c], p.D[s]);
+    fc[c] = (uint8_t)((fc[c] & ~kPlainCell) | (plain ? kPlainCell : 0));
+  }
+}
+
 Dims dims_of(const ibm_ctx *c) {
   Dims d;
   d.nx = c->g.nx; d.ny = c->g.ny; d.nz = c->g.nz;
@@ -738,8 +850,69 @@ void ensure_rhs_df(ibm_ctx *c) {
   c->df_u.alloc(c->g.NU); c->df_v.alloc(c->g.NV); c->df_w.alloc(c->g.NW); c->df_p.alloc(c->g.NP);
 }
 
+// The record (W values) that appears most often among a sample of n records;
+// records of zeros only when there are no others.
+static void common_record(ibm_ctx *c, const double *a, long ld, const double *a2, int W, long n, double *out) {
+  constexpr int kSamples = 512;
+  for (int w = 0; w < W; ++w) out[w] = 0.0;
+  if (n <= 0) return;
+  DBuf<double> d;
+  d.alloc((size_t)kSamples * W);
+  {
+    LaunchScope ls(K_SETUP, c->st, 0.0);
+    k_sample<<<(kSamples + kThreads - 1) / kThreads, kThreads, 0, c->st>>>(a, ld, a2, W, n, kSamples, d.p);
+  }
+  std::vector<double> h((size_t)kSamples * W);
+  IBM_CUDA_TRY(cudaMemcpyAsync(h.data(), d.p, d.bytes(), cudaMemcpyDeviceToHost, c->st));
+  IBM_CUDA_TRY(cudaStreamSynchronize(c->st));
+  std::map<std::vector<uint64_t>, int> count;
+  std::vector<uint64_t> key((size_t)W), best;
+  int most = 0;
+  for (int t = 0; t < kSamples; ++t) {
+    bool zero = true;
+    for (int w = 0; w < W; ++w) {
+      memcpy(&key[(size_t)w], &h[(size_t)t * W + w], 8);
+      zero = zero && h[(size_t)t * W + w] == 0.0;
+    }
+    if (!zero && ++count[key] > most) { most = count[key]; best = key; }
+  }
+  if (most > 0) memcpy(out, best.data(), 8 * (size_t)W);
+}
+
+void ensure_plain(ibm_ctx *c) {
+  if (c->plain_ready) return;
+  const Geometry &g = c->g;
+  const Dims d = dims_of(c);
+  uint8_t *fl[3] = {c->fu.p, c->fv.p, c->fw.p};
+  const double *G[3] = {c->Gu.p, c->Gv.p, c->Gw.p};
+  const long NF[3] = {g.NU, g.NV, g.NW};
+  const Box *box[3] = {&g.bu, &g.bv, &g.bw};
+  Plain &p = c->plain;
+  for (int f = 0; f < 3; ++f) {
+    double r[2];
+    common_record(c, G[f], NF[f], nullptr, 2, NF[f], r);
+    p.gl[f] = r[0]; p.gr[f] = r[1];
+    common_record(c, c->scale_box[f].p, 0, c->bc_box[f].p, 2, box[f]->n, r);
+    p.sc[f] = r[0]; p.bc[f] = r[1];
+    LaunchScope ls(K_SETUP, c->st, 0.0, 2);
+    k_mark_faces<<<blocks_for(NF[f]), kThreads, 0, c->st>>>(fl[f], c->fc.p, G[f], NF[f], d, f, p.gl[f], p.gr[f]);
+    k_mark_rows<<<blocks_for(box[f]->n), kThreads, 0, c->st>>>(fl[f], c->scale_box[f].p, c->bc_box[f].p, box[f]->n, d, f,
+                                                              p.sc[f], p.bc[f]);
+  }
+  common_record(c, c->Dc.p, g.NP, nullptr, 6, g.NP, p.D);
+  {
+    LaunchScope ls(K_SETUP, c->st, 0.0);
+    k_mark_cells<<<blocks_for(g.NP), kThreads, 0, c->st>>>(c->fc.p, fl[0], fl[1], fl[2], c->Dc.p, c->div_bc_cell.p, d, p);
+  }
+  IBM_CUDA_TRY(cudaStreamSynchronize(c->st));
+  IBM_CUDA_TRY(cudaGetLastError());
+  c->graph_ready = false;  // a captured step holds the coefficients in its kernels' parameters
+  c->plain_ready = true;
+}
+
 void launch_momentum_rhs(ibm_ctx *c) {
   RhsArgs A;
+  A.plain = c->plain;
   A.d = dims_of(c);
   A.u = c->u.p; A.v = c->v.p; A.w = c->w.p; A.p = c->p.p;
   A.fu = c->fu.p; A.fv = c->fv.p; A.fw = c->fw.p; A.fc = c->fc.p;
@@ -763,7 +936,7 @@ void launch_momentum_rhs(ibm_ctx *c) {
   A.da = split(A.a); A.drho = split(A.rho);
   A.drx = split(1.0 / (2 * c->g.dx)); A.dry = split(1.0 / (2 * c->g.dy)); A.drz = split(1.0 / (2 * c->g.dz));
   const double faces = (double)(c->g.NU + c->g.NV + c->g.NW), nbox = (double)(A.nb[0] + A.nb[1] + A.nb[2]);
-  const long rows = A.nb[0] + A.nb[1] + A.nb[2];
+  const long rows = std::max(std::max(A.nb[0], A.nb[1]), A.nb[2]);  // of the longest of the three loops
   if (momentum_rhs_df(c->prm)) {
     if (!c->df_u.p || !c->df_v.p || !c->df_w.p || !c->df_p.p)
       throw Error(IBM_ERR_STATE, "double-float field copies not allocated");
@@ -941,10 +1114,11 @@ void launch_projection(ibm_ctx *c) {
   A.Gu = c->Gu.p; A.Gv = c->Gv.p; A.Gw = c->Gw.p;
   A.factor = c->g.dt / c->g.rho;
   A.dg = c->diag.p;
+  A.plain = c->plain;
   const double faces = (double)(c->g.NU + c->g.NV + c->g.NW);
   {
     LaunchScope ls(K_PROJECT, c->st, 33.0 * faces + 25.0 * c->g.NP);
-    k_project<<<wave_blocks(k_project, c->g.NU + c->g.NV + c->g.NW + c->g.NP), kThreads, 0, c->st>>>(A);
+    k_project<<<wave_blocks(k_project, std::max(std::max(c->g.NU, c->g.NV), c->g.NW)), kThreads, 0, c->st>>>(A);
   }
   launch_bc(c, c->u.p, c->v.p, c->w.p);
   DiagArgs D;
@@ -954,9 +1128,10 @@ void launch_projection(ibm_ctx *c) {
   D.fu = c->fu.p; D.fv = c->fv.p; D.fw = c->fw.p; D.fc = c->fc.p;
   D.Gu = c->Gu.p; D.Gv = c->Gv.p; D.Gw = c->Gw.p; D.Dc = c->Dc.p; D.div_bc = c->div_bc_cell.p;
   D.factor = A.factor;
+  D.plain = c->plain;
   D.ramp = c->dramp.p;
   // one wave: four resident blocks per SM (launch bounds), at most the 1024 partials of c->part
-  const int nb = std::min(std::min(blocks_for(c->g.NP + c->g.NU + c->g.NV + c->g.NW), 4 * sm_count()), 1024);
+  const int nb = std::min(std::min(blocks_for(c->g.NP), 4 * sm_count()), 1024);
   D.part = c->part.p;
   D.dg = c->diag.p;
   D.np_active = c->np_active;

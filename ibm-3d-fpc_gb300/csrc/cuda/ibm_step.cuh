@@ -11,6 +11,8 @@ void launch_momentum_rhs(ibm_ctx *c);
 // (df_rhs); its field copies are allocated outside any graph capture.
 bool momentum_rhs_df(const ibm_solver_params &p);
 void ensure_rhs_df(ibm_ctx *c);
+// Derives the kPlain* flags when an input changed (outside any graph capture).
+void ensure_plain(ibm_ctx *c);
 void launch_tilde(ibm_ctx *c);
 void launch_pressure_rhs(ibm_ctx *c);
 void launch_projection(ibm_ctx *c);
