@@ -1793,8 +1793,16 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 // Blocks of the dense level's solve: one warp per row.
 int dense_grid(long n) { return std::max(1, (int)std::min<long>((n + 7) / 8, (long)sm_count() * 4)); }
 
+// Threads per block of the V-cycle's kernels over n items. With fewer than
+// kThreads items per SM a small level is spread over more SMs in blocks of 64:
+// an FP64 multiply-add takes a warp 64 clocks on its quarter of an SM, so a
+// 27-point phase of 1280 points in five blocks of 256 took 5.4 us, two thirds
+// of it waiting for 40 warps' FP64 work on five SMs; 4.9 in twenty of 64.
+int block_of(long n) { return n <= (long)kThreads * sm_count() ? 64 : kThreads; }
+
 int grid_for(long n) {
-  long b = (n + kThreads - 1) / kThreads;
+  const int t = block_of(n);
+  long b = (n + t - 1) / t;
   const long cap = (long)sm_count() * 8;
   if (b > cap) b = cap;
   return (int)std::max(1L, b);
@@ -1803,7 +1811,10 @@ int grid_for(long n) {
 // One thread per element for the V-cycle's streaming kernels: every block
 // retires after one element per thread, so the GPU keeps many independent
 // loads in flight without a serial loop per thread.
-int grid_all(long n) { return (int)std::max(1L, std::min((n + kThreads - 1) / kThreads, 1L << 30)); }
+int grid_all(long n) {
+  const int t = block_of(n);
+  return (int)std::max(1L, std::min((n + t - 1) / t, 1L << 30));
+}
 
 // Blocks for a grid-stride kernel over n items: one per kThreads items, at
 // most as many as stay resident (one wave). A resident grid loops over its
@@ -1826,7 +1837,8 @@ int resident_grid(K kernel, long n) {
     std::lock_guard<std::mutex> lock(mu);
     cache[(const void *)kernel] = per_sm;
   }
-  return (int)std::min<long>(grid_all(n), (long)per_sm * sm_count());
+  const int all = grid_all(n);
+  return block_of(n) < kThreads ? all : (int)std::min<long>(all, (long)per_sm * sm_count());
 }
 
 // Blocks of k_relax_rb_sweep: one tile each, at most as many as stay resident.
@@ -1902,8 +1914,8 @@ static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
   R.alloc((size_t)W * F.b.n);
   {
     LaunchScope ls(K_SETUP, st, 0.0);
-    if (F.ns == 7) k_split_colors<T><<<grid_for(F.b.n), kThreads, 0, st>>>(F.A, F.invd.p, F.b, R.p);
-    else k_split_colors27<T><<<grid_for(F.b.n), kThreads, 0, st>>>(F.A, F.invd.p, F.b, R.p);
+    if (F.ns == 7) k_split_colors<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p);
+    else k_split_colors27<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p);
   }
   if (prm.classes && build_classes<T>(st, R.p, W, F.b.n, F.rbc)) {
     R.release();
@@ -1941,7 +1953,7 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
     L[0].Aown.alloc((size_t)7 * b0.n);
     {
       LaunchScope ls(K_SETUP, st, 0.0);
-      k_scale_rows<<<grid_for(7 * b0.n), kThreads, 0, st>>>(A7, winv_, b0.n, L[0].Aown.p);
+      k_scale_rows<<<grid_for(7 * b0.n), block_of(7 * b0.n), 0, st>>>(A7, winv_, b0.n, L[0].Aown.p);
     }
     L[0].A = L[0].Aown.p;
   }
@@ -1957,7 +1969,7 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
     const double *diag = F.A + (F.ns == 27 ? 13L * n : 0L);
     {
       LaunchScope ls(K_SETUP, st, 0.0);
-      k_diag<<<grid_for(n), kThreads, 0, st>>>(diag, n, prm.omega, F.invd.p, F.wd.p);
+      k_diag<<<grid_for(n), block_of(n), 0, st>>>(diag, n, prm.omega, F.invd.p, F.wd.p);
     }
     split_colors(st, F, prm);
     const int dims[3] = {F.b.nx, F.b.ny, F.b.nz};
@@ -2005,8 +2017,8 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
     coupled.alloc(n);
     {
       LaunchScope ls(K_SETUP, st, 0.0);
-      k_coupled<<<grid_for(n), kThreads, 0, st>>>(F.A, F.ns, n, coupled.p);
-      k_interp_weights<<<grid_for(n), kThreads, 0, st>>>(F.A, F.ns, F.b, d, coupled.p, aware, F.pm.p, F.pp.p);
+      k_coupled<<<grid_for(n), block_of(n), 0, st>>>(F.A, F.ns, n, coupled.p);
+      k_interp_weights<<<grid_for(n), block_of(n), 0, st>>>(F.A, F.ns, F.b, d, coupled.p, aware, F.pm.p, F.pp.p);
     }
     const Box cb = make_box(d == 0 ? (F.b.nx + 1) / 2 : F.b.nx, d == 1 ? (F.b.ny + 1) / 2 : F.b.ny,
                             d == 2 ? (F.b.nz + 1) / 2 : F.b.nz);
@@ -2018,7 +2030,7 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
     a27.alloc((size_t)27 * cb.n);
     {
       LaunchScope ls(K_SETUP, st, 0.0);
-      k_rap<<<grid_for(cb.n), kThreads, 0, st>>>(Fr.A, Fr.ns, Fr.b, Fr.pm.p, Fr.pp.p, d, cb, a27.p);
+      k_rap<<<grid_for(cb.n), block_of(cb.n), 0, st>>>(Fr.A, Fr.ns, Fr.b, Fr.pm.p, Fr.pp.p, d, cb, a27.p);
     }
     if (prm.rap == 1) {
       C.Aown.alloc((size_t)7 * cb.n);
@@ -2026,8 +2038,8 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
       ccoupled.alloc(cb.n);
       {
         LaunchScope ls(K_SETUP, st, 0.0);
-        k_coupled<<<grid_for(cb.n), kThreads, 0, st>>>(a27.p, 27, cb.n, ccoupled.p);
-        k_collapse7<<<grid_for(cb.n), kThreads, 0, st>>>(a27.p, cb, ccoupled.p, aware, C.Aown.p);
+        k_coupled<<<grid_for(cb.n), block_of(cb.n), 0, st>>>(a27.p, 27, cb.n, ccoupled.p);
+        k_collapse7<<<grid_for(cb.n), block_of(cb.n), 0, st>>>(a27.p, cb, ccoupled.p, aware, C.Aown.p);
       }
       IBM_CUDA_TRY(cudaStreamSynchronize(st));
       C.ns = 7;
@@ -2054,7 +2066,7 @@ void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const flo
   if (winv) {
     winvf_.alloc(b.n);
     LaunchScope ls(K_SETUP, st, 0.0);
-    k_convert<float><<<grid_for(b.n), kThreads, 0, st>>>(winv, winvf_.p, b.n);
+    k_convert<float><<<grid_for(b.n), block_of(b.n), 0, st>>>(winv, winvf_.p, b.n);
   }
   (void)fp64;
   build<double>(st, L64, b, A7, h);
@@ -2538,14 +2550,14 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
           const bool z = zero && color == 0;
           if (z && fin) {
             LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? 2.0 : T_) + (winvf ? 4.0 : 3.0) * T_ * n);
-            k_relax_rb_quad_in<<<resident_grid(k_relax_rb_quad_in, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, *fin, winvf, gate);
+            k_relax_rb_quad_in<<<resident_grid(k_relax_rb_quad_in, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, *fin, winvf, gate);
           } else if (color == 1 && last && fout) {
             LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 2.5 * T_ * n);
-            k_relax_rb_quad_out<<<resident_grid(k_relax_rb_quad_out, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, 1, *fout, gate);
+            k_relax_rb_quad_out<<<resident_grid(k_relax_rb_quad_out, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, 1, *fout, gate);
           } else {
             LaunchScope ls(K_MG_RELAX_FINE, st, z ? 0.5 * n * (R7.code ? 2.0 : T_) + 1.5 * T_ * n
                                                   : 0.5 * n * rec7 + 1.5 * T_ * n);
-            k_relax_rb_quad<<<resident_grid(k_relax_rb_quad, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, color, z, gate);
+            k_relax_rb_quad<<<resident_grid(k_relax_rb_quad, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, color, z, gate);
           }
         }
         return;
@@ -2555,11 +2567,11 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
       {
         LaunchScope ls(K_MG_RELAX_FINE, st, zero ? 0.5 * n * (R7.code ? 2.0 : T_) + 1.5 * T_ * n
                                                  : 0.5 * n * rec7 + 1.5 * T_ * n);
-        if (zero) k_relax_rb_zero<T><<<grid_all(h), kThreads, 0, st>>>(R7, F.bv.p, cur, F.b, gate);
-        else k_relax_rb<T><<<grid_all(h), kThreads, 0, st>>>(R7, F.bv.p, cur, F.b, 0, gate);
+        if (zero) k_relax_rb_zero<T><<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, gate);
+        else k_relax_rb<T><<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, 0, gate);
       }
       LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 1.5 * T_ * n);
-      k_relax_rb<T><<<grid_all(h), kThreads, 0, st>>>(R7, F.bv.p, cur, F.b, 1, gate);
+      k_relax_rb<T><<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, 1, gate);
     } else if (p.relax == 2 && rb27) {
       for (int color = 0; color < 2; ++color) {
         const bool z = zero && color == 0;
@@ -2568,28 +2580,28 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
         bool done = false;
         if constexpr (sizeof(T) == 4) {
           if (p.quads && F.b.nx % 4 == 0) {
-            k_relax_rb27_quad<<<resident_grid(k_relax_rb27_quad, n / 4), kThreads, 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
+            k_relax_rb27_quad<<<resident_grid(k_relax_rb27_quad, n / 4), block_of(n / 4), 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
             done = true;
           }
         }
-        if (!done) k_relax_rb27<T><<<grid_all(h), kThreads, 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
+        if (!done) k_relax_rb27<T><<<grid_all(h), block_of(h), 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
         std::swap(cur, oth);
       }
     } else if (p.relax == 2) {
       for (int color = 0; color < 2; ++color) {
         const bool z = zero && color == 0;
         LaunchScope ls(K_MG_RELAX, st, z ? 3.0 * T_ * n : sweep_bytes);
-        if (F.ns == 7) k_relax_color<T, 7><<<g, kThreads, 0, st>>>(F.A, F.invd.p, F.bv.p, cur, oth, F.b, color, z, gate);
-        else k_relax_color<T, 27><<<g, kThreads, 0, st>>>(F.A, F.invd.p, F.bv.p, cur, oth, F.b, color, z, gate);
+        if (F.ns == 7) k_relax_color<T, 7><<<g, block_of(n), 0, st>>>(F.A, F.invd.p, F.bv.p, cur, oth, F.b, color, z, gate);
+        else k_relax_color<T, 27><<<g, block_of(n), 0, st>>>(F.A, F.invd.p, F.bv.p, cur, oth, F.b, color, z, gate);
         std::swap(cur, oth);
       }
     } else if (zero) {
       LaunchScope ls(K_MG_RELAX, st, 3.0 * T_ * n);
-      k_relax_zero<T><<<g, kThreads, 0, st>>>(F.wd.p, F.bv.p, cur, n, gate);
+      k_relax_zero<T><<<g, block_of(n), 0, st>>>(F.wd.p, F.bv.p, cur, n, gate);
     } else {
       LaunchScope ls(K_MG_RELAX, st, sweep_bytes);
-      if (F.ns == 7) k_relax_jacobi<T, 7><<<g, kThreads, 0, st>>>(F.A, F.wd.p, F.bv.p, cur, oth, F.b, gate);
-      else k_relax_jacobi<T, 27><<<g, kThreads, 0, st>>>(F.A, F.wd.p, F.bv.p, cur, oth, F.b, gate);
+      if (F.ns == 7) k_relax_jacobi<T, 7><<<g, block_of(n), 0, st>>>(F.A, F.wd.p, F.bv.p, cur, oth, F.b, gate);
+      else k_relax_jacobi<T, 27><<<g, block_of(n), 0, st>>>(F.A, F.wd.p, F.bv.p, cur, oth, F.b, gate);
       std::swap(cur, oth);
     }
   };
@@ -2606,27 +2618,27 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
     bool done = false;
     if constexpr (sizeof(T) == 4) {
       if (quad) {
-        k_residual_rb_quad<<<resident_grid(k_residual_rb_quad, n / 4), kThreads, 0, st>>>(R7, U7, Q, F.bv.p, cur, F.r.p, F.b, gate);
+        k_residual_rb_quad<<<resident_grid(k_residual_rb_quad, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.r.p, F.b, gate);
         done = true;
       }
     }
-    if (!done) k_residual_rb<T><<<grid_all(n / 2), kThreads, 0, st>>>(R7, F.bv.p, cur, F.r.p, F.b, gate);
+    if (!done) k_residual_rb<T><<<grid_all(n / 2), block_of(n / 2), 0, st>>>(R7, F.bv.p, cur, F.r.p, F.b, gate);
     res = F.r.p;
   } else if (nu1 > 0 && p.relax == 2 && rb27) {
     LaunchScope ls(K_MG_RESID, st, n * rec27 + 3.0 * T_ * n);
     bool done = false;
     if constexpr (sizeof(T) == 4) {
       if (p.quads && F.b.nx % 4 == 0) {
-        k_residual_rb27_quad<<<resident_grid(k_residual_rb27_quad, n / 4), kThreads, 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
+        k_residual_rb27_quad<<<resident_grid(k_residual_rb27_quad, n / 4), block_of(n / 4), 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
         done = true;
       }
     }
-    if (!done) k_residual_rb27<T><<<grid_all(n), kThreads, 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
+    if (!done) k_residual_rb27<T><<<grid_all(n), block_of(n), 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
     res = F.r.p;
   } else if (nu1 > 0) {
     LaunchScope ls(K_MG_RESID, st, T_ * n * (F.ns + 3.0));
-    if (F.ns == 7) k_residual<T, 7><<<grid_all(n), kThreads, 0, st>>>(F.A, F.bv.p, cur, F.r.p, F.b, gate);
-    else k_residual<T, 27><<<grid_all(n), kThreads, 0, st>>>(F.A, F.bv.p, cur, F.r.p, F.b, gate);
+    if (F.ns == 7) k_residual<T, 7><<<grid_all(n), block_of(n), 0, st>>>(F.A, F.bv.p, cur, F.r.p, F.b, gate);
+    else k_residual<T, 27><<<grid_all(n), block_of(n), 0, st>>>(F.A, F.bv.p, cur, F.r.p, F.b, gate);
     res = F.r.p;
   }
   // the stages of this level's coarsening group, up to where a fused part begins
@@ -2639,18 +2651,18 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
     // a group reads the level once and writes the group's last level (the weights of the levels between: n)
     LaunchScope ls(K_MG_RESTRICT, st, T_ * ((G.n > 1 ? 2.0 : 3.0) * n + C.b.n));
     if (G.n == 3)
-      k_restrict_group<T, 3><<<resident_grid(k_restrict_group<T, 3>, C.b.n), kThreads, 0, st>>>(G, res, C.bv.p, gate);
+      k_restrict_group<T, 3><<<resident_grid(k_restrict_group<T, 3>, C.b.n), block_of(C.b.n), 0, st>>>(G, res, C.bv.p, gate);
     else if (G.n == 2)
-      k_restrict_group<T, 2><<<resident_grid(k_restrict_group<T, 2>, C.b.n), kThreads, 0, st>>>(G, res, C.bv.p, gate);
+      k_restrict_group<T, 2><<<resident_grid(k_restrict_group<T, 2>, C.b.n), block_of(C.b.n), 0, st>>>(G, res, C.bv.p, gate);
     else if constexpr (sizeof(T) == 4) {
       if (F.cdir != 0 && F.b.nx % 4 == 0)
-        k_restrict_yz4<<<resident_grid(k_restrict_yz4, C.b.n / 4), kThreads, 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
+        k_restrict_yz4<<<resident_grid(k_restrict_yz4, C.b.n / 4), block_of(C.b.n / 4), 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
       else if (p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0)
-        k_restrict_x4<<<resident_grid(k_restrict_x4, C.b.n / 4), kThreads, 0, st>>>(res, F.pm.p, F.pp.p, F.b, C.bv.p, C.b, gate);
+        k_restrict_x4<<<resident_grid(k_restrict_x4, C.b.n / 4), block_of(C.b.n / 4), 0, st>>>(res, F.pm.p, F.pp.p, F.b, C.bv.p, C.b, gate);
       else
-        k_restrict<T><<<grid_all(C.b.n), kThreads, 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
+        k_restrict<T><<<grid_all(C.b.n), block_of(C.b.n), 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
     } else {
-      k_restrict<T><<<grid_all(C.b.n), kThreads, 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
+      k_restrict<T><<<grid_all(C.b.n), block_of(C.b.n), 0, st>>>(res, F.pm.p, F.pp.p, F.b, F.cdir, C.bv.p, C.b, gate);
     }
   }
   T *xc = nullptr;
@@ -2663,18 +2675,18 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   {
     LaunchScope ls(K_MG_PROLONG, st, T_ * ((nu1 > 0 ? 4.0 : 3.0) * n + C.b.n));
     if (G.n == 3)
-      k_prolong_group<T, 3><<<resident_grid(k_prolong_group<T, 3>, n), kThreads, 0, st>>>(G, xc, cur, nu1 > 0, gate);
+      k_prolong_group<T, 3><<<resident_grid(k_prolong_group<T, 3>, n), block_of(n), 0, st>>>(G, xc, cur, nu1 > 0, gate);
     else if (G.n == 2)
-      k_prolong_group<T, 2><<<resident_grid(k_prolong_group<T, 2>, n), kThreads, 0, st>>>(G, xc, cur, nu1 > 0, gate);
+      k_prolong_group<T, 2><<<resident_grid(k_prolong_group<T, 2>, n), block_of(n), 0, st>>>(G, xc, cur, nu1 > 0, gate);
     else if constexpr (sizeof(T) == 4) {
       if (F.cdir != 0 && F.b.nx % 4 == 0)
-        k_prolong_yz4<<<resident_grid(k_prolong_yz4, n / 4), kThreads, 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
+        k_prolong_yz4<<<resident_grid(k_prolong_yz4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
       else if (p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0)
-        k_prolong_x4<<<resident_grid(k_prolong_x4, n / 4), kThreads, 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, cur, nu1 > 0, gate);
+        k_prolong_x4<<<resident_grid(k_prolong_x4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, cur, nu1 > 0, gate);
       else
-        k_prolong<T><<<grid_all(n), kThreads, 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
+        k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
     } else {
-      k_prolong<T><<<grid_all(n), kThreads, 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
+      k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
     }
   }
   for (int s = 0; s < nu2; ++s) relax(false, s == nu2 - 1);
@@ -2717,15 +2729,15 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
     {
       if (in.basef && F.b.n % 4 == 0 && (in.ld % 4) == 0) {
         LaunchScope ls(K_MG_LOAD, st, (winv_ ? 12.0 : 8.0) * F.b.n);
-        k_load_input_f4<<<resident_grid(k_load_input_f4, F.b.n / 4), kThreads, 0, st>>>(F.bv.p, F.b.n, in, winvf_.p, gate);
+        k_load_input_f4<<<resident_grid(k_load_input_f4, F.b.n / 4), block_of(F.b.n / 4), 0, st>>>(F.bv.p, F.b.n, in, winvf_.p, gate);
       } else {
         LaunchScope ls(K_MG_LOAD, st, (winv_ ? 20.0 : 12.0) * F.b.n);
-        k_load_input<float><<<grid_for(F.b.n), kThreads, 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
+        k_load_input<float><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
       }
     }
     float *x = vcycle<float>(st, L32, 0, prm, gate, nullptr, nullptr, nullptr, tp, c32);
     LaunchScope ls(K_MG_STORE, st, (4.0 + ob) * F.b.n);
-    k_store_output<float><<<grid_for(F.b.n), kThreads, 0, st>>>(x, F.b.n, out, gate);
+    k_store_output<float><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(x, F.b.n, out, gate);
   } else {
     MgLevelT<double> &F = L64[0];
     if (cluster && clu64_.blocks && clu64_.level == 0) {
@@ -2734,11 +2746,11 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
     }
     {
       LaunchScope ls(K_MG_LOAD, st, (winv_ ? 24.0 : 16.0) * F.b.n);
-      k_load_input<double><<<grid_for(F.b.n), kThreads, 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
+      k_load_input<double><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
     }
     double *x = vcycle<double>(st, L64, 0, prm, gate, nullptr, nullptr, nullptr, nullptr, c64);
     LaunchScope ls(K_MG_STORE, st, (8.0 + ob) * F.b.n);
-    k_store_output<double><<<grid_for(F.b.n), kThreads, 0, st>>>(x, F.b.n, out, gate);
+    k_store_output<double><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(x, F.b.n, out, gate);
   }
 }
 
