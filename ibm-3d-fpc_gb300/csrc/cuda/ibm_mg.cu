@@ -228,6 +228,12 @@ __global__ void k_collapse7(const double *A27, Box b, const unsigned char *coupl
   }
 }
 
+// Input scaling of a finest level stored with `pre`: winv (null: 1) over the diagonal.
+__global__ void k_input_scale(const double *winv, const double *invd, double *out, long n) {
+  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
+    out[r] = winv ? winv[r] * invd[r] : invd[r];
+}
+
 template <class T>
 __global__ void k_convert(const double *src, T *dst, long n) {
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
@@ -384,6 +390,7 @@ struct Recs {
   const T *R = nullptr;            // [c][m][W]
   const uint16_t *code = nullptr;  // [c][m] when classed
   const T *tab = nullptr;          // [K][W]
+  int pre = 0;                     // 7-point records scaled by the inverse diagonal
 };
 template <class T, int W>
 __device__ __forceinline__ void load_recs(const Recs<T, W> &s, long idx, T (&v)[W]) {
@@ -403,8 +410,15 @@ __device__ __forceinline__ const T *rec_ptr(const Recs<T, W> &s, long idx) {
   return s.code ? s.tab + (long)__ldcs(s.code + idx) * W : s.R + idx * W;
 }
 
+// pre: the finest FP64 level, whose phases are bound by the FP64 rate (two
+// operations per clock and SM): the record holds the diagonal, then the
+// negated couplings times the inverse diagonal, and the level's right-hand
+// side is stored times the inverse diagonal, so a phase takes six FMAs a point
+// (x = b' + sum c' x) instead of six FMAs, a subtraction and a product, and the
+// first phase from a zero guess none. FP64 step 640x128x128: 33.96 -> 32.05 ms,
+// 160x32x32 4155 -> 4042 us.
 template <class T>
-__global__ void k_split_colors(const T *A, const T *invd, Box bx, T *R) {
+__global__ void k_split_colors(const T *A, const T *invd, Box bx, T *R, int pre) {
   const long h = bx.n / 2;
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < 2 * h; t += (long)gridDim.x * blockDim.x) {
     const int c = (int)(t / h);
@@ -412,9 +426,9 @@ __global__ void k_split_colors(const T *A, const T *invd, Box bx, T *R) {
     int i, j, k;
     const long r = rb_row(m, c, bx, i, j, k);
     T *o = R + ((long)c * h + m) * 8;
-    o[0] = invd[r];
-    for (int s = 1; s < 7; ++s) o[s] = A[(long)s * bx.n + r];
-    o[7] = A[r];
+    o[0] = pre ? A[r] : invd[r];
+    for (int s = 1; s < 7; ++s) o[s] = pre ? -(A[(long)s * bx.n + r] * invd[r]) : A[(long)s * bx.n + r];
+    o[7] = pre ? invd[r] : A[r];
   }
 }
 
@@ -422,8 +436,8 @@ __global__ void k_split_colors(const T *A, const T *invd, Box bx, T *R) {
 // other colour's points). Points of one colour are not coupled to each other
 // in a 7-point stencil, so the phase reads only values it does not write.
 template <class T>
-__device__ __forceinline__ void relax_rb_body(const Recs<T, 8> &R, const T *b, T *x, const Box &bx, int color, long t0,
-                                              long ts) {
+__device__ __forceinline__ void relax_rb_body(const Recs<T, 8> &R, const T *b, T *x, const Box &bx, int color, T *zout,
+                                              long t0, long ts) {
   const long h = bx.n / 2;
   const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
   const long sy = nx, sz = (long)nx * ny;
@@ -438,21 +452,55 @@ __device__ __forceinline__ void relax_rb_body(const Recs<T, 8> &R, const T *b, T
     const T xn = j < ny - 1 ? x[r + sy] : T(0);
     const T xb = k > 0 ? x[r - sz] : T(0);
     const T xt = k < nz - 1 ? x[r + sz] : T(0);
-    T acc = T(0);
+    const bool pre = sizeof(T) == 8 && R.pre;
+    T acc = pre ? b[r] : T(0);
     acc = fmat<T>(c[1], xw, acc);
     acc = fmat<T>(c[2], xe, acc);
     acc = fmat<T>(c[3], xs, acc);
     acc = fmat<T>(c[4], xn, acc);
     acc = fmat<T>(c[5], xb, acc);
     acc = fmat<T>(c[6], xt, acc);
-    x[r] = c[0] * (b[r] - acc);
+    if (!pre) acc = c[0] * (b[r] - acc);
+    x[r] = acc;
+    if (zout) {  // the V-cycle's result: this point and the other colour's of its pair
+      zout[r] = acc;
+      zout[r ^ 1] = x[r ^ 1];
+    }
   }
 }
 template <class T>
 __global__ void __launch_bounds__(kThreads) k_relax_rb(Recs<T, 8> R, const T *__restrict__ b, T *x,
                                                        Box bx, int color, const int *gate) {
   if (gate_off(gate)) return;
-  relax_rb_body<T>(R, b, x, bx, color, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
+  relax_rb_body<T>(R, b, x, bx, color, nullptr, (long)blockIdx.x * blockDim.x + threadIdx.x,
+                   (long)gridDim.x * blockDim.x);
+}
+// FP64: the finest level's first phase from a zero guess with the V-cycle's
+// input load fused in (k_load_input, then k_relax_rb_zero), and its last phase
+// with the output store: two launches and two passes over the level less.
+__global__ void __launch_bounds__(kThreads) k_relax_rb_in64(Recs<double, 8> R, double *bv, double *x, Box bx, VecRef in,
+                                                            const double *winv, const int *gate) {
+  if (gate_off(gate)) return;
+  const long h = bx.n / 2;
+  const double *src = in.base + (in.idx ? (long)(*in.idx) * in.ld : 0);
+  const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
+  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < h; m += (long)gridDim.x * blockDim.x) {
+    int i, j, k;
+    const long r = rb_row(m, 0, bx, i, j, k);
+    double v[2] = {src[r], src[r ^ 1]};
+    if (in.inu) { v[0] = v[0] * sc; v[1] = v[1] * sc; }
+    if (winv) { v[0] = v[0] * winv[r]; v[1] = v[1] * winv[r ^ 1]; }
+    bv[r] = v[0];
+    bv[r ^ 1] = v[1];
+    x[r] = R.pre ? v[0] : rec_ptr<double, 8>(R, m)[0] * v[0];
+    x[r ^ 1] = 0.0;
+  }
+}
+__global__ void __launch_bounds__(kThreads) k_relax_rb_out64(Recs<double, 8> R, const double *__restrict__ b, double *x,
+                                                             Box bx, OutRef out, const int *gate) {
+  if (gate_off(gate)) return;
+  relax_rb_body<double>(R, b, x, bx, 1, out.d + (out.idx ? (long)(*out.idx) * out.ld : 0),
+                        (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
 // 27-point levels: diagonal neighbours share a colour, so a phase cannot
@@ -703,15 +751,15 @@ __device__ __forceinline__ void residual_rb_body(const Recs<T, 8> &R, const T *b
     const T xn = j < ny - 1 ? x[r + sy] : T(0);
     const T xb = k > 0 ? x[r - sz] : T(0);
     const T xt = k < nz - 1 ? x[r + sz] : T(0);
-    T acc = T(0);
-    acc = fmat<T>(c[7], xc, acc);
+    const bool pre = sizeof(T) == 8 && R.pre;
+    T acc = pre ? b[r] - xc : fmat<T>(c[7], xc, T(0));
     acc = fmat<T>(c[1], xw, acc);
     acc = fmat<T>(c[2], xe, acc);
     acc = fmat<T>(c[3], xs, acc);
     acc = fmat<T>(c[4], xn, acc);
     acc = fmat<T>(c[5], xb, acc);
     acc = fmat<T>(c[6], xt, acc);
-    res[r] = b[r] - acc;
+    res[r] = pre ? c[0] * acc : b[r] - acc;
     res[r ^ 1] = T(0);
   }
 }
@@ -1134,7 +1182,7 @@ __device__ __forceinline__ void relax_rb_zero_body(const Recs<T, 8> &R, const T 
   for (long m = t0; m < h; m += ts) {
     int i, j, k;
     const long r = rb_row(m, 0, bx, i, j, k);
-    x[r] = rec_ptr<T, 8>(R, m)[0] * b[r];
+    x[r] = sizeof(T) == 8 && R.pre ? b[r] : rec_ptr<T, 8>(R, m)[0] * b[r];
     x[r ^ 1] = T(0);
   }
 }
@@ -1660,7 +1708,7 @@ enum ClusterKind : int {
 template <class T>
 struct alignas(16) ClusterOp {
   int kind = 0, color = 0, zero = 0, d = 0;  // zero: zero guess (relaxation); d: direction (transfers)
-  int accumulate = 0;
+  int accumulate = 0, pre = 0;
   Box fb, cb;
   QuadMap quads;
   const T *rec = nullptr, *tab = nullptr;  // colour-split records: the records, or the class table
@@ -1694,7 +1742,7 @@ __device__ __forceinline__ void cluster_barrier() {
 template <class T, int W>
 __device__ __forceinline__ Recs<T, W> op_recs(const ClusterOp<T> &o) {
   Recs<T, W> r;
-  r.R = o.rec; r.code = o.code; r.tab = o.tab;
+  r.R = o.rec; r.code = o.code; r.tab = o.tab; r.pre = o.pre;
   return r;
 }
 
@@ -1739,7 +1787,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         relax_color_body<T, 27>(op.A, op.wd, op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
         break;
       case CK_RB_ZERO: relax_rb_zero_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, t0, ts); break;
-      case CK_RB: relax_rb_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, op.color, t0, ts); break;
+      case CK_RB: relax_rb_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, op.color, nullptr, t0, ts); break;
       case CK_RB27:
         relax_rb27_body<T>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
         break;
@@ -1914,7 +1962,7 @@ static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
   R.alloc((size_t)W * F.b.n);
   {
     LaunchScope ls(K_SETUP, st, 0.0);
-    if (F.ns == 7) k_split_colors<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p);
+    if (F.ns == 7) k_split_colors<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p, F.pre);
     else k_split_colors27<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p);
   }
   if (prm.classes && build_classes<T>(st, R.p, W, F.b.n, F.rbc)) {
@@ -1971,6 +2019,7 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
       LaunchScope ls(K_SETUP, st, 0.0);
       k_diag<<<grid_for(n), block_of(n), 0, st>>>(diag, n, prm.omega, F.invd.p, F.wd.p);
     }
+    F.pre = l == 0 && prm.relax == 2 && F.b.nx % 2 == 0 && prm.nu1 > 0;
     split_colors(st, F, prm);
     const int dims[3] = {F.b.nx, F.b.ny, F.b.nz};
     // A group starts at a relaxed level: every direction whose spacing is
@@ -2070,6 +2119,12 @@ void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const flo
   }
   (void)fp64;
   build<double>(st, L64, b, A7, h);
+  winvd_.release();
+  if (L64[0].pre) {
+    winvd_.alloc(b.n);
+    LaunchScope ls(K_SETUP, st, 0.0);
+    k_input_scale<<<grid_for(b.n), block_of(b.n), 0, st>>>(winv, L64[0].invd.p, winvd_.p, b.n);
+  }
   L32.clear();
   if (fp32) {
     L32.reserve(L64.size());
@@ -2269,7 +2324,7 @@ static T *record_cluster(std::vector<MgLevelT<T>> &L, int l, const MgParams &p, 
   const bool rb7 = R7.R || R7.code, rb27 = R27.R || R27.code;
   const bool quad = f32 && p.quads && F.b.nx % 4 == 0;
   auto recs = [&](ClusterOp<T> &op) {
-    if (rb7) { op.rec = R7.R; op.tab = R7.tab; op.code = R7.code; }
+    if (rb7) { op.rec = R7.R; op.tab = R7.tab; op.code = R7.code; op.pre = F.pre; }
     else { op.rec = R27.R; op.tab = R27.tab; op.code = R27.code; }
   };
   T *cur = F.x.p, *oth = F.t.p;
@@ -2510,7 +2565,7 @@ template <class T>
 // the levels on one cluster.
 static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgParams &p, const int *gate,
                  const VecRef *fin = nullptr, const OutRef *fout = nullptr, const float *winvf = nullptr,
-                 const TailLaunch *tail = nullptr, const ClusterPlan *clu = nullptr) {
+                 const TailLaunch *tail = nullptr, const ClusterPlan *clu = nullptr, const double *winv = nullptr) {
   MgLevelT<T> &F = L[l];
   const long n = F.b.n;
   const double T_ = sizeof(T);
@@ -2526,7 +2581,8 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   // Colour-split records, plain or classed. Algorithmic bytes of a phase: the
   // records of its colour, b of its colour, x of the other colour read and
   // the phase's writes of x.
-  const Recs<T, 8> R7 = recs_of<T, 8>(F.rb, F.rbc);
+  Recs<T, 8> R7 = recs_of<T, 8>(F.rb, F.rbc);
+  R7.pre = F.pre;
   const Recs<T, 28> R27 = recs_of<T, 28>(F.rb27, F.rbc);
   const bool rb7 = R7.R || R7.code, rb27 = R27.R || R27.code;
   const bool quad = F.b.nx % 4 == 0 && p.quads;  // quartet kernels (FP32)
@@ -2559,6 +2615,25 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
                                                   : 0.5 * n * rec7 + 1.5 * T_ * n);
             k_relax_rb_quad<<<resident_grid(k_relax_rb_quad, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, color, z, gate);
           }
+        }
+        return;
+      }
+    }
+    if constexpr (sizeof(T) == 8) {
+      if (p.relax == 2 && rb7 && (zero ? fin != nullptr : last && fout)) {
+        if (zero) {
+          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.pre ? 0.0 : R7.code ? 2.0 : T_) + (winv ? 4.0 : 3.0) * T_ * n);
+          k_relax_rb_in64<<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, *fin, winv, gate);
+        } else {
+          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 1.5 * T_ * n);
+          k_relax_rb<T><<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, 0, gate);
+        }
+        if (last && fout) {
+          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 2.5 * T_ * n);
+          k_relax_rb_out64<<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, *fout, gate);
+        } else {
+          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 1.5 * T_ * n);
+          k_relax_rb<T><<<grid_all(h), block_of(h), 0, st>>>(R7, F.bv.p, cur, F.b, 1, gate);
         }
         return;
       }
@@ -2740,13 +2815,19 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
     k_store_output<float><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(x, F.b.n, out, gate);
   } else {
     MgLevelT<double> &F = L64[0];
+    const double *winv = F.pre ? winvd_.p : winv_;
     if (cluster && clu64_.blocks && clu64_.level == 0) {
-      run_cluster<double>(st, L64, clu64_, in, out, winv_, nullptr, gate);
+      run_cluster<double>(st, L64, clu64_, in, out, winv, nullptr, gate);
+      return;
+    }
+    if (in.base && out.d && prm.relax == 2 && F.relax && F.cdir >= 0 && F.ns == 7 && (F.rb.p || F.rbc.ok()) &&
+        prm.nu1 > 0 && prm.nu2 > 0) {
+      vcycle<double>(st, L64, 0, prm, gate, &in, &out, nullptr, nullptr, c64, winv);
       return;
     }
     {
       LaunchScope ls(K_MG_LOAD, st, (winv_ ? 24.0 : 16.0) * F.b.n);
-      k_load_input<double><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
+      k_load_input<double><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.bv.p, F.b.n, in, winv, gate);
     }
     double *x = vcycle<double>(st, L64, 0, prm, gate, nullptr, nullptr, nullptr, nullptr, c64);
     LaunchScope ls(K_MG_STORE, st, (8.0 + ob) * F.b.n);
