@@ -1553,7 +1553,7 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
     in.base = slot[s].z.p;
     OutRef out;
     out.d = slot[s].z2.p;
-    pc.apply(pc.ctx, st, s, in, out, &scal.p[s].cycle_end);
+    pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].cycle_end : nullptr);
     cb = true;
   }
   if (cb) {
@@ -1567,6 +1567,9 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
 void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl, unsigned mask) {
   const dim3 grid(nblk, nsys), gridu(nblk * 2, nsys);
   auto rows = [&](int s) { return ((mask >> s) & 1u) ? (double)slot[s].host.n : 0.0; };
+  // A single system is active whenever an Arnoldi step runs (the host loop and
+  // the graph's WHILE and SWITCH see to that), so its preconditioner needs no
+  // gate: one dependent load less at the start of each of its kernels.
   for (int s = 0; s < nsys; ++s) {
     if (!((mask >> s) & 1u) || (fl && !fl[s].active)) continue;
     const KSysHost &h = slot[s].host;
@@ -1576,7 +1579,7 @@ void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl
       OutRef out;
       out.d = slot[s].z.p;
       if (slot[s].Zd.p) { out.d = slot[s].Zd.p; out.ld = h.n; out.idx = &scal.p[s].i; }
-      pc.apply(pc.ctx, st, s, in, out, &scal.p[s].active);
+      pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].active : nullptr);
     } else if (h.pc == 2 && h.pc_cb) {
       VecRef in;
       if (h.a32) in.basef = slot[s].Vf.p;
@@ -1584,7 +1587,7 @@ void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl
       in.ld = h.n; in.idx = &scal.p[s].i; in.inu = scal.p[s].inu;
       OutRef out;
       out.f = slot[s].Z.p; out.ld = h.n; out.idx = &scal.p[s].i;
-      pc.apply(pc.ctx, st, s, in, out, &scal.p[s].active);
+      pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].active : nullptr);
     }
   }
   int inner_sweeps = 0;

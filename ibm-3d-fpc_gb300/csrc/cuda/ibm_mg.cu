@@ -1952,6 +1952,7 @@ void dense_inverse(const std::vector<double> &A, int ns, const Box &b, std::vect
 // level), used by the in-place two-colour relaxation.
 // With record classes on, the records are replaced by their classes when
 // there are at most kMaxClasses distinct ones.
+constexpr long kPlainRecords = 32768;
 template <class T>
 static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
   if (prm.relax != 2 || (F.b.nx & 1) || F.b.n < 2) return;
@@ -1963,6 +1964,11 @@ static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
     if (F.ns == 7) k_split_colors<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p, F.pre);
     else k_split_colors27<T><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.A, F.invd.p, F.b, R.p);
   }
+  // A small 27-point level keeps its records: they stay in L2 whole, and a
+  // phase there is a chain of memory latencies of which the class is one (step
+  // 97x33x21 4690 -> 4500 us, FP64 160x32x32 4017 -> 3955, with the gate's load
+  // of a single system's V-cycle taken out).
+  if (F.ns == 27 && F.b.n <= kPlainRecords) return;
   if (prm.classes && build_classes<T>(st, R.p, W, F.b.n, F.rbc)) {
     R.release();
     if (sizeof(T) == 4 && F.b.nx % 4 == 0 && prm.quads) mark_runs<T>(st, F.rbc, F.b);
