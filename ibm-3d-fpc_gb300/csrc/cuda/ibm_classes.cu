@@ -108,22 +108,27 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
   IBM_CUDA_TRY(cudaStreamSynchronize(st));
   dh.release();
   std::vector<uint16_t> code((size_t)nrec);
-  std::vector<long> rep;
+  std::vector<long> rep, count;  // first record and number of records of each class
   std::unordered_map<unsigned long long, int> id;
   unsigned long long prev_h = 0;
   int prev_c = -1;
+  long run = 0;  // records since the class last changed
   for (long t = 0; t < nrec; ++t) {
     const unsigned long long v = h[(size_t)t];
     int c;
     if (prev_c >= 0 && v == prev_h) {
       c = prev_c;
+      ++run;
     } else {
+      if (prev_c >= 0) count[(size_t)prev_c] += run;
+      run = 1;
       auto it = id.find(v);
       if (it == id.end()) {
         if ((int)rep.size() >= kMaxClasses) return false;
         c = (int)rep.size();
         id.emplace(v, c);
         rep.push_back(t);
+        count.push_back(0);
       } else {
         c = it->second;
       }
@@ -161,8 +166,7 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
     return false;
   }
   out.K = K;
-  std::vector<long> count((size_t)K, 0);
-  for (long t = 0; t < nrec; ++t) ++count[code[(size_t)t]];
+  count[(size_t)prev_c] += run;
   out.major = (int)(std::max_element(count.begin(), count.end()) - count.begin());
   out.major_rec.resize((size_t)W);
   IBM_CUDA_TRY(cudaMemcpyAsync(out.major_rec.data(), out.tab.p + (size_t)out.major * W, sizeof(T) * W,
