@@ -9,7 +9,7 @@
 // entry point of this library works through a context, and creating a context
 // allocates; this one needs none.
 //
-// Its only scratch is the file-scope array below: per-tile partial sums of the
+// Its only scratch is the file-scope array below: per-block partial sums of the
 // two norms and the counter that elects the block finishing the reduction.
 // The array lives in the library's module and is held on every device that
 // loads the library until the process exits. Its address in the current
@@ -18,6 +18,7 @@
 // device is followed; a call made while its stream is being captured reuses
 // the address found by the last uncaptured call on that device. In host code
 // the array's name is only a stand-in for the symbol, never a device address.
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -32,8 +33,8 @@ constexpr int kNaMaxDevices = 64;
 static_assert(kNaMaxRows % kTile == 0, "the row limit is a whole number of tiles");
 
 struct NoAllocScratch {
-  double part[2 * kNaMaxTiles];  // per tile: sum r^2, sum b^2
-  unsigned ticket;               // tiles finished; cleared before every launch
+  double part[2 * kNaMaxTiles];  // per block: sum r^2, sum b^2
+  unsigned ticket;               // blocks finished; cleared before every launch
 };
 
 }  // namespace
@@ -43,41 +44,97 @@ static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 
 namespace {
 
-// One block per tile of kTile rows. The stencil is evaluated in the same order
-// as the context path's operator apply (centre, -x, +x, -y, +y, -z, +z, one fma
-// each), so r is bitwise equal to b - ibm_apply_operator(x). The norms are
-// summed in a fixed order (rows within a thread, lanes, warps, tiles), so the
-// result does not depend on which block finishes last.
-__global__ void __launch_bounds__(kThreads)
-    k_residual_noalloc(const double *__restrict__ vals, int nx, int ny, int nz, long n,
-                       const double *__restrict__ x, const double *__restrict__ b, double *__restrict__ r,
-                       double *__restrict__ norms, NoAllocScratch *sc) {
+// A warp takes 32 rows at a time and keeps kNaStages such chunks on their way.
+constexpr int kNaStages = 3;
+constexpr int kNaBlocksPerSm = 4;
+constexpr int kNaChunk = 32 * 7;  // coefficients of a chunk
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(double *smem, const double *g) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(g) : "memory");
+}
+
+// The rows' coefficients lie row by row (56 bytes each): read by the thread of
+// each row they are seven 8-byte loads 56 bytes apart across the lanes, which
+// touch the same 14 lines seven times. So a warp copies the rows of its next
+// chunks to shared memory as they lie, 16 bytes a lane (8 when vals is aligned
+// to 8 only), while it sums the present one; a row's values are then 14 words
+// apart between neighbouring lanes, which no two lanes of a half-warp have in
+// one bank. Warps run free of each other, so that one's FP64 work (10
+// operations a row, 75 us at 512x96x96) covers another's loads (57 us at the
+// copy bandwidth). A call at that size took 125 us and takes 100; with one copy
+// of a whole tile per block and a barrier it took 156, since blocks then load
+// and compute in step.
+//
+// The stencil is evaluated in the same order as the context path's operator
+// apply (centre, -x, +x, -y, +y, -z, +z, one fma each), so r is bitwise equal
+// to b - ibm_apply_operator(x). The norms are summed in a fixed order (chunks
+// of a warp, lanes, warps, blocks), so the result does not depend on which
+// block finishes last.
+__global__ void __launch_bounds__(kThreads, kNaBlocksPerSm)
+    k_residual_noalloc(const double *__restrict__ vals, Box bx, int aligned16, const double *__restrict__ x,
+                       const double *__restrict__ b, double *__restrict__ r, double *__restrict__ norms,
+                       NoAllocScratch *sc) {
+  __shared__ __align__(16) double rows[kWarps][kNaStages][kNaChunk];
   __shared__ double srr[kWarps], sbb[kWarps];
   __shared__ int last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long sy = nx, sz = (long)nx * ny;
-  double rr = 0.0, bb = 0.0;
+  const int nx = bx.nx, ny = bx.ny, nz = bx.nz;
+  const long n = bx.n, sy = nx, sz = (long)nx * ny;
+  const int chunks = (int)((n + 31) / 32), step = gridDim.x * kWarps;
+  // copies chunk c (none past the end); every call commits one group
+  auto fetch = [&](int c, int stage) {
+    if (c < chunks) {
+      const double *src = vals + (long)c * kNaChunk;
+      double *dst = rows[warp][stage];
+      const int count = (int)(n - 32l * c < 32 ? (n - 32l * c) * 7 : kNaChunk);
+      if (aligned16) {
+        for (int e = 2 * lane; e < count; e += 64) {
+          if (e + 1 < count) copy_async<16>(dst + e, src + e);
+          else copy_async<8>(dst + e, src + e);
+        }
+      } else {
+        for (int e = lane; e < count; e += 32) copy_async<8>(dst + e, src + e);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int c = blockIdx.x * kWarps + warp;
 #pragma unroll
-  for (int t = 0; t < kRowsPerThread; ++t) {
-    const long row = (long)blockIdx.x * kTile + t * kThreads + threadIdx.x;
-    if (row < n) {
-      int i, j, k;
-      row_ijk((int)row, nx, ny, i, j, k);
-      const double *c = vals + 7 * row;
+  for (int q = 0; q < kNaStages - 1; ++q) fetch(c + q * step, q);
+  double rr = 0.0, bb = 0.0;
+  for (int stage = 0; c < chunks; c += step) {
+    const long row = 32l * c + lane;
+    const bool in = row < n;
+    int i = 0, j = 0, k = 0;
+    if (in) box_ijk(row, bx, i, j, k);
+    const double x0 = in ? x[row] : 0.0, xw = in && i > 0 ? x[row - 1] : 0.0, xe = in && i < nx - 1 ? x[row + 1] : 0.0,
+                 xs = in && j > 0 ? x[row - sy] : 0.0, xn = in && j < ny - 1 ? x[row + sy] : 0.0,
+                 xb = in && k > 0 ? x[row - sz] : 0.0, xt = in && k < nz - 1 ? x[row + sz] : 0.0;
+    const double bv = in ? b[row] : 0.0;
+    asm volatile("cp.async.wait_group %0;" ::"n"(kNaStages - 2) : "memory");
+    __syncwarp();  // every lane's copies are in, and the stage refilled next has been read by all
+    int next = stage + kNaStages - 1;
+    if (next >= kNaStages) next -= kNaStages;
+    fetch(c + (kNaStages - 1) * step, next);
+    if (in) {
+      const double *v = rows[warp][stage] + 7 * lane;
       double acc = 0.0;
-      acc = fma(c[0], x[row], acc);
-      acc = fma(c[1], i > 0 ? x[row - 1] : 0.0, acc);
-      acc = fma(c[2], i < nx - 1 ? x[row + 1] : 0.0, acc);
-      acc = fma(c[3], j > 0 ? x[row - sy] : 0.0, acc);
-      acc = fma(c[4], j < ny - 1 ? x[row + sy] : 0.0, acc);
-      acc = fma(c[5], k > 0 ? x[row - sz] : 0.0, acc);
-      acc = fma(c[6], k < nz - 1 ? x[row + sz] : 0.0, acc);
-      const double bv = b[row];
+      acc = fma(v[0], x0, acc);
+      acc = fma(v[1], xw, acc);
+      acc = fma(v[2], xe, acc);
+      acc = fma(v[3], xs, acc);
+      acc = fma(v[4], xn, acc);
+      acc = fma(v[5], xb, acc);
+      acc = fma(v[6], xt, acc);
       const double rv = bv - acc;
       r[row] = rv;
       rr = fma(rv, rv, rr);
       bb = fma(bv, bv, bb);
     }
+    if (++stage == kNaStages) stage = 0;
   }
   rr = warp_sum(rr);
   bb = warp_sum(bb);
@@ -188,7 +245,12 @@ extern "C" int ibm_residual_noalloc(const double *vals, int nx, int ny, int nz, 
   NoAllocScratch *sc = nullptr;
   if (scratch_on_device(dev, cs != cudaStreamCaptureStatusNone, &sc) != cudaSuccess) return IBM_ERR_CUDA;
   if (cudaMemsetAsync(&sc->ticket, 0, sizeof(unsigned), st) != cudaSuccess) return IBM_ERR_CUDA;
-  const int tiles = (int)((n + kTile - 1) / kTile);
-  k_residual_noalloc<<<tiles, kThreads, 0, st>>>(vals, nx, ny, nz, n, x, b, r, norms, sc);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return IBM_ERR_CUDA;
+  // one chunk per warp up to one resident wave; 152 x 4 blocks are within the scratch's tiles on any device
+  const long blocks = (n + 32 * kWarps - 1) / (32 * kWarps);
+  const int grid = (int)std::min({blocks, (long)sms * kNaBlocksPerSm, (long)kNaMaxTiles});
+  k_residual_noalloc<<<grid, kThreads, 0, st>>>(vals, make_box(nx, ny, nz),
+                                                reinterpret_cast<uintptr_t>(vals) % 16 == 0, x, b, r, norms, sc);
   return cudaGetLastError() == cudaSuccess ? IBM_OK : IBM_ERR_CUDA;
 }
