@@ -1691,8 +1691,9 @@ __global__ void __launch_bounds__(kThreads) k_mg_tail(const TailOp *__restrict__
 // cluster barrier between them, whose release / acquire orders their global
 // stores and loads; the phase list is copied to shared memory once. A phase
 // then takes 2.5 to 3 us (the barrier's flush to L2 and the loads back). A
-// launch inside a captured step takes no longer than that, so captured steps
-// keep one launch per phase. Per point the arithmetic is the stand-alone
+// launch inside a captured step takes no longer than that (steps on this form:
+// mixed 320x64x64 4997 -> 5654 us, 97x33x21 4308 -> 6109), so captured steps
+// keep launches, with a level's sweeps in one (k_smooth27) where it is small. Per point the arithmetic is the stand-alone
 // kernels' (the shared bodies), so results do not depend on which form ran.
 // ---------------------------------------------------------------------------
 enum ClusterKind : int {
@@ -1833,6 +1834,133 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       }
     }
     if (o + 1 < nops) cluster_barrier();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// All sweeps of one 27-point level on one cluster. As launches, a colour phase
+// of a level of some thousand points is a chain of latencies (launch, record
+// and x from L2, x back to L2), 3.5 to 4 us at any size. Here each thread keeps
+// a pair of points: their coefficients (the same for every phase), right-hand
+// sides and values stay in registers, and a block holds the x values that its
+// points' stencils touch in shared memory. After a phase a thread stores its
+// new value there and into the shared memory of the neighbouring blocks whose
+// points touch it, and a cluster barrier ends the phase; nothing goes through
+// L2 between the phases. Steps in us, one launch per phase against this: mixed
+// 97x33x21 4308 -> 3866, 320x64x64 4997 -> 4804, FP64 160x32x32 3716 -> 3593,
+// twelve channels 30.9 -> 29.1 ms.
+//
+// A phase reads its own colour's values of the sweep before (a 27-point stencil
+// couples points of one colour), so each colour has two buffers of which the
+// phase writes the other. Per point the arithmetic and its order are those of
+// k_relax_rb27 / k_relax_color and k_residual, so results are the same bits.
+// ---------------------------------------------------------------------------
+// Most pairs (threads) of a block: two records of 28 values per thread have to
+// fit the register file.
+template <class T>
+constexpr int kSmoothThreads = sizeof(T) == 4 ? 640 : 320;
+
+__device__ __forceinline__ void store_cluster(uint32_t at, int rank, float v) {
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f32 [a], %2;\n\t}" ::"r"(at),
+               "r"(rank), "f"(v)
+               : "memory");
+}
+__device__ __forceinline__ void store_cluster(uint32_t at, int rank, double v) {
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f64 [a], %2;\n\t}" ::"r"(at),
+               "r"(rank), "d"(v)
+               : "memory");
+}
+
+// sweeps two-colour sweeps of A x = b from x, or from zero (zero != 0), and the
+// residual when res is given. One cluster of gridDim.x blocks; block q keeps
+// pairs [q, q + 1) * blockDim.x, which are points [q, q + 1) * span, and the x
+// values of its points and of `halo` points on either side. halo is even and
+// more than the stencil's reach of nx ny + nx + 1 points, so a pair lies inside
+// or outside of a block's values as a whole. A pair holds one point of either
+// colour (nx even: one line; nx odd: consecutive rows of a plane alternate).
+template <class T>
+__global__ void __launch_bounds__(kSmoothThreads<T>, 1)
+    k_smooth27(const T *A, const T *invd, const T *b, T *x, T *res, Box bx, int sweeps, int zero, int halo,
+               const int *gate) {
+  if (gate_off(gate)) return;
+  extern __shared__ __align__(16) unsigned char smem_x[];
+  const int n = bx.n, span = 2 * blockDim.x, held = span + 2 * halo, lo = (int)blockIdx.x * span;
+  T *const x0 = reinterpret_cast<T *>(smem_x), *const x1 = x0 + held;
+  const int r0 = lo + 2 * (int)threadIdx.x;
+  int at[2];       // the pair's point of each colour
+  bool own[2] = {false, false};
+  T c[2][28], bv[2], xv[2];
+  {
+    int i, j, k;
+    box_ijk(r0 < n ? r0 : 0, bx, i, j, k);
+    const int first = (i + j + k) & 1;
+    at[0] = r0 + first;
+    at[1] = r0 + 1 - first;
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    own[q] = at[q] < n;
+    int i, j, k;
+    box_ijk(own[q] ? at[q] : 0, bx, i, j, k);
+#pragma unroll
+    for (int s = 0; s < 27; ++s) {
+      const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+      const bool in = own[q] && ii >= 0 && ii < bx.nx && jj >= 0 && jj < bx.ny && kk >= 0 && kk < bx.nz;
+      c[q][s] = in ? A[(long)s * n + at[q]] : T(0);  // 0: the value read in its place is finite
+    }
+    c[q][27] = own[q] ? invd[at[q]] : T(0);
+    bv[q] = own[q] ? b[at[q]] : T(0);
+    xv[q] = own[q] && !zero ? x[at[q]] : T(0);
+  }
+  for (int e = threadIdx.x; e < held; e += blockDim.x) {
+    const int r = lo - halo + e;
+    x0[e] = !zero && r >= 0 && r < n ? x[r] : T(0);
+    x1[e] = T(0);
+  }
+  // blocks that hold the pair's values
+  const int last = (n - 1) / span;
+  const int b0 = r0 >= halo ? (r0 - halo) / span : 0, b1 = r0 < n ? min(last, (r0 + halo) / span) : -1;
+  cluster_barrier();
+  const int sy = bx.nx, sz = bx.nx * bx.ny;
+  auto sum = [&](int q, const T *same, const T *opp) {  // A x at the pair's point of colour q
+    const int l = at[q] - lo + halo;
+    T acc = T(0);
+#pragma unroll
+    for (int s = 0; s < 27; ++s) {
+      const int di = s % 3 - 1, dj = (s / 3) % 3 - 1, dk = s / 9 - 1;
+      const T v = s == 13 ? xv[q] : ((di + dj + dk) & 1 ? opp : same)[l + di + dj * sy + dk * sz];
+      acc = fmat<T>(c[q][s], v, acc);
+    }
+    return acc;
+  };
+  T *cur[2] = {x0, x0}, *oth[2] = {x1, x1};
+  for (int w = 0; w < sweeps; ++w) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const bool ends = w == sweeps - 1 && q == 1 && !res;  // no value is read any more
+      if (own[q]) {
+        if (zero && w == 0 && q == 0) xv[q] = c[q][27] * bv[q];
+        else xv[q] = fmat<T>(c[q][27], bv[q] - sum(q, cur[q], cur[q ^ 1]), xv[q]);
+        if (!ends) {
+          T *to = oth[q] + (at[q] - lo + halo);
+          *to = xv[q];
+          const uint32_t to32 = (uint32_t)__cvta_generic_to_shared(to);
+          for (int d = b0; d <= b1; ++d)
+            if (d != (int)blockIdx.x)
+              store_cluster(to32 + (uint32_t)(((int)blockIdx.x - d) * span * (int)sizeof(T)), d, xv[q]);
+        }
+      }
+      T *const t = cur[q];
+      cur[q] = oth[q];
+      oth[q] = t;
+      if (!ends) cluster_barrier();
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    if (!own[q]) continue;
+    x[at[q]] = xv[q];
+    if (res) res[at[q]] = bv[q] - sum(q, cur[q], cur[q ^ 1]);
   }
 }
 
@@ -2425,11 +2553,12 @@ static void launch_cluster(cudaStream_t st, const ClusterOp<T> *ops, int count, 
   IBM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_mg_cluster<T>, ops, count, in, load4, out, winv, winvf, gate));
 }
 
-// Blocks of the cluster: 16 where the device can place such a cluster, else
-// the portable 8, else 0 (one launch per phase). Asked once per device: the
+// Blocks of a cluster of kernel K's blocks (threads, dynamic shared memory as
+// given): 16 where the device can place such a cluster, else the portable 8,
+// else 0 (one launch per phase). Asked once per device and kernel: the
 // occupancy query takes milliseconds.
-template <class T>
-static int cluster_blocks() {
+template <auto K>
+static int cluster_blocks(int threads, int smem) {
   static std::mutex mu;
   static std::unordered_map<int, int> known;
   int dev = 0;
@@ -2439,17 +2568,16 @@ static int cluster_blocks() {
   if (it != known.end()) return it->second;
   int &found = known[dev];
   found = 0;
-  if (cudaFuncSetAttribute(k_mg_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaFuncSetAttribute(k_mg_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(ClusterOp<T>) * kClusterOps) != cudaSuccess) {
+  if (cudaFuncSetAttribute(K, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   for (int blocks : {16, 8}) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(kClusterThreads);
-    cfg.dynamicSmemBytes = sizeof(ClusterOp<T>) * (size_t)kClusterOps;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)blocks;
@@ -2457,7 +2585,7 @@ static int cluster_blocks() {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_mg_cluster<T>, &cfg) == cudaSuccess && n > 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, K, &cfg) == cudaSuccess && n > 0) {
       found = blocks;
       break;
     }
@@ -2465,6 +2593,9 @@ static int cluster_blocks() {
   }
   return found;
 }
+constexpr int kSmoothShared = 96 * 1024;  // k_smooth27; more is only needed by levels a few points thick
+template <class T>
+static int smooth_blocks() { return cluster_blocks<&k_smooth27<T>>(kSmoothThreads<T>, kSmoothShared); }
 
 // Algorithmic bytes of the recorded phases (each operand of a phase once).
 template <class T>
@@ -2512,7 +2643,7 @@ static void plan_cluster(cudaStream_t st, std::vector<MgLevelT<T>> &L, const MgP
       if (ops[(size_t)o].kind == CK_DENSE) down = o;
   const int up = (int)ops.size() - down - 1;  // phases after the dense level, when it stands alone
   if (down > kClusterOps || up > kClusterOps) return;
-  c.blocks = cluster_blocks<T>();
+  c.blocks = cluster_blocks<&k_mg_cluster<T>>(kClusterThreads, (int)sizeof(ClusterOp<T>) * kClusterOps);
   if (c.blocks == 0) return;
   c.ops.alloc(sizeof(ClusterOp<T>) * ops.size());
   IBM_CUDA_TRY(cudaMemcpyAsync(c.ops.p, ops.data(), c.ops.n, cudaMemcpyHostToDevice, st));
@@ -2542,6 +2673,51 @@ static T *run_cluster(cudaStream_t st, std::vector<MgLevelT<T>> &L, const Cluste
   return (T *)c.out;
 }
 
+// How k_smooth27 takes a level; threads == 0: not at all.
+struct SmoothPlan {
+  int threads = 0, blocks = 0, halo = 0, smem = 0;
+};
+// A level goes to one cluster when its pairs fit the registers of its blocks
+// (20480 points in FP32, 10240 in FP64). Above that a launch per phase spreads
+// the level over all SMs.
+template <class T>
+static SmoothPlan smooth_plan(const MgLevelT<T> &F, const MgParams &p) {
+  SmoothPlan s;
+  const long reach = (long)F.b.nx * F.b.ny + F.b.nx + 1, pairs = ((long)F.b.n + 1) / 2;
+  if (p.relax != 2 || F.ns != 27 || pairs > 16L * kSmoothThreads<T>) return s;
+  const int most = smooth_blocks<T>();
+  if (most == 0) return s;
+  const int threads = std::max(64, (int)((pairs + most - 1) / most + 31) / 32 * 32);
+  if (threads > kSmoothThreads<T>) return s;
+  s.halo = (int)(reach + 2) / 2 * 2;
+  s.smem = 2 * (2 * threads + 2 * s.halo) * (int)sizeof(T);
+  if (s.smem > kSmoothShared) return s;
+  s.blocks = 1;
+  while ((long)s.blocks * threads < pairs) s.blocks *= 2;
+  s.threads = threads;
+  return s;
+}
+
+template <class T>
+static void launch_smooth(cudaStream_t st, const SmoothPlan &s, const MgLevelT<T> &F, T *x, T *res, int sweeps, bool zero,
+                          const int *gate) {
+  // algorithmic bytes: coefficients, b, x in (unless zero) and out, the residual
+  LaunchScope ls(K_MG_RELAX, st, sizeof(T) * (double)F.b.n * (28.0 + 2.0 + (zero ? 0.0 : 1.0) + (res ? 1.0 : 0.0)));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)s.blocks);
+  cfg.blockDim = dim3((unsigned)s.threads);
+  cfg.dynamicSmemBytes = (size_t)s.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)s.blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  IBM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_smooth27<T>, F.A, (const T *)F.invd.p, (const T *)F.bv.p, x, res, F.b, sweeps,
+                                  zero ? 1 : 0, s.halo, gate));
+}
+
 // One cooperative launch of the fused coarse levels (a memset clears the
 // barrier state first); returns the buffer holding the first fused level's
 // correction.
@@ -2569,7 +2745,8 @@ template <class T>
 // the levels on one cluster.
 static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgParams &p, const int *gate,
                  const VecRef *fin = nullptr, const OutRef *fout = nullptr, const float *winvf = nullptr,
-                 const TailLaunch *tail = nullptr, const ClusterPlan *clu = nullptr, const double *winv = nullptr) {
+                 const TailLaunch *tail = nullptr, const ClusterPlan *clu = nullptr, const double *winv = nullptr,
+                 bool fused = false) {
   MgLevelT<T> &F = L[l];
   const long n = F.b.n;
   const double T_ = sizeof(T);
@@ -2690,9 +2867,15 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   // each way when it is set
   const int c1 = (l > 0 && p.nu_coarse > 0) ? p.nu_coarse : p.nu1, c2 = (l > 0 && p.nu_coarse > 0) ? p.nu_coarse : p.nu2;
   const int nu1 = F.relax ? c1 : 0, nu2 = F.relax ? c2 : 0;
-  for (int s = 0; s < nu1; ++s) relax(s == 0, false);
+  const SmoothPlan sp = fused && nu1 + nu2 > 0 ? smooth_plan<T>(F, p) : SmoothPlan();
   const T *res = F.bv.p;  // residual of a zero initial guess is b
-  if (nu1 > 0 && p.relax == 2 && rb7) {
+  if (sp.threads && nu1 > 0) {
+    launch_smooth<T>(st, sp, F, cur, F.r.p, nu1, true, gate);
+    res = F.r.p;
+  }
+  for (int s = 0; s < nu1 && !sp.threads; ++s) relax(s == 0, false);
+  if (sp.threads) {
+  } else if (nu1 > 0 && p.relax == 2 && rb7) {
     LaunchScope ls(K_MG_RESID, st, 0.5 * n * rec7 + 2.5 * T_ * n);
     bool done = false;
     if constexpr (sizeof(T) == 4) {
@@ -2750,7 +2933,7 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   }
   if (!xc && clu && clu->blocks && l + G.n == clu->level)
     xc = run_cluster<T>(st, L, *clu, VecRef(), OutRef(), nullptr, nullptr, gate);
-  if (!xc) xc = vcycle<T>(st, L, l + G.n, p, gate, nullptr, nullptr, nullptr, tail, clu);
+  if (!xc) xc = vcycle<T>(st, L, l + G.n, p, gate, nullptr, nullptr, nullptr, tail, clu, nullptr, fused);
   {
     LaunchScope ls(K_MG_PROLONG, st, T_ * ((nu1 > 0 ? 4.0 : 3.0) * n + C.b.n));
     if (G.n == 3)
@@ -2768,7 +2951,8 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
       k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
     }
   }
-  for (int s = 0; s < nu2; ++s) relax(false, s == nu2 - 1);
+  if (sp.threads && nu2 > 0) launch_smooth<T>(st, sp, F, cur, nullptr, nu2, false, gate);
+  for (int s = 0; s < nu2 && !sp.threads; ++s) relax(false, s == nu2 - 1);
   return cur;
 }
 
@@ -2802,7 +2986,7 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
       return;
     }
     if (fuse) {
-      vcycle<float>(st, L32, 0, prm, gate, &in, &out, winvf_.p, tp, c32);
+      vcycle<float>(st, L32, 0, prm, gate, &in, &out, winvf_.p, tp, c32, nullptr, fused);
       return;
     }
     {
@@ -2814,7 +2998,7 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
         k_load_input<float><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.bv.p, F.b.n, in, winv_, gate);
       }
     }
-    float *x = vcycle<float>(st, L32, 0, prm, gate, nullptr, nullptr, nullptr, tp, c32);
+    float *x = vcycle<float>(st, L32, 0, prm, gate, nullptr, nullptr, nullptr, tp, c32, nullptr, fused);
     LaunchScope ls(K_MG_STORE, st, (4.0 + ob) * F.b.n);
     k_store_output<float><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(x, F.b.n, out, gate);
   } else {
@@ -2826,14 +3010,14 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
     }
     if (in.base && out.d && prm.relax == 2 && F.relax && F.cdir >= 0 && F.ns == 7 && (F.rb.p || F.rbc.ok()) &&
         prm.nu1 > 0 && prm.nu2 > 0) {
-      vcycle<double>(st, L64, 0, prm, gate, &in, &out, nullptr, nullptr, c64, winv);
+      vcycle<double>(st, L64, 0, prm, gate, &in, &out, nullptr, nullptr, c64, winv, fused);
       return;
     }
     {
       LaunchScope ls(K_MG_LOAD, st, (winv_ ? 24.0 : 16.0) * F.b.n);
       k_load_input<double><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(F.bv.p, F.b.n, in, winv, gate);
     }
-    double *x = vcycle<double>(st, L64, 0, prm, gate, nullptr, nullptr, nullptr, nullptr, c64);
+    double *x = vcycle<double>(st, L64, 0, prm, gate, nullptr, nullptr, nullptr, nullptr, c64, nullptr, fused);
     LaunchScope ls(K_MG_STORE, st, (8.0 + ob) * F.b.n);
     k_store_output<double><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(x, F.b.n, out, gate);
   }
