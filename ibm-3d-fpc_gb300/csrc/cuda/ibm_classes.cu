@@ -63,8 +63,9 @@ __global__ void k_verify_classes(const unsigned *__restrict__ words, int wpr, lo
   }
 }
 
-// runs[w] = 1 when the four points of every quad 32 w .. 32 w + 31 have codes
-// `major`. One warp per run, one quad per lane.
+// runs[w] = 1 when the points of every quad (octet) 32 w .. 32 w + 31 have
+// codes `major`. One warp per run, one quad per lane.
+template <int unit>
 __global__ void k_mark_runs(const uint16_t *__restrict__ code, Box b, QuadMap Q, int major, uint8_t *__restrict__ runs,
                             long nruns) {
   const long w0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, ws = ((long)gridDim.x * blockDim.x) >> 5;
@@ -73,9 +74,9 @@ __global__ void k_mark_runs(const uint16_t *__restrict__ code, Box b, QuadMap Q,
   for (long w = w0; w < nruns; w += ws) {
     const long q = 32 * w + lane;
     bool same = true;
-    if (q < b.n / 4) {
-      const long m = quad_of(q, Q, b).r0 / 2;
-      same = code[m] == major && code[m + 1] == major && code[h + m] == major && code[h + m + 1] == major;
+    if (q < b.n / unit) {
+      const long m = unit_of<unit>(q, Q, b).r0 / 2;
+      for (int t = 0; t < unit / 2; ++t) same = same && code[m + t] == major && code[h + m + t] == major;
     }
     same = __all_sync(0xffffffffu, same);
     if (lane == 0) runs[w] = same ? 1 : 0;
@@ -92,6 +93,7 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
   out.code.release();
   out.tab.release();
   out.runs.release();
+  out.runs8.release();
   out.K = 0;
   out.W = W;
   if (nrec <= 0 || W <= 0) return false;
@@ -180,7 +182,12 @@ void mark_runs(cudaStream_t st, Classes<T> &c, const Box &b) {
   const long nruns = (b.n / 4 + 31) / 32;
   c.runs.alloc((size_t)nruns);
   LaunchScope ls(K_SETUP, st, 0.0);
-  k_mark_runs<<<grid_of(32 * nruns), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b), c.major, c.runs.p, nruns);
+  k_mark_runs<4><<<grid_of(32 * nruns), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b), c.major, c.runs.p, nruns);
+  if (b.nx % 8 == 0) {
+    const long n8 = (b.n / 8 + 31) / 32;
+    c.runs8.alloc((size_t)n8);
+    k_mark_runs<8><<<grid_of(32 * n8), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b, 8), c.major, c.runs8.p, n8);
+  }
 }
 
 template void mark_runs<float>(cudaStream_t, Classes<float> &, const Box &);

@@ -91,13 +91,14 @@ struct Classes {
   int K = 0, W = 0;
   int major = 0;             // the class of most records
   std::vector<T> major_rec;  // its record
-  DBuf<uint8_t> runs;        // per 32 quads of a level: all their records are of the major class (mark_runs)
+  DBuf<uint8_t> runs, runs8; // per 32 quads (octets) of a level: all their records are of the major class (mark_runs)
   bool ok() const { return code.p != nullptr; }
-  size_t bytes() const { return code.bytes() + tab.bytes() + runs.bytes(); }
+  size_t bytes() const { return code.bytes() + tab.bytes() + runs.bytes() + runs8.bytes(); }
 };
 struct Box;
 // Fills c.runs for colour-split codes ([colour][n / 2]) of a level of box b
-// (b.nx % 4 == 0), quads in the order of QuadMap.
+// (b.nx % 4 == 0), quads in the order of QuadMap, and c.runs8 for its octets
+// when b.nx % 8 == 0.
 template <class T>
 void mark_runs(cudaStream_t st, Classes<T> &c, const Box &b);
 // Fills c for the records rec[t * W .. t * W + W) (device memory, t < nrec).
@@ -144,30 +145,32 @@ struct QuadMap {
   long nint = 0;  // ... of all lines
   FastDiv dw;
 };
-inline QuadMap make_quad_map(const Box &b) {
+// (unit 8: octets, eight points, nx % 8 == 0.)
+inline QuadMap make_quad_map(const Box &b, int unit = 4) {
   QuadMap m;
-  m.w = b.nx / 4 > 2 ? b.nx / 4 - 2 : 0;
+  m.w = b.nx / unit > 2 ? b.nx / unit - 2 : 0;
   m.nint = (long)m.w * b.ny * b.nz;
   m.dw = make_fastdiv((unsigned)(m.w > 0 ? m.w : 1));
   return m;
 }
-// Quad q: the points r0 .. r0 + 3 of line (j, k) from column i0.
+// Quad (octet) q: the points r0 .. r0 + unit - 1 of line (j, k) from column i0.
 struct Quad {
   long r0;
   int i0, j, k;
 };
 __device__ __forceinline__ unsigned fast_div(unsigned n, FastDiv f);
-__device__ __forceinline__ Quad quad_of(long q, const QuadMap &m, const Box &b) {
+template <int unit>
+__device__ __forceinline__ Quad unit_of(long q, const QuadMap &m, const Box &b) {
   Quad g;
   unsigned line;
   if (q < m.nint) {
     line = fast_div((unsigned)q, m.dw);
-    g.i0 = 4 * (int)((unsigned)q - line * (unsigned)m.w + 1u);
+    g.i0 = unit * (int)((unsigned)q - line * (unsigned)m.w + 1u);
   } else {
     const unsigned e = (unsigned)(q - m.nint);
-    if (b.nx > 4) {
+    if (b.nx > unit) {
       line = e >> 1;
-      g.i0 = (e & 1) ? b.nx - 4 : 0;
+      g.i0 = (e & 1) ? b.nx - unit : 0;
     } else {  // one quad a line
       line = e;
       g.i0 = 0;
@@ -179,6 +182,7 @@ __device__ __forceinline__ Quad quad_of(long q, const QuadMap &m, const Box &b) 
   g.r0 = (long)line * b.nx + g.i0;
   return g;
 }
+__device__ __forceinline__ Quad quad_of(long q, const QuadMap &m, const Box &b) { return unit_of<4>(q, m, b); }
 
 // 7-point operator on a solve box: coefficient planes [7][n] (C,-x,+x,-y,+y,-z,+z).
 struct Op7 {

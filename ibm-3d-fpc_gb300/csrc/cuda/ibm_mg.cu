@@ -983,6 +983,251 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_quad(Recs<float, 8> R, Un
                      (long)gridDim.x * blockDim.x);
 }
 
+// Colour-split form of the finest FP32 level within one V-cycle (nx a multiple
+// of 8): x and b are kept as [colour][n / 2], a point at the index of its pair,
+// so a phase reads the other colour's x and its own colour's b and writes its
+// own colour's x, 6 bytes a point of the level where the pairs in one array
+// move 12 (every sector holds both colours), and a thread makes four points
+// from the 16-byte loads that make two otherwise. A point's y and z neighbours
+// have its own pair index in their lines; of its x neighbours one is of its own
+// pair, the other of the pair before (even column) or after. The input load
+// splits, the output store joins, the residual is written joined for the
+// restriction, and the interpolation adds to colour 1 only: a phase needs no
+// values of its own colour, so what the first phase after it overwrites is not
+// read. Per point the arithmetic is k_relax_rb's, in the same order. Bound: L2
+// (HBM above about 20M points). Steps, joined against split: mixed 640x128x128
+// 17.10 -> 15.53 ms, 320x64x64 4854 -> 4711 us, pressure solve 512x96x96 with FP64
+// basis 6975 -> 6418 us, twelve channels 29.4 -> 28.2 ms (78 registers; four
+// blocks per SM at 64 with spills: 15.54 ms, 4812, 6423, 28.8).
+struct OctX {
+  float4 c, s, n, b, t;  // the other colour on the octet's line and the four lines around it
+  float side;            // and its value beyond the octet that the first (last) point needs
+};
+// xo: the other colour's values; e: the phase's points lie on columns 2 m + e.
+__device__ __forceinline__ OctX load_oct(const float *xo, const Quad &g, const Box &bx, int e) {
+  const long m = g.r0 / 2, sy = bx.nx / 2, sz = (long)(bx.nx / 2) * bx.ny;
+  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float *p = xo + m;
+  OctX v;
+  v.c = *reinterpret_cast<const float4 *>(p);
+  v.s = g.j > 0 ? *reinterpret_cast<const float4 *>(p - sy) : z4;
+  v.n = g.j < bx.ny - 1 ? *reinterpret_cast<const float4 *>(p + sy) : z4;
+  v.b = g.k > 0 ? *reinterpret_cast<const float4 *>(p - sz) : z4;
+  v.t = g.k < bx.nz - 1 ? *reinterpret_cast<const float4 *>(p + sz) : z4;
+  const bool has = e ? g.i0 + 8 < bx.nx : g.i0 > 0;
+  v.side = has ? p[e ? 4 : -1] : 0.0f;
+  return v;
+}
+__device__ __forceinline__ void oct_row(const OctX &v, int e, int u, float (&x)[6]) {
+  const float c[4] = {v.c.x, v.c.y, v.c.z, v.c.w}, s[4] = {v.s.x, v.s.y, v.s.z, v.s.w},
+              n[4] = {v.n.x, v.n.y, v.n.z, v.n.w}, b[4] = {v.b.x, v.b.y, v.b.z, v.b.w},
+              t[4] = {v.t.x, v.t.y, v.t.z, v.t.w};
+  x[0] = e ? c[u] : u > 0 ? c[u > 0 ? u - 1 : 0] : v.side;
+  x[1] = e ? (u < 3 ? c[u < 3 ? u + 1 : 3] : v.side) : c[u];
+  x[2] = s[u]; x[3] = n[u]; x[4] = b[u]; x[5] = t[u];
+}
+__device__ __forceinline__ float relax_point(const float *c, float b, const float (&x)[6]) {
+  float acc = 0.0f;
+#pragma unroll
+  for (int s = 0; s < 6; ++s) acc = fmaf(c[1 + s], x[s], acc);
+  return c[0] * (b - acc);
+}
+__device__ __forceinline__ float resid_point(const float *c, float b, float xc, const float (&x)[6]) {
+  float acc = fmaf(c[7], xc, 0.0f);
+#pragma unroll
+  for (int s = 0; s < 6; ++s) acc = fmaf(c[1 + s], x[s], acc);
+  return b - acc;
+}
+// Eight points of a line from its two colours' values, the first on even
+// columns or (odd) on odd ones.
+__device__ __forceinline__ void join(const float (&a)[4], const float (&b)[4], int odd, float (&o)[8]) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    o[2 * u] = odd ? b[u] : a[u];
+    o[2 * u + 1] = odd ? a[u] : b[u];
+  }
+}
+__device__ __forceinline__ float4 vec(const float *a) { return make_float4(a[0], a[1], a[2], a[3]); }
+
+// The input load and the first phase from a zero guess: b split, colour 0 of x.
+// vec4: FP32 source, 16-byte aligned, scaled in FP32 (k_load_input_f4's
+// arithmetic); else k_load_input's.
+__global__ void __launch_bounds__(kThreads) k_split_in(Recs<float, 8> R, Uni8 U, QuadMap Q, float *bs, float *xs, Box bx,
+                                                       VecRef in, int vec4, const double *winv, const float *winvf,
+                                                       const int *gate) {
+  if (gate_off(gate)) return;
+  const long n8 = bx.n / 8, h = bx.n / 2;
+  const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
+  const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
+  const double *src = in.base + off;
+  const float *srcf = in.basef ? in.basef + off : nullptr;
+  const bool wide = !srcf && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n8; q += (long)gridDim.x * blockDim.x) {
+    const Quad g = unit_of<8>(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    float a[8];
+    if (vec4) {
+      const float f = in.inu ? (float)sc : 1.0f;
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        float4 w = *reinterpret_cast<const float4 *>(srcf + g.r0 + 4 * v);
+        w.x *= f; w.y *= f; w.z *= f; w.w *= f;
+        if (winvf) {
+          const float4 d = *reinterpret_cast<const float4 *>(winvf + g.r0 + 4 * v);
+          w.x *= d.x; w.y *= d.y; w.z *= d.z; w.w *= d.w;
+        }
+        a[4 * v] = w.x; a[4 * v + 1] = w.y; a[4 * v + 2] = w.z; a[4 * v + 3] = w.w;
+      }
+    } else {
+      double d[8];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        if (wide) {
+          const double2 w = *reinterpret_cast<const double2 *>(src + g.r0 + 2 * v);
+          d[2 * v] = w.x;
+          d[2 * v + 1] = w.y;
+        } else {
+          d[2 * v] = srcf ? (double)srcf[g.r0 + 2 * v] : src[g.r0 + 2 * v];
+          d[2 * v + 1] = srcf ? (double)srcf[g.r0 + 2 * v + 1] : src[g.r0 + 2 * v + 1];
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        double w = in.inu ? d[v] * sc : d[v];
+        if (winv) w = w * winv[g.r0 + v];
+        a[v] = (float)w;
+      }
+    }
+    const int e = (g.j + g.k) & 1;  // columns of colour 0
+    const long m = g.r0 / 2;
+    float b0[4], b1[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      b0[u] = e ? a[2 * u + 1] : a[2 * u];
+      b1[u] = e ? a[2 * u] : a[2 * u + 1];
+    }
+    *reinterpret_cast<float4 *>(bs + m) = vec(b0);
+    *reinterpret_cast<float4 *>(bs + h + m) = vec(b1);
+    if (uni) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) b0[u] = U.c[0] * b0[u];
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; u += 2) {
+        float c[2][8];
+        load_quad_recs(R, m + u, c);
+        b0[u] = c[0][0] * b0[u];
+        b0[u + 1] = c[1][0] * b0[u + 1];
+      }
+    }
+    *reinterpret_cast<float4 *>(xs + m) = vec(b0);
+  }
+}
+
+// A phase; the last one (OUT, colour 1) writes the joined level to the output
+// instead.
+template <bool OUT>
+__global__ void __launch_bounds__(kThreads, 3) k_split_phase(Recs<float, 8> R, Uni8 U, QuadMap Q,
+                                                          const float *__restrict__ bs, float *xs, Box bx, int color,
+                                                          OutRef out, const int *gate) {
+  if (gate_off(gate)) return;
+  const long n8 = bx.n / 8, h = bx.n / 2, own = color ? h : 0;
+  const float *xo = xs + (h - own);
+  const long off = OUT && out.idx ? (long)(*out.idx) * out.ld : 0;
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n8; q += (long)gridDim.x * blockDim.x) {
+    const Quad g = unit_of<8>(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    const int e = (g.j + g.k + color) & 1;
+    const long m = g.r0 / 2;
+    const OctX v = load_oct(xo, g, bx, e);
+    const float4 b4 = *reinterpret_cast<const float4 *>(bs + own + m);
+    const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
+    float o[4], x[6];
+    if (uni) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        oct_row(v, e, u, x);
+        o[u] = relax_point(U.c, bb[u], x);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; u += 2) {
+        float c[2][8];
+        load_quad_recs(R, own + m + u, c);
+        oct_row(v, e, u, x);
+        o[u] = relax_point(c[0], bb[u], x);
+        oct_row(v, e, u + 1, x);
+        o[u + 1] = relax_point(c[1], bb[u + 1], x);
+      }
+    }
+    if constexpr (OUT) {
+      const float other[4] = {v.c.x, v.c.y, v.c.z, v.c.w};
+      float z[8];
+      join(o, other, e, z);
+      if (out.d) {
+        double *zd = out.d + off + g.r0;
+        if ((reinterpret_cast<uintptr_t>(zd) & 15) == 0) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            reinterpret_cast<double2 *>(zd)[u] = make_double2((double)z[2 * u], (double)z[2 * u + 1]);
+        } else {
+          for (int u = 0; u < 8; ++u) zd[u] = (double)z[u];
+        }
+      } else {
+        float *zf = out.f + off + g.r0;
+        if ((reinterpret_cast<uintptr_t>(zf) & 15) == 0) {
+          reinterpret_cast<float4 *>(zf)[0] = vec(z);
+          reinterpret_cast<float4 *>(zf)[1] = vec(z + 4);
+        } else {
+          for (int u = 0; u < 8; ++u) zf[u] = z[u];
+        }
+      }
+    } else {
+      *reinterpret_cast<float4 *>(xs + own + m) = vec(o);
+    }
+  }
+}
+
+// The residual after a colour-1 phase, joined: colour 0 as computed, colour 1
+// zero.
+__global__ void __launch_bounds__(kThreads, 3) k_split_residual(Recs<float, 8> R, Uni8 U, QuadMap Q,
+                                                             const float *__restrict__ bs, const float *__restrict__ xs,
+                                                             float *__restrict__ res, Box bx, const int *gate) {
+  if (gate_off(gate)) return;
+  const long n8 = bx.n / 8, h = bx.n / 2;
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n8; q += (long)gridDim.x * blockDim.x) {
+    const Quad g = unit_of<8>(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    const int e = (g.j + g.k) & 1;
+    const long m = g.r0 / 2;
+    const OctX v = load_oct(xs + h, g, bx, e);
+    const float4 b4 = *reinterpret_cast<const float4 *>(bs + m), x4 = *reinterpret_cast<const float4 *>(xs + m);
+    const float bb[4] = {b4.x, b4.y, b4.z, b4.w}, xc[4] = {x4.x, x4.y, x4.z, x4.w};
+    const float zero[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float o[4], x[6], z[8];
+    if (uni) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        oct_row(v, e, u, x);
+        o[u] = resid_point(U.c, bb[u], xc[u], x);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; u += 2) {
+        float c[2][8];
+        load_quad_recs(R, m + u, c);
+        oct_row(v, e, u, x);
+        o[u] = resid_point(c[0], bb[u], xc[u], x);
+        oct_row(v, e, u + 1, x);
+        o[u + 1] = resid_point(c[1], bb[u + 1], xc[u + 1], x);
+      }
+    }
+    join(o, zero, e, z);
+    *reinterpret_cast<float4 *>(res + g.r0) = vec(z);
+    *reinterpret_cast<float4 *>(res + g.r0 + 4) = vec(z + 4);
+  }
+}
+
 // One whole two-colour sweep of a 7-point FP32 level (colour 0, then colour
 // 1) in one kernel, out of place: x_new = sweep(x_old). A block takes a tile
 // of kSwJ x kSwK lines and kSwX points of each, loads x_old over the tile
@@ -1283,8 +1528,18 @@ __global__ void k_restrict_yz4(const float *__restrict__ res, const float *__res
                     (long)gridDim.x * blockDim.x);
 }
 
+// Adds four points' corrections to a colour-split level: the two of colour 1,
+// on columns 2 m + e.
+__device__ __forceinline__ void add_split(float *x, const Box &fb, long r0, int e, const float4 &corr) {
+  float2 *xo = reinterpret_cast<float2 *>(x + fb.n / 2 + r0 / 2);
+  float2 v = *xo;
+  v.x = v.x + (e ? corr.y : corr.x);
+  v.y = v.y + (e ? corr.w : corr.z);
+  *xo = v;
+}
 __device__ __forceinline__ void prolong_yz4_body(const float *xc, const Box &cb, const float *pm, const float *pp,
-                                                 const Box &fb, int d, float *x, int accumulate, long t0, long ts) {
+                                                 const Box &fb, int d, float *x, int accumulate, long t0, long ts,
+                                                 int split = 0) {
   const long n4 = fb.n / 4;
   const long plane_c = (long)cb.nx * cb.ny;
   const int ncd = d == 1 ? cb.ny : cb.nz;
@@ -1310,6 +1565,10 @@ __device__ __forceinline__ void prolong_yz4_body(const float *xc, const Box &cb,
       corr.z = fmaf(a.z, x1.z, b.z * x0.z);
       corr.w = fmaf(a.w, x1.w, b.w * x0.w);
     }
+    if (split) {
+      add_split(x, fb, 4 * t, (y + k + 1) & 1, corr);
+      continue;
+    }
     float4 *xo = reinterpret_cast<float4 *>(x + 4 * t);
     if (accumulate) {
       const float4 xv = *xo;
@@ -1319,11 +1578,11 @@ __device__ __forceinline__ void prolong_yz4_body(const float *xc, const Box &cb,
   }
 }
 __global__ void k_prolong_yz4(const float *__restrict__ xc, Box cb, const float *__restrict__ pm,
-                              const float *__restrict__ pp, Box fb, int d, float *x, int accumulate,
+                              const float *__restrict__ pp, Box fb, int d, float *x, int accumulate, int split,
                               const int *gate) {
   if (gate_off(gate)) return;
   prolong_yz4_body(xc, cb, pm, pp, fb, d, x, accumulate, (long)blockIdx.x * blockDim.x + threadIdx.x,
-                   (long)gridDim.x * blockDim.x);
+                   (long)gridDim.x * blockDim.x, split);
 }
 
 // Restriction / interpolation along x on FP32 levels with fine nx = 2 coarse
@@ -1373,7 +1632,8 @@ __global__ void k_restrict_x4(const float *__restrict__ res, const float *__rest
 }
 
 __device__ __forceinline__ void prolong_x4_body(const float *xc, const Box &cb, const float *pm, const float *pp,
-                                                const Box &fb, float *x, int accumulate, long t0, long ts) {
+                                                const Box &fb, float *x, int accumulate, long t0, long ts,
+                                                int split = 0) {
   const long n4 = fb.n / 4;
   for (long t = t0; t < n4; t += ts) {
     const long r0 = 4 * t;
@@ -1389,6 +1649,11 @@ __device__ __forceinline__ void prolong_x4_body(const float *xc, const Box &cb, 
     corr.y = fmaf(a.y, c01.y, m.y * c01.x);
     corr.z = c01.y;
     corr.w = fmaf(a.w, c2, m.w * c01.y);
+    if (split) {
+      const unsigned k = fast_div(line, fb.dy), j = line - k * (unsigned)fb.ny;
+      add_split(x, fb, r0, (int)((j + k + 1) & 1), corr);
+      continue;
+    }
     float4 *xo = reinterpret_cast<float4 *>(x + r0);
     if (accumulate) {
       const float4 xv = *xo;
@@ -1398,10 +1663,10 @@ __device__ __forceinline__ void prolong_x4_body(const float *xc, const Box &cb, 
   }
 }
 __global__ void k_prolong_x4(const float *__restrict__ xc, Box cb, const float *__restrict__ pm,
-                             const float *__restrict__ pp, Box fb, float *x, int accumulate, const int *gate) {
+                             const float *__restrict__ pp, Box fb, float *x, int accumulate, int split, const int *gate) {
   if (gate_off(gate)) return;
   prolong_x4_body(xc, cb, pm, pp, fb, x, accumulate, (long)blockIdx.x * blockDim.x + threadIdx.x,
-                  (long)gridDim.x * blockDim.x);
+                  (long)gridDim.x * blockDim.x, split);
 }
 
 template <class T>
@@ -1520,21 +1785,25 @@ __device__ __forceinline__ T prolonged(const Group<T> &G, const T *xc, int i, in
 }
 template <class T, int M>
 __device__ __forceinline__ void prolong_group_body(const Group<T> &G, const T *xc, T *x, int accumulate, long t0,
-                                                   long ts) {
+                                                   long ts, int split = 0) {
   const Box &b = G.s[0].b;
   for (long r = t0; r < b.n; r += ts) {
     int i, j, k;
     box_ijk(r, b, i, j, k);
     const T corr = prolonged<T, 0, M>(G, xc, i, j, k, true);
+    if (split) {  // a colour-split level: colour 1 only
+      if ((i + j + k) & 1) x[b.n / 2 + (r >> 1)] = x[b.n / 2 + (r >> 1)] + corr;
+      continue;
+    }
     x[r] = accumulate ? x[r] + corr : corr;
   }
 }
 template <class T, int M>
 __global__ void __launch_bounds__(kThreads) k_prolong_group(Group<T> G, const T *__restrict__ xc, T *x, int accumulate,
-                                                            const int *gate) {
+                                                            int split, const int *gate) {
   if (gate_off(gate)) return;
   prolong_group_body<T, M>(G, xc, x, accumulate, (long)blockIdx.x * blockDim.x + threadIdx.x,
-                           (long)gridDim.x * blockDim.x);
+                           (long)gridDim.x * blockDim.x, split);
 }
 
 // Coarsest level: x = Ainv b (one warp per row).
@@ -2117,6 +2386,11 @@ static Uni8 uni8_of(const Classes<float> &c) {
     std::copy(c.major_rec.begin(), c.major_rec.end(), u.c);
     u.runs = c.runs.p;
   }
+  return u;
+}
+static Uni8 uni8_octs(const Classes<float> &c) {
+  Uni8 u = uni8_of(c);
+  u.runs = c.runs8.p;
   return u;
 }
 
@@ -2746,7 +3020,7 @@ template <class T>
 static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgParams &p, const int *gate,
                  const VecRef *fin = nullptr, const OutRef *fout = nullptr, const float *winvf = nullptr,
                  const TailLaunch *tail = nullptr, const ClusterPlan *clu = nullptr, const double *winv = nullptr,
-                 bool fused = false) {
+                 bool fused = false, bool split = false) {
   MgLevelT<T> &F = L[l];
   const long n = F.b.n;
   const double T_ = sizeof(T);
@@ -2771,8 +3045,29 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   if constexpr (sizeof(T) == 4) U7 = uni8_of(F.rbc);
   const QuadMap Q = make_quad_map(F.b);
   const double rec7 = R7.code ? 2.0 : 8.0 * T_, rec27 = R27.code ? 2.0 : 28.0 * T_;
+  const QuadMap O = make_quad_map(F.b, 8);
+  Uni8 U8;
+  if constexpr (sizeof(T) == 4) {
+    if (split) U8 = uni8_octs(F.rbc);
+  }
   auto relax = [&](bool zero, bool last) {
     if constexpr (sizeof(T) == 4) {
+      if (split) {
+        const long n8 = n / 8;
+        const double phase = 0.5 * n * rec7 + 1.5 * T_ * n;
+        if (zero) {
+          const int vec4 = fin->basef && fin->ld % 4 == 0;
+          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? 2.0 : T_) + (vec4 ? (winvf ? 4.0 : 3.0) : (winv ? 6.0 : 4.0)) * T_ * n);
+          k_split_in<<<resident_grid(k_split_in, n8), block_of(n8), 0, st>>>(R7, U8, O, F.bv.p, cur, F.b, *fin, vec4, winv, winvf, gate);
+        } else {
+          LaunchScope ls(K_MG_RELAX_FINE, st, phase);
+          k_split_phase<false><<<resident_grid(k_split_phase<false>, n8), block_of(n8), 0, st>>>(R7, U8, O, F.bv.p, cur, F.b, 0, OutRef(), gate);
+        }
+        LaunchScope ls(K_MG_RELAX_FINE, st, last ? phase + (fout->d ? 1.5 : 0.5) * T_ * n : phase);
+        if (last) k_split_phase<true><<<resident_grid(k_split_phase<true>, n8), block_of(n8), 0, st>>>(R7, U8, O, F.bv.p, cur, F.b, 1, *fout, gate);
+        else k_split_phase<false><<<resident_grid(k_split_phase<false>, n8), block_of(n8), 0, st>>>(R7, U8, O, F.bv.p, cur, F.b, 1, OutRef(), gate);
+        return;
+      }
       if (p.relax == 2 && rb7 && quad && p.fused_sweep && !(zero && fin) && !(last && fout)) {
         // both colour phases in one kernel, out of place
         LaunchScope ls(K_MG_RELAX_FINE, st, (zero ? 0.5 * n * (R7.code ? 2.0 : T_) + 1.5 * T_ * n
@@ -2879,7 +3174,10 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
     LaunchScope ls(K_MG_RESID, st, 0.5 * n * rec7 + 2.5 * T_ * n);
     bool done = false;
     if constexpr (sizeof(T) == 4) {
-      if (quad) {
+      if (split) {
+        k_split_residual<<<resident_grid(k_split_residual, n / 8), block_of(n / 8), 0, st>>>(R7, U8, O, F.bv.p, cur, F.r.p, F.b, gate);
+        done = true;
+      } else if (quad) {
         k_residual_rb_quad<<<resident_grid(k_residual_rb_quad, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.r.p, F.b, gate);
         done = true;
       }
@@ -2937,14 +3235,14 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   {
     LaunchScope ls(K_MG_PROLONG, st, T_ * ((nu1 > 0 ? 4.0 : 3.0) * n + C.b.n));
     if (G.n == 3)
-      k_prolong_group<T, 3><<<resident_grid(k_prolong_group<T, 3>, n), block_of(n), 0, st>>>(G, xc, cur, nu1 > 0, gate);
+      k_prolong_group<T, 3><<<resident_grid(k_prolong_group<T, 3>, n), block_of(n), 0, st>>>(G, xc, cur, nu1 > 0, split, gate);
     else if (G.n == 2)
-      k_prolong_group<T, 2><<<resident_grid(k_prolong_group<T, 2>, n), block_of(n), 0, st>>>(G, xc, cur, nu1 > 0, gate);
+      k_prolong_group<T, 2><<<resident_grid(k_prolong_group<T, 2>, n), block_of(n), 0, st>>>(G, xc, cur, nu1 > 0, split, gate);
     else if constexpr (sizeof(T) == 4) {
       if (F.cdir != 0 && F.b.nx % 4 == 0)
-        k_prolong_yz4<<<resident_grid(k_prolong_yz4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
+        k_prolong_yz4<<<resident_grid(k_prolong_yz4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, split, gate);
       else if (p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0)
-        k_prolong_x4<<<resident_grid(k_prolong_x4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, cur, nu1 > 0, gate);
+        k_prolong_x4<<<resident_grid(k_prolong_x4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, cur, nu1 > 0, split, gate);
       else
         k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
     } else {
@@ -2985,8 +3283,13 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
       run_cluster<float>(st, L32, clu32_, in, out, winv_, winvf_.p, gate);
       return;
     }
-    if (fuse) {
-      vcycle<float>(st, L32, 0, prm, gate, &in, &out, winvf_.p, tp, c32, nullptr, fused);
+    // x and b of the finest level by colour (k_split_phase) where its lines are
+    // whole octets; a single application keeps the joined form, whose input load
+    // and output store are launches of their own in the profile
+    const bool split = fused && prm.quads && !prm.fused_sweep && prm.relax == 2 && F.relax && F.cdir >= 0 && F.ns == 7 &&
+                       (F.rb.p || F.rbc.ok()) && F.b.nx % 8 == 0 && prm.nu1 > 0 && prm.nu2 > 0;
+    if (split || fuse) {
+      vcycle<float>(st, L32, 0, prm, gate, &in, &out, winvf_.p, tp, c32, winv_, fused, split);
       return;
     }
     {
