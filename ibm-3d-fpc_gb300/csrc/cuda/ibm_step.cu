@@ -414,37 +414,59 @@ __global__ void __launch_bounds__(kThreads) k_split_fields(SplitArgs A) {
 
 // ------------------------------------------------------------------ tilde
 // ut = u, interior faces <- solve-box x (gpu_dense_ops.hpp:20-22); flags non-finite x.
-__global__ void k_scatter(const double *u, const double *v, const double *w, const double *xu, const double *xv,
-                          const double *xw, double *ut, double *vt, double *wt, Dims d, StepDiag *dg) {
+// A copy: one loop per field, four faces of a thread in flight together, and u
+// only read where it is kept. 640x128x128: 237 -> 77 us (before: u read
+// everywhere, one load in flight).
+constexpr int kFlight = 4;
+__global__ void __launch_bounds__(kThreads) k_scatter(const double *__restrict__ u, const double *__restrict__ v,
+                                                      const double *__restrict__ w, const double *__restrict__ xu,
+                                                      const double *__restrict__ xv, const double *__restrict__ xw,
+                                                      double *__restrict__ ut, double *__restrict__ vt,
+                                                      double *__restrict__ wt, Dims d, StepDiag *dg) {
   const long NU = (long)(d.nx + 1) * d.ny * d.nz, NV = (long)d.nx * (d.ny + 1) * d.nz,
              NW = (long)d.nx * d.ny * (d.nz + 1);
+  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
   int bad = 0;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < NU + NV + NW; t += (long)gridDim.x * blockDim.x) {
-    if (t < NU) {
-      const long f = t;
-      long q;
-      const int i = udivmod(f, d.dnx1, q);
-      double val = u[f];
-      if (i >= 1 && i <= d.nx - 1) { val = xu[q * (d.nx - 1) + (i - 1)]; bad |= !isfinite(val); }
-      ut[f] = val;
-    } else if (t < NU + NV) {
-      const long f = t - NU;
-      long q;
-      const int i = udivmod(f, d.dnx, q);
-      long kq;
-      const int j = udivmod(q, d.dny1, kq), k = (int)kq;
-      double val = v[f];
-      if (j >= 1 && j <= d.ny - 1) { val = xv[((long)k * (d.ny - 1) + (j - 1)) * d.nx + i]; bad |= !isfinite(val); }
-      vt[f] = val;
-    } else {
-      const long f = t - NU - NV;
-      const long plane = (long)d.nx * d.ny;
-      const int k = (int)(f / plane);
-      double val = w[f];
-      if (k >= 1 && k <= d.nz - 1) { val = xw[f - plane]; bad |= !isfinite(val); }
-      wt[f] = val;
+  // faces t, t + ts, ...: from(f, inner) gives the address of the value and whether it is x's
+  auto copy = [&](double *out, long n, auto from) {
+    for (long t = t0; t < n; t += kFlight * ts) {
+      double val[kFlight];
+      bool inner[kFlight];
+#pragma unroll
+      for (int q = 0; q < kFlight; ++q) {
+        const long f = t + q * ts;
+        inner[q] = false;
+        val[q] = 0.0;
+        if (f < n) val[q] = *from(f, inner[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < kFlight; ++q) {
+        const long f = t + q * ts;
+        if (f >= n) break;
+        bad |= inner[q] && !isfinite(val[q]);
+        out[f] = val[q];
+      }
     }
-  }
+  };
+  copy(ut, NU, [&](long f, bool &inner) {
+    long q;
+    const int i = udivmod(f, d.dnx1, q);
+    inner = i >= 1 && i <= d.nx - 1;
+    return inner ? xu + q * (d.nx - 1) + (i - 1) : u + f;
+  });
+  copy(vt, NV, [&](long f, bool &inner) {
+    long q;
+    const int i = udivmod(f, d.dnx, q);
+    long kq;
+    const int j = udivmod(q, d.dny1, kq), k = (int)kq;
+    inner = j >= 1 && j <= d.ny - 1;
+    return inner ? xv + ((long)k * (d.ny - 1) + (j - 1)) * d.nx + i : v + f;
+  });
+  const long plane = (long)d.nx * d.ny;
+  copy(wt, NW, [&](long f, bool &inner) {
+    inner = f >= plane && f < NW - plane;
+    return inner ? xw + f - plane : w + f;
+  });
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(&dg->nonfinite_mom, 1);
 }
 
@@ -473,6 +495,38 @@ __device__ __forceinline__ double div_cell(const double *Dc, long NPc, long c, d
   s = fma(Dc[5 * NPc + c], qt, s);
   return s;
 }
+
+// A cell's six face values and its flag.
+struct CellFaces {
+  double w, e, s, n, b, t;
+  int i, j, k;
+  uint8_t fl;
+};
+__device__ __forceinline__ CellFaces cell_faces(const Dims &d, const double *u, const double *v, const double *w,
+                                                const uint8_t *fc, long c) {
+  CellFaces q;
+  q.fl = fc[c];
+  long r, kq;
+  q.i = udivmod(c, d.dnx, r);
+  q.j = udivmod(r, d.dny, kq);
+  q.k = (int)kq;
+  const long fw_ = U3(d, q.i, q.j, q.k), fs = V3(d, q.i, q.j, q.k);
+  q.w = u[fw_]; q.e = u[fw_ + 1];
+  q.s = v[fs]; q.n = v[fs + d.nx];
+  q.b = w[c]; q.t = w[c + (long)d.nx * d.ny];
+  return q;
+}
+// D q of a cell with the common row and q faces all around.
+__device__ __forceinline__ double div_plain(const Plain &p, const CellFaces &q) {
+  double s = fma(p.D[0], q.w, 0.0);
+  s = fma(p.D[1], q.e, s);
+  s = fma(p.D[2], q.s, s);
+  s = fma(p.D[3], q.n, s);
+  s = fma(p.D[4], q.b, s);
+  s = fma(p.D[5], q.t, s);
+  return s;
+}
+constexpr int kCellsAhead = 2;  // cells of a thread whose loads are in flight together
 
 __global__ void __launch_bounds__(kThreads) k_pressure_rhs(DivArgs A) {
   const Dims &d = A.d;
@@ -510,8 +564,6 @@ struct ProjArgs {
   Plain plain;
 };
 
-__device__ __forceinline__ double phi_at(const ProjArgs &A, long c) { return (A.fc[c] & kFluid) ? A.phi[c] : 0.0; }
-
 // q = q~ - (dt/rho) G phi on q-faces, other faces keep q~; p += phi on fluid cells.
 __global__ void __launch_bounds__(kThreads, 4) k_project(ProjArgs A) {
   const Dims &d = A.d;
@@ -520,41 +572,60 @@ __global__ void __launch_bounds__(kThreads, 4) k_project(ProjArgs A) {
   const double nf = -A.factor;
   int bad = 0;
   const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
-  // One loop per field. The common face reads its flag, its value and the two
-  // phi and nothing else (no G pair, no cell flags), and none of its loads
-  // waits for another but the flag. 640x128x128: 519 -> 390 us, bound by HBM
-  // (8.6 values a cell) and three FP64 operations a face.
-  auto face = [&](uint8_t fl, double val, int f, long lo, long hi, bool has_lo, bool has_hi, const double *G, long NF,
-                  long g) {
-    if (fl & kPlainFace) return fma(nf, grad_face(A.plain.gl[f], A.phi[lo], A.plain.gr[f], A.phi[hi]), val);
-    if (!(fl & kQFace)) return val;
-    const double pl = has_lo ? phi_at(A, lo) : 0.0, pr = has_hi ? phi_at(A, hi) : 0.0;
-    return fma(nf, grad_face(G[g], pl, G[NF + g], pr), val);
+  // One loop per field, two faces of a thread at a time with their flags,
+  // values and phi loaded before the flags say which are used; the common face
+  // needs no more (no G pair, no cell flags). 640x128x128: 519 us with G read
+  // and cells tested everywhere, 390 with phi loaded after the flag, 310 now (HBM and FP64 floors 130 and 150).
+  auto faces = [&](const uint8_t *fl, const double *qt, double *out, long n, int f, long below, const double *G, auto cell) {
+    for (long t = t0; t < n; t += kCellsAhead * ts) {
+      uint8_t m[kCellsAhead];
+      double val[kCellsAhead], pl[kCellsAhead], pr[kCellsAhead];
+      long c[kCellsAhead];
+      bool lo[kCellsAhead], hi[kCellsAhead];
+#pragma unroll
+      for (int h = 0; h < kCellsAhead; ++h) {
+        const long g = t + h * ts < n ? t + h * ts : t;
+        m[h] = fl[g];
+        val[h] = qt[g];
+        c[h] = cell(g, lo[h], hi[h]);  // the cell above the face
+        pl[h] = lo[h] ? A.phi[c[h] - below] : 0.0;
+        pr[h] = hi[h] ? A.phi[c[h]] : 0.0;
+      }
+#pragma unroll
+      for (int h = 0; h < kCellsAhead; ++h) {
+        const long g = t + h * ts;
+        if (g >= n) break;
+        double r = val[h];
+        if (m[h] & kPlainFace) {
+          r = fma(nf, grad_face(A.plain.gl[f], pl[h], A.plain.gr[f], pr[h]), r);
+        } else if (m[h] & kQFace) {
+          const double a = lo[h] && (A.fc[c[h] - below] & kFluid) ? pl[h] : 0.0;
+          const double b = hi[h] && (A.fc[c[h]] & kFluid) ? pr[h] : 0.0;
+          r = fma(nf, grad_face(G[g], a, G[n + g], b), r);
+        }
+        out[g] = r;
+      }
+    }
   };
-  for (long f = t0; f < NU; f += ts) {
-    const uint8_t fl = A.fu[f];
-    const double val = A.ut[f];
+  const long plane = (long)d.nx * d.ny;
+  faces(A.fu, A.ut, A.u, NU, 0, 1, A.Gu, [&](long g, bool &lo, bool &hi) {
     long q;
-    const int i = udivmod(f, d.dnx1, q);
-    const long c = q * d.nx + i;  // cell i of the face's line
-    A.u[f] = face(fl, val, 0, c - 1, c, i > 0, i < d.nx, A.Gu, NU, f);
-  }
-  for (long f = t0; f < NV; f += ts) {
-    const uint8_t fl = A.fv[f];
-    const double val = A.vt[f];
+    const int i = udivmod(g, d.dnx1, q);
+    lo = i > 0; hi = i < d.nx;
+    return q * d.nx + i;
+  });
+  faces(A.fv, A.vt, A.v, NV, 1, d.nx, A.Gv, [&](long g, bool &lo, bool &hi) {
     long q;
-    const int i = udivmod(f, d.dnx, q);
+    const int i = udivmod(g, d.dnx, q);
     long kq;
     const int j = udivmod(q, d.dny1, kq), k = (int)kq;
-    const long c = P3(d, i, j, k);
-    A.v[f] = face(fl, val, 1, c - d.nx, c, j > 0, j < d.ny, A.Gv, NV, f);
-  }
-  const long plane = (long)d.nx * d.ny;
-  for (long f = t0; f < NW; f += ts) {
-    const uint8_t fl = A.fw[f];
-    const double val = A.wt[f];
-    A.w[f] = face(fl, val, 2, f - plane, f, f >= plane, f < NP, A.Gw, NW, f);
-  }
+    lo = j > 0; hi = j < d.ny;
+    return P3(d, i, j, k);
+  });
+  faces(A.fw, A.wt, A.w, NW, 2, plane, A.Gw, [&](long g, bool &lo, bool &hi) {
+    lo = g >= plane; hi = g < NP;
+    return g;
+  });
   for (long c = t0; c < NP; c += ts) {
     const double phi = A.phi[c];
     bad |= !isfinite(phi);
@@ -633,52 +704,51 @@ __global__ void __launch_bounds__(kThreads, 4) k_diagnostics(DiagArgs A) {
   unsigned long long um = 0, vm = 0, wm = 0;
   // Each cell reads its six faces: their magnitudes (the lower three, and the
   // upper ones on the last planes, so that every face is taken once or more),
-  // and for fluid cells their divergence. The common cell needs nothing else.
+  // and for fluid cells their divergence. The common cell needs nothing else: 8
+  // FP64 operations, a floor of 134 us at 640x128x128. Two cells of a thread
+  // in flight take 372, one took 421.
   const long plane = (long)d.nx * d.ny;
   auto top = [](unsigned long long &m, double x) {
     const unsigned long long key = mag_key(x);
     m = key > m ? key : m;
   };
-  for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < NP; c += (long)gridDim.x * blockDim.x) {
-    const uint8_t fl = A.fc[c];
-    long q;
-    const int i = udivmod(c, d.dnx, q);
-    long kq;
-    const int j = udivmod(q, d.dny, kq), k = (int)kq;
-    const long fw_ = U3(d, i, j, k), fe = fw_ + 1, fs = V3(d, i, j, k), fn = fs + d.nx, fb = c, ft = c + plane;
-    double qw = A.u[fw_], qe = A.u[fe], qs = A.v[fs], qn = A.v[fn], qb = A.w[fb], qt = A.w[ft];
-    top(um, qw); top(vm, qs); top(wm, qb);
-    if (i == d.nx - 1) top(um, qe);
-    if (j == d.ny - 1) top(vm, qn);
-    if (k == d.nz - 1) top(wm, qt);
-    if (!(fl & kFluid)) continue;
-    double s, lift;
-    if (fl & kPlainCell) {
-      s = fma(A.plain.D[0], qw, 0.0);
-      s = fma(A.plain.D[1], qe, s);
-      s = fma(A.plain.D[2], qs, s);
-      s = fma(A.plain.D[3], qn, s);
-      s = fma(A.plain.D[4], qb, s);
-      s = fma(A.plain.D[5], qt, s);
-      lift = 0.0;
-    } else {
-      const uint8_t mw = A.fu[fw_], me = A.fu[fe], ms = A.fv[fs], mn = A.fv[fn], mb = A.fw[fb], mt = A.fw[ft];
-      if (!((mw | me | ms | mn | mb | mt) & kBcSet)) {
-        // the six corrected values are the projected field
-        qw = (mw & kQFace) ? qw : 0.0;
-        qe = (me & kQFace) ? qe : 0.0;
-        qs = (ms & kQFace) ? qs : 0.0;
-        qn = (mn & kQFace) ? qn : 0.0;
-        qb = (mb & kQFace) ? qb : 0.0;
-        qt = (mt & kQFace) ? qt : 0.0;
+  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, ts = (long)gridDim.x * blockDim.x;
+  for (long t = t0; t < NP; t += kCellsAhead * ts) {
+    CellFaces cf[kCellsAhead];
+#pragma unroll
+    for (int h = 0; h < kCellsAhead; ++h) cf[h] = cell_faces(d, A.u, A.v, A.w, A.fc, t + h * ts < NP ? t + h * ts : t);
+#pragma unroll
+    for (int h = 0; h < kCellsAhead; ++h) {
+      const long c = t + h * ts;
+      if (c >= NP) break;
+      CellFaces &q = cf[h];
+      top(um, q.w); top(vm, q.s); top(wm, q.b);
+      if (q.i == d.nx - 1) top(um, q.e);
+      if (q.j == d.ny - 1) top(vm, q.n);
+      if (q.k == d.nz - 1) top(wm, q.t);
+      if (!(q.fl & kFluid)) continue;
+      double dv;
+      if (q.fl & kPlainCell) {
+        dv = div_plain(A.plain, q);
       } else {
-        boundary_q(A, c, i, j, k, qw, qe, qs, qn, qb, qt);
+        const long fw_ = U3(d, q.i, q.j, q.k), fs = V3(d, q.i, q.j, q.k);
+        const uint8_t mw = A.fu[fw_], me = A.fu[fw_ + 1], ms = A.fv[fs], mn = A.fv[fs + d.nx], mb = A.fw[c],
+                      mt = A.fw[c + plane];
+        if (!((mw | me | ms | mn | mb | mt) & kBcSet)) {
+          // the six corrected values are the projected field
+          q.w = (mw & kQFace) ? q.w : 0.0;
+          q.e = (me & kQFace) ? q.e : 0.0;
+          q.s = (ms & kQFace) ? q.s : 0.0;
+          q.n = (mn & kQFace) ? q.n : 0.0;
+          q.b = (mb & kQFace) ? q.b : 0.0;
+          q.t = (mt & kQFace) ? q.t : 0.0;
+        } else {
+          boundary_q(A, c, q.i, q.j, q.k, q.w, q.e, q.s, q.n, q.b, q.t);
+        }
+        dv = __dadd_rn(div_cell(A.Dc, NP, c, q.w, q.e, q.s, q.n, q.b, q.t), __dmul_rn(*A.ramp, A.div_bc[c]));
       }
-      s = div_cell(A.Dc, NP, c, qw, qe, qs, qn, qb, qt);
-      lift = A.div_bc[c];
+      div2 = __dadd_rn(div2, __dmul_rn(dv, dv));
     }
-    const double dv = __dadd_rn(s, __dmul_rn(*A.ramp, lift));
-    div2 = __dadd_rn(div2, __dmul_rn(dv, dv));
   }
   __shared__ double s_div[kWarps];
   __shared__ unsigned long long s_max[3][kWarps];
