@@ -1724,38 +1724,73 @@ struct Group {
   int n = 0;
 };
 
-// The vector after S restrictions at point (i, j, k) of its level (0, with
-// nothing loaded, when `in` is false). Every load is predicated and none waits
-// for a branch, so a thread's 27 values and their weights are in flight
-// together.
-template <class T, int S>
-__device__ __forceinline__ T restricted(const Group<T> &G, const T *r, int i, int j, int k, bool in) {
-  if constexpr (S == 0) {
-    const Box &b = G.s[0].b;
-    return in ? r[((long)k * b.ny + j) * b.nx + i] : T(0);
-  } else {
-    const GroupStage<T> &L = G.s[S - 1];
-    const int nd = L.d == 0 ? L.b.nx : L.d == 1 ? L.b.ny : L.b.nz, c2 = 2 * (L.d == 0 ? i : L.d == 1 ? j : k);
-    T acc = T(0);
+// A group's directions differ, so a stage moves a point's index on every level
+// by a constant: the indices of all points that a thread touches are its base
+// on the level plus a stride for each stage's step. (Each point's index from
+// its coordinates, with the directions looked up, was most of the kernels'
+// instructions. Steps in us: FP64 160x32x32 3625 -> 3544, mixed 97x33x21 3853 ->
+// 3795, 320x64x64 4632 -> 4437, twelve channels 28.0 -> 27.2 ms.)
+__device__ __forceinline__ int group_stride(const Box &b, int d) { return d == 0 ? 1 : d == 1 ? b.nx : b.nx * b.ny; }
+__device__ __forceinline__ int along(int d, const int (&c)[3]) { return d == 0 ? c[0] : d == 1 ? c[1] : c[2]; }
+__device__ __forceinline__ void set_along(int d, int v, int (&c)[3]) {
+  c[0] = d == 0 ? v : c[0];
+  c[1] = d == 1 ? v : c[1];
+  c[2] = d == 2 ? v : c[2];
+}
+__device__ __forceinline__ int extent(const Box &b, int d) { return d == 0 ? b.nx : d == 1 ? b.ny : b.nz; }
+__device__ __forceinline__ int index_of(const Box &b, const int (&c)[3]) { return (c[2] * b.ny + c[1]) * b.nx + c[0]; }
+
+// Restriction to a point of the group's last level: st[q][t], the step of
+// stage t on level q <= t; lo / hi: the stage's lower / upper fine point exists.
+template <int M>
+struct RestrictSteps {
+  int st[M][M];
+  bool lo[M], hi[M];
+};
+// The vector after S restrictions at the point whose indices on the levels
+// below S are id (0, with nothing loaded, when `in` is false). Every load is
+// predicated and none waits for a branch, so a thread's 27 values and their
+// weights are in flight together.
+template <class T, int M, int S>
+__device__ __forceinline__ T restricted(const Group<T> &G, const RestrictSteps<M> &C, const T *r, const int (&id)[M],
+                                        bool in) {
+  constexpr int s = S - 1;
+  const GroupStage<T> &L = G.s[s];
+  T acc = T(0);
 #pragma unroll
-    for (int fo = -1; fo <= 1; ++fo) {
-      const int f = c2 + fo;
-      const bool has = in && f >= 0 && f < nd;
-      const int fi = L.d == 0 ? f : i, fj = L.d == 1 ? f : j, fk = L.d == 2 ? f : k;
-      T w = T(1);
-      if (fo != 0) w = has ? (fo < 0 ? L.pp : L.pm)[((long)fk * L.b.ny + fj) * L.b.nx + fi] : T(0);
-      const T v = restricted<T, S - 1>(G, r, fi, fj, fk, has);
-      acc = has ? fmat<T>(w, v, acc) : acc;
-    }
-    return acc;
+  for (int fo = -1; fo <= 1; ++fo) {
+    const bool has = in && (fo < 0 ? C.lo[s] : fo > 0 ? C.hi[s] : true);
+    int to[M] = {};
+#pragma unroll
+    for (int q = 0; q <= s; ++q) to[q] = id[q] + fo * C.st[q][s];
+    T w = T(1);
+    if (fo != 0) w = has ? (fo < 0 ? L.pp : L.pm)[to[s]] : T(0);
+    T v;
+    if constexpr (s == 0) v = has ? r[to[0]] : T(0);
+    else v = restricted<T, M, S - 1>(G, C, r, to, has);
+    acc = has ? fmat<T>(w, v, acc) : acc;
   }
+  return acc;
 }
 template <class T, int M>
 __device__ __forceinline__ void restrict_group_body(const Group<T> &G, const T *r, T *bc, long t0, long ts) {
+  RestrictSteps<M> C;
+#pragma unroll
+  for (int t = 0; t < M; ++t)
+#pragma unroll
+    for (int q = 0; q <= t; ++q) C.st[q][t] = group_stride(G.s[q].b, G.s[t].d);
   for (long I = t0; I < G.cb.n; I += ts) {
-    int i, j, k;
-    box_ijk(I, G.cb, i, j, k);
-    bc[I] = restricted<T, M>(G, r, i, j, k, true);
+    int c[3], id[M];
+    box_ijk(I, G.cb, c[0], c[1], c[2]);
+#pragma unroll
+    for (int t = M - 1; t >= 0; --t) {
+      const int d = G.s[t].d, f = 2 * along(d, c);
+      C.lo[t] = f > 0;
+      C.hi[t] = f + 1 < extent(G.s[t].b, d);
+      set_along(d, f, c);
+      id[t] = index_of(G.s[t].b, c);
+    }
+    bc[I] = restricted<T, M, M>(G, C, r, id, true);
   }
 }
 template <class T, int M>
@@ -1765,21 +1800,30 @@ __global__ void __launch_bounds__(kThreads) k_restrict_group(Group<T> G, const T
   restrict_group_body<T, M>(G, r, bc, (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
-// The interpolation of xc at point (i, j, k) of the group's level S (0, with
-// nothing loaded, when `in` is false).
+// Interpolation to a point of the group's first level: st[q][t], the step of
+// stage t on level q > t (level M: the group's last); odd: the point lies
+// between two of the stage's coarse points; two: the upper one exists.
+template <int M>
+struct ProlongSteps {
+  int st[M + 1][M];
+  bool odd[M], two[M];
+};
+// The interpolation of xc at the point of level S whose indices on the levels
+// from S on are id (0, with nothing loaded, when `in` is false).
 template <class T, int S, int M>
-__device__ __forceinline__ T prolonged(const Group<T> &G, const T *xc, int i, int j, int k, bool in) {
+__device__ __forceinline__ T prolonged(const Group<T> &G, const ProlongSteps<M> &C, const T *xc, const int (&id)[M + 1],
+                                       bool in) {
   if constexpr (S == M) {
-    return in ? xc[((long)k * G.cb.ny + j) * G.cb.nx + i] : T(0);
+    return in ? xc[id[M]] : T(0);
   } else {
     const GroupStage<T> &L = G.s[S];
-    const int nd = L.d == 0 ? L.b.nx : L.d == 1 ? L.b.ny : L.b.nz, f = L.d == 0 ? i : L.d == 1 ? j : k, c = f >> 1;
-    const bool odd = in && (f & 1), two = odd && c + 1 < (nd + 1) / 2;
-    const T x0 = prolonged<T, S + 1, M>(G, xc, L.d == 0 ? c : i, L.d == 1 ? c : j, L.d == 2 ? c : k, in);
-    const T x1 =
-        prolonged<T, S + 1, M>(G, xc, L.d == 0 ? c + 1 : i, L.d == 1 ? c + 1 : j, L.d == 2 ? c + 1 : k, two);
-    const long r = ((long)k * L.b.ny + j) * L.b.nx + i;
-    const T wp = odd ? L.pp[r] : T(0), wm = odd ? L.pm[r] : T(0);
+    const bool odd = in && C.odd[S], two = odd && C.two[S];
+    int up[M + 1] = {};
+#pragma unroll
+    for (int q = S + 1; q <= M; ++q) up[q] = id[q] + C.st[q][S];
+    const T x0 = prolonged<T, S + 1, M>(G, C, xc, id, in);
+    const T x1 = prolonged<T, S + 1, M>(G, C, xc, up, two);
+    const T wp = odd ? L.pp[id[S]] : T(0), wm = odd ? L.pm[id[S]] : T(0);
     return odd ? fmat<T>(wp, x1, wm * x0) : x0;
   }
 }
@@ -1787,15 +1831,28 @@ template <class T, int M>
 __device__ __forceinline__ void prolong_group_body(const Group<T> &G, const T *xc, T *x, int accumulate, long t0,
                                                    long ts, int split = 0) {
   const Box &b = G.s[0].b;
+  ProlongSteps<M> C;
+#pragma unroll
+  for (int t = 0; t < M; ++t)
+#pragma unroll
+    for (int q = t + 1; q <= M; ++q) C.st[q][t] = group_stride(q < M ? G.s[q < M ? q : 0].b : G.cb, G.s[t].d);
   for (long r = t0; r < b.n; r += ts) {
-    int i, j, k;
-    box_ijk(r, b, i, j, k);
-    const T corr = prolonged<T, 0, M>(G, xc, i, j, k, true);
-    if (split) {  // a colour-split level: colour 1 only
-      if ((i + j + k) & 1) x[b.n / 2 + (r >> 1)] = x[b.n / 2 + (r >> 1)] + corr;
-      continue;
+    int c[3], id[M + 1];
+    box_ijk(r, b, c[0], c[1], c[2]);
+    const int odd = (c[0] + c[1] + c[2]) & 1;
+    if (split && !odd) continue;  // a colour-split level takes colour 1 only
+    id[0] = (int)r;
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      const int d = G.s[t].d, f = along(d, c), h = f >> 1;
+      C.odd[t] = f & 1;
+      C.two[t] = h + 1 < (extent(G.s[t].b, d) + 1) / 2;
+      set_along(d, h, c);
+      id[t + 1] = index_of(t + 1 < M ? G.s[t + 1 < M ? t + 1 : 0].b : G.cb, c);
     }
-    x[r] = accumulate ? x[r] + corr : corr;
+    const T corr = prolonged<T, 0, M>(G, C, xc, id, true);
+    if (split) x[b.n / 2 + (r >> 1)] = x[b.n / 2 + (r >> 1)] + corr;
+    else x[r] = accumulate ? x[r] + corr : corr;
   }
 }
 template <class T, int M>
