@@ -63,9 +63,18 @@ __device__ inline T apply_row(const T *__restrict__ A, long n, const T *__restri
     acc = fmat<T>(A[4 * n + r], j < ny - 1 ? x[r + sy] : T(0), acc);
     acc = fmat<T>(A[5 * n + r], k > 0 ? x[r - sz] : T(0), acc);
     acc = fmat<T>(A[6 * n + r], k < nz - 1 ? x[r + sz] : T(0), acc);
+  } else if constexpr (sizeof(T) == 8) {
+#pragma unroll
+    for (int s = 0; s < 27; ++s) {
+      const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+      const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
+      const T xv = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
+      acc = fmat<T>(A[(long)s * n + r], xv, acc);
+    }
   } else {
-    // all 54 loads before the sum: small levels wait for one memory latency
-    // and not for one per handful of slots (step 97x33x21 with its odd lines: 5530 -> 4690 us)
+    // FP32: all 54 loads before the sum: small levels wait for one memory latency
+    // and not for one per handful of slots (step 97x33x21 with its odd lines:
+    // 5530 -> 4690 us). In FP64 they would take 108 registers.
     T av[27], xv[27];
 #pragma unroll
     for (int s = 0; s < 27; ++s) {
@@ -526,7 +535,12 @@ __global__ void k_split_colors27(const T *A, const T *invd, Box bx, T *R) {
   }
 }
 
-template <class T>
+// AHEAD: the record and the window of x come in before the sum, so that their
+// loads are in flight together, at 112 (FP32 60) registers: for levels of few
+// warps per SM, which wait for latencies. A large FP64 level is bound by the
+// FP64 rate and wants warps instead (FP64 step 640x128x128 with AHEAD everywhere
+// 32.56 ms, below kPlainRecords points 31.30).
+template <class T, bool AHEAD = true>
 __device__ __forceinline__ void relax_rb27_body(const Recs<T, 28> &R, const T *b, const T *x, T *t, const Box &bx,
                                                 int color, int zero_x, long t0, long ts) {
   const long h = bx.n / 2;
@@ -540,30 +554,41 @@ __device__ __forceinline__ void relax_rb27_body(const Recs<T, 28> &R, const T *b
       t[r ^ 1] = T(0);
       continue;
     }
-    // the record and the window of x before the sum, so that their loads are
-    // in flight together
-    T c[28], xv[27];
-    load_recs<T, 28>(R, idx, c);
-#pragma unroll
-    for (int s = 0; s < 27; ++s) {
-      const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
-      const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
-      xv[s] = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
-    }
-    const T bv = b[r], other = x[r ^ 1];
     T acc = T(0);
+    if constexpr (AHEAD) {
+      T c[28], xv[27];
+      load_recs<T, 28>(R, idx, c);
 #pragma unroll
-    for (int s = 0; s < 27; ++s) acc = fmat<T>(c[s], xv[s], acc);
-    t[r] = fmat<T>(c[27], bv - acc, xv[13]);
-    t[r ^ 1] = other;
+      for (int s = 0; s < 27; ++s) {
+        const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+        const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
+        xv[s] = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
+      }
+      const T bv = b[r], other = x[r ^ 1];
+#pragma unroll
+      for (int s = 0; s < 27; ++s) acc = fmat<T>(c[s], xv[s], acc);
+      t[r] = fmat<T>(c[27], bv - acc, xv[13]);
+      t[r ^ 1] = other;
+    } else {
+      const T *__restrict__ pr = rec_ptr<T, 28>(R, idx);
+#pragma unroll
+      for (int s = 0; s < 27; ++s) {
+        const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+        const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
+        const T xv = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
+        acc = fmat<T>(pr[s], xv, acc);
+      }
+      t[r] = fmat<T>(pr[27], b[r] - acc, x[r]);
+      t[r ^ 1] = x[r ^ 1];
+    }
   }
 }
-template <class T>
-__global__ void __launch_bounds__(kThreads, 2) k_relax_rb27(Recs<T, 28> R, const T *__restrict__ b,
+template <class T, bool AHEAD>
+__global__ void __launch_bounds__(kThreads, AHEAD ? 2 : 4) k_relax_rb27(Recs<T, 28> R, const T *__restrict__ b,
                                                          const T *__restrict__ x, T *__restrict__ t, Box bx,
                                                          int color, int zero_x, const int *gate) {
   if (gate_off(gate)) return;
-  relax_rb27_body<T>(R, b, x, t, bx, color, zero_x, (long)blockIdx.x * blockDim.x + threadIdx.x,
+  relax_rb27_body<T, AHEAD>(R, b, x, t, bx, color, zero_x, (long)blockIdx.x * blockDim.x + threadIdx.x,
                      (long)gridDim.x * blockDim.x);
 }
 
@@ -693,7 +718,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_rb27_quad(Recs<float, 28>
 // Residual of a 27-point level from its colour-split records: every point
 // (both colours; same-colour points are coupled), b - A x in apply_row's slot
 // order, so the result equals k_residual<T, 27> bit for bit.
-template <class T>
+template <class T, bool AHEAD = true>
 __device__ __forceinline__ void residual_rb27_body(const Recs<T, 28> &R, const T *b, const T *x, T *res,
                                                    const Box &bx, long t0, long ts) {
   const long h = bx.n / 2;
@@ -703,27 +728,40 @@ __device__ __forceinline__ void residual_rb27_body(const Recs<T, 28> &R, const T
     const long m = t - color * h;
     int i, j, k;
     const long r = rb_row(m, color, bx, i, j, k);
-    T c[28], xv[27];
-    load_recs<T, 28>(R, t, c);
+    if constexpr (AHEAD) {
+      T c[28], xv[27];
+      load_recs<T, 28>(R, t, c);
 #pragma unroll
-    for (int s = 0; s < 27; ++s) {
-      const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
-      const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
-      xv[s] = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
+      for (int s = 0; s < 27; ++s) {
+        const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+        const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
+        xv[s] = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
+      }
+      const T bv = b[r];
+      T acc = T(0);
+#pragma unroll
+      for (int s = 0; s < 27; ++s) acc = fmat<T>(c[s], xv[s], acc);
+      res[r] = bv - acc;
+    } else {
+      const T *__restrict__ pr = rec_ptr<T, 28>(R, t);
+      T acc = T(0);
+#pragma unroll
+      for (int s = 0; s < 27; ++s) {
+        const int ii = i + s % 3 - 1, jj = j + (s / 3) % 3 - 1, kk = k + s / 9 - 1;
+        const bool in = ii >= 0 && ii < nx && jj >= 0 && jj < ny && kk >= 0 && kk < nz;
+        const T xv = in ? x[((long)kk * ny + jj) * nx + ii] : T(0);
+        acc = fmat<T>(pr[s], xv, acc);
+      }
+      res[r] = b[r] - acc;
     }
-    const T bv = b[r];
-    T acc = T(0);
-#pragma unroll
-    for (int s = 0; s < 27; ++s) acc = fmat<T>(c[s], xv[s], acc);
-    res[r] = bv - acc;
   }
 }
-template <class T>
-__global__ void __launch_bounds__(kThreads, 2) k_residual_rb27(Recs<T, 28> R, const T *__restrict__ b,
+template <class T, bool AHEAD>
+__global__ void __launch_bounds__(kThreads, AHEAD ? 2 : 4) k_residual_rb27(Recs<T, 28> R, const T *__restrict__ b,
                                                             const T *__restrict__ x, T *__restrict__ res, Box bx,
                                                             const int *gate) {
   if (gate_off(gate)) return;
-  residual_rb27_body<T>(R, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x,
+  residual_rb27_body<T, AHEAD>(R, b, x, res, bx, (long)blockIdx.x * blockDim.x + threadIdx.x,
                         (long)gridDim.x * blockDim.x);
 }
 
@@ -2402,11 +2440,11 @@ void dense_inverse(const std::vector<double> &A, int ns, const Box &b, std::vect
 }  // namespace
 
 // ---------------------------------------------------------------- host side
+constexpr long kPlainRecords = 32768;  // see split_colors
 // Colour-split copy of a relaxed 7-point level with an even nx (the fine
 // level), used by the in-place two-colour relaxation.
 // With record classes on, the records are replaced by their classes when
 // there are at most kMaxClasses distinct ones.
-constexpr long kPlainRecords = 32768;
 template <class T>
 static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
   if (prm.relax != 2 || (F.b.nx & 1) || F.b.n < 2) return;
@@ -3103,6 +3141,7 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   const QuadMap Q = make_quad_map(F.b);
   const double rec7 = R7.code ? 2.0 : 8.0 * T_, rec27 = R27.code ? 2.0 : 28.0 * T_;
   const QuadMap O = make_quad_map(F.b, 8);
+  const bool ahead = sizeof(T) == 4 || n <= kPlainRecords;  // k_relax_rb27
   Uni8 U8;
   if constexpr (sizeof(T) == 4) {
     if (split) U8 = uni8_octs(F.rbc);
@@ -3192,7 +3231,9 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
             done = true;
           }
         }
-        if (!done) k_relax_rb27<T><<<grid_all(h), block_of(h), 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
+        if (done) {
+        } else if (ahead) k_relax_rb27<T, true><<<grid_all(h), block_of(h), 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
+        else if constexpr (sizeof(T) == 8) k_relax_rb27<T, false><<<grid_all(h), block_of(h), 0, st>>>(R27, F.bv.p, cur, oth, F.b, color, z, gate);
         std::swap(cur, oth);
       }
     } else if (p.relax == 2) {
@@ -3250,7 +3291,9 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
         done = true;
       }
     }
-    if (!done) k_residual_rb27<T><<<grid_all(n), block_of(n), 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
+    if (done) {
+    } else if (ahead) k_residual_rb27<T, true><<<grid_all(n), block_of(n), 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
+    else if constexpr (sizeof(T) == 8) k_residual_rb27<T, false><<<grid_all(n), block_of(n), 0, st>>>(R27, F.bv.p, cur, F.r.p, F.b, gate);
     res = F.r.p;
   } else if (nu1 > 0) {
     LaunchScope ls(K_MG_RESID, st, T_ * n * (F.ns + 3.0));
