@@ -275,6 +275,8 @@ void use_classes(const Op7 &o, KSysHost &h) {
   }
   if (o.clsj.ok()) {
     h.clsj = o.clsj.code.p; h.tabj = o.clsj.tab.p;
+    h.majorj = o.clsj.major;
+    std::copy(o.clsj.major_rec.begin(), o.clsj.major_rec.end(), h.uj);
   }
 }
 

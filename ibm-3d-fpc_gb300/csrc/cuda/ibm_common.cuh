@@ -261,12 +261,12 @@ struct KSys {
   const uint16_t *clsj; // class of each FP32 Jacobi record
   const float *tabj;    // [K][8] {invdf, Ajf_1..Ajf_6, 0}
   const float *tabdf;   // [K][16] rows of Ar as double-float pairs
-  // The class of most rows: its code, and the rows of tabf and tabdf for
-  // it. Kernels that take four rows a thread compare the four codes with it and
+  // The class of most rows: its code, and the rows of tabf, tabdf and
+  // tabj for it. Kernels that take four rows a thread compare the four codes with it and
   // use these values, which are in constant memory, instead of table loads.
-  int major;
-  float uf[8], udf[16];
-  int quad;             // nx % 4 == 0: four rows from a multiple of four lie on one line, 16-byte aligned
+  int major, majorj;
+  float uf[8], udf[16], uj[8];
+  int quad;             // 1: nx % 4 == 0, four rows from a multiple of four lie on one line; 2: n % 4 == 0 only; else 0
   int df_resid;         // FP32 cycles with classes: true residuals in double-float (FP32 pipe)
   float2 *xs;           // df_resid: x as double-float pairs, written with every update of x
   int df_spmv;          // pc 2, FP64 cycles, classes: A z_j in double-float (tabdf) on the FP32 pipe

@@ -78,33 +78,61 @@ __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 __device__ __forceinline__ float f4(const float4 &v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
 
-// A quad: rows r0 .. r0 + 3 of one line (nx and r0 multiples of 4), with the
-// values of an FP32 vector there and around, 0 outside the box: seven loads
-// instead of 28.
+// Rows r0 .. r0 + 3 (r0 a multiple of 4) with the values of an FP32 vector
+// there and around, 0 outside the box.
 struct QuadRows {
-  float4 c, s, n, b, t;  // the quad; its neighbours at y - 1, y + 1, z - 1, z + 1
-  float l, r;            // x neighbours of the first and the last row
-  bool hl, hr, hs, hn, hb, ht;
+  float4 c, w, e, s, n, b, t;  // the rows; their neighbours at x -+ 1, y -+ 1, z -+ 1
 };
+// LINE: nx is a multiple of 4, the rows are of one line: seven loads instead
+// of 28. Else only n is: the rows may go over to the next line (and plane), and
+// lines start anywhere, so the y neighbours are single loads.
+template <bool LINE>
 __device__ __forceinline__ QuadRows load_quad_rows(const KSys &S, const float *z, long r0) {
   int i, j, k;
   sys_ijk(r0, S, i, j, k);
-  const long sy = S.nx, sz = (long)S.nx * S.ny;
+  const int nx = S.nx, ny = S.ny, nz = S.nz;
+  const long sy = nx, sz = (long)nx * ny;
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
   QuadRows q;
-  q.hl = i > 0; q.hr = i + 4 < S.nx; q.hs = j > 0; q.hn = j < S.ny - 1; q.hb = k > 0; q.ht = k < S.nz - 1;
   q.c = ld4(z + r0);
-  q.s = q.hs ? ld4(z + r0 - sy) : z4;
-  q.n = q.hn ? ld4(z + r0 + sy) : z4;
-  q.b = q.hb ? ld4(z + r0 - sz) : z4;
-  q.t = q.ht ? ld4(z + r0 + sz) : z4;
-  q.l = q.hl ? z[r0 - 1] : 0.0f;
-  q.r = q.hr ? z[r0 + 4] : 0.0f;
+  if constexpr (LINE) {
+    q.s = j > 0 ? ld4(z + r0 - sy) : z4;
+    q.n = j < ny - 1 ? ld4(z + r0 + sy) : z4;
+    q.b = k > 0 ? ld4(z + r0 - sz) : z4;
+    q.t = k < nz - 1 ? ld4(z + r0 + sz) : z4;
+    const float l = i > 0 ? z[r0 - 1] : 0.0f, r = i + 4 < nx ? z[r0 + 4] : 0.0f;
+    q.w = make_float4(l, q.c.x, q.c.y, q.c.z);
+    q.e = make_float4(q.c.y, q.c.z, q.c.w, r);
+  } else {
+    const float c[4] = {q.c.x, q.c.y, q.c.z, q.c.w};
+    float w[4], e[4], s[4], n[4], b[4], t[4];
+    const bool vec = (sz & 3) == 0;
+    const bool over = i + 3 >= nx && j == ny - 1;  // the last rows are of the next plane
+    const bool below = vec && k > 0, above = vec && (over ? k + 1 : k) < nz - 1;
+    if (below) q.b = ld4(z + r0 - sz);
+    if (above) q.t = ld4(z + r0 + sz);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool wrap = i + u >= nx;
+      const int iu = wrap ? i + u - nx : i + u, j1 = wrap ? j + 1 : j;
+      const int ju = j1 == ny ? 0 : j1, ku = j1 == ny ? k + 1 : k;
+      const long r = r0 + u;
+      w[u] = iu > 0 ? (u > 0 ? c[u > 0 ? u - 1 : 0] : z[r - 1]) : 0.0f;
+      e[u] = iu < nx - 1 ? (u < 3 ? c[u < 3 ? u + 1 : 3] : z[r + 1]) : 0.0f;
+      s[u] = ju > 0 ? z[r - sy] : 0.0f;
+      n[u] = ju < ny - 1 ? z[r + sy] : 0.0f;
+      if (!below) b[u] = ku > 0 ? z[r - sz] : 0.0f;
+      if (!above) t[u] = ku < nz - 1 ? z[r + sz] : 0.0f;
+    }
+    q.w = make_float4(w[0], w[1], w[2], w[3]);
+    q.e = make_float4(e[0], e[1], e[2], e[3]);
+    q.s = make_float4(s[0], s[1], s[2], s[3]);
+    q.n = make_float4(n[0], n[1], n[2], n[3]);
+    if (!below) q.b = make_float4(b[0], b[1], b[2], b[3]);
+    if (!above) q.t = make_float4(t[0], t[1], t[2], t[3]);
+  }
   return q;
 }
-// x neighbours of row q of the quad
-__device__ __forceinline__ float quad_w(const QuadRows &v, int q) { return q == 0 ? v.l : f4(v.c, q - 1); }
-__device__ __forceinline__ float quad_e(const QuadRows &v, int q) { return q == 3 ? v.r : f4(v.c, q + 1); }
 // whether all four codes are `major`
 __device__ __forceinline__ bool all_major(ushort4 c, int major) {
   return c.x == major && c.y == major && c.z == major && c.w == major;
@@ -114,8 +142,8 @@ __device__ __forceinline__ float quad_row32(const QuadRows &v, int q, float c0, 
                                             float c5, float c6) {
   float a = 0.0f;
   a = fmaf(c0, f4(v.c, q), a);
-  a = fmaf(c1, quad_w(v, q), a);
-  a = fmaf(c2, quad_e(v, q), a);
+  a = fmaf(c1, f4(v.w, q), a);
+  a = fmaf(c2, f4(v.e, q), a);
   a = fmaf(c3, f4(v.s, q), a);
   a = fmaf(c4, f4(v.n, q), a);
   a = fmaf(c5, f4(v.b, q), a);
@@ -127,8 +155,8 @@ template <class C>
 __device__ __forceinline__ double quad_row_df(const QuadRows &v, int q, const C &c) {
   float ah = 0.0f, al = 0.0f;
   df_fma1(ah, al, c[0], c[8], f4(v.c, q));
-  df_fma1(ah, al, c[1], c[9], quad_w(v, q));
-  df_fma1(ah, al, c[2], c[10], quad_e(v, q));
+  df_fma1(ah, al, c[1], c[9], f4(v.w, q));
+  df_fma1(ah, al, c[2], c[10], f4(v.e, q));
   df_fma1(ah, al, c[3], c[11], f4(v.s, q));
   df_fma1(ah, al, c[4], c[12], f4(v.n, q));
   df_fma1(ah, al, c[5], c[13], f4(v.b, q));
@@ -467,7 +495,7 @@ __device__ __forceinline__ void spmv_pass64_quad(const KSys &S, const float *zj,
     double w[4];
     if (c0 == 0) {
       const ushort4 c4 = __ldcs(reinterpret_cast<const ushort4 *>(S.cls + r0));
-      const QuadRows v = load_quad_rows(S, zj, r0);
+      const QuadRows v = load_quad_rows<true>(S, zj, r0);
       if (all_major(c4, S.major)) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) w[q] = quad_row_df(v, q, S.udf);
@@ -517,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_arnoldi_spmv(const __grid_const
     double pd[kDots64];
 #pragma unroll
     for (int kk = 0; kk < kDots64; ++kk) pd[kk] = 0.0;
-    if (S.df_spmv && S.quad) spmv_pass64_quad(S, zj, c0, ndc, pd);
+    if (S.df_spmv && S.quad == 1) spmv_pass64_quad(S, zj, c0, ndc, pd);
     else if (S.df_spmv) spmv_pass64<0>(S, z, zj, inv_nu, c0, ndc, pd);
     else if (S.pc != 2) spmv_pass64<1>(S, z, zj, inv_nu, c0, ndc, pd);
     else spmv_pass64<2>(S, z, zj, inv_nu, c0, ndc, pd);
@@ -916,11 +944,11 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_spmv32(const __grid_consta
       const long r0 = t0 + 4 * threadIdx.x;
       if (r0 >= n) continue;
       float w[4];
-      if (S.quad && S.cls) {
+      if (S.quad == 1 && S.cls) {
         // 85 us at 10.5M rows with 28 loads of z and eight of the table per
         // thread, 64 as quads
         const ushort4 c4 = __ldcs(reinterpret_cast<const ushort4 *>(S.cls + r0));
-        const QuadRows v = load_quad_rows(S, zj, r0);
+        const QuadRows v = load_quad_rows<true>(S, zj, r0);
         if (all_major(c4, S.major)) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
@@ -1255,6 +1283,42 @@ __device__ __forceinline__ void jacobi_two_rows(const KSys &S, const VT *__restr
   }
 }
 
+// The same, four consecutive rows per thread (S.quad, classed records): 112 us
+// over 3 x 10.5M rows with 28 loads of v and eight of the table per thread;
+// 76 so. Lines of an odd number of rows (the u system) take the second form.
+template <bool LINE>
+__device__ __forceinline__ void jacobi_two_quads(const KSys &S, const float *__restrict__ vj, float inv_nu,
+                                                 float *__restrict__ out) {
+  auto scaled = [&](float4 &a) { a.x *= inv_nu; a.y *= inv_nu; a.z *= inv_nu; a.w *= inv_nu; };
+  for (long r0 = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x); r0 < S.n; r0 += 4L * gridDim.x * blockDim.x) {
+    const ushort4 c4 = __ldcs(reinterpret_cast<const ushort4 *>(S.clsj + r0));
+    QuadRows v = load_quad_rows<LINE>(S, vj, r0);
+    scaled(v.c); scaled(v.w); scaled(v.e); scaled(v.s); scaled(v.n); scaled(v.b); scaled(v.t);
+    auto row = [&](int q, float id, float c1, float c2, float c3, float c4_, float c5, float c6) {
+      float acc = f4(v.c, q);
+      acc = fmaf(-c1, f4(v.w, q), acc);
+      acc = fmaf(-c2, f4(v.e, q), acc);
+      acc = fmaf(-c3, f4(v.s, q), acc);
+      acc = fmaf(-c4_, f4(v.n, q), acc);
+      acc = fmaf(-c5, f4(v.b, q), acc);
+      acc = fmaf(-c6, f4(v.t, q), acc);
+      return id * acc;
+    };
+    float z[4];
+    if (all_major(c4, S.majorj)) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) z[q] = row(q, S.uj[0], S.uj[1], S.uj[2], S.uj[3], S.uj[4], S.uj[5], S.uj[6]);
+    } else {
+      float4 cp[7];
+      load_rows4(S.tabj, c4, cp);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        z[q] = row(q, f4(cp[0], q), f4(cp[1], q), f4(cp[2], q), f4(cp[3], q), f4(cp[4], q), f4(cp[5], q), f4(cp[6], q));
+    }
+    st4(out + r0, make_float4(z[0], z[1], z[2], z[3]));
+  }
+}
+
 // Four consecutive rows per thread with 16-byte loads of the coefficient
 // planes and stores of z (FP32 basis, n % 4 == 0).
 __device__ __forceinline__ void jacobi_two_rows4(const KSys &S, const float *__restrict__ vj, float inv_nu,
@@ -1302,7 +1366,9 @@ __global__ void __launch_bounds__(kThreads) k_jacobi32_two(const __grid_constant
   // values ((float) V_j), one conversion per row where the vector is formed
   // instead of one per row and neighbour here
   const float *vf = S.a32 ? S.Vf + (long)j * S.ldv : S.vcur;
-  if (vf && S.vec4) jacobi_two_rows4(S, vf, inv_nu, out);
+  if (vf && S.clsj && S.quad == 1) jacobi_two_quads<true>(S, vf, inv_nu, out);
+  else if (vf && S.clsj && S.quad == 2) jacobi_two_quads<false>(S, vf, inv_nu, out);
+  else if (vf && S.vec4) jacobi_two_rows4(S, vf, inv_nu, out);
   else if (vf) jacobi_two_rows<float>(S, vf, inv_nu, out);
   else jacobi_two_rows<double>(S, S.V + (long)j * S.ldv, inv_nu, out);
 }
@@ -1484,10 +1550,11 @@ void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, uns
     k.A = h.A; k.Ar = h.Ar; k.invd = h.invd; k.Af = h.Af; k.invdf = h.invdf; k.Ajf = h.Ajf;
     k.cls = h.cls; k.tab = h.tab; k.tabf = h.tabf; k.clsj = h.clsj; k.tabj = h.tabj;
     k.tabdf = h.tabdf;
-    k.major = h.major;
+    k.major = h.major; k.majorj = h.majorj;
     std::copy(h.uf, h.uf + 8, k.uf);
     std::copy(h.udf, h.udf + 16, k.udf);
-    k.quad = (h.nx % 4 == 0) ? 1 : 0;
+    std::copy(h.uj, h.uj + 8, k.uj);
+    k.quad = h.nx % 4 == 0 ? 1 : h.n % 4 == 0 && h.nx >= 4 ? 2 : 0;
     k.df_resid = (h.a32 && h.cls && h.tabdf && h.df_residual) ? 1 : 0;
     k.df_spmv = (h.pc == 2 && !h.a32 && h.cls && h.tabdf && h.A == h.Ar && h.df_spmv) ? 1 : 0;
     k.xs = slot[s].xs.p;

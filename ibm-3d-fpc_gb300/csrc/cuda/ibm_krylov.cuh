@@ -49,8 +49,8 @@ struct KSysHost {
   const float *tabf = nullptr;
   const uint16_t *clsj = nullptr;
   const float *tabj = nullptr;
-  int major = 0;     // the class of most rows, and its rows of tabf and tabdf
-  float uf[8] = {}, udf[16] = {};
+  int major = 0, majorj = 0;     // the class of most rows, and its rows of tabf, tabdf and tabj
+  float uf[8] = {}, udf[16] = {}, uj[8] = {};
   const float *tabdf = nullptr;  // with a32: true residuals in double-float
   int df_residual = 1;           // use them when a32 and tabdf are set
   int df_spmv = 1;               // pc 2 without a32: A z_j in double-float from tabdf
