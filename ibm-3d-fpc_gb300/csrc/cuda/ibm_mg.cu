@@ -1266,6 +1266,156 @@ __global__ void __launch_bounds__(kThreads, 3) k_split_residual(Recs<float, 8> R
   }
 }
 
+// The same for the finest FP64 level (nx a multiple of 4, records scaled by the
+// inverse diagonal): two points of a colour per thread. FP64 sets the floor of a
+// phase (six multiply-adds a point, 50 us at 640x128x128); one point per thread
+// on joined arrays took 78, with two table and class loads a point before its
+// multiply-adds and twice the bytes. The major record's values are operands in
+// constant memory. FP64 steps, joined against split: 640x128x128 31.30 -> 30.15 ms,
+// two forward and two adjoint steps 256x48x48 (590k points) 20.99 -> 20.57 ms; 160x32x32
+// (164k points) 3510 -> 3611 us, a thread's two chains of multiply-adds being
+// longer than one where few warps share an SM: levels below kSplitPoints64 stay
+// joined.
+constexpr long kSplitPoints64 = 300000;
+struct Uni8d {
+  double c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const uint8_t *runs = nullptr;
+};
+struct QuadX64 {
+  double2 c, s, n, b, t;  // the other colour on the quad's line and the four lines around it
+  double side;
+};
+__device__ __forceinline__ QuadX64 load_quad64(const double *xo, const Quad &g, const Box &bx, int e) {
+  const long sy = bx.nx / 2, sz = (long)(bx.nx / 2) * bx.ny;
+  const double2 z2 = make_double2(0.0, 0.0);
+  const double *p = xo + g.r0 / 2;
+  QuadX64 v;
+  v.c = *reinterpret_cast<const double2 *>(p);
+  v.s = g.j > 0 ? *reinterpret_cast<const double2 *>(p - sy) : z2;
+  v.n = g.j < bx.ny - 1 ? *reinterpret_cast<const double2 *>(p + sy) : z2;
+  v.b = g.k > 0 ? *reinterpret_cast<const double2 *>(p - sz) : z2;
+  v.t = g.k < bx.nz - 1 ? *reinterpret_cast<const double2 *>(p + sz) : z2;
+  const bool has = e ? g.i0 + 4 < bx.nx : g.i0 > 0;
+  v.side = has ? p[e ? 2 : -1] : 0.0;
+  return v;
+}
+// acc + sum of couplings times neighbours at the quad's point u of the phase's colour
+__device__ __forceinline__ double row64(const double *c, const QuadX64 &v, int e, int u, double acc) {
+  const double w = u == 0 ? (e ? v.c.x : v.side) : (e ? v.c.y : v.c.x);
+  const double x = u == 0 ? (e ? v.c.y : v.c.x) : (e ? v.side : v.c.y);
+  acc = fma(c[1], w, acc);
+  acc = fma(c[2], x, acc);
+  acc = fma(c[3], u == 0 ? v.s.x : v.s.y, acc);
+  acc = fma(c[4], u == 0 ? v.n.x : v.n.y, acc);
+  acc = fma(c[5], u == 0 ? v.b.x : v.b.y, acc);
+  acc = fma(c[6], u == 0 ? v.t.x : v.t.y, acc);
+  return acc;
+}
+// Four points of a line, a on columns 2 m + odd, b on the others.
+__device__ __forceinline__ void store_joined64(double *p, const double2 &a, const double2 &b, int odd, bool wide) {
+  const double2 lo = odd ? make_double2(b.x, a.x) : make_double2(a.x, b.x);
+  const double2 hi = odd ? make_double2(b.y, a.y) : make_double2(a.y, b.y);
+  if (wide) {
+    reinterpret_cast<double2 *>(p)[0] = lo;
+    reinterpret_cast<double2 *>(p)[1] = hi;
+  } else {
+    p[0] = lo.x; p[1] = lo.y; p[2] = hi.x; p[3] = hi.y;
+  }
+}
+__device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+__global__ void __launch_bounds__(kThreads) k_split_in64(QuadMap Q, double *bs, double *xs, Box bx, VecRef in,
+                                                         const double *winv, const int *gate) {
+  if (gate_off(gate)) return;
+  const long n4 = bx.n / 4, h = bx.n / 2;
+  const double *src = in.base + (in.idx ? (long)(*in.idx) * in.ld : 0);
+  const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
+  const bool wide = aligned16(src);
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+    const Quad g = quad_of(q, Q, bx);
+    double a[4];
+    if (wide) {
+      const double2 lo = *reinterpret_cast<const double2 *>(src + g.r0), hi = *reinterpret_cast<const double2 *>(src + g.r0 + 2);
+      a[0] = lo.x; a[1] = lo.y; a[2] = hi.x; a[3] = hi.y;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] = src[g.r0 + u];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (in.inu) a[u] = a[u] * sc;
+      if (winv) a[u] = a[u] * winv[g.r0 + u];
+    }
+    const int e = (g.j + g.k) & 1;  // columns of colour 0
+    const long m = g.r0 / 2;
+    const double2 b0 = e ? make_double2(a[1], a[3]) : make_double2(a[0], a[2]);
+    const double2 b1 = e ? make_double2(a[0], a[2]) : make_double2(a[1], a[3]);
+    *reinterpret_cast<double2 *>(bs + m) = b0;
+    *reinterpret_cast<double2 *>(bs + h + m) = b1;
+    *reinterpret_cast<double2 *>(xs + m) = b0;  // the right-hand side is scaled by the inverse diagonal
+  }
+}
+
+template <bool OUT>
+__global__ void __launch_bounds__(kThreads) k_split_phase64(Recs<double, 8> R, Uni8d U, QuadMap Q,
+                                                            const double *__restrict__ bs, double *xs, Box bx, int color,
+                                                            OutRef out, const int *gate) {
+  if (gate_off(gate)) return;
+  const long n4 = bx.n / 4, h = bx.n / 2, own = color ? h : 0;
+  const double *xo = xs + (h - own);
+  double *zd = OUT ? out.d + (out.idx ? (long)(*out.idx) * out.ld : 0) : nullptr;
+  const bool wide = OUT && aligned16(zd);
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+    const Quad g = quad_of(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    const int e = (g.j + g.k + color) & 1;
+    const long m = g.r0 / 2;
+    const QuadX64 v = load_quad64(xo, g, bx, e);
+    const double2 b = *reinterpret_cast<const double2 *>(bs + own + m);
+    double2 o;
+    if (uni) {
+      o.x = row64(U.c, v, e, 0, b.x);
+      o.y = row64(U.c, v, e, 1, b.y);
+    } else {
+      double c[8];
+      load_recs<double, 8>(R, own + m, c);
+      o.x = row64(c, v, e, 0, b.x);
+      load_recs<double, 8>(R, own + m + 1, c);
+      o.y = row64(c, v, e, 1, b.y);
+    }
+    if constexpr (OUT) store_joined64(zd + g.r0, o, v.c, e, wide);
+    else *reinterpret_cast<double2 *>(xs + own + m) = o;
+  }
+}
+
+__global__ void __launch_bounds__(kThreads) k_split_residual64(Recs<double, 8> R, Uni8d U, QuadMap Q,
+                                                               const double *__restrict__ bs,
+                                                               const double *__restrict__ xs, double *__restrict__ res,
+                                                               Box bx, const int *gate) {
+  if (gate_off(gate)) return;
+  const long n4 = bx.n / 4, h = bx.n / 2;
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
+    const Quad g = quad_of(q, Q, bx);
+    const bool uni = U.runs && U.runs[q >> 5];
+    const int e = (g.j + g.k) & 1;
+    const long m = g.r0 / 2;
+    const QuadX64 v = load_quad64(xs + h, g, bx, e);
+    const double2 b = *reinterpret_cast<const double2 *>(bs + m), x = *reinterpret_cast<const double2 *>(xs + m);
+    double2 o;
+    if (uni) {
+      o.x = U.c[0] * row64(U.c, v, e, 0, b.x - x.x);
+      o.y = U.c[0] * row64(U.c, v, e, 1, b.y - x.y);
+    } else {
+      double c[8];
+      load_recs<double, 8>(R, m, c);
+      o.x = c[0] * row64(c, v, e, 0, b.x - x.x);
+      load_recs<double, 8>(R, m + 1, c);
+      o.y = c[0] * row64(c, v, e, 1, b.y - x.y);
+    }
+    store_joined64(res + g.r0, o, make_double2(0.0, 0.0), e, true);
+  }
+}
+
 // One whole two-colour sweep of a 7-point FP32 level (colour 0, then colour
 // 1) in one kernel, out of place: x_new = sweep(x_old). A block takes a tile
 // of kSwJ x kSwK lines and kSwX points of each, loads x_old over the tile
@@ -1709,11 +1859,12 @@ __global__ void k_prolong_x4(const float *__restrict__ xc, Box cb, const float *
 
 template <class T>
 __device__ __forceinline__ void prolong_body(const T *xc, const Box &cb, const T *pm, const T *pp, const Box &fb,
-                                             int d, T *x, int accumulate, long t0, long ts) {
+                                             int d, T *x, int accumulate, long t0, long ts, int split = 0) {
   const int cn[3] = {cb.nx, cb.ny, cb.nz};
   for (long r = t0; r < fb.n; r += ts) {
     int f[3];
     box_ijk(r, fb, f[0], f[1], f[2]);
+    if (split && !((f[0] + f[1] + f[2]) & 1)) continue;  // a colour-split level takes colour 1 only
     T corr;
     if ((f[d] & 1) == 0) {
       int c[3] = {f[0], f[1], f[2]};
@@ -1731,15 +1882,16 @@ __device__ __forceinline__ void prolong_body(const T *xc, const Box &cb, const T
       }
       corr = fmat<T>(pp[r], x1, pm[r] * x0);
     }
-    x[r] = accumulate ? x[r] + corr : corr;
+    if (split) x[fb.n / 2 + (r >> 1)] = x[fb.n / 2 + (r >> 1)] + corr;
+    else x[r] = accumulate ? x[r] + corr : corr;
   }
 }
 template <class T>
-__global__ void k_prolong(const T *xc, Box cb, const T *pm, const T *pp, Box fb, int d, T *x, int accumulate,
+__global__ void k_prolong(const T *xc, Box cb, const T *pm, const T *pp, Box fb, int d, T *x, int accumulate, int split,
                           const int *gate) {
   if (gate_off(gate)) return;
   prolong_body<T>(xc, cb, pm, pp, fb, d, x, accumulate, (long)blockIdx.x * blockDim.x + threadIdx.x,
-                  (long)gridDim.x * blockDim.x);
+                  (long)gridDim.x * blockDim.x, split);
 }
 
 // Transfers of a whole coarsening group: the levels between two relaxed ones
@@ -2463,7 +2615,7 @@ static void split_colors(cudaStream_t st, MgLevelT<T> &F, const MgParams &prm) {
   if (F.ns == 27 && F.b.n <= kPlainRecords) return;
   if (prm.classes && build_classes<T>(st, R.p, W, F.b.n, F.rbc)) {
     R.release();
-    if (sizeof(T) == 4 && F.b.nx % 4 == 0 && prm.quads) mark_runs<T>(st, F.rbc, F.b);
+    if (F.b.nx % 4 == 0 && prm.quads && (sizeof(T) == 4 || F.pre)) mark_runs<T>(st, F.rbc, F.b);
   }
 }
 
@@ -2477,6 +2629,14 @@ static Recs<T, W> recs_of(const DBuf<T> &plain, const Classes<T> &c) {
 
 static Uni8 uni8_of(const Classes<float> &c) {
   Uni8 u;
+  if (c.ok() && c.W == 8 && c.runs.p) {
+    std::copy(c.major_rec.begin(), c.major_rec.end(), u.c);
+    u.runs = c.runs.p;
+  }
+  return u;
+}
+static Uni8d uni8d_of(const Classes<double> &c) {
+  Uni8d u;
   if (c.ok() && c.W == 8 && c.runs.p) {
     std::copy(c.major_rec.begin(), c.major_rec.end(), u.c);
     u.runs = c.runs.p;
@@ -2607,6 +2767,8 @@ static float *record_tail(std::vector<MgLevelT<float>> &L, int l, const MgParams
                           double &bytes);
 template <class T>
 static void plan_cluster(cudaStream_t st, std::vector<MgLevelT<T>> &L, const MgParams &p, ClusterPlan &c);
+template <class T>
+static int smooth_blocks();
 
 void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const float *A7f, const double h[3],
                       const MgParams &p, bool fp64, bool fp32, const double *winv) {
@@ -2657,6 +2819,10 @@ void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const flo
       F.x.alloc(n); F.bv.alloc(n); F.r.alloc(n); F.t.alloc(n);
     }
     IBM_CUDA_TRY(cudaStreamSynchronize(st));
+  }
+  if (prm.relax == 2) {  // asked here, where no stream is being captured
+    smooth_blocks<double>();
+    if (fp32) smooth_blocks<float>();
   }
   build_tail(st);
   clu32_ = ClusterPlan();
@@ -3192,6 +3358,22 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
       }
     }
     if constexpr (sizeof(T) == 8) {
+      if (split) {
+        const long n4 = n / 4;
+        const double phase = 0.5 * n * rec7 + 1.5 * T_ * n;
+        const Uni8d U = uni8d_of(F.rbc);
+        if (zero) {
+          LaunchScope ls(K_MG_RELAX_FINE, st, (winv ? 3.5 : 2.5) * T_ * n);
+          k_split_in64<<<resident_grid(k_split_in64, n4), block_of(n4), 0, st>>>(Q, F.bv.p, cur, F.b, *fin, winv, gate);
+        } else {
+          LaunchScope ls(K_MG_RELAX_FINE, st, phase);
+          k_split_phase64<false><<<resident_grid(k_split_phase64<false>, n4), block_of(n4), 0, st>>>(R7, U, Q, F.bv.p, cur, F.b, 0, OutRef(), gate);
+        }
+        LaunchScope ls(K_MG_RELAX_FINE, st, last ? phase + 0.5 * T_ * n : phase);
+        if (last) k_split_phase64<true><<<resident_grid(k_split_phase64<true>, n4), block_of(n4), 0, st>>>(R7, U, Q, F.bv.p, cur, F.b, 1, *fout, gate);
+        else k_split_phase64<false><<<resident_grid(k_split_phase64<false>, n4), block_of(n4), 0, st>>>(R7, U, Q, F.bv.p, cur, F.b, 1, OutRef(), gate);
+        return;
+      }
       if (p.relax == 2 && rb7 && (zero ? fin != nullptr : last && fout)) {
         if (zero) {
           LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.pre ? 0.0 : R7.code ? 2.0 : T_) + (winv ? 4.0 : 3.0) * T_ * n);
@@ -3280,6 +3462,12 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
         done = true;
       }
     }
+    if constexpr (sizeof(T) == 8) {
+      if (split) {
+        k_split_residual64<<<resident_grid(k_split_residual64, n / 4), block_of(n / 4), 0, st>>>(R7, uni8d_of(F.rbc), Q, F.bv.p, cur, F.r.p, F.b, gate);
+        done = true;
+      }
+    }
     if (!done) k_residual_rb<T><<<grid_all(n / 2), block_of(n / 2), 0, st>>>(R7, F.bv.p, cur, F.r.p, F.b, gate);
     res = F.r.p;
   } else if (nu1 > 0 && p.relax == 2 && rb27) {
@@ -3344,9 +3532,9 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
       else if (p.quads && F.cdir == 0 && F.b.nx == 2 * C.b.nx && C.b.nx % 4 == 0)
         k_prolong_x4<<<resident_grid(k_prolong_x4, n / 4), block_of(n / 4), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, cur, nu1 > 0, split, gate);
       else
-        k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
+        k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, split, gate);
     } else {
-      k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, gate);
+      k_prolong<T><<<grid_all(n), block_of(n), 0, st>>>(xc, C.b, F.pm.p, F.pp.p, F.b, F.cdir, cur, nu1 > 0, split, gate);
     }
   }
   if (sp.threads && nu2 > 0) launch_smooth<T>(st, sp, F, cur, nullptr, nu2, false, gate);
@@ -3413,7 +3601,8 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
     }
     if (in.base && out.d && prm.relax == 2 && F.relax && F.cdir >= 0 && F.ns == 7 && (F.rb.p || F.rbc.ok()) &&
         prm.nu1 > 0 && prm.nu2 > 0) {
-      vcycle<double>(st, L64, 0, prm, gate, &in, &out, nullptr, nullptr, c64, winv, fused);
+      const bool split = fused && prm.quads && F.pre && F.b.nx % 4 == 0 && F.b.n >= kSplitPoints64;
+      vcycle<double>(st, L64, 0, prm, gate, &in, &out, nullptr, nullptr, c64, winv, fused, split);
       return;
     }
     {

@@ -102,8 +102,9 @@ typedef struct ibm_solver_params {
                             per row and the row from a table of the distinct rows; results are bitwise
                             those of the plain layout. 0: plain layout */
   int mg_quads;          /* 1 (default): FP32 levels with nx % 4 == 0 relax (two-colour phases), form
-                            residuals and transfer along x four points per thread (same arithmetic,
-                            bitwise equal results) */
+                            residuals and transfer along x four points per thread, and within a solve
+                            the finest level keeps x and b by colour (FP32: nx % 8 == 0, FP64:
+                            nx % 4 == 0 from 300000 points); same arithmetic, bitwise equal results */
   int df_residual;       /* precision 2 with row classes, 1 (default): the true residual at each restart
                             is computed in double-float on the FP32 pipe (about 48 significant bits;
                             GB300's FP64 rate makes the FP64 stencil the bound there). 0: FP64 */
