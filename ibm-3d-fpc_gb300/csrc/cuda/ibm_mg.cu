@@ -2304,12 +2304,12 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       case CK_RB_ZERO: relax_rb_zero_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, t0, ts); break;
       case CK_RB: relax_rb_body<T>(op_recs<T, 8>(op), op.b, op.dst, op.fb, op.color, nullptr, t0, ts); break;
       case CK_RB27:
-        relax_rb27_body<T>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
+        relax_rb27_body<T, sizeof(T) == 4>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, op.color, op.zero, t0, ts);
         break;
       case CK_RESID7: residual_body<T, 7>(op.A, op.b, op.src, op.dst, op.fb, t0, ts); break;
       case CK_RESID27: residual_body<T, 27>(op.A, op.b, op.src, op.dst, op.fb, t0, ts); break;
       case CK_RESID_RB: residual_rb_body<T>(op_recs<T, 8>(op), op.b, op.src, op.dst, op.fb, t0, ts); break;
-      case CK_RESID_RB27: residual_rb27_body<T>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, t0, ts); break;
+      case CK_RESID_RB27: residual_rb27_body<T, sizeof(T) == 4>(op_recs<T, 28>(op), op.b, op.src, op.dst, op.fb, t0, ts); break;
       case CK_RESTRICT: restrict_body<T>(op.src, op.pm, op.pp, op.fb, op.d, op.dst, op.cb, t0, ts); break;
       case CK_PROLONG:
         prolong_body<T>(op.src, op.cb, op.pm, op.pp, op.fb, op.d, op.dst, op.accumulate, t0, ts);

@@ -112,14 +112,15 @@ typedef struct ibm_solver_params {
                             coarse end of the V-cycle, from the first level below the finest with at
                             most this many points, runs as one persistent cooperative kernel per
                             V-cycle (one phase per former launch, grid-wide barriers between them;
-                            bitwise the same results). 0 (default): one launch per phase; 1: from
+                            bitwise the same results). 0 (default): launches per phase, a small
+                            level's sweeps in one; 1: from
                             the first level of at most 262144 points. Measured on the 640x128x128
                             channel: no faster (each fused phase stays bound by the latency of its
                             dependent loads plus the grid barrier, about 5 us) */
   int mg_fused_sweep;    /* 1: an FP32 7-point level's two-colour sweep (both phases) runs as one kernel
                             on shared-memory tiles with a halo, out of place (bitwise the two in-place
                             phases); 0 (default): one launch per phase. Measured on the 640x128x128
-                            channel: about 96 us a sweep against 62 us for the two phases */
+                            channel: about 96 us a sweep against 29 us for the two phases by colour */
   int vel_precision;     /* precision of the three momentum solves (0, 1, 2 as `precision`); -1
                             (default): `precision` */
   int df_spmv;           /* precision 1 with row classes, 1 (default): the Arnoldi product A z_j of the
