@@ -1033,9 +1033,10 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_quad(Recs<float, 8> R, Un
 // restriction, and the interpolation adds to colour 1 only: a phase needs no
 // values of its own colour, so what the first phase after it overwrites is not
 // read. Per point the arithmetic is k_relax_rb's, in the same order. Bound: L2
-// (HBM above about 20M points). Steps, joined against split: mixed 640x128x128
+// (HBM above about 20M points). A phase at 640x128x128 takes 14.3 us, 24.3
+// joined. Steps, joined against split: mixed 640x128x128
 // 17.10 -> 15.53 ms, 320x64x64 4854 -> 4711 us, pressure solve 512x96x96 with FP64
-// basis 6975 -> 6418 us, twelve channels 29.4 -> 28.2 ms (78 registers; four
+// basis 6975 -> 6418 us, twelve channels 29.4 -> 28.2 ms (80 registers; four
 // blocks per SM at 64 with spills: 15.54 ms, 4812, 6423, 28.8).
 struct OctX {
   float4 c, s, n, b, t;  // the other colour on the octet's line and the four lines around it
