@@ -1,16 +1,15 @@
 """FP32 multigrid levels with nx % 4 == 0 relax and form residuals four points
-a thread, take runs of one record from the kernel's parameters, and march over
-the planes of large levels; one point at a time (mg_quads 0) is the same
-arithmetic, so V-cycles must agree bit for bit."""
+a thread and take runs of one record from the kernel's parameters; one point at
+a time (mg_quads 0) is the same arithmetic, so V-cycles must agree bit for
+bit."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 # one, two and three quads a line (no inner quads, one); runs cut by line ends;
-# 32 and 33 inner quads; lines in y and z that leave partial tiles; above two
-# million points the marching sweep, with 81 = 3 x 27 quads a line, and with one
-# tile along x and lines short of a whole tile
+# 32 and 33 inner quads; lines in y and z that leave partial runs; above two
+# million points with 81 and 30 quads a line
 SHAPES = [(4, 8, 8), (8, 8, 8), (12, 9, 8), (136, 12, 12), (140, 13, 11), (324, 81, 83), (120, 129, 137)]
 
 
@@ -32,7 +31,7 @@ def test_quads_equal_single_points(ibm, shape, rap):
         b.close()
 
 
-def test_marching_solve_equals_single_points(ibm):
+def test_solve_equals_single_points(ibm):
     """The whole FP32 solve: the V-cycle's input and output fused into the
     finest level's first and last sweeps."""
     shape = (324, 81, 83)
