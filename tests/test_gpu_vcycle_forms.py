@@ -1,5 +1,5 @@
 """The V-cycle of a host-driven solve runs its small levels on one
-thread-block cluster, a captured one as a launch per phase, and both take a
+thread-block cluster, a captured one in launches of their own, and both take a
 coarsening group's transfers in one launch on small levels. The arithmetic per
 point is the same, so host-driven and captured steps must agree bit for bit:
 FP64 and FP32 hierarchies, 7- and 27-point levels, Jacobi and two-colour
