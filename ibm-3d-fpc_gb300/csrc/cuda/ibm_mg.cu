@@ -2681,8 +2681,6 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
       LaunchScope ls(K_SETUP, st, 0.0);
       k_diag<<<grid_for(n), block_of(n), 0, st>>>(diag, n, prm.omega, F.invd.p, F.wd.p);
     }
-    F.pre = l == 0 && prm.relax == 2 && F.b.nx % 2 == 0 && prm.nu1 > 0;
-    split_colors(st, F, prm);
     const int dims[3] = {F.b.nx, F.b.ny, F.b.nz};
     // A group starts at a relaxed level: every direction whose spacing is
     // within group_ratio of the smallest is coarsened once (smallest spacing
@@ -2724,6 +2722,10 @@ void Multigrid::build<double>(cudaStream_t st, std::vector<MgLevelT<double>> &L,
     }
     F.cdir = d;
     h[d] *= 2.0;
+    // below the dense level's exit: it is not relaxed, and its inverse takes the
+    // right-hand side unscaled
+    F.pre = l == 0 && prm.relax == 2 && F.b.nx % 2 == 0 && prm.nu1 > 0;
+    split_colors(st, F, prm);
     F.pm.alloc(n); F.pp.alloc(n);
     coupled.alloc(n);
     {
@@ -2816,7 +2818,7 @@ void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const flo
         }
       };
       conv(D.wd, F.wd); conv(D.invd, F.invd); conv(D.pm, F.pm); conv(D.pp, F.pp); conv(D.dense, F.dense);
-      split_colors(st, F, prm);
+      if (F.cdir >= 0) split_colors(st, F, prm);
       F.x.alloc(n); F.bv.alloc(n); F.r.alloc(n); F.t.alloc(n);
     }
     IBM_CUDA_TRY(cudaStreamSynchronize(st));
