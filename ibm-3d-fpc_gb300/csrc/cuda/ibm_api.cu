@@ -286,6 +286,13 @@ int precision_key(const ibm_solver_params &p) {
   return 4 * p.precision + vp;
 }
 
+// The captured reverse sweeps that hold this context's buffers: its own, and for
+// a transposed context its owner's.
+void drop_adjoint_graph(ibm_ctx *c) {
+  if (c->adj) c->adj->graph_ready = false;
+  if (c->adj_owner && c->adj_owner->adj) c->adj_owner->adj->graph_ready = false;
+}
+
 void ensure_solvers(ibm_ctx *c) {
   if (c->solvers_ready && c->solvers_precision == precision_key(c->prm)) return;
   const ibm_solver_params &p = c->prm;
@@ -362,6 +369,7 @@ void ensure_solvers(ibm_ctx *c) {
   c->solvers_precision = precision_key(p);
   c->graph_ready = false;
   c->graph_bound = false;
+  drop_adjoint_graph(c);
 }
 
 int worst(int a, int b) { return std::max(a, b); }
@@ -377,6 +385,7 @@ void invalidate_graph(ibm_ctx *c) {
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   c->gexec = nullptr;
   c->graph_ready = false;
+  drop_adjoint_graph(c);
 }
 
 // Captures one timestep into c->gexec. Launch accounting during the capture
@@ -1713,6 +1722,7 @@ int ibm_step_backward(ibm_ctx *c, double ramp, double weight, ibm_step_stats *st
     ibm::AdjState &a = adj_of(c);
     if (a.tape.empty()) throw Error(IBM_ERR_STATE, "ibm_step_backward: no step on the tape (ibm_step_forward)");
     if (ramp != a.tape.back().ramp) throw Error(IBM_ERR_ARG, "ibm_step_backward: ramp differs from the taped step's");
+    ensure_solvers(c);  // parameters or operators may have changed since the step
     sync_transposed_params(c);
     ibm::TapeEntry e = std::move(a.tape.back());
     a.tape.pop_back();
