@@ -47,7 +47,7 @@ struct AdjState {
   bool graph_ready = false;
   bool graph_bound = false;               // the transposed Krylov systems are bound to the graph's vectors
   long long graph_fixed_launches = 0;
-  long long graph_body_launches[4] = {0, 0, 0, 0};
+  long long graph_body_launches[2] = {0, 0};
   KResult last[4];                        // the last reverse sweep's transposed solves (u, v, w, p)
   ~AdjState();
 };

@@ -405,7 +405,7 @@ void build_step_graph(ibm_ctx *c, const Precond &none, const Precond &mgp) {
     IBM_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     IBM_CUDA_TRY(cudaMemcpyAsync(c->dramp.p, c->hramp, sizeof(double), cudaMemcpyHostToDevice, st));
     IBM_CUDA_TRY(cudaMemsetAsync(c->diag.p, 0, sizeof(StepDiag), st));
-    IBM_CUDA_TRY(cudaMemsetAsync(c->dloops.p, 0, sizeof(unsigned long long) * 4, st));
+    IBM_CUDA_TRY(cudaMemsetAsync(c->dloops.p, 0, sizeof(unsigned long long) * 2, st));
     IBM_CUDA_TRY(cudaEventRecordWithFlags(c->ev[0], st, cudaEventRecordExternal));
     launch_bc(c, c->u.p, c->v.p, c->w.p);
     launch_momentum_rhs(c);
@@ -415,12 +415,12 @@ void build_step_graph(ibm_ctx *c, const Precond &none, const Precond &mgp) {
     launch_tilde(c);
     launch_pressure_rhs(c);
     IBM_CUDA_TRY(cudaEventRecordWithFlags(c->ev[5], st, cudaEventRecordExternal));
-    gp = c->kp.enqueue_graph(st, c->cap, mgp, c->hflags_graph + 3, c->dloops.p + 2);
+    gp = c->kp.enqueue_graph(st, c->cap, mgp, c->hflags_graph + 3, c->dloops.p + 1);
     IBM_CUDA_TRY(cudaEventRecordWithFlags(c->ev[3], st, cudaEventRecordExternal));
     launch_projection(c);
     IBM_CUDA_TRY(cudaEventRecordWithFlags(c->ev[4], st, cudaEventRecordExternal));
     IBM_CUDA_TRY(cudaMemcpyAsync(c->hdiag, c->diag.p, sizeof(StepDiag), cudaMemcpyDeviceToHost, st));
-    IBM_CUDA_TRY(cudaMemcpyAsync(c->hloops, c->dloops.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st));
+    IBM_CUDA_TRY(cudaMemcpyAsync(c->hloops, c->dloops.p, sizeof(unsigned long long) * 2, cudaMemcpyDeviceToHost, st));
     IBM_CUDA_TRY(cudaStreamEndCapture(st, &graph));
   } catch (...) {
     cudaGraph_t junk = nullptr;
@@ -436,10 +436,8 @@ void build_step_graph(ibm_ctx *c, const Precond &none, const Precond &mgp) {
   cudaGraphDestroy(graph);
   IBM_CUDA_TRY(e);
   c->graph_fixed_launches = cap_count - gm.loop - gp.loop;
-  c->graph_body_launches[0] = gm.end_body;
-  c->graph_body_launches[1] = gm.arnoldi_body;
-  c->graph_body_launches[2] = gp.end_body;
-  c->graph_body_launches[3] = gp.arnoldi_body;
+  c->graph_body_launches[0] = gm.loop;
+  c->graph_body_launches[1] = gp.loop;
   c->graph_ready = true;
 }
 
@@ -521,12 +519,12 @@ int ibm_create(const ibm_grid_desc *grid, ibm_ctx **out) {
     c->u.zero(c->st); c->v.zero(c->st); c->w.zero(c->st); c->p.zero(c->st);
     c->diag.alloc(1);
     c->dramp.alloc(1);
-    c->dloops.alloc(4);
+    c->dloops.alloc(2);
     IBM_CUDA_TRY(cudaMallocHost((void **)&c->hramp, sizeof(double)));
     *c->hramp = 1.0;
     IBM_CUDA_TRY(cudaMallocHost((void **)&c->hflags_graph, sizeof(KFlags) * 4));
-    IBM_CUDA_TRY(cudaMallocHost((void **)&c->hloops, sizeof(unsigned long long) * 4));
-    for (auto &s : c->cap) IBM_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    IBM_CUDA_TRY(cudaMallocHost((void **)&c->hloops, sizeof(unsigned long long) * 2));
+    IBM_CUDA_TRY(cudaStreamCreateWithFlags(&c->cap, cudaStreamNonBlocking));
     c->part.alloc(4 * 1024);
     IBM_CUDA_TRY(cudaMallocHost((void **)&c->hdiag, sizeof(StepDiag)));
     IBM_CUDA_TRY(cudaStreamSynchronize(c->st));
@@ -557,8 +555,7 @@ void ibm_destroy(ibm_ctx *c) {
   if (c->hramp) cudaFreeHost(c->hramp);
   if (c->hflags_graph) cudaFreeHost(c->hflags_graph);
   if (c->hloops) cudaFreeHost(c->hloops);
-  for (auto s : c->cap)
-    if (s) cudaStreamDestroy(s);
+  if (c->cap) cudaStreamDestroy(c->cap);
   cudaStream_t st = c->st;
   delete c;
   if (st) cudaStreamDestroy(st);
@@ -1106,8 +1103,7 @@ int step_collect(ibm_ctx *c, double ramp, ibm_step_stats *stats) {
     }
     const unsigned long long *lp = c->hloops;
     c->launches += c->graph_fixed_launches + (long long)lp[0] * c->graph_body_launches[0] +
-                   (long long)lp[1] * c->graph_body_launches[1] + (long long)lp[2] * c->graph_body_launches[2] +
-                   (long long)lp[3] * c->graph_body_launches[3];
+                   (long long)lp[1] * c->graph_body_launches[1];
   }
   int rc = IBM_OK;
   const StepDiag &dg = *c->hdiag;
@@ -1513,7 +1509,7 @@ void build_adjoint_graph(ibm_ctx *c) {
   try {
     IBM_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     IBM_CUDA_TRY(cudaMemcpyAsync(a.dweight.p, a.hweight, sizeof(double), cudaMemcpyHostToDevice, st));
-    IBM_CUDA_TRY(cudaMemsetAsync(t->dloops.p, 0, sizeof(unsigned long long) * 4, st));
+    IBM_CUDA_TRY(cudaMemsetAsync(t->dloops.p, 0, sizeof(unsigned long long) * 2, st));
     launch_bc(c, a.u1.p, a.v1.p, a.w1.p);
     adj_force(c, a.dweight.p);
     adj_bc(c, a.lu.p, a.lv.p, a.lw.p, ramp);
@@ -1521,12 +1517,12 @@ void build_adjoint_graph(ibm_ctx *c) {
       adj_projection(c, a.mu.p);
       adj_wscale(c, a.mu.p, c->bb[3].p, true);
       IBM_CUDA_TRY(cudaMemsetAsync(c->xb[3].p, 0, sizeof(double) * c->g.NP, st));
-      gp = c->kp.enqueue_graph(st, c->cap, mgc, c->hflags_graph + 3, t->dloops.p + 2);
+      gp = c->kp.enqueue_graph(st, c->cap, mgc, c->hflags_graph + 3, t->dloops.p + 1);
       adj_wscale(c, c->xb[3].p, a.mu.p, false);
     } else {
       adj_projection(c, t->bb[3].p);
       IBM_CUDA_TRY(cudaMemsetAsync(t->xb[3].p, 0, sizeof(double) * t->g.bp.n, st));
-      gp = t->kp.enqueue_graph(st, t->cap, mgp, t->hflags_graph + 3, t->dloops.p + 2);
+      gp = t->kp.enqueue_graph(st, t->cap, mgp, t->hflags_graph + 3, t->dloops.p + 1);
       IBM_CUDA_TRY(cudaMemcpyAsync(a.mu.p, t->xb[3].p, sizeof(double) * c->g.NP, cudaMemcpyDeviceToDevice, st));
     }
     adj_divergence(c, a.mu.p, ramp);
@@ -1540,7 +1536,7 @@ void build_adjoint_graph(ibm_ctx *c) {
     adj_momentum(c, lb);
     adj_gradient(c);
     adj_bc(c, a.lu.p, a.lv.p, a.lw.p, ramp);
-    IBM_CUDA_TRY(cudaMemcpyAsync(t->hloops, t->dloops.p, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st));
+    IBM_CUDA_TRY(cudaMemcpyAsync(t->hloops, t->dloops.p, sizeof(unsigned long long) * 2, cudaMemcpyDeviceToHost, st));
     IBM_CUDA_TRY(cudaStreamEndCapture(st, &graph));
   } catch (...) {
     cudaGraph_t junk = nullptr;
@@ -1556,10 +1552,8 @@ void build_adjoint_graph(ibm_ctx *c) {
   cudaGraphDestroy(graph);
   IBM_CUDA_TRY(e);
   a.graph_fixed_launches = cap_count - gm.loop - gp.loop;
-  a.graph_body_launches[0] = gm.end_body;
-  a.graph_body_launches[1] = gm.arnoldi_body;
-  a.graph_body_launches[2] = gp.end_body;
-  a.graph_body_launches[3] = gp.arnoldi_body;
+  a.graph_body_launches[0] = gm.loop;
+  a.graph_body_launches[1] = gp.loop;
   a.graph_ready = true;
 }
 
@@ -1585,8 +1579,7 @@ int reverse_graph(ibm_ctx *c) {
   IBM_CUDA_TRY(cudaGetLastError());
   const unsigned long long *lp = t->hloops;
   c->launches += a.graph_fixed_launches + (long long)lp[0] * a.graph_body_launches[0] +
-                 (long long)lp[1] * a.graph_body_launches[1] + (long long)lp[2] * a.graph_body_launches[2] +
-                 (long long)lp[3] * a.graph_body_launches[3];
+                 (long long)lp[1] * a.graph_body_launches[1];
   int rc = IBM_OK;
   for (int s = 0; s < 4; ++s) {
     const KFlags &f = (s == 3 && c->p_sym) ? c->hflags_graph[3] : t->hflags_graph[s];

@@ -115,12 +115,12 @@ struct ibm_ctx {
   cudaGraphExec_t gexec = nullptr;
   bool graph_ready = false;
   bool graph_bound = false;           // the Krylov system tables hold the step's full masks
-  cudaStream_t cap[2] = {};           // streams that capture conditional-node bodies
+  cudaStream_t cap = nullptr;         // captures conditional-node bodies
   ibm::KFlags *hflags_graph = nullptr;  // pinned: u, v, w, p solve flags after a graph step
-  ibm::DBuf<unsigned long long> dloops;  // loop-body counters (momentum x2, pressure x2)
+  ibm::DBuf<unsigned long long> dloops;  // loop-body counters (momentum, pressure)
   unsigned long long *hloops = nullptr;  // pinned copy
   long long graph_fixed_launches = 0;
-  long long graph_body_launches[4] = {0, 0, 0, 0};
+  long long graph_body_launches[2] = {0, 0};
   // Adjoint extension: transposed-operator context, lambdas, tape, checkpoints.
   ibm::AdjState *adj = nullptr;
   ibm_ctx *adj_owner = nullptr;       // a transposed-operator context: the context it serves

@@ -193,6 +193,31 @@ __device__ bool block_partials_and_last(double *sacc, int nd, double *part, unsi
   return last != 0;
 }
 
+// pc 1 keeps a cycle's preconditioned directions M V_k, as the flexible form
+// does, so that the update is x += sum c_k M V_k and not M (V c): one V-cycle
+// less per GMRES cycle (six instead of seven for a solve of six iterations; FP64
+// step 640x128x128 36.8 -> 34.7 ms, 160x32x32 4.58 -> 4.24). They lie in the
+// vectors of V that a short cycle does not reach, from its end down: direction
+// k in vector kdim - k, up to kdim / 2 of them (vectors 0 .. kdim / 2 of the
+// basis lie below). A longer cycle's basis runs over them; its later directions
+// go to the spare vector kdim + 1, and its end takes V c there and applies the
+// preconditioner to it, into vector kdim. Solves here take six to seven
+// iterations of the default 50.
+__device__ __forceinline__ int direction_slot(int k, int kdim) { return k < kdim / 2 ? kdim - k : kdim + 1; }
+// Whether a system's finished cycle applies the preconditioner at its end.
+__device__ __forceinline__ bool end_applies(const KSys &S) { return S.pc == 1 && S.s->i > S.s->kdim / 2; }
+// The next V-cycle: of Arnoldi step i; of a finished cycle's V c.
+__device__ __forceinline__ void pc_of_step(KScal *sc, int i, int on) {
+  sc->pc_in = i;
+  sc->pc_out = direction_slot(i, sc->kdim);
+  sc->pc_on = on;
+}
+__device__ __forceinline__ void pc_of_end(KScal *sc) {
+  sc->pc_in = sc->kdim + 1;
+  sc->pc_out = sc->kdim;
+  sc->pc_on = 2;
+}
+
 // r = b - Ar x; V_0 = r; |b|^2, |r|^2. Last block: norms, tolerance, state.
 __global__ void __launch_bounds__(kThreads) k_init(const __grid_constant__ KSysPack P) {
   const KSys &S = P.s[blockIdx.y];
@@ -274,6 +299,7 @@ __global__ void __launch_bounds__(kThreads) k_init(const __grid_constant__ KSysP
     else if (rn == 0.0 || rn <= sc->eps) { sc->status = 1; sc->active = 0; }
     else if (sc->maxit <= 0) { sc->status = 2; sc->active = 0; }
     else { sc->status = 0; sc->active = 1; }
+    pc_of_step(sc, 0, sc->active);
     sc->nu[0] = rn;
     sc->inu[0] = 1.0 / rn;
     sc->g[0] = rn;
@@ -335,6 +361,7 @@ __device__ void arnoldi_finalize(KScal *sc, int j, double hn) {
       sc->active = 0;
       sc->cycle_end = 1;
     }
+    pc_of_step(sc, m, end ? 0 : 1);
     ended = end;
   }
   __syncthreads();
@@ -538,7 +565,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_arnoldi_spmv(const __grid_const
   const double inv_nu = sc->inu[j];
   __shared__ double sacc[(kMaxKdim + 1) * kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double *z = S.pc == 0 ? S.V + (long)j * S.ldv : S.Zd ? S.Zd + (long)j * S.ldv : S.z;
+  const double *z = S.V + (long)(S.pc == 1 ? sc->pc_out : j) * S.ldv;
   const float *zj = S.Z + (long)j * S.ldv;
   for (int c0 = 0; c0 < nd; c0 += kDots64) {
     const int ndc = min(nd - c0, kDots64);
@@ -685,9 +712,9 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next(const __grid_constant
   arnoldi_finalize(sc, j, sqrt(tot[0]));
 }
 
-// Cycle end, solution update. pc 0: x += invd * (V c); pc 1: x += Zd c, or
-// without the directions z = V c (the caller applies the preconditioner and
-// then k_add_z); pc 2: x += Z y.
+// Cycle end, solution update. pc 0: x += invd * (V c); pc 1: x += sum of c_k
+// times direction k, or where the cycle outgrew them (end_applies) V c is left
+// for the preconditioner, and x += M (V c) once that has run; pc 2: x += Z y.
 __global__ void __launch_bounds__(kThreads) k_cycle_update(const __grid_constant__ KSysPack P) {
   const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
@@ -769,26 +796,27 @@ __global__ void __launch_bounds__(kThreads) k_cycle_update(const __grid_constant
     }
     return;
   }
+  const bool kept = S.pc == 1 && !end_applies(S);
+  double *const last = S.V + (long)sc->kdim * S.ldv;
+  const double *basis = kept ? last : S.V;
+  const long step = kept ? -S.ldv : S.ldv;
+  if (S.pc == 1 && sc->pc_on == 2) {
+    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x)
+      S.x[r] = S.x[r] + last[r];
+    return;
+  }
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x) {
     double acc = 0.0;
     if (S.pc == 2) {
       for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], widen(S.Z[(long)kk * S.ldv + r]), acc);
       S.x[r] = S.x[r] + acc;
     } else {
-      const double *basis = S.Zd ? S.Zd : S.V;
-      for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], basis[(long)kk * S.ldv + r], acc);
+      for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], basis[(long)kk * step + r], acc);
       if (S.pc == 0) S.x[r] = fma(S.invd[r], acc, S.x[r]);
-      else if (S.Zd) S.x[r] = S.x[r] + acc;
-      else S.z[r] = acc;
+      else if (kept) S.x[r] = S.x[r] + acc;
+      else last[S.ldv + r] = acc;
     }
   }
-}
-
-__global__ void k_add_z(const __grid_constant__ KSysPack P) {
-  const KSys &S = P.s[blockIdx.y];
-  if (!S.s->cycle_end || S.pc != 1 || S.Zd) return;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x)
-    S.x[r] = S.x[r] + S.z2[r];
 }
 
 // Relative bound on the double-float residual of one row: |r_df - r| <=
@@ -803,10 +831,11 @@ constexpr double kDfRowBound = 4.547473508864641e-13;  // 2^-41
 // the per-row bounds; a decision closer to the tolerance than
 // kDfRowBound * M is taken again from an FP64 residual, and the rest of the
 // solve stays in FP64, so convergence is always decided within FP64 rounding.
+// Systems whose x waits for the preconditioner are left alone.
 __global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_constant__ KSysPack P) {
   const KSys &S = P.s[blockIdx.y];
   KScal *sc = S.s;
-  if (!sc->cycle_end) return;
+  if (!sc->cycle_end || (end_applies(S) && sc->pc_on != 2)) return;
   const bool df = S.df_resid && !sc->use64;
   __shared__ double sacc[2 * kWarps];
   if (threadIdx.x < 2 * kWarps) sacc[threadIdx.x] = 0.0;
@@ -881,6 +910,7 @@ __global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_consta
     sc->ticket = 0;
     const double rt = sqrt(tot[0]);
     sc->cycle_end = 0;
+    sc->pc_on = 0;
     sc->r_norm = rt;
     if (!isfinite(rt)) { sc->nonfinite = 1; sc->status = 2; sc->active = 0; return; }
     if (df) {
@@ -902,6 +932,7 @@ __global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_consta
     sc->real_old = rt;
     sc->cyc_eps = fmax(sc->eps, sc->cyc_rtol * rt);
     sc->i = 0;
+    pc_of_step(sc, 0, 1);
     sc->claimed = 0;
     sc->nu[0] = rt;
     sc->inu[0] = 1.0 / rt;
@@ -1431,27 +1462,30 @@ __global__ void k_flags(const __grid_constant__ KSysPack P, int nsys, KFlags *ou
   }
 }
 
-// Loop control of the graph form: WHILE runs while any system is active or
-// has a finished cycle to close. Its body is an Arnoldi step and the cycle's
-// end, whose kernels return at once for systems with no finished cycle; with
-// explicit preconditioning at the cycle's end (no stored directions) a SWITCH
-// picks the cycle-end body (0) when any system closed a cycle, else the
-// Arnoldi body (1). loops (may be null): bodies run.
-__global__ void k_set_while(const __grid_constant__ KSysPack P, int nsys, cudaGraphConditionalHandle hw,
-                            unsigned long long *loops) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (loops) loops[1] += 1;
-  unsigned run = 0;
-  for (int s = 0; s < nsys; ++s) run |= (P.s[s].s->active | P.s[s].s->cycle_end) ? 1u : 0u;
-  cudaGraphSetConditional(hw, run);
+// Systems whose finished cycle waits for the preconditioner: the next V-cycle is
+// its. (In a launch of its own: the kernels that read the state run in many blocks.)
+__device__ void wait_for_pc(const KSys &S) {
+  if (S.s->cycle_end && end_applies(S)) pc_of_end(S.s);
+}
+__global__ void k_pc_of_end(const __grid_constant__ KSysPack P, int nsys) {
+  if ((int)threadIdx.x < nsys) wait_for_pc(P.s[threadIdx.x]);
 }
 
-__global__ void k_set_switch(const __grid_constant__ KSysPack P, int nsys, cudaGraphConditionalHandle hs, unsigned long long *loops) {
+// Loop control of the graph form: WHILE runs while any system is active or
+// has a finished cycle to close. Its body is an Arnoldi step and the cycle's
+// end, whose kernels return at once for systems with no finished cycle. A cycle
+// that waits for the preconditioner takes the next body's V-cycle, in which its
+// Arnoldi kernels return at once. count (may be null): bodies run.
+__global__ void k_set_while(const __grid_constant__ KSysPack P, int nsys, cudaGraphConditionalHandle hw,
+                            unsigned long long *count) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int end = 0;
-  for (int s = 0; s < nsys; ++s) end |= P.s[s].s->cycle_end;
-  cudaGraphSetConditional(hs, end ? 0u : 1u);
-  loops[end ? 0 : 1] += 1;
+  if (count) *count += 1;
+  unsigned run = 0;
+  for (int s = 0; s < nsys; ++s) {
+    wait_for_pc(P.s[s]);
+    run |= (P.s[s].s->active | P.s[s].s->cycle_end) ? 1u : 0u;
+  }
+  cudaGraphSetConditional(hw, run);
 }
 
 }  // namespace
@@ -1487,26 +1521,8 @@ void Krylov::configure(int nsys_, const KSysHost *hs) {
       sl.wf.alloc(h.n);
     } else {
       sl.Vf.release(); sl.wf.release();
-      sl.V.alloc((size_t)(h.kdim + 1) * h.n);
+      sl.V.alloc((size_t)(h.kdim + (h.pc == 1 ? 2 : 1)) * h.n);  // pc 1: the spare vector (direction_slot)
       sl.w.alloc(h.n);
-    }
-    // An explicit preconditioner keeps the cycle's directions M V_k, as the
-    // flexible form does, so the update is x += sum c_k M V_k and not M (V c):
-    // one V-cycle less per GMRES cycle (seven instead of six for a solve of six
-    // iterations; FP64 step 640x128x128 36.8 -> 34.7 ms, 160x32x32 4.58 -> 4.24). Where the device has no room for
-    // kdim more vectors the update applies the preconditioner again.
-    sl.Zd.release();
-    sl.z.release();
-    sl.z2.release();
-    if (h.pc == 1) {
-      try {
-        sl.Zd.alloc((size_t)h.kdim * h.n);
-      } catch (const Error &e) {
-        if (e.code != IBM_ERR_NOMEM) throw;
-        cudaGetLastError();
-        sl.z.alloc(h.n);
-        sl.z2.alloc(h.n);
-      }
     }
     if (h.a32 && h.cls && h.tabdf && h.df_residual) sl.xs.alloc(h.n);
     else sl.xs.release();
@@ -1527,7 +1543,7 @@ size_t Krylov::bytes() const {
   size_t b = 0;
   for (int s = 0; s < nsys; ++s) {
     const Slot &sl = slot[s];
-    b += sl.Zd.bytes() + sl.V.bytes() + sl.w.bytes() + sl.z.bytes() + sl.z2.bytes() + sl.part.bytes() +
+    b += sl.V.bytes() + sl.w.bytes() + sl.part.bytes() +
          sl.Z.bytes() + sl.zf.bytes() + sl.zf2.bytes() + sl.Vf.bytes() + sl.wf.bytes() + sl.xs.bytes() +
          sl.vcur.bytes();
   }
@@ -1560,8 +1576,7 @@ void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, uns
     k.xs = slot[s].xs.p;
     k.V = slot[s].V.p; k.ldv = h.n;
     k.Z = slot[s].Z.p;
-    k.Zd = slot[s].Zd.p;
-    k.w = slot[s].w.p; k.z = slot[s].z.p; k.z2 = slot[s].z2.p;
+    k.w = slot[s].w.p;
     k.zf = slot[s].zf.p; k.zf2 = slot[s].zf2.p;
     k.Vf = slot[s].Vf.p; k.wf = slot[s].wf.p; k.a32 = h.a32;
     k.vcur = slot[s].vcur.p;
@@ -1603,55 +1618,63 @@ void Krylov::read_flags(cudaStream_t st) {
 void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *fl, unsigned mask) {
   const dim3 grid(nblk, nsys), gridu(nblk * 2, nsys);
   auto rows = [&](int s) { return ((mask >> s) & 1u) ? (double)slot[s].host.n : 0.0; };
-  double bu = 0.0, br = 0.0, ba = 0.0;
+  double bu = 0.0, br = 0.0;
   if (fl) {
     for (int s = 0; s < nsys; ++s) {
       if (!fl[s].cycle_end) continue;
       const int m = fl[s].i, pcm = slot[s].host.pc;
-      bu += rows(s) * (pcm == 2 ? 4.0 * m + 16.0 : pcm == 1 ? 8.0 * m + (slot[s].Zd.p ? 16.0 : 8.0) : 8.0 * m + 24.0);
+      bu += rows(s) * (pcm == 2 ? 4.0 * m + 16.0 : pcm == 1 ? 8.0 * m + (m > slot[s].host.kdim / 2 ? 8.0 : 16.0) : 8.0 * m + 24.0);
       // a classed row is its 2-byte class instead of 7 FP64 coefficients
-      br += ((slot[s].host.cls ? 34.0 : 88.0) + (slot[s].vcur.p ? 4.0 : 0.0)) * rows(s);
-      if (pcm == 1 && !slot[s].Zd.p) ba += 24.0 * rows(s);
+      if (pcm != 1 || m <= slot[s].host.kdim / 2)
+        br += ((slot[s].host.cls ? 34.0 : 88.0) + (slot[s].vcur.p ? 4.0 : 0.0)) * rows(s);
     }
   }
-  {
-    LaunchScope ls(K_GM_UPDATE, st, bu);
-    k_cycle_update<<<wave(k_cycle_update), kThreads, 0, st>>>(pack);
+  auto update = [&](KernelId id, double b_update, double b_resid) {
+    {
+      LaunchScope ls(id, st, b_update);
+      k_cycle_update<<<wave(k_cycle_update), kThreads, 0, st>>>(pack);
+    }
+    LaunchScope ls(K_GM_RESID, st, b_resid);
+    k_cycle_residual<<<wave(k_cycle_residual), kThreads, 0, st>>>(pack);
+  };
+  update(K_GM_UPDATE, bu, br);
+  // cycles that outgrew their stored directions (captured: the next loop body's V-cycle takes them)
+  bool applies = false;
+  double ba = 0.0, bar = 0.0;
+  for (int s = 0; fl && s < nsys; ++s) {
+    if (slot[s].host.pc != 1 || !fl[s].cycle_end || fl[s].i <= slot[s].host.kdim / 2) continue;
+    if (!applies) {
+      LaunchScope ls(K_GM_UPDATE, st, 0.0);
+      k_pc_of_end<<<1, 32, 0, st>>>(pack, nsys);
+    }
+    apply_explicit(st, pc, s);
+    ba += 24.0 * rows(s);
+    bar += (slot[s].host.cls ? 34.0 : 88.0) * rows(s);
+    applies = true;
   }
-  bool cb = false;
-  for (int s = 0; s < nsys; ++s) {
-    if (slot[s].host.pc != 1 || slot[s].Zd.p || !((mask >> s) & 1u) || (fl && !fl[s].cycle_end)) continue;
-    VecRef in;
-    in.base = slot[s].z.p;
-    OutRef out;
-    out.d = slot[s].z2.p;
-    pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].cycle_end : nullptr);
-    cb = true;
-  }
-  if (cb) {
-    LaunchScope ls(K_GM_ADDZ, st, ba);
-    k_add_z<<<wave(k_add_z), kThreads, 0, st>>>(pack);
-  }
-  LaunchScope ls(K_GM_RESID, st, br);
-  k_cycle_residual<<<wave(k_cycle_residual), kThreads, 0, st>>>(pack);
+  if (applies) update(K_GM_ADDZ, ba, bar);
+}
+
+// The V-cycle that a pc 1 system's scalars name (pc_of_step, pc_of_end).
+void Krylov::apply_explicit(cudaStream_t st, const Precond &pc, int s) {
+  VecRef in;
+  in.base = slot[s].V.p; in.ld = slot[s].host.n; in.idx = &scal.p[s].pc_in;
+  OutRef out;
+  out.d = slot[s].V.p; out.ld = slot[s].host.n; out.idx = &scal.p[s].pc_out;
+  pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].pc_on : nullptr);
 }
 
 void Krylov::launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *fl, unsigned mask) {
   const dim3 grid(nblk, nsys), gridu(nblk * 2, nsys);
   auto rows = [&](int s) { return ((mask >> s) & 1u) ? (double)slot[s].host.n : 0.0; };
   // A single system is active whenever an Arnoldi step runs (the host loop and
-  // the graph's WHILE and SWITCH see to that), so its preconditioner needs no
-  // gate: one dependent load less at the start of each of its kernels.
+  // the graph's WHILE see to that), so its preconditioner needs no gate: one
+  // dependent load less at the start of each of its kernels.
   for (int s = 0; s < nsys; ++s) {
     if (!((mask >> s) & 1u) || (fl && !fl[s].active)) continue;
     const KSysHost &h = slot[s].host;
     if (h.pc == 1) {
-      VecRef in;
-      in.base = slot[s].V.p; in.ld = h.n; in.idx = &scal.p[s].i;
-      OutRef out;
-      out.d = slot[s].z.p;
-      if (slot[s].Zd.p) { out.d = slot[s].Zd.p; out.ld = h.n; out.idx = &scal.p[s].i; }
-      pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].active : nullptr);
+      apply_explicit(st, pc, s);
     } else if (h.pc == 2 && h.pc_cb) {
       VecRef in;
       if (h.a32) in.basef = slot[s].Vf.p;
@@ -1824,7 +1847,7 @@ long long capture_body(cudaGraph_t body, cudaStream_t bs, F &&fn) {
 
 }  // namespace
 
-Krylov::GraphCounts Krylov::enqueue_graph(cudaStream_t st, const cudaStream_t body_st[2], const Precond &pc,
+Krylov::GraphCounts Krylov::enqueue_graph(cudaStream_t st, cudaStream_t body_st, const Precond &pc,
                                           KFlags *host_flags, unsigned long long *loops) {
   GraphCounts gc;
   const long long t0 = launches();
@@ -1842,50 +1865,32 @@ Krylov::GraphCounts Krylov::enqueue_graph(cudaStream_t st, const cudaStream_t bo
   }
   cudaGraph_t wbody;
   add_conditional(st, &hw, cudaGraphCondTypeWhile, 1, &wbody);
-  bool explicit_end = false;  // the cycle's end applies the preconditioner
-  for (int s = 0; s < nsys; ++s) explicit_end |= slot[s].host.pc == 1 && !slot[s].Zd.p;
-  long long end_l = 0, arn_l = 0;
-  const long long loop_l = capture_body(wbody, body_st[0], [&](cudaStream_t b0) {
-    if (explicit_end) {
-      cudaGraphConditionalHandle hs;
-      IBM_CUDA_TRY(cudaGraphConditionalHandleCreate(&hs, wbody, 0, 0));
-      {
-        LaunchScope ls(K_GM_UPDATE, b0, 0.0);
-        k_set_switch<<<1, 32, 0, b0>>>(pack, nsys, hs, loops);
-      }
-      cudaGraph_t cases[2];
-      add_conditional(b0, &hs, cudaGraphCondTypeSwitch, 2, cases);
-      end_l = capture_body(cases[0], body_st[1], [&](cudaStream_t b1) { launch_cycle_end(b1, pc, nullptr, mask); });
-      arn_l = capture_body(cases[1], body_st[1], [&](cudaStream_t b1) { launch_arnoldi(b1, pc, nullptr, mask); });
-    } else {
-      // One body for both: a SWITCH node and its control kernel cost about
-      // 6 us an iteration and a cycle's end an iteration of its own, the
-      // three kernels that mostly return at once 1.2 us each. The residual
-      // is launched again for systems whose double-float one was too close
-      // to the tolerance to call. Steps in us: FP64 160x32x32 3955 -> 3712,
-      // 97x33x21 4495 -> 4255, 320x64x64 270 less, twelve channels 38.2 -> 36.9 ms.
-      launch_arnoldi(b0, pc, nullptr, mask);
-      launch_cycle_end(b0, pc, nullptr, mask);
-      bool df = false;
-      for (int s = 0; s < nsys; ++s) df |= pack.s[s].df_resid != 0;
-      if (df) {
-        LaunchScope ls(K_GM_RESID, b0, 0.0);
-        k_cycle_residual<<<wave(k_cycle_residual), kThreads, 0, b0>>>(pack);
-      }
+  gc.loop = capture_body(wbody, body_st, [&](cudaStream_t b0) {
+    // One body for the step and the cycle's end: a SWITCH node and its control
+    // kernel cost about 6 us an iteration and a cycle's end an iteration of its
+    // own, the three kernels that mostly return at once 1.2 us each. The residual
+    // is launched again for systems whose double-float one was too close to the
+    // tolerance to call. Steps in us: FP64 160x32x32 3955 -> 3712, 97x33x21
+    // 4495 -> 4255, 320x64x64 270 less, twelve channels 38.2 -> 36.9 ms. (A second
+    // loop for the ends that apply the preconditioner, inside or beside this one,
+    // cost 20 us a solve without any.)
+    launch_arnoldi(b0, pc, nullptr, mask);
+    launch_cycle_end(b0, pc, nullptr, mask);
+    bool df = false;
+    for (int s = 0; s < nsys; ++s) df |= pack.s[s].df_resid != 0;
+    if (df) {
+      LaunchScope ls(K_GM_RESID, b0, 0.0);
+      k_cycle_residual<<<wave(k_cycle_residual), kThreads, 0, b0>>>(pack);
     }
     LaunchScope ls(K_GM_UPDATE, b0, 0.0);
-    k_set_while<<<1, 32, 0, b0>>>(pack, nsys, hw, explicit_end ? nullptr : loops);
+    k_set_while<<<1, 32, 0, b0>>>(pack, nsys, hw, loops);
   });
   {
     LaunchScope ls(K_GM_UPDATE, st, 0.0);
     k_flags<<<1, 32, 0, st>>>(pack, nsys, dflags.p);
   }
   IBM_CUDA_TRY(cudaMemcpyAsync(host_flags, dflags.p, sizeof(KFlags) * nsys, cudaMemcpyDeviceToHost, st));
-  const long long per_iter = loop_l - end_l - arn_l;  // the two control kernels
-  gc.end_body = end_l + per_iter;
-  gc.arnoldi_body = arn_l + per_iter;
-  gc.fixed = (launches() - t0) - loop_l;
-  gc.loop = loop_l;
+  gc.fixed = (launches() - t0) - gc.loop;
   return gc;
 }
 

@@ -88,21 +88,20 @@ class Krylov {
 
   // Graph form. bind() fixes the vectors (outside any capture); enqueue_graph()
   // records the whole solve into the capture running on `st`: the restart /
-  // Arnoldi loop is a WHILE node whose body SWITCHes between the cycle-end
-  // and the Arnoldi-step bodies, captured on body_st[0] / body_st[1].
+  // Arnoldi loop is a WHILE node whose body, captured on body_st, is an Arnoldi
+  // step and the cycle's end.
   // After the solve the per-system flags land in host_flags (pinned) and the
-  // numbers of cycle-end / Arnoldi bodies run in loops[0] / loops[1].
-  // Returns the launches recorded outside the loop and per body kind.
-  struct GraphCounts { long long fixed = 0, end_body = 0, arnoldi_body = 0, loop = 0; };
+  // number of bodies run in *loops.
+  // Returns the launches recorded outside the loop and in its body.
+  struct GraphCounts { long long fixed = 0, loop = 0; };
   void bind(cudaStream_t st, const double *const *b, double *const *x, unsigned mask, bool x_zero = false);
-  GraphCounts enqueue_graph(cudaStream_t st, const cudaStream_t body_st[2], const Precond &pc, KFlags *host_flags,
+  GraphCounts enqueue_graph(cudaStream_t st, cudaStream_t body_st, const Precond &pc, KFlags *host_flags,
                             unsigned long long *loops);
 
  private:
   struct Slot {
     KSysHost host;
-    DBuf<double> V, w, z, z2, part;
-    DBuf<double> Zd;  // pc 1: the preconditioned directions of the cycle
+    DBuf<double> V, w, part;
     DBuf<float> Z, zf, zf2, Vf, wf;
     DBuf<float> vcur;  // FP64 basis with FP32 Jacobi: FP32 copy of the current basis vector
     DBuf<float2> xs;  // double-float copy of x for the double-float residual
@@ -114,6 +113,7 @@ class Krylov {
   // flags == nullptr every launch is recorded (each kernel is gated on the
   // device flags of its system); otherwise only what the flags require.
   void launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *flags, unsigned mask);
+  void apply_explicit(cudaStream_t st, const Precond &pc, int sys);
   void launch_arnoldi(cudaStream_t st, const Precond &pc, const KFlags *flags, unsigned mask);
   unsigned bound_mask = ~0u;
   bool bound_x_zero = false;
