@@ -2785,11 +2785,10 @@ void Multigrid::setup(cudaStream_t st, const Box &b, const double *A7, const flo
   }
   (void)fp64;
   build<double>(st, L64, b, A7, h);
-  winvd_.release();
   if (L64[0].pre) {
-    winvd_.alloc(b.n);
+    // in wd, which two-colour relaxation does not read
     LaunchScope ls(K_SETUP, st, 0.0);
-    k_input_scale<<<grid_for(b.n), block_of(b.n), 0, st>>>(winv, L64[0].invd.p, winvd_.p, b.n);
+    k_input_scale<<<grid_for(b.n), block_of(b.n), 0, st>>>(winv, L64[0].invd.p, L64[0].wd.p, b.n);
   }
   L32.clear();
   if (fp32) {
@@ -3597,7 +3596,7 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
     k_store_output<float><<<grid_for(F.b.n), block_of(F.b.n), 0, st>>>(x, F.b.n, out, gate);
   } else {
     MgLevelT<double> &F = L64[0];
-    const double *winv = F.pre ? winvd_.p : winv_;
+    const double *winv = F.pre ? F.wd.p : winv_;
     if (cluster && clu64_.blocks && clu64_.level == 0) {
       run_cluster<double>(st, L64, clu64_, in, out, winv, nullptr, gate);
       return;

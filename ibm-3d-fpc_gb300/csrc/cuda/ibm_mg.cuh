@@ -33,7 +33,7 @@ struct MgLevelT {
   DBuf<T> Aown, wd, invd, pm, pp, x, bv, r, t, dense;
   DBuf<T> rb;           // colour-split coefficients for the in-place two-colour relaxation (7-point, even nx)
   DBuf<T> rb27;         // colour-split 27-point coefficients + inverse diagonal (two-colour relaxation)
-  int pre = 0;          // rb (or its classes) holds couplings scaled by the inverse diagonal (k_split_colors)
+  int pre = 0;          // rb (or its classes) holds couplings scaled by the inverse diagonal (k_split_colors), wd the input's scaling
   Classes<T> rbc;       // the classes of rb or rb27 (W 8 or 28); the plain records are then released
 };
 
@@ -83,7 +83,6 @@ class Multigrid {
   double tail_bytes_ = 0.0;
   ClusterPlan clu32_, clu64_;
   const double *winv_ = nullptr;
-  DBuf<double> winvd_;  // FP64 input scaling of a finest level with pre: winv_ / diagonal
   DBuf<float> winvf_;   // FP32 copy of winv_ for the FP32 hierarchy
 };
 
