@@ -93,7 +93,6 @@ struct Classes {
   std::vector<T> major_rec;  // its record
   DBuf<uint8_t> runs, runs8; // per 32 quads (octets) of a level: all their records are of the major class (mark_runs)
   bool ok() const { return code.p != nullptr; }
-  size_t bytes() const { return code.bytes() + tab.bytes() + runs.bytes() + runs8.bytes(); }
 };
 struct Box;
 // Fills c.runs for colour-split codes ([colour][n / 2]) of a level of box b

@@ -1539,17 +1539,6 @@ void Krylov::configure(int nsys_, const KSysHost *hs) {
   if (!hflags) IBM_CUDA_TRY(cudaMallocHost((void **)&hflags, sizeof(KFlags) * kMaxSys));
 }
 
-size_t Krylov::bytes() const {
-  size_t b = 0;
-  for (int s = 0; s < nsys; ++s) {
-    const Slot &sl = slot[s];
-    b += sl.V.bytes() + sl.w.bytes() + sl.part.bytes() +
-         sl.Z.bytes() + sl.zf.bytes() + sl.zf2.bytes() + sl.Vf.bytes() + sl.wf.bytes() + sl.xs.bytes() +
-         sl.vcur.bytes();
-  }
-  return b;
-}
-
 Krylov::~Krylov() {
   if (hflags) cudaFreeHost(hflags);
 }

@@ -84,7 +84,6 @@ class Krylov {
   // x_zero: the caller guarantees x = 0 on entry (the first residual is b).
   void solve(cudaStream_t st, const double *const *b, double *const *x, const Precond &pc, KResult *res,
              unsigned mask = ~0u, bool x_zero = false);
-  size_t bytes() const;
 
   // Graph form. bind() fixes the vectors (outside any capture); enqueue_graph()
   // records the whole solve into the capture running on `st`: the restart /

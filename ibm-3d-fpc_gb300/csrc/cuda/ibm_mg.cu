@@ -3637,11 +3637,4 @@ void Multigrid::level_coef27(cudaStream_t st, int l, double *host_out) const {
   }
 }
 
-size_t Multigrid::bytes() const {
-  size_t b = 0;
-  for (const auto &F : L64) b += F.Aown.bytes() + F.wd.bytes() + F.invd.bytes() + F.pm.bytes() + F.pp.bytes() + F.x.bytes() + F.bv.bytes() + F.r.bytes() + F.t.bytes() + F.dense.bytes() + F.rb.bytes() + F.rb27.bytes() + F.rbc.bytes();
-  for (const auto &F : L32) b += F.Aown.bytes() + F.wd.bytes() + F.invd.bytes() + F.pm.bytes() + F.pp.bytes() + F.x.bytes() + F.bv.bytes() + F.r.bytes() + F.t.bytes() + F.dense.bytes() + F.rb.bytes() + F.rb27.bytes() + F.rbc.bytes();
-  return b;
-}
-
 }  // namespace ibm

@@ -62,7 +62,6 @@ class Multigrid {
   void level_info(int l, int dims[3], int *cdir, int *ns) const;
   // Copies level l's coefficients as [n][27] (FP64 hierarchy).
   void level_coef27(cudaStream_t st, int l, double *host_out) const;
-  size_t bytes() const;
   MgParams prm;
 
  private:
