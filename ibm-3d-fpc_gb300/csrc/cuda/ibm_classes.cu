@@ -94,6 +94,7 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
   out.tab.release();
   out.runs.release();
   out.runs8.release();
+  out.read = out.read8 = 1.0;
   out.K = 0;
   out.W = W;
   if (nrec <= 0 || W <= 0) return false;
@@ -177,17 +178,26 @@ bool build_classes(cudaStream_t st, const T *rec, int W, long nrec, Classes<T> &
   return true;
 }
 
+template <int unit, class T>
+static double mark_runs_of(cudaStream_t st, const Classes<T> &c, const Box &b, DBuf<uint8_t> &runs) {
+  const long units = b.n / unit, nruns = (units + 31) / 32;
+  runs.alloc((size_t)nruns);
+  {
+    LaunchScope ls(K_SETUP, st, 0.0);
+    k_mark_runs<unit><<<grid_of(32 * nruns), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b, unit), c.major, runs.p, nruns);
+  }
+  std::vector<uint8_t> h((size_t)nruns);
+  IBM_CUDA_TRY(cudaMemcpyAsync(h.data(), runs.p, (size_t)nruns, cudaMemcpyDeviceToHost, st));
+  IBM_CUDA_TRY(cudaStreamSynchronize(st));
+  long out = 0;
+  for (long w = 0; w < nruns; ++w)
+    if (!h[(size_t)w]) out += std::min(32L, units - 32 * w);
+  return (double)out / (double)units;
+}
 template <class T>
 void mark_runs(cudaStream_t st, Classes<T> &c, const Box &b) {
-  const long nruns = (b.n / 4 + 31) / 32;
-  c.runs.alloc((size_t)nruns);
-  LaunchScope ls(K_SETUP, st, 0.0);
-  k_mark_runs<4><<<grid_of(32 * nruns), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b), c.major, c.runs.p, nruns);
-  if (b.nx % 8 == 0) {
-    const long n8 = (b.n / 8 + 31) / 32;
-    c.runs8.alloc((size_t)n8);
-    k_mark_runs<8><<<grid_of(32 * n8), kThreads, 0, st>>>(c.code.p, b, make_quad_map(b, 8), c.major, c.runs8.p, n8);
-  }
+  c.read = mark_runs_of<4>(st, c, b, c.runs);
+  if (b.nx % 8 == 0) c.read8 = mark_runs_of<8>(st, c, b, c.runs8);
 }
 
 template void mark_runs<float>(cudaStream_t, Classes<float> &, const Box &);

@@ -92,6 +92,7 @@ struct Classes {
   int major = 0;             // the class of most records
   std::vector<T> major_rec;  // its record
   DBuf<uint8_t> runs, runs8; // per 32 quads (octets) of a level: all their records are of the major class (mark_runs)
+  double read = 1.0, read8 = 1.0;  // the shares of the records outside such runs
   bool ok() const { return code.p != nullptr; }
 };
 struct Box;

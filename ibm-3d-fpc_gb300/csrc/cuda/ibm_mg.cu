@@ -3307,7 +3307,9 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
   Uni8 U7;
   if constexpr (sizeof(T) == 4) U7 = uni8_of(F.rbc);
   const QuadMap Q = make_quad_map(F.b);
-  const double rec7 = R7.code ? 2.0 : 8.0 * T_, rec27 = R27.code ? 2.0 : 28.0 * T_;
+  const double share = split && sizeof(T) == 4 ? F.rbc.read8 : split || (quad && sizeof(T) == 4) ? F.rbc.read : 1.0;
+  const double code7 = 2.0 * share;  // a class code, where the common record's runs do not stand for it
+  const double rec7 = R7.code ? code7 : 8.0 * T_, rec27 = R27.code ? 2.0 : 28.0 * T_;
   const QuadMap O = make_quad_map(F.b, 8);
   const bool ahead = sizeof(T) == 4 || n <= kPlainRecords;  // k_relax_rb27
   Uni8 U8;
@@ -3321,7 +3323,7 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
         const double phase = 0.5 * n * rec7 + 1.5 * T_ * n;
         if (zero) {
           const int vec4 = fin->basef && fin->ld % 4 == 0;
-          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? 2.0 : T_) + (vec4 ? (winvf ? 4.0 : 3.0) : (winv ? 6.0 : 4.0)) * T_ * n);
+          LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? code7 : T_) + (vec4 ? (winvf ? 4.0 : 3.0) : (winv ? 6.0 : 4.0)) * T_ * n);
           k_split_in<<<resident_grid(k_split_in, n8), block_of(n8), 0, st>>>(R7, U8, O, F.bv.p, cur, F.b, *fin, vec4, winv, winvf, gate);
         } else {
           LaunchScope ls(K_MG_RELAX_FINE, st, phase);
@@ -3334,9 +3336,10 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
       }
       if (p.relax == 2 && rb7 && quad && p.fused_sweep && !(zero && fin) && !(last && fout)) {
         // both colour phases in one kernel, out of place
+        const double rec = R7.code ? 2.0 : 8.0 * T_;
         LaunchScope ls(K_MG_RELAX_FINE, st, (zero ? 0.5 * n * (R7.code ? 2.0 : T_) + 1.5 * T_ * n
-                                                  : 0.5 * n * rec7 + 1.5 * T_ * n) +
-                                                0.5 * n * rec7 + 1.5 * T_ * n);
+                                                  : 0.5 * n * rec + 1.5 * T_ * n) +
+                                                0.5 * n * rec + 1.5 * T_ * n);
         k_relax_rb_sweep<<<sweep_grid(F.b), kThreads, 0, st>>>(R7, F.bv.p, cur, oth, F.b, zero ? 1 : 0, gate);
         std::swap(cur, oth);
         return;
@@ -3345,13 +3348,13 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
         for (int color = 0; color < 2; ++color) {
           const bool z = zero && color == 0;
           if (z && fin) {
-            LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? 2.0 : T_) + (winvf ? 4.0 : 3.0) * T_ * n);
+            LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * (R7.code ? code7 : T_) + (winvf ? 4.0 : 3.0) * T_ * n);
             k_relax_rb_quad_in<<<resident_grid(k_relax_rb_quad_in, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, *fin, winvf, gate);
           } else if (color == 1 && last && fout) {
             LaunchScope ls(K_MG_RELAX_FINE, st, 0.5 * n * rec7 + 2.5 * T_ * n);
             k_relax_rb_quad_out<<<resident_grid(k_relax_rb_quad_out, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, 1, *fout, gate);
           } else {
-            LaunchScope ls(K_MG_RELAX_FINE, st, z ? 0.5 * n * (R7.code ? 2.0 : T_) + 1.5 * T_ * n
+            LaunchScope ls(K_MG_RELAX_FINE, st, z ? 0.5 * n * (R7.code ? code7 : T_) + 1.5 * T_ * n
                                                   : 0.5 * n * rec7 + 1.5 * T_ * n);
             k_relax_rb_quad<<<resident_grid(k_relax_rb_quad, n / 4), block_of(n / 4), 0, st>>>(R7, U7, Q, F.bv.p, cur, F.b, color, z, gate);
           }
