@@ -91,6 +91,7 @@ struct ibm_ctx {
 
   ibm::DBuf<double> u, v, w, p, ut, vt, wt;
   ibm::Plain plain;
+  double plain_faces = 0.0, plain_rows = 0.0, plain_cells = 0.0;  // how many carry the flags (booked bytes)
   bool plain_ready = false;      // flags and coefficients above derived from the current inputs
   ibm::DBuf<float2> df_u, df_v, df_w, df_p;  // double-float copies of u, v, w, p (df_rhs)
   ibm::DBuf<double> xb[4], bb[4];

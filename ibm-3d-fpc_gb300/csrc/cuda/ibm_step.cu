@@ -826,7 +826,8 @@ __global__ void k_sample(const double *a, long ld, const double *a2, int W, long
 // kPlainFace of one field's faces. d3: the direction of the field; the cells
 // below and above a face (none outside the box).
 __global__ void k_mark_faces(uint8_t *fl, const uint8_t *fc, const double *G, long NF, Dims d, int d3, double gl,
-                             double gr) {
+                             double gr, unsigned long long *count) {
+  unsigned long long marked = 0;
   for (long f = (long)blockIdx.x * blockDim.x + threadIdx.x; f < NF; f += (long)gridDim.x * blockDim.x) {
     long q, kq;
     const int i = udivmod(f, d3 == 0 ? d.dnx1 : d.dnx, q);
@@ -838,10 +839,14 @@ __global__ void k_mark_faces(uint8_t *fl, const uint8_t *fc, const double *G, lo
       if ((fc[lo] & kFluid) && (fc[hi] & kFluid)) v |= kPlainFace;
     }
     fl[f] = v;
+    marked += (v & kPlainFace) != 0;
   }
+  if (marked) atomicAdd(count, marked);
 }
 // kPlainRow of one field's solve-box rows.
-__global__ void k_mark_rows(uint8_t *fl, const double *sc, const double *bc, long n, Dims d, int d3, double s, double b) {
+__global__ void k_mark_rows(uint8_t *fl, const double *sc, const double *bc, long n, Dims d, int d3, double s, double b,
+                            unsigned long long *count) {
+  unsigned long long marked = 0;
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
     long q, kq;
     const int i = udivmod(r, d3 == 0 ? d.dnxm : d.dnx, q) + (d3 == 0);
@@ -849,12 +854,15 @@ __global__ void k_mark_rows(uint8_t *fl, const double *sc, const double *bc, lon
     const long f = d3 == 0 ? U3(d, i, j, k) : d3 == 1 ? V3(d, i, j, k) : W3(d, i, j, k);
     const bool same = same_bits(sc[r], s) && same_bits(bc[r], b);
     fl[f] = (uint8_t)((fl[f] & ~kPlainRow) | (same ? kPlainRow : 0));
+    marked += same;
   }
+  if (marked) atomicAdd(count, marked);
 }
 // kPlainCell. Cells of the inlet column never are: ibm_set_inflow rewrites their lift.
 __global__ void k_mark_cells(uint8_t *fc, const uint8_t *fu, const uint8_t *fv, const uint8_t *fw, const double *Dc,
-                             const double *div_bc, Dims d, Plain p) {
+                             const double *div_bc, Dims d, Plain p, unsigned long long *count) {
   const long NP = (long)d.nx * d.ny * d.nz;
+  unsigned long long marked = 0;
   for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < NP; c += (long)gridDim.x * blockDim.x) {
     long q, kq;
     const int i = udivmod(c, d.dnx, q);
@@ -864,7 +872,9 @@ __global__ void k_mark_cells(uint8_t *fc, const uint8_t *fu, const uint8_t *fv, 
     bool plain = (fc[c] & kFluid) && i > 0 && same_bits(div_bc[c], 0.0);
     for (int s = 0; s < 6; ++s) plain = plain && (f[s] & kQFace) && !(f[s] & kBcSet) && same_bits(Dc[s * NP + c], p.D[s]);
     fc[c] = (uint8_t)((fc[c] & ~kPlainCell) | (plain ? kPlainCell : 0));
+    marked += plain;
   }
+  if (marked) atomicAdd(count, marked);
 }
 
 Dims dims_of(const ibm_ctx *c) {
@@ -958,6 +968,9 @@ void ensure_plain(ibm_ctx *c) {
   const long NF[3] = {g.NU, g.NV, g.NW};
   const Box *box[3] = {&g.bu, &g.bv, &g.bw};
   Plain &p = c->plain;
+  DBuf<unsigned long long> count;  // faces, rows, cells marked
+  count.alloc(3);
+  count.zero(c->st);
   for (int f = 0; f < 3; ++f) {
     double r[2];
     common_record(c, G[f], NF[f], nullptr, 2, NF[f], r);
@@ -965,17 +978,22 @@ void ensure_plain(ibm_ctx *c) {
     common_record(c, c->scale_box[f].p, 0, c->bc_box[f].p, 2, box[f]->n, r);
     p.sc[f] = r[0]; p.bc[f] = r[1];
     LaunchScope ls(K_SETUP, c->st, 0.0, 2);
-    k_mark_faces<<<blocks_for(NF[f]), kThreads, 0, c->st>>>(fl[f], c->fc.p, G[f], NF[f], d, f, p.gl[f], p.gr[f]);
+    k_mark_faces<<<blocks_for(NF[f]), kThreads, 0, c->st>>>(fl[f], c->fc.p, G[f], NF[f], d, f, p.gl[f], p.gr[f],
+                                                           count.p);
     k_mark_rows<<<blocks_for(box[f]->n), kThreads, 0, c->st>>>(fl[f], c->scale_box[f].p, c->bc_box[f].p, box[f]->n, d, f,
-                                                              p.sc[f], p.bc[f]);
+                                                              p.sc[f], p.bc[f], count.p + 1);
   }
   common_record(c, c->Dc.p, g.NP, nullptr, 6, g.NP, p.D);
   {
     LaunchScope ls(K_SETUP, c->st, 0.0);
-    k_mark_cells<<<blocks_for(g.NP), kThreads, 0, c->st>>>(c->fc.p, fl[0], fl[1], fl[2], c->Dc.p, c->div_bc_cell.p, d, p);
+    k_mark_cells<<<blocks_for(g.NP), kThreads, 0, c->st>>>(c->fc.p, fl[0], fl[1], fl[2], c->Dc.p, c->div_bc_cell.p, d, p,
+                                                              count.p + 2);
   }
+  unsigned long long marked[3];
+  IBM_CUDA_TRY(cudaMemcpyAsync(marked, count.p, sizeof(marked), cudaMemcpyDeviceToHost, c->st));
   IBM_CUDA_TRY(cudaStreamSynchronize(c->st));
   IBM_CUDA_TRY(cudaGetLastError());
+  c->plain_faces = (double)marked[0]; c->plain_rows = (double)marked[1]; c->plain_cells = (double)marked[2];
   c->graph_ready = false;  // a captured step holds the coefficients in its kernels' parameters
   c->plain_ready = true;
 }
@@ -1007,6 +1025,10 @@ void launch_momentum_rhs(ibm_ctx *c) {
   A.drx = split(1.0 / (2 * c->g.dx)); A.dry = split(1.0 / (2 * c->g.dy)); A.drz = split(1.0 / (2 * c->g.dz));
   const double faces = (double)(c->g.NU + c->g.NV + c->g.NW), nbox = (double)(A.nb[0] + A.nb[1] + A.nb[2]);
   const long rows = std::max(std::max(A.nb[0], A.nb[1]), A.nb[2]);  // of the longest of the three loops
+  // velocities, p, a row's flag, right-hand side and guess; scale and boundary
+  // term, G and the cells' flags where they are not the common ones
+  const double bytes = 8.0 * faces + 8.0 * c->g.NP + 17.0 * nbox + 16.0 * (nbox - c->plain_rows) +
+                       18.0 * (nbox - c->plain_faces);
   if (momentum_rhs_df(c->prm)) {
     if (!c->df_u.p || !c->df_v.p || !c->df_w.p || !c->df_p.p)
       throw Error(IBM_ERR_STATE, "double-float field copies not allocated");
@@ -1021,11 +1043,11 @@ void launch_momentum_rhs(ibm_ctx *c) {
       k_split_fields<<<grid, kThreads, 0, c->st>>>(S);
     }
     A.u2 = c->df_u.p; A.v2 = c->df_v.p; A.w2 = c->df_w.p; A.p2 = c->df_p.p;
-    LaunchScope ls(K_RHS, c->st, 8.0 * faces + 9.0 * c->g.NP + nbox * (1 + 16 + 32));
+    LaunchScope ls(K_RHS, c->st, bytes);
     k_momentum_rhs<RhsDF><<<wave_blocks(k_momentum_rhs<RhsDF>, rows), kThreads, 0, c->st>>>(A);
   } else {
     A.u2 = A.v2 = A.w2 = A.p2 = nullptr;
-    LaunchScope ls(K_RHS, c->st, 8.0 * faces + 9.0 * c->g.NP + nbox * (1 + 16 + 32));
+    LaunchScope ls(K_RHS, c->st, bytes);
     k_momentum_rhs<RhsF64><<<wave_blocks(k_momentum_rhs<RhsF64>, rows), kThreads, 0, c->st>>>(A);
   }
 }
@@ -1034,7 +1056,7 @@ void launch_tilde(ibm_ctx *c) {
   const Dims d = dims_of(c);
   {
     const double faces = (double)(c->g.NU + c->g.NV + c->g.NW);
-    LaunchScope ls(K_SCATTER, c->st, 16.0 * faces + 8.0 * (c->g.bu.n + c->g.bv.n + c->g.bw.n));
+    LaunchScope ls(K_SCATTER, c->st, 16.0 * faces);  // x or u in, out
     k_scatter<<<wave_blocks(k_scatter, c->g.NU + c->g.NV + c->g.NW), kThreads, 0, c->st>>>(
         c->u.p, c->v.p, c->w.p, c->xb[0].p, c->xb[1].p, c->xb[2].p, c->ut.p, c->vt.p, c->wt.p, d, c->diag.p);
   }
@@ -1187,7 +1209,7 @@ void launch_projection(ibm_ctx *c) {
   A.plain = c->plain;
   const double faces = (double)(c->g.NU + c->g.NV + c->g.NW);
   {
-    LaunchScope ls(K_PROJECT, c->st, 33.0 * faces + 25.0 * c->g.NP);
+    LaunchScope ls(K_PROJECT, c->st, 17.0 * faces + 18.0 * (faces - c->plain_faces) + 25.0 * c->g.NP);
     k_project<<<wave_blocks(k_project, std::max(std::max(c->g.NU, c->g.NV), c->g.NW)), kThreads, 0, c->st>>>(A);
   }
   launch_bc(c, c->u.p, c->v.p, c->w.p);
@@ -1206,7 +1228,7 @@ void launch_projection(ibm_ctx *c) {
   D.dg = c->diag.p;
   D.np_active = c->np_active;
   {
-    LaunchScope ls(K_DIAG, c->st, 33.0 * faces + 65.0 * c->g.NP);
+    LaunchScope ls(K_DIAG, c->st, 8.0 * faces + c->g.NP + 62.0 * (c->g.NP - c->plain_cells));
     k_diagnostics<<<nb, kThreads, 0, c->st>>>(D);
   }
   if (c->prm.compute_forces) launch_forces(c);

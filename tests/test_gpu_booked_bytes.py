@@ -47,3 +47,64 @@ def test_bytes_of_fine_phases(ibm, form):
         assert abs(p.bytes[k] - n * (fixed + 12 * share)) <= 1e-9 * p.bytes[k]
     finally:
         s.close()
+
+
+def common(records):
+    """Which records are the most frequent one that is not all zeros."""
+    _, code, count = np.unique(np.ascontiguousarray(records).view(np.uint64), axis=0, return_inverse=True,
+                               return_counts=True)
+    code = code.reshape(-1)
+    zeros = ~records.any(axis=1)
+    count[np.unique(code[zeros])] = 0
+    return code == np.argmax(count)
+
+
+def common_faces(case):
+    """Faces between two cells whose G pair is their field's common one."""
+    ptr, val = case.array("G_rowptr"), case.array("G_val")
+    n, first = 0, 0
+    for name in ("nqu", "nqv", "nqw"):
+        rows = np.arange(first, first + case.counts[name])
+        first += case.counts[name]
+        two = rows[np.diff(ptr)[rows] == 2]
+        n += common(np.stack([val[ptr[two]], val[ptr[two] + 1]], axis=1)).sum()
+    return int(n)
+
+
+def common_rows(case):
+    nx, ny, nz = case.shape
+    n = 0
+    for f, shape, inner in (("u", (nz, ny, nx + 1), np.s_[:, :, 1:-1]), ("v", (nz, ny + 1, nx), np.s_[:, 1:-1, :]),
+                            ("w", (nz + 1, ny, nx), np.s_[1:-1, :, :])):
+        ids = case.array("id_" + f).reshape(shape)[inner].ravel()
+        active = case.array("active_" + f).reshape(shape)[inner].ravel()
+        ids = np.where(active != 0, ids, 0)
+        rec = np.stack([case.array("scale_" + f)[ids], case.array(f"rhs_{f}_bc")[ids]], axis=1)
+        rec[ids == 0] = 0.0
+        n += int(common(rec).sum())
+    return n
+
+
+def test_bytes_of_dense_kernels(ibm):
+    """Scale, boundary term, G and cell flags are booked only for the rows and
+    faces that do not share the common ones."""
+    nx, ny, nz = shape = (64, 24, 20)
+    case = ibm.Case(ibm.channel_params(*shape, Um=1.0, dt=1e-3))
+    s = ibm.Solver(case, ibm.solver_params())
+    try:
+        s.step(1.0)
+        s.profile_reset()
+        s.step(1.0)
+        p, names = s.profile(), ibm.kernel_names()
+        booked = {name: p.bytes[k] for k, name in enumerate(names)}
+        faces = (nx + 1) * ny * nz + nx * (ny + 1) * nz + nx * ny * (nz + 1)
+        box = (nx - 1) * ny * nz + nx * (ny - 1) * nz + nx * ny * (nz - 1)
+        cells = nx * ny * nz
+        pf, pr = common_faces(case), common_rows(case)
+        assert 0.5 * faces < pf < faces and 0.3 * box < pr < box
+        assert booked["scatter"] == 16 * faces
+        assert booked["project"] == 17 * faces + 18 * (faces - pf) + 25 * cells
+        assert booked["momentum_rhs"] == 8 * faces + 8 * cells + 17 * box + 16 * (box - pr) + 18 * (box - pf)
+        assert 8 * faces + cells < booked["diagnostics"] < 8 * faces + 63 * cells
+    finally:
+        s.close()
