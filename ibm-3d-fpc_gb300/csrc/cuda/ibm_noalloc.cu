@@ -46,7 +46,7 @@ namespace {
 
 // A warp takes 32 rows at a time and keeps kNaStages such chunks on their way.
 constexpr int kNaStages = 3;
-constexpr int kNaBlocksPerSm = 4;
+constexpr int kNaBlocksPerSm = 2;
 constexpr int kNaChunk = 32 * 7;  // coefficients of a chunk
 
 template <int BYTES>
@@ -64,9 +64,15 @@ __device__ __forceinline__ void copy_async(double *smem, const double *g) {
 // apart between neighbouring lanes, which no two lanes of a half-warp have in
 // one bank. Warps run free of each other, so that one's FP64 work (10
 // operations a row, 75 us at 512x96x96) covers another's loads (57 us at the
-// copy bandwidth). A call at that size took 125 us and takes 100; with one copy
+// copy bandwidth). A call at that size took 125 us and takes 94; with one copy
 // of a whole tile per block and a barrier it took 156, since blocks then load
 // and compute in step.
+//
+// The norms' sums count beside ten operations a row: with four blocks an SM and
+// a butterfly of both sums in every warp, a call on 131072 rows (one chunk a
+// warp) spent as much FP64 issue there as on its rows, 16.5 us in a graph. With
+// two blocks an SM, twice the chunks a warp, and the sums by two warps of a block
+// it takes 12.4, as a block per 1024 rows did; 1M rows 28.4 (31.7; 35.0 so).
 //
 // The stencil is evaluated in the same order as the context path's operator
 // apply (centre, -x, +x, -y, +y, -z, +z, one fma each), so r is bitwise equal
@@ -136,21 +142,22 @@ __global__ void __launch_bounds__(kThreads, kNaBlocksPerSm)
     }
     if (++stage == kNaStages) stage = 0;
   }
-  rr = warp_sum(rr);
-  bb = warp_sum(bb);
-  if (lane == 0) {
-    srr[warp] = rr;
-    sbb[warp] = bb;
+  // the block's sums by two warps, each lane first the eight warps' values of
+  // its place: 26 warp-wide FP64 instructions a block, not 80
+  double(*const sums)[kThreads] = reinterpret_cast<double(*)[kThreads]>(&rows[0][0][0]);
+  __syncthreads();  // every warp has read its rows
+  sums[0][threadIdx.x] = rr;
+  sums[1][threadIdx.x] = bb;
+  __syncthreads();
+  if (warp < 2) {
+    double a = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) a += sums[warp][32 * w + lane];
+    a = warp_sum(a);
+    if (lane == 0) sc->part[2 * blockIdx.x + warp] = a;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double a = 0.0, e = 0.0;
-    for (int w = 0; w < kWarps; ++w) {
-      a += srr[w];
-      e += sbb[w];
-    }
-    sc->part[2 * blockIdx.x] = a;
-    sc->part[2 * blockIdx.x + 1] = e;
     __threadfence();
     last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
   }
@@ -247,7 +254,7 @@ extern "C" int ibm_residual_noalloc(const double *vals, int nx, int ny, int nz, 
   if (cudaMemsetAsync(&sc->ticket, 0, sizeof(unsigned), st) != cudaSuccess) return IBM_ERR_CUDA;
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return IBM_ERR_CUDA;
-  // one chunk per warp up to one resident wave; 152 x 4 blocks are within the scratch's tiles on any device
+  // one chunk per warp up to one resident wave; 152 x 2 blocks are within the scratch's tiles on any device
   const long blocks = (n + 32 * kWarps - 1) / (32 * kWarps);
   const int grid = (int)std::min({blocks, (long)sms * kNaBlocksPerSm, (long)kNaMaxTiles});
   k_residual_noalloc<<<grid, kThreads, 0, st>>>(vals, make_box(nx, ny, nz),
