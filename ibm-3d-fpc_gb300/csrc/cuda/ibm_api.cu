@@ -364,7 +364,9 @@ void ensure_solvers(ibm_ctx *c) {
     ensure_classes(c, c->op[3]);
     use_classes(op, hp);
   }
-  c->kp.configure(1, &hp);
+  size_t idle_n = 0;
+  double *const idle = c->kmom.idle(idle_n);  // no momentum solve runs beside a pressure solve
+  c->kp.configure(1, &hp, idle, idle_n);
   c->solvers_ready = true;
   c->solvers_precision = precision_key(p);
   c->graph_ready = false;

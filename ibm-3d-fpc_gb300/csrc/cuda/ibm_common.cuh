@@ -211,8 +211,8 @@ struct KScal {
   int active;         // 1 while an Arnoldi cycle is running
   int cycle_end;      // 1 when the cycle stopped and the solution update is due
   int i;              // Arnoldi vectors built in this cycle
-  int pc_in, pc_out;  // pc 1: the vectors of V that the next V-cycle reads and writes
-  int pc_on;          // pc 1: 1 the next V-cycle is an Arnoldi step's, 2 a finished cycle's, 0 there is none
+  double *pc_in, *pc_out;  // pc 1: the vectors that the next V-cycle reads and writes
+  int pc_on;               // pc 1: 1 the next V-cycle is an Arnoldi step's, 2 a finished cycle's, 0 there is none
   int iters;
   int status;         // 0 running, 1 converged, 2 iteration limit, 3 stagnation
   int claimed;        // the Givens estimate reached the tolerance
@@ -244,6 +244,8 @@ struct KSys {
   long ldv;
   float *Z;             // flexible basis (FP32), vector k at Z + k*ldv
   double *w, *x;
+  double *lent;         // pc 1: the cycle's first nlent preconditioned directions, k at lent - k*ldv
+  int nlent, nkept;     // ... and the most that are kept (direction_of)
   const double *b;
   float *zf, *zf2;      // FP32 work for the inner sweeps
   double *part;         // block partial sums [nblk][kMaxKdim + 2]

@@ -196,26 +196,36 @@ __device__ bool block_partials_and_last(double *sacc, int nd, double *part, unsi
 // pc 1 keeps a cycle's preconditioned directions M V_k, as the flexible form
 // does, so that the update is x += sum c_k M V_k and not M (V c): one V-cycle
 // less per GMRES cycle (six instead of seven for a solve of six iterations; FP64
-// step 640x128x128 36.8 -> 34.7 ms, 160x32x32 4.58 -> 4.24). They lie in the
-// vectors of V that a short cycle does not reach, from its end down: direction
-// k in vector kdim - k, up to kdim / 2 of them (vectors 0 .. kdim / 2 of the
-// basis lie below). A longer cycle's basis runs over them; its later directions
-// go to the spare vector kdim + 1, and its end takes V c there and applies the
-// preconditioner to it, into vector kdim. Solves here take six to seven
-// iterations of the default 50.
-__device__ __forceinline__ int direction_slot(int k, int kdim) { return k < kdim / 2 ? kdim - k : kdim + 1; }
-// Whether a system's finished cycle applies the preconditioner at its end.
-__device__ __forceinline__ bool end_applies(const KSys &S) { return S.pc == 1 && S.s->i > S.s->kdim / 2; }
-// The next V-cycle: of Arnoldi step i; of a finished cycle's V c.
-__device__ __forceinline__ void pc_of_step(KScal *sc, int i, int on) {
-  sc->pc_in = i;
-  sc->pc_out = direction_slot(i, sc->kdim);
-  sc->pc_on = on;
+// step 640x128x128 36.8 -> 34.7 ms, 160x32x32 4.58 -> 4.24). They take no memory of
+// their own. The first nlent lie in another solver's basis that is idle meanwhile
+// (the momentum systems': with the default restart lengths all of them), from its
+// end down, which that solver's own cycles seldom reach; the next ones in the
+// vectors of V that the cycle does not reach, from vector kdim + 1 down. A cycle
+// longer than nkept iterations has its basis run over these; its later directions
+// go to the spare vector kdim + 1 one after the other, and its end takes V c there
+// and applies the preconditioner to it, into vector kdim.
+__device__ __forceinline__ double *direction_of(const KSys &S, int k, int kdim) {
+  if (k < S.nlent) return S.lent - (long)k * S.ldv;
+  return S.V + (long)(kdim + 1 - (k < S.nkept ? k - S.nlent : 0)) * S.ldv;
 }
-__device__ __forceinline__ void pc_of_end(KScal *sc) {
-  sc->pc_in = sc->kdim + 1;
-  sc->pc_out = sc->kdim;
-  sc->pc_on = 2;
+// The most directions that a cycle can keep: vectors 0 .. m of V are its basis
+// (the last only for m < kdim), m - lent of kdim + 2 above them directions.
+int kept_directions(int kdim, int lent) {
+  return lent >= kdim - 2 ? kdim : std::min(kdim - 1, (kdim + 1 + lent) / 2);
+}
+// Whether a system's finished cycle applies the preconditioner at its end.
+__device__ __forceinline__ bool end_applies(const KSys &S) { return S.pc == 1 && S.s->i > S.nkept; }
+// The next V-cycle: of Arnoldi step i; of a finished cycle's V c.
+__device__ __forceinline__ void pc_of_step(const KSys &S, int i, int kdim, int on) {
+  if (S.pc != 1) return;
+  S.s->pc_in = S.V + (long)i * S.ldv;
+  S.s->pc_out = direction_of(S, i, kdim);
+  S.s->pc_on = on;
+}
+__device__ __forceinline__ void pc_of_end(const KSys &S) {
+  S.s->pc_in = S.V + (long)(S.s->kdim + 1) * S.ldv;
+  S.s->pc_out = S.V + (long)S.s->kdim * S.ldv;
+  S.s->pc_on = 2;
 }
 
 // r = b - Ar x; V_0 = r; |b|^2, |r|^2. Last block: norms, tolerance, state.
@@ -299,7 +309,7 @@ __global__ void __launch_bounds__(kThreads) k_init(const __grid_constant__ KSysP
     else if (rn == 0.0 || rn <= sc->eps) { sc->status = 1; sc->active = 0; }
     else if (sc->maxit <= 0) { sc->status = 2; sc->active = 0; }
     else { sc->status = 0; sc->active = 1; }
-    pc_of_step(sc, 0, sc->active);
+    pc_of_step(S, 0, sc->kdim, sc->active);
     sc->nu[0] = rn;
     sc->inu[0] = 1.0 / rn;
     sc->g[0] = rn;
@@ -314,7 +324,8 @@ __global__ void __launch_bounds__(kThreads) k_init(const __grid_constant__ KSysP
 // many threads at once (one memory latency each for the column and, at a
 // cycle's end, the triangle), and one thread then works there. One thread
 // walking global memory paid a latency per rotation and per matrix entry.
-__device__ void arnoldi_finalize(KScal *sc, int j, double hn) {
+__device__ void arnoldi_finalize(const KSys &S, int j, double hn) {
+  KScal *sc = S.s;
   constexpr int K = kMaxKdim;
   __shared__ double col[K + 1], rc[K], rs[K], tri[K * (K + 1) / 2];
   __shared__ int ended;
@@ -361,7 +372,7 @@ __device__ void arnoldi_finalize(KScal *sc, int j, double hn) {
       sc->active = 0;
       sc->cycle_end = 1;
     }
-    pc_of_step(sc, m, end ? 0 : 1);
+    pc_of_step(S, m, kdim, end ? 0 : 1);
     ended = end;
   }
   __syncthreads();
@@ -565,7 +576,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_arnoldi_spmv(const __grid_const
   const double inv_nu = sc->inu[j];
   __shared__ double sacc[(kMaxKdim + 1) * kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double *z = S.V + (long)(S.pc == 1 ? sc->pc_out : j) * S.ldv;
+  const double *z = S.pc == 1 ? sc->pc_out : S.V + (long)j * S.ldv;
   const float *zj = S.Z + (long)j * S.ldv;
   for (int c0 = 0; c0 < nd; c0 += kDots64) {
     const int ndc = min(nd - c0, kDots64);
@@ -709,7 +720,7 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next(const __grid_constant
   reduce_partials(S.part, gridDim.x, 1, tot);
   __syncthreads();
   if (threadIdx.x == 0) sc->ticket = 0;
-  arnoldi_finalize(sc, j, sqrt(tot[0]));
+  arnoldi_finalize(S, j, sqrt(tot[0]));
 }
 
 // Cycle end, solution update. pc 0: x += invd * (V c); pc 1: x += sum of c_k
@@ -796,25 +807,31 @@ __global__ void __launch_bounds__(kThreads) k_cycle_update(const __grid_constant
     }
     return;
   }
-  const bool kept = S.pc == 1 && !end_applies(S);
-  double *const last = S.V + (long)sc->kdim * S.ldv;
-  const double *basis = kept ? last : S.V;
-  const long step = kept ? -S.ldv : S.ldv;
+  const int kdim = sc->kdim;
   if (S.pc == 1 && sc->pc_on == 2) {
+    const double *z = sc->pc_out;
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x)
-      S.x[r] = S.x[r] + last[r];
+      S.x[r] = S.x[r] + z[r];
     return;
   }
+  const bool kept = S.pc == 1 && !end_applies(S);
+  // the vectors of the sum: the basis' from V up or the directions in lent
+  // memory from its end down, then directions from the spare vector down
+  double *const spare = S.V + (long)(kdim + 1) * S.ldv;
+  const double *const first = kept ? S.lent : S.V;
+  const long step = kept ? -S.ldv : S.ldv;
+  const int nfirst = kept ? min(m, S.nlent) : m;
   for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < S.n; r += (long)gridDim.x * blockDim.x) {
     double acc = 0.0;
     if (S.pc == 2) {
       for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], widen(S.Z[(long)kk * S.ldv + r]), acc);
       S.x[r] = S.x[r] + acc;
     } else {
-      for (int kk = 0; kk < m; ++kk) acc = fma(cf[kk], basis[(long)kk * step + r], acc);
+      for (int kk = 0; kk < nfirst; ++kk) acc = fma(cf[kk], first[(long)kk * step + r], acc);
+      for (int kk = nfirst; kk < m; ++kk) acc = fma(cf[kk], spare[r - (long)(kk - nfirst) * S.ldv], acc);
       if (S.pc == 0) S.x[r] = fma(S.invd[r], acc, S.x[r]);
       else if (kept) S.x[r] = S.x[r] + acc;
-      else last[S.ldv + r] = acc;
+      else spare[r] = acc;
     }
   }
 }
@@ -932,7 +949,7 @@ __global__ void __launch_bounds__(kThreads) k_cycle_residual(const __grid_consta
     sc->real_old = rt;
     sc->cyc_eps = fmax(sc->eps, sc->cyc_rtol * rt);
     sc->i = 0;
-    pc_of_step(sc, 0, 1);
+    pc_of_step(S, 0, sc->kdim, 1);
     sc->claimed = 0;
     sc->nu[0] = rt;
     sc->inu[0] = 1.0 / rt;
@@ -1284,7 +1301,7 @@ __global__ void __launch_bounds__(kThreads) k_arnoldi_next32(const __grid_consta
   reduce_partials(S.part, gridDim.x, 1, tot);
   __syncthreads();
   if (threadIdx.x == 0) sc->ticket = 0;
-  arnoldi_finalize(sc, j, sqrt(tot[0]));
+  arnoldi_finalize(S, j, sqrt(tot[0]));
 }
 
 // Two FP32 Jacobi sweeps from zero in one pass (momentum preconditioner of
@@ -1465,7 +1482,7 @@ __global__ void k_flags(const __grid_constant__ KSysPack P, int nsys, KFlags *ou
 // Systems whose finished cycle waits for the preconditioner: the next V-cycle is
 // its. (In a launch of its own: the kernels that read the state run in many blocks.)
 __device__ void wait_for_pc(const KSys &S) {
-  if (S.s->cycle_end && end_applies(S)) pc_of_end(S.s);
+  if (S.s->cycle_end && end_applies(S)) pc_of_end(S);
 }
 __global__ void k_pc_of_end(const __grid_constant__ KSysPack P, int nsys) {
   if ((int)threadIdx.x < nsys) wait_for_pc(P.s[threadIdx.x]);
@@ -1478,13 +1495,15 @@ __global__ void k_pc_of_end(const __grid_constant__ KSysPack P, int nsys) {
 // Arnoldi kernels return at once. count (may be null): bodies run.
 __global__ void k_set_while(const __grid_constant__ KSysPack P, int nsys, cudaGraphConditionalHandle hw,
                             unsigned long long *count) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (count) *count += 1;
-  unsigned run = 0;
-  for (int s = 0; s < nsys; ++s) {
+  const int s = threadIdx.x;  // one warp: a system's flags by a lane each, one memory latency for all
+  bool runs = false;
+  if (s < nsys) {
+    runs = P.s[s].s->active | P.s[s].s->cycle_end;
     wait_for_pc(P.s[s]);
-    run |= (P.s[s].s->active | P.s[s].s->cycle_end) ? 1u : 0u;
   }
+  const unsigned run = __any_sync(0xffffffffu, runs) ? 1u : 0u;
+  if (s != 0) return;
+  if (count) *count += 1;
   cudaGraphSetConditional(hw, run);
 }
 
@@ -1493,7 +1512,7 @@ __global__ void k_set_while(const __grid_constant__ KSysPack P, int nsys, cudaGr
 // ---------------------------------------------------------------------------
 // Host driver
 // ---------------------------------------------------------------------------
-void Krylov::configure(int nsys_, const KSysHost *hs) {
+void Krylov::configure(int nsys_, const KSysHost *hs, double *lent, size_t lent_n) {
   if (nsys_ < 1 || nsys_ > kMaxSys) throw Error(IBM_ERR_ARG, "Krylov: bad system count");
   nsys = nsys_;
   int maxn = 0;
@@ -1521,9 +1540,12 @@ void Krylov::configure(int nsys_, const KSysHost *hs) {
       sl.wf.alloc(h.n);
     } else {
       sl.Vf.release(); sl.wf.release();
-      sl.V.alloc((size_t)(h.kdim + (h.pc == 1 ? 2 : 1)) * h.n);  // pc 1: the spare vector (direction_slot)
+      sl.V.alloc((size_t)(h.kdim + (h.pc == 1 ? 2 : 1)) * h.n);  // pc 1: the spare vector (direction_of)
       sl.w.alloc(h.n);
     }
+    sl.nlent = h.pc == 1 && nsys == 1 ? (int)std::min((size_t)h.kdim, lent_n / (size_t)h.n) : 0;
+    sl.lent = sl.nlent ? lent + (lent_n - (size_t)h.n) : nullptr;
+    sl.nkept = h.pc == 1 ? kept_directions(h.kdim, sl.nlent) : 0;
     if (h.a32 && h.cls && h.tabdf && h.df_residual) sl.xs.alloc(h.n);
     else sl.xs.release();
     if (h.pc == 2) {
@@ -1537,6 +1559,17 @@ void Krylov::configure(int nsys_, const KSysHost *hs) {
   scal.alloc(nsys);
   dflags.alloc(nsys);
   if (!hflags) IBM_CUDA_TRY(cudaMallocHost((void **)&hflags, sizeof(KFlags) * kMaxSys));
+}
+
+double *Krylov::idle(size_t &n) const {
+  double *p = nullptr;
+  n = 0;
+  for (int s = 0; s < nsys; ++s) {
+    const size_t v = slot[s].V.n, f = slot[s].Vf.n / 2;
+    if (v > n) { n = v; p = slot[s].V.p; }
+    if (f > n) { n = f; p = reinterpret_cast<double *>(slot[s].Vf.p); }
+  }
+  return p;
 }
 
 Krylov::~Krylov() {
@@ -1566,6 +1599,7 @@ void Krylov::bind(cudaStream_t st, const double *const *b, double *const *x, uns
     k.V = slot[s].V.p; k.ldv = h.n;
     k.Z = slot[s].Z.p;
     k.w = slot[s].w.p;
+    k.lent = slot[s].lent; k.nlent = slot[s].nlent; k.nkept = slot[s].nkept;
     k.zf = slot[s].zf.p; k.zf2 = slot[s].zf2.p;
     k.Vf = slot[s].Vf.p; k.wf = slot[s].wf.p; k.a32 = h.a32;
     k.vcur = slot[s].vcur.p;
@@ -1612,9 +1646,9 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
     for (int s = 0; s < nsys; ++s) {
       if (!fl[s].cycle_end) continue;
       const int m = fl[s].i, pcm = slot[s].host.pc;
-      bu += rows(s) * (pcm == 2 ? 4.0 * m + 16.0 : pcm == 1 ? 8.0 * m + (m > slot[s].host.kdim / 2 ? 8.0 : 16.0) : 8.0 * m + 24.0);
+      bu += rows(s) * (pcm == 2 ? 4.0 * m + 16.0 : pcm == 1 ? 8.0 * m + (m > slot[s].nkept ? 8.0 : 16.0) : 8.0 * m + 24.0);
       // a classed row is its 2-byte class instead of 7 FP64 coefficients
-      if (pcm != 1 || m <= slot[s].host.kdim / 2)
+      if (pcm != 1 || m <= slot[s].nkept)
         br += ((slot[s].host.cls ? 34.0 : 88.0) + (slot[s].vcur.p ? 4.0 : 0.0)) * rows(s);
     }
   }
@@ -1631,7 +1665,7 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
   bool applies = false;
   double ba = 0.0, bar = 0.0;
   for (int s = 0; fl && s < nsys; ++s) {
-    if (slot[s].host.pc != 1 || !fl[s].cycle_end || fl[s].i <= slot[s].host.kdim / 2) continue;
+    if (slot[s].host.pc != 1 || !fl[s].cycle_end || fl[s].i <= slot[s].nkept) continue;
     if (!applies) {
       LaunchScope ls(K_GM_UPDATE, st, 0.0);
       k_pc_of_end<<<1, 32, 0, st>>>(pack, nsys);
@@ -1647,9 +1681,9 @@ void Krylov::launch_cycle_end(cudaStream_t st, const Precond &pc, const KFlags *
 // The V-cycle that a pc 1 system's scalars name (pc_of_step, pc_of_end).
 void Krylov::apply_explicit(cudaStream_t st, const Precond &pc, int s) {
   VecRef in;
-  in.base = slot[s].V.p; in.ld = slot[s].host.n; in.idx = &scal.p[s].pc_in;
+  in.at = &scal.p[s].pc_in;
   OutRef out;
-  out.d = slot[s].V.p; out.ld = slot[s].host.n; out.idx = &scal.p[s].pc_out;
+  out.at = &scal.p[s].pc_out;
   pc.apply(pc.ctx, st, s, in, out, nsys > 1 ? &scal.p[s].pc_on : nullptr);
 }
 

@@ -4,10 +4,11 @@
 
 namespace ibm {
 
-// A vector whose location is resolved on the device: base + (*idx) * ld,
+// A vector whose location is resolved on the device: base + (*idx) * ld, or *at,
 // optionally scaled by inu[*idx] (1 / norm of the unnormalised Krylov basis vector).
 struct VecRef {
   const double *base = nullptr;
+  double *const *at = nullptr;   // FP64 source (used instead of base when set)
   const float *basef = nullptr;  // FP32 source (used instead of base when set)
   long ld = 0;
   const int *idx = nullptr;
@@ -18,7 +19,12 @@ struct OutRef {
   float *f = nullptr;   // FP32 destination
   long ld = 0;
   const int *idx = nullptr;
+  double *const *at = nullptr;  // FP64 destination (used instead of d when set)
+  __host__ __device__ bool fp64() const { return d || at; }
 };
+__device__ __forceinline__ long ref_offset(const int *idx, long ld) { return idx ? (long)(*idx) * ld : 0; }
+__device__ __forceinline__ const double *ref64(const VecRef &r) { return r.at ? *r.at : r.base + ref_offset(r.idx, r.ld); }
+__device__ __forceinline__ double *ref64(const OutRef &r) { return r.at ? *r.at : r.d + ref_offset(r.idx, r.ld); }
 
 // Preconditioner callback: out = M in, every kernel gated on *gate != 0.
 struct Precond {
@@ -79,7 +85,12 @@ struct KResult {
 class Krylov {
  public:
   ~Krylov();
-  void configure(int nsys, const KSysHost *systems);
+  // lent: FP64 memory that is idle while these systems are solved (pc 1: the
+  // directions of a cycle; direction_of), of lent_n values; it must stay where it
+  // is until the next configure.
+  void configure(int nsys, const KSysHost *systems, double *lent = nullptr, size_t lent_n = 0);
+  // The largest of these systems' basis buffers, for another solver's use between their solves.
+  double *idle(size_t &n) const;
   // mask: bit s set = solve system s (the others are skipped).
   // x_zero: the caller guarantees x = 0 on entry (the first residual is b).
   void solve(cudaStream_t st, const double *const *b, double *const *x, const Precond &pc, KResult *res,
@@ -101,6 +112,8 @@ class Krylov {
   struct Slot {
     KSysHost host;
     DBuf<double> V, w, part;
+    double *lent = nullptr;      // pc 1: where the first of the nlent directions in lent memory goes
+    int nlent = 0, nkept = 0;
     DBuf<float> Z, zf, zf2, Vf, wf;
     DBuf<float> vcur;  // FP64 basis with FP32 Jacobi: FP32 copy of the current basis vector
     DBuf<float2> xs;  // double-float copy of x for the double-float residual

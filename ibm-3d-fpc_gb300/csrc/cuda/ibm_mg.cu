@@ -257,10 +257,9 @@ __global__ void k_convert(const double *src, T *dst, long n) {
 // ---------------------------------------------------------------- V-cycle
 template <class T>
 __device__ __forceinline__ void load_input_body(T *bv, long n, const VecRef &in, const double *winv, long t0, long ts) {
-  const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
   const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
-  const double *src = in.base + off;
-  const float *srcf = in.basef ? in.basef + off : nullptr;
+  const double *src = ref64(in);
+  const float *srcf = in.basef ? in.basef + ref_offset(in.idx, in.ld) : nullptr;
   for (long r = t0; r < n; r += ts) {
     const double a = srcf ? (double)srcf[r] : src[r];
     double v = in.inu ? a * sc : a;
@@ -298,10 +297,12 @@ __global__ void k_load_input_f4(float *bv, long n, VecRef in, const float *winvf
 
 template <class T>
 __device__ __forceinline__ void store_output_body(const T *x, long n, const OutRef &out, long t0, long ts) {
-  const long off = out.idx ? (long)(*out.idx) * out.ld : 0;
+  const bool wide = out.fp64();
+  double *d = wide ? ref64(out) : nullptr;
+  float *f = wide ? nullptr : out.f + ref_offset(out.idx, out.ld);
   for (long r = t0; r < n; r += ts) {
-    if (out.d) out.d[off + r] = (double)x[r];
-    else out.f[off + r] = (float)x[r];
+    if (wide) d[r] = (double)x[r];
+    else f[r] = (float)x[r];
   }
 }
 template <class T>
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_in64(Recs<double, 8> R, d
                                                             const double *winv, const int *gate) {
   if (gate_off(gate)) return;
   const long h = bx.n / 2;
-  const double *src = in.base + (in.idx ? (long)(*in.idx) * in.ld : 0);
+  const double *src = ref64(in);
   const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
   for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < h; m += (long)gridDim.x * blockDim.x) {
     int i, j, k;
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(kThreads) k_relax_rb_in64(Recs<double, 8> R, d
 __global__ void __launch_bounds__(kThreads) k_relax_rb_out64(Recs<double, 8> R, const double *__restrict__ b, double *x,
                                                              Box bx, OutRef out, const int *gate) {
   if (gate_off(gate)) return;
-  relax_rb_body<double>(R, b, x, bx, 1, out.d + (out.idx ? (long)(*out.idx) * out.ld : 0),
+  relax_rb_body<double>(R, b, x, bx, 1, ref64(out),
                         (long)blockIdx.x * blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
@@ -1096,10 +1097,9 @@ __global__ void __launch_bounds__(kThreads) k_split_in(Recs<float, 8> R, Uni8 U,
                                                        const int *gate) {
   if (gate_off(gate)) return;
   const long n8 = bx.n / 8, h = bx.n / 2;
-  const long off = in.idx ? (long)(*in.idx) * in.ld : 0;
   const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
-  const double *src = in.base + off;
-  const float *srcf = in.basef ? in.basef + off : nullptr;
+  const double *src = ref64(in);
+  const float *srcf = in.basef ? in.basef + ref_offset(in.idx, in.ld) : nullptr;
   const bool wide = !srcf && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n8; q += (long)gridDim.x * blockDim.x) {
     const Quad g = unit_of<8>(q, Q, bx);
@@ -1329,7 +1329,7 @@ __global__ void __launch_bounds__(kThreads) k_split_in64(QuadMap Q, double *bs, 
                                                          const double *winv, const int *gate) {
   if (gate_off(gate)) return;
   const long n4 = bx.n / 4, h = bx.n / 2;
-  const double *src = in.base + (in.idx ? (long)(*in.idx) * in.ld : 0);
+  const double *src = ref64(in);
   const double sc = in.inu ? in.inu[in.idx ? *in.idx : 0] : 1.0;
   const bool wide = aligned16(src);
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
@@ -1364,7 +1364,7 @@ __global__ void __launch_bounds__(kThreads) k_split_phase64(Recs<double, 8> R, U
   if (gate_off(gate)) return;
   const long n4 = bx.n / 4, h = bx.n / 2, own = color ? h : 0;
   const double *xo = xs + (h - own);
-  double *zd = OUT ? out.d + (out.idx ? (long)(*out.idx) * out.ld : 0) : nullptr;
+  double *zd = OUT ? ref64(out) : nullptr;
   const bool wide = OUT && aligned16(zd);
   for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (long)gridDim.x * blockDim.x) {
     const Quad g = quad_of(q, Q, bx);
@@ -3555,7 +3555,7 @@ static T *vcycle(cudaStream_t st, std::vector<MgLevelT<T>> &L, int l, const MgPa
 void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, const int *gate, bool use_fp32,
                       bool fused) {
   if (prm.cycles != 1) throw Error(IBM_ERR_UNSUPPORTED, "multigrid: only one V-cycle per application");
-  const double ob = out.d ? 8.0 : 4.0;
+  const double ob = out.fp64() ? 8.0 : 4.0;
   // captured solves keep a launch per phase (see k_mg_cluster)
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   IBM_CUDA_TRY(cudaStreamIsCapturing(st, &capturing));
@@ -3609,7 +3609,7 @@ void Multigrid::apply(cudaStream_t st, const VecRef &in, const OutRef &out, cons
       run_cluster<double>(st, L64, clu64_, in, out, winv, nullptr, gate);
       return;
     }
-    if (in.base && out.d && prm.relax == 2 && F.relax && F.cdir >= 0 && F.ns == 7 && (F.rb.p || F.rbc.ok()) &&
+    if ((in.base || in.at) && out.fp64() && prm.relax == 2 && F.relax && F.cdir >= 0 && F.ns == 7 && (F.rb.p || F.rbc.ok()) &&
         prm.nu1 > 0 && prm.nu2 > 0) {
       const bool split = fused && prm.quads && F.pre && F.b.nx % 4 == 0 && F.b.n >= kSplitPoints64;
       vcycle<double>(st, L64, 0, prm, gate, &in, &out, nullptr, nullptr, c64, winv, fused, split);
